@@ -547,17 +547,18 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         }
         const uint32_t x = __ldg(ccsr + head + col);
         n_trials++;
-        {
-            // accept_candidate searches N(prev) when neither the rand value
-            // nor x == prev (nor prev == cur) decides the trial
-            const bool cm = ZC ? s_mapped[cb] != 0 : true, pm = ZC ? s_mapped[pb] != 0 : true;
-            if (cm) zc_sectors += 1u;
-            if (pcsr != nullptr && pm && !(rv <= thr_min<SOPR>(a.c, t)) && x != prev && prev != cur)
-                zc_sectors += search_sectors(pdeg);
+        // N(prev) is searched only when the verdict depends on it, and then
+        // only if its block is resident (or mapped); each search and each
+        // candidate counts its sectors
+        int verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
+        if (!ZC || s_mapped[cb]) zc_sectors += 1u;
+        if (verdict < 0 && pcsr != nullptr) {
+            if (!ZC || s_mapped[pb]) zc_sectors += search_sectors(pdeg);
+            verdict = (csr_contains(CsrIndex{pcsr, {}, 0}, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
+                                                                           : rv < thr_notfound<SOPR>(a.c, t))
+                          ? 1
+                          : 0;
         }
-        const int verdict = pcsr != nullptr
-                                ? (accept_candidate<SOPR>(a.c, t, rv, x, prev, cur, CsrIndex{pcsr, {}, 0}, phead, pdeg) ? 1 : 0)
-                                : accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
         if (verdict < 0) {
             // Needs N(prev), whose block is absent: park the walker flagged in
             // bucket (prev block, cur block).  The step restarts at attempt 0

@@ -161,23 +161,9 @@ __device__ __forceinline__ bool csr_contains(const CsrIndex &ix, uint64_t lo, ui
     return p < lo + n && __ldg(ix.csr + p) == x;
 }
 
-// Acceptance of candidate x drawn with rand value rv (engine/engine.hpp:209-258,
-// 334-375); N(prev) is pix.csr[phead, phead + pdeg).
-template <bool SOPR>
-__device__ __forceinline__ bool accept_candidate(const StepConsts &c, const StepThr &t, float rv, uint32_t x,
-                                                 uint32_t prev, uint32_t cur, const CsrIndex &pix, uint64_t phead,
-                                                 uint32_t pdeg)
-{
-    if (rv <= thr_min<SOPR>(c, t)) return true;
-    if (x == prev) return rv < thr_prev<SOPR>(c, t);
-    // x is drawn from N(cur); when prev == cur the search must succeed.
-    const bool found = (prev == cur) ? true : csr_contains(pix, phead, pdeg, x);
-    return found ? (rv < thr_found<SOPR>(c, t)) : (rv < thr_notfound<SOPR>(c, t));
-}
-
-// The same verdict without N(prev), for a walker whose previous block is not
-// resident: 1 accept, 0 reject, -1 when it depends on x in N(prev) (the
-// found and not-found thresholds disagree at rv).
+// Verdict on candidate x drawn with rand value rv (engine/engine.hpp:209-258,
+// 334-375) without N(prev): 1 accept, 0 reject, -1 when it depends on x in
+// N(prev) (the found and not-found thresholds disagree at rv).
 template <bool SOPR>
 __device__ __forceinline__ int accept_without_prev(const StepConsts &c, const StepThr &t, float rv, uint32_t x,
                                                    uint32_t prev, uint32_t cur)
@@ -185,9 +171,28 @@ __device__ __forceinline__ int accept_without_prev(const StepConsts &c, const St
     if (rv <= thr_min<SOPR>(c, t)) return 1;
     if (x == prev) return rv < thr_prev<SOPR>(c, t) ? 1 : 0;
     const bool af = rv < thr_found<SOPR>(c, t);
+    // x is drawn from N(cur); when prev == cur the search must succeed.
     if (prev == cur) return af ? 1 : 0;
     const bool an = rv < thr_notfound<SOPR>(c, t);
     return af == an ? (af ? 1 : 0) : -1;
+}
+
+// The verdict with N(prev) = pix.csr[phead, phead + pdeg) at hand.  N(prev)
+// is searched only when the verdict depends on it: for Node2vec a trial whose
+// rand value lies on the same side of both thresholds (1 and 1/q) needs no
+// search, so p = 0.5, q = 2 searches on a quarter of the trials and p = 2,
+// q = 0.5 on a half, where every rand value above the smallest threshold
+// (three quarters of them) used to search.  The step kernels are bound by the
+// distinct lines their loads touch (one L1 tag access per cycle), most of
+// them probes of this search.
+template <bool SOPR>
+__device__ __forceinline__ bool accept_candidate(const StepConsts &c, const StepThr &t, float rv, uint32_t x,
+                                                 uint32_t prev, uint32_t cur, const CsrIndex &pix, uint64_t phead,
+                                                 uint32_t pdeg)
+{
+    const int v = accept_without_prev<SOPR>(c, t, rv, x, prev, cur);
+    if (v >= 0) return v != 0;
+    return csr_contains(pix, phead, pdeg, x) ? (rv < thr_found<SOPR>(c, t)) : (rv < thr_notfound<SOPR>(c, t));
 }
 
 // A walker whose step has already rejected this many attempts is served by

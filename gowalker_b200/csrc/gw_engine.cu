@@ -210,10 +210,13 @@ void gw_handle::release()
     cudaFree(d_hashes);
     cudaFree(d_ctr);
     cudaFree(d_err);
-    cudaFree(d_index);
-    d_index = nullptr;
-    index_cap = 0;
-    index_nlvl = 0;
+    cudaFree(d_verts);
+    cudaFree(d_heads_hi);
+    cudaFree(d_table);
+    d_verts = nullptr;
+    d_heads_hi = nullptr;
+    d_table = nullptr;
+    verts_cap = heads_hi_cap = table_cap = 0;
     if (h_ctr) cudaFreeHost(h_ctr);
     ooc_release();
     if (ev_start) cudaEventDestroy(ev_start);
@@ -501,38 +504,72 @@ extern "C" int gw_num_walkers(gw_handle *h, uint64_t *n)
 
 // ------------------------------------------------------------------ ABI: run
 
-// Sample levels of the resident CSR (CsrIndex): level L holds csr[j * 32^L]
-// for every j, ceil(nedges / 32^L) words, about 3% of the CSR in all.  Built
-// once per graph, after validation.
-int gw_handle::build_index(cudaStream_t s)
+// Device memory for `n` elements in *p, kept when it already holds as many.
+// An index is worth having, not needed: false when there is no room.
+template <typename T>
+static bool index_room(T **p, uint64_t *cap, uint64_t n, uint64_t bytes_each)
 {
-    index_nlvl = 0;
-    uint64_t n[kIdxLevels], total = 0;
-    uint32_t nl = 0;
-    for (uint64_t m = nedges; nl < (uint32_t)kIdxLevels && m > 64; ++nl) {
-        m = (m + 31) / 32;
-        n[nl] = m;
-        total += m;
+    if (n <= *cap) return true;
+    cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    if (cudaMalloc((void **)p, n * bytes_each) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    if (nl == 0) return GW_OK;
-    if (total > index_cap) {
-        cudaFree(d_index);
-        d_index = nullptr;
-        index_cap = 0;
-        int st;
-        if ((st = cuda(cudaMalloc(&d_index, total * sizeof(uint32_t)), "CSR sample levels"))) return st;
-        index_cap = total;
+    *cap = n;
+    return true;
+}
+
+// Checks the resident CSR and builds its index, once per graph: per vertex 16
+// bytes (first edge, degree, first bucket, the degree's reciprocal), which a
+// step loads at once in place of two offsets and a division, and the
+// membership tables (10 bytes per edge and up to 32 per vertex).  Where the
+// device has no room for them walks read the offsets and halve.
+int gw_handle::validate_graph(cudaStream_t s)
+{
+    int st;
+    index_ready = false;
+    index_wide = nedges >= (1ull << 32);
+    const bool index = index_room(&d_verts, &verts_cap, nverts, sizeof(uint4)) &&
+                       (!index_wide || index_room(&d_heads_hi, &heads_hi_cap, nverts, sizeof(uint32_t)));
+    CsrCheck check{};
+    check.beg = dev_beg;
+    check.csr = dev_csr;
+    check.nverts = nverts;
+    check.nedges = nedges;
+    check.err = d_err;
+    if (index) {
+        check.verts = d_verts;
+        check.heads_hi = index_wide ? d_heads_hi : nullptr;
+        check.nbuckets = d_ctr;
     }
-    uint32_t *dst = d_index;
-    const uint32_t *src = dev_csr;
-    for (uint32_t L = 0; L < nl; ++L) {
-        int st;
-        if ((st = cuda(launch_sample_level(src, n[L], dst, num_sms, s), "CSR sample level"))) return st;
-        index_lvl[L] = dst;
-        src = dst;
-        dst += n[L];
+    uint64_t ends[2] = {1, 0};
+    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long), s), "memset")) ||
+        (st = cuda(launch_validate_csr(check, num_sms, s), "validate")) ||
+        (st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s), "buckets")) ||
+        (st = cuda(cudaMemcpyAsync(h_ctr + kCtrCount, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
+                   "error word D2H")) ||
+        (st = cuda(cudaMemcpyAsync(&ends[0], dev_beg, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "beg[0]")) ||
+        (st = cuda(cudaMemcpyAsync(&ends[1], dev_beg + nverts, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "beg[V]")) ||
+        (st = cuda(cudaStreamSynchronize(s), "validate")))
+        return st;
+    if ((uint32_t)h_ctr[kCtrCount] != 0) {
+        h_ctr[kCtrCount] = 0;
+        return fail(GW_ERR_GRAPH, "graph failed validation: offsets not monotone or a neighbour id >= %u", nverts);
     }
-    index_nlvl = nl;
+    if (ends[0] != 0 || ends[1] != nedges)
+        return fail(GW_ERR_GRAPH, "graph offsets must run from 0 to nedges (%llu..%llu)", (unsigned long long)ends[0],
+                    (unsigned long long)ends[1]);
+    const uint64_t buckets = h_ctr[0];
+    if (index && buckets < (1ull << 32) && index_room(&d_table, &table_cap, buckets ? buckets : 1, 32)) {
+        if ((st = cuda(cudaMemsetAsync(d_table, 0xFF, buckets * 32, s), "memset")) ||
+            (st = cuda(launch_build_table(dev_beg, d_verts, nverts, dev_csr, nedges, d_table, num_sms, s),
+                       "membership tables")))
+            return st;
+        index_ready = true;
+    }
+    validated = true;
     return GW_OK;
 }
 
@@ -577,30 +614,7 @@ int gw_handle::run_incore(gw_stats *stats)
         if ((st = upload_whole_graph(s, &h2d))) return st;
     }
     if ((st = cuda(cudaMemsetAsync(d_err, 0, sizeof(uint32_t), s), "memset"))) return st;
-    if (!validated) {
-        // One pass over the resident CSR before any walk indexes through it.
-        if ((st = cuda(launch_validate_csr(dev_beg, dev_csr, nverts, nedges, d_err, num_sms, s), "validate")))
-            return st;
-        if ((st = cuda(cudaMemcpyAsync(h_ctr + kCtrCount, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-                       "error word D2H")))
-            return st;
-        if ((st = cuda(cudaStreamSynchronize(s), "validate"))) return st;
-        if ((uint32_t)h_ctr[kCtrCount] != 0) {
-            h_ctr[kCtrCount] = 0;
-            return fail(GW_ERR_GRAPH, "graph failed validation: offsets not monotone or a neighbour id >= %u",
-                        nverts);
-        }
-        uint64_t ends[2] = {1, 0};
-        if ((st = cuda(cudaMemcpy(&ends[0], dev_beg, sizeof(uint64_t), cudaMemcpyDeviceToHost), "beg[0]")))
-            return st;
-        if ((st = cuda(cudaMemcpy(&ends[1], dev_beg + nverts, sizeof(uint64_t), cudaMemcpyDeviceToHost), "beg[V]")))
-            return st;
-        if (ends[0] != 0 || ends[1] != nedges)
-            return fail(GW_ERR_GRAPH, "graph offsets must run from 0 to nedges (%llu..%llu)",
-                        (unsigned long long)ends[0], (unsigned long long)ends[1]);
-        if ((st = build_index(s))) return st;
-        validated = true;
-    }
+    if (!validated && (st = validate_graph(s))) return st;
     if (weighted) {
         if (cfg.algorithm != GW_NODE2VEC)
             return fail(GW_ERR_ARG, "weighted walks are Node2vec walks (algorithm %u given)", cfg.algorithm);
@@ -616,9 +630,12 @@ int gw_handle::run_incore(gw_stats *stats)
     a.init.key0 = (uint32_t)cfg.seed;
     a.init.key1 = (uint32_t)(cfg.seed >> 32);
     a.beg = dev_beg;
-    a.ix.csr = dev_csr;
-    a.ix.nlvl = index_nlvl;
-    for (uint32_t L = 0; L < index_nlvl; ++L) a.ix.lvl[L] = index_lvl[L];
+    a.csr = dev_csr;
+    if (index_ready) {
+        a.verts = d_verts;
+        a.heads_hi = index_wide ? d_heads_hi : nullptr;
+        a.table = d_table;
+    }
     a.nverts = nverts;
     a.nwalkers = (uint32_t)nwalkers;
     a.wid_base = wid_first;

@@ -41,11 +41,11 @@ struct gw_handle {
     bool resident = false;
     bool device_graph = false;
     bool validated = false;
-    // sample levels of the resident CSR, rebuilt whenever it is validated
-    uint32_t *d_index = nullptr;
-    uint64_t index_cap = 0;
-    const uint32_t *index_lvl[gw::kIdxLevels] = {};
-    uint32_t index_nlvl = 0;
+    // index of the resident CSR, rebuilt whenever it is validated
+    uint4 *d_verts = nullptr;
+    uint32_t *d_heads_hi = nullptr, *d_table = nullptr;
+    uint64_t verts_cap = 0, heads_hi_cap = 0, table_cap = 0;  // entries, entries, buckets
+    bool index_wide = false, index_ready = false;             // heads_hi in use; there is an index
 
     // edge weights (weighted Node2vec, in-core): per host block, or resident
     std::vector<const float *> host_w;
@@ -96,7 +96,7 @@ struct gw_handle {
     bool host_graph_complete() const;
     int upload_whole_graph(cudaStream_t s, uint64_t *h2d);
     int ensure_outputs();
-    int build_index(cudaStream_t s);
+    int validate_graph(cudaStream_t s);
     int build_alias(cudaStream_t s);
     int run_incore(gw_stats *stats);
     int run_ooc(uint32_t policy, gw_stats *stats);

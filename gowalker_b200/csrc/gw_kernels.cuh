@@ -70,7 +70,11 @@ struct IncoreArgs {
     StepConsts c;
     WalkerInit init;
     const uint64_t *beg;       // nverts+1 global offsets
-    CsrIndex ix;               // nedges neighbour ids and their sample levels
+    const uint32_t *csr;       // nedges neighbour ids
+    // index of the resident CSR, built once per graph (verts null: none)
+    const uint4 *verts;        // {first edge (low word), degree, first bucket, mod_magic(degree)} per vertex
+    const uint32_t *heads_hi;  // high words of the first edges; null when all are 0
+    const uint32_t *table;     // membership tables (table_has); set with verts
     uint32_t nverts;
     uint32_t nwalkers;         // walkers of this launch: ids wid_base + i * wid_stride, i < nwalkers
     uint32_t wid_base;
@@ -97,6 +101,24 @@ __device__ __forceinline__ uint32_t walker_source(const WalkerInit &in, uint32_t
     }
     const U4 r = philox4x32_10(wid, 0xFFFFFFFFu, 0u, kTagInit, in.key0, in.key1);
     return r.x % in.nverts;
+}
+
+// What a step reads of a vertex v < nverts.
+struct Vertex {
+    uint64_t head;   // first edge
+    uint32_t deg;
+    uint32_t bucket; // first bucket of its membership table
+    uint32_t magic;  // mod_magic(deg)
+};
+__device__ __forceinline__ Vertex load_vertex(const IncoreArgs &a, uint32_t v)
+{
+    if (a.verts) {
+        const uint4 e = __ldg(a.verts + v);
+        return Vertex{a.heads_hi ? ((uint64_t)__ldg(a.heads_hi + v) << 32) | e.x : e.x, e.y, e.z, e.w};
+    }
+    const uint64_t head = __ldg(a.beg + v);
+    const uint32_t deg = (uint32_t)(__ldg(a.beg + v + 1) - head);
+    return Vertex{head, deg, 0u, deg ? mod_magic(deg) : 0u};
 }
 
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
@@ -133,9 +155,23 @@ inline bool needs_coop(uint32_t algo, const StepConsts &c)
 {
     return algo != 0u || c.n2v_maxv > 8.0f * c.n2v_minv;
 }
-// One sample level: dst[j] = src[32 * j] for j < n.
-cudaError_t launch_sample_level(const uint32_t *src, uint64_t n, uint32_t *dst, int num_sms, cudaStream_t s);
-cudaError_t launch_validate_csr(const uint64_t *beg, const uint32_t *csr, uint32_t nverts, uint64_t nedges,
-                                uint32_t *err, int num_sms, cudaStream_t s);
+// One pass over a resident CSR before any walk reads it: error bits for
+// offsets that are not monotone within [0, nedges] and ids >= nverts, and, in
+// the same pass, the vertex index (verts null: none) with a place for every
+// vertex's table; *nbuckets counts the buckets.
+struct CsrCheck {
+    const uint64_t *beg;
+    const uint32_t *csr;
+    uint32_t nverts;
+    uint64_t nedges;
+    uint32_t *err;
+    uint4 *verts;
+    uint32_t *heads_hi;            // null: offsets below 2^32
+    unsigned long long *nbuckets;
+};
+cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s);
+// Fills the membership tables of a validated CSR; every slot is kEmptySlot before.
+cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t nverts, const uint32_t *csr,
+                               uint64_t nedges, uint32_t *table, int num_sms, cudaStream_t s);
 
 }  // namespace gw

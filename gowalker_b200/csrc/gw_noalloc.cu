@@ -146,7 +146,13 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     // returns them (the kernel writes only the visited entries)
     if (e == cudaSuccess && cfg->record_paths == GW_PATHS_FULL)
         e = cudaMemsetAsync(d_paths, 0, nwalkers * ((uint64_t)cfg->maxhops + 1) * sizeof(uint32_t), s);
-    if (e == cudaSuccess) e = launch_validate_csr(d_beg, d_csr, nverts, nedges, err, num_sms, s);
+    CsrCheck check{};
+    check.beg = d_beg;
+    check.csr = d_csr;
+    check.nverts = nverts;
+    check.nedges = nedges;
+    check.err = err;
+    if (e == cudaSuccess) e = launch_validate_csr(check, num_sms, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, sizeof(host_ctr), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&ends[0], d_beg, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&ends[1], d_beg + nverts, sizeof(uint64_t), cudaMemcpyDeviceToHost, s);
@@ -167,7 +173,7 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     a.init.key0 = (uint32_t)cfg->seed;
     a.init.key1 = (uint32_t)(cfg->seed >> 32);
     a.beg = d_beg;
-    a.ix = CsrIndex{d_csr, {}, 0};  // no sample levels: this entry point allocates nothing
+    a.csr = d_csr;  // no index: this entry point allocates nothing
     a.nverts = nverts;
     a.nwalkers = (uint32_t)nwalkers;
     a.wid_stride = 1;

@@ -31,25 +31,16 @@ struct U4 {
     uint32_t x, y, z, w;
 };
 
-GW_HD uint32_t mulhi32(uint32_t a, uint32_t b)
-{
-#if defined(__CUDA_ARCH__)
-    return __umulhi(a, b);
-#else
-    return (uint32_t)(((uint64_t)a * b) >> 32);
-#endif
-}
-
 GW_HD U4 philox4x32_10(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3, uint32_t k0, uint32_t k1)
 {
 #if defined(__CUDA_ARCH__)
 #pragma unroll
 #endif
     for (int r = 0; r < 10; ++r) {
-        const uint32_t lo0 = kPhiloxM0 * c0;
-        const uint32_t hi0 = mulhi32(kPhiloxM0, c0);
-        const uint32_t lo1 = kPhiloxM1 * c2;
-        const uint32_t hi1 = mulhi32(kPhiloxM1, c2);
+        // both halves of each product from one wide multiply
+        const uint64_t p0 = (uint64_t)kPhiloxM0 * c0, p1 = (uint64_t)kPhiloxM1 * c2;
+        const uint32_t lo0 = (uint32_t)p0, hi0 = (uint32_t)(p0 >> 32);
+        const uint32_t lo1 = (uint32_t)p1, hi1 = (uint32_t)(p1 >> 32);
         const uint32_t n0 = hi1 ^ c1 ^ k0;
         const uint32_t n2 = hi0 ^ c3 ^ k1;
         c0 = n0;
@@ -71,10 +62,10 @@ GW_HD U4 philox4x32_10_sched(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3,
 #pragma unroll
 #endif
     for (int r = 0; r < 10; ++r) {
-        const uint32_t lo0 = kPhiloxM0 * c0;
-        const uint32_t hi0 = mulhi32(kPhiloxM0, c0);
-        const uint32_t lo1 = kPhiloxM1 * c2;
-        const uint32_t hi1 = mulhi32(kPhiloxM1, c2);
+        // both halves of each product from one wide multiply
+        const uint64_t p0 = (uint64_t)kPhiloxM0 * c0, p1 = (uint64_t)kPhiloxM1 * c2;
+        const uint32_t lo0 = (uint32_t)p0, hi0 = (uint32_t)(p0 >> 32);
+        const uint32_t lo1 = (uint32_t)p1, hi1 = (uint32_t)(p1 >> 32);
         const uint32_t n0 = hi1 ^ c1 ^ rk0[r];
         const uint32_t n2 = hi0 ^ c3 ^ rk1[r];
         c0 = n0;

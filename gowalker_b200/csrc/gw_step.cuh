@@ -97,6 +97,17 @@ __device__ __forceinline__ U4 draw(const StepConsts &c, uint32_t wid, uint32_t h
     return philox4x32_10_sched(wid, hop, attempt, kTagWalk, c.rk0, c.rk1);
 }
 
+// x % d with a precomputed m = floor((2^32 - 1) / d): m > 2^32 / d - 1 - 1 / d
+// and an integer, so m >= 2^32 / d - 1 and x m / 2^32 > x / d - 1; the quotient
+// falls short by at most one and one correction gives the remainder exactly.
+__host__ __device__ __forceinline__ uint32_t mod_magic(uint32_t d) { return 0xFFFFFFFFu / d; }
+__device__ __forceinline__ uint32_t mod_by(uint32_t x, uint32_t d, uint32_t m)
+{
+    uint32_t r = x - __umulhi(x, m) * d;
+    if (r >= d) r -= d;
+    return r;
+}
+
 __device__ __forceinline__ float rand_val(uint32_t y, float maxv)
 {
     return __fmul_rn(__uint2float_rn(y >> 8) * 0x1p-24f, maxv);
@@ -107,44 +118,62 @@ __device__ __forceinline__ bool terminates(const StepConsts &c, uint32_t z)
     return c.term_prob > 0.0f && __uint2float_rn(z >> 8) * 0x1p-24f < c.term_prob;
 }
 
-// Neighbour array of the graph (or of one block) with its sample levels:
-// lvl[L-1][j] = csr[j * 32^L].  Inside one vertex's sorted neighbours the
-// entries of level L are every 32^L-th neighbour (by global position), so a
-// search walks down the levels, each a binary search over at most 65
-// contiguous entries (one or two lines, then L1 hits), and ends in fewer than
-// 32 neighbours: about one new line per level where a plain binary search
-// takes a miss per halving.  nlvl = 0 is a plain binary search.
-constexpr int kIdxLevels = 6;
+// Neighbour array of the graph (or of one block), with the membership table of
+// its vertices when `table` is set (table_has); without it a search is a plain
+// binary search.
 struct CsrIndex {
     const uint32_t *csr;
-    const uint32_t *lvl[kIdxLevels];
-    uint32_t nlvl;
+    const uint32_t *table;  // buckets of eight ids, on 32-byte boundaries
 };
 
-// First position p in [lo, hi) with csr[p] >= y, or hi (csr[lo, hi) sorted,
-// hi - lo < 2^32).  Ranges of at most 64 go straight to the last binary
-// search; longer ones start at the highest level with more than two entries
-// inside (level L qualifies when hi - lo > 2 * 32^L).
-__device__ __forceinline__ uint64_t csr_lower_bound(const CsrIndex &ix, uint64_t lo, uint64_t hi, uint32_t y)
+// Membership table of one vertex's neighbours: table_buckets(d) buckets of
+// eight slots, an id in its home bucket (table_home) or, that one being full,
+// in the next that was not, slots filled in order, empty ones kEmptySlot.  The
+// slots number more than d, so a search ends at a bucket with room.
+constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;  // no id: ids are below a 32-bit vertex count
+__host__ __device__ __forceinline__ uint32_t table_buckets(uint32_t d)
 {
-    if (hi - lo > 64 && ix.nlvl != 0) {
-        int L = min((int)ix.nlvl, (62 - __clzll((long long)(hi - lo))) / 5);  // (floor(log2 n) - 1) / 5
-        for (; L >= 1; --L) {
-            const uint32_t sh = 5u * (uint32_t)L;
-            if (hi - lo <= (2ull << sh)) continue;
-            const uint32_t *__restrict__ g = ix.lvl[L - 1];
-            const uint64_t j0 = (lo + (1ull << sh) - 1) >> sh, j1 = (hi - 1) >> sh;
-            uint32_t a = 0, b = (uint32_t)(j1 - j0) + 1;  // first j in [j0, j1] with csr[j << sh] >= y
-            while (a < b) {
-                const uint32_t m = (a + b) >> 1;
-                if (__ldg(g + j0 + m) < y) a = m + 1;
-                else b = m;
-            }
-            if (a > 0) lo = ((j0 + a - 1) << sh) + 1;
-            if (j0 + a <= j1) hi = (j0 + a) << sh;
-        }
+    return d ? (d >> 2) + (d >> 4) + 1u : 0u;  // 3.2 ids a bucket: fewer than 1 in 100 buckets overflow
+}
+__device__ __forceinline__ uint32_t table_home(uint32_t id, uint32_t buckets)
+{
+    // two rounds: the product alone sends some arithmetic progressions to one bucket
+    uint32_t h = id * 0x9E3779B1u;
+    h = (h ^ (h >> 15)) * 0x85EBCA77u;
+    return __umulhi(h, buckets);
+}
+
+// One aligned 32-byte sector: eight consecutive words in one load.
+__device__ __forceinline__ void load_sector(const uint32_t *p, uint32_t (&v)[8])
+{
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(p));
+}
+
+// Whether x is among the d ids whose table starts at bucket `first`.
+__device__ __forceinline__ bool table_has(const uint32_t *table, uint32_t first, uint32_t d, uint32_t x)
+{
+    const uint32_t n = table_buckets(d);
+    uint32_t b = n ? table_home(x, n) : 0u;
+    for (uint32_t i = 0; i < n; ++i) {
+        uint32_t v[8];
+        load_sector(table + ((uint64_t)first + b) * 8u, v);
+        bool found = false;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) found |= v[k] == x;
+        if (found) return true;
+        if (v[7] == kEmptySlot) return false;
+        b = b + 1 == n ? 0u : b + 1;
     }
-    const uint32_t *__restrict__ p = ix.csr + lo;
+    return false;
+}
+
+// First position p in [lo, hi) with csr[p] >= y, or hi (csr[lo, hi) sorted,
+// hi - lo < 2^32).
+__device__ __forceinline__ uint64_t csr_lower_bound(const uint32_t *csr, uint64_t lo, uint64_t hi, uint32_t y)
+{
+    const uint32_t *__restrict__ p = csr + lo;
     uint32_t a = 0, b = (uint32_t)(hi - lo);
     while (a < b) {
         const uint32_t m = (a + b) >> 1;
@@ -154,10 +183,19 @@ __device__ __forceinline__ uint64_t csr_lower_bound(const CsrIndex &ix, uint64_t
     return lo + a;
 }
 
-// Membership of x in the sorted csr[lo, lo + n).
-__device__ __forceinline__ bool csr_contains(const CsrIndex &ix, uint64_t lo, uint32_t n, uint32_t x)
+// Membership of x in the sorted csr[lo, lo + n), whose table (if any) starts
+// at bucket `first`.
+//
+// What bounds it: every probe of a search is a dependent load of a line of its
+// own and a warp waits for the longest chain of its lanes.  Halving takes 12
+// probes (a hundred instructions) for the thousands of neighbours of the
+// vertices walks visit most; a bucket is one load and eight compares.  Sample
+// levels of 32, eight-way levels and eight-way trees were all measured too:
+// fewer lines than halving, but no fewer instructions.
+__device__ __forceinline__ bool csr_contains(const CsrIndex &ix, uint32_t first, uint64_t lo, uint32_t n, uint32_t x)
 {
-    const uint64_t p = csr_lower_bound(ix, lo, lo + n, x);
+    if (ix.table != nullptr) return table_has(ix.table, first, n, x);
+    const uint64_t p = csr_lower_bound(ix.csr, lo, lo + n, x);
     return p < lo + n && __ldg(ix.csr + p) == x;
 }
 
@@ -187,16 +225,16 @@ __device__ __forceinline__ int accept_without_prev(const StepConsts &c, const St
 // them probes of this search.
 template <bool SOPR>
 __device__ __forceinline__ bool accept_candidate(const StepConsts &c, const StepThr &t, float rv, uint32_t x,
-                                                 uint32_t prev, uint32_t cur, const CsrIndex &pix, uint64_t phead,
-                                                 uint32_t pdeg)
+                                                 uint32_t prev, uint32_t cur, const CsrIndex &pix, uint32_t pbucket,
+                                                 uint64_t phead, uint32_t pdeg)
 {
     const int v = accept_without_prev<SOPR>(c, t, rv, x, prev, cur);
     if (v >= 0) return v != 0;
-    return csr_contains(pix, phead, pdeg, x) ? (rv < thr_found<SOPR>(c, t)) : (rv < thr_notfound<SOPR>(c, t));
+    return csr_contains(pix, pbucket, phead, pdeg, x) ? (rv < thr_found<SOPR>(c, t)) : (rv < thr_notfound<SOPR>(c, t));
 }
 
-// A walker whose step has already rejected this many attempts is served by
-// the whole warp (warp_first_accept).
+// A walker whose step has rejected this many attempts is served by the whole
+// warp (warp_first_accept).
 constexpr uint32_t kHardAttempts = 4;
 
 __device__ __forceinline__ uint64_t shfl64(uint64_t v, int src)
@@ -305,7 +343,7 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
     uint32_t lo = 0, hi = 0;
     if (lane <= pdeg) {
         const uint32_t y = (lane < pdeg) ? __ldg(pix.csr + phead + lane) : prev;
-        lo = (uint32_t)(csr_lower_bound(cix, head, head + deg, y) - head);
+        lo = (uint32_t)(csr_lower_bound(cix.csr, head, head + deg, y) - head);
         hi = lo;
         while (hi < deg && __ldg(cix.csr + head + hi) == y) hi++;
     }
@@ -402,7 +440,8 @@ __device__ __forceinline__ uint32_t warp_first_accept(const StepConsts &c, const
                                                       uint32_t hop, uint32_t p0, uint32_t limit,
                                                       const CsrIndex &cix, uint64_t head, uint32_t deg,
                                                       uint32_t prev, uint32_t cur, const CsrIndex &pix,
-                                                      uint64_t phead, uint32_t pdeg, uint32_t *iv, uint32_t *x_out)
+                                                      uint32_t pbucket, uint64_t phead, uint32_t pdeg, uint32_t *iv,
+                                                      uint32_t *x_out)
 {
     if (pdeg < 32 && prev != cur)
         return warp_first_accept_runs<SOPR>(c, t, wid, hop, p0, limit, cix, head, deg, prev, pix, phead, pdeg, iv,
@@ -419,9 +458,7 @@ __device__ __forceinline__ uint32_t warp_first_accept(const StepConsts &c, const
             const uint32_t pos = fastmod(r.x, M, deg);
             const float rv = rand_val(r.y, maxv);
             x = __ldg(cix.csr + head + pos);
-            // N(prev) serves every attempt of the step and stays in L1: a
-            // plain binary search beats the sample levels here.
-            acc = accept_candidate<SOPR>(c, t, rv, x, prev, cur, CsrIndex{pix.csr, {}, 0}, phead, pdeg);
+            acc = accept_candidate<SOPR>(c, t, rv, x, prev, cur, pix, pbucket, phead, pdeg);
         }
         const unsigned m = __ballot_sync(0xFFFFFFFFu, acc);
         if (m) {

@@ -21,28 +21,39 @@
 namespace gw {
 
 // Words of a lane's walker parked in shared memory while its warp serves hard
-// steps (kPkAstar receives the accepting attempt found for it).
+// steps.
 enum ParkWord : int {
     kPkWid = 0, kPkPrev, kPkCur, kPkHop, kPkAttempt, kPkDeg, kPkPdeg, kPkHeadLo, kPkHeadHi, kPkPheadLo,
-    kPkPheadHi, kPkHashLo, kPkHashHi, kPkThr0, kPkThr1, kPkThr2, kPkRx, kPkRy, kPkTrials, kPkAstar, kPkCount
+    kPkPheadHi, kPkBucket, kPkPbucket, kPkMagic, kPkHashLo, kPkHashHi, kPkThr0, kPkThr1, kPkThr2, kPkTrials, kPkCount
 };
 
 // W: weighted Node2vec -- the trial's candidate is alias column r.x % deg,
 // kept when float(r.w >> 8) * 2^-24 < its probability, else its alias (the
 // alias tables of gw_weighted.cu); everything else is the unweighted step.
+//
+// One round of the loop is one trial of every active lane: the draw, the
+// candidate, then the new vertex's record and (where the verdict needs it) the
+// search of N(prev), in flight together.  A warp spends the time of its
+// longest lane in each part, so the parts that differ between lanes are kept
+// short: one draw for accepted, rejected and new walkers alike, a membership
+// table (csr_contains), one load for a vertex's record.
 template <bool SOPR, bool PATHS, bool COOP, int MINB, bool W = false>
 __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid_constant__ IncoreArgs a)
 {
-    __shared__ uint32_t s_iv[kWalkThreads / 32][kCoopScratchWords];  // per-warp scratch of warp_first_accept
+    __shared__ uint32_t s_iv[COOP ? kWalkThreads / 32 : 1][kCoopScratchWords];  // scratch of warp_first_accept
     __shared__ unsigned long long s_ws[kWalkThreads / 32][kWsCount];  // per-warp statistics
+    __shared__ unsigned long long s_hash[kWalkThreads], s_steps[kWalkThreads];  // per lane, of finished walkers
+    __shared__ uint32_t s_done[kWalkThreads];
     __shared__ uint32_t s_park[COOP ? kWalkThreads / 32 : 1][kPkCount][32];  // lane state during hard steps
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt_mask = (1u << lane) - 1u;
     if (lane < kWsCount) s_ws[warp][lane] = 0;
+    s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
+    s_done[threadIdx.x] = 0;
     __syncwarp();
-    const uint64_t *__restrict__ beg = a.beg;
-    const uint32_t *__restrict__ csr = a.ix.csr;
+    const CsrIndex ix{a.csr, a.table};
+    const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     const uint32_t chunk = a.chunk ? a.chunk : kChunk;
 
@@ -50,27 +61,22 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
     bool exhausted = false;          // warp-uniform
     bool active = false;
 
-    // Lane state.  Statistics live in s_ws and the path row is recomputed
-    // from wid, so the registers hold only what the next trial reads.
+    // Lane state.  Statistics live in shared memory and the path row is
+    // recomputed from wid, so the registers hold only what the next trial
+    // reads.  `attempt` is the attempt the next trial evaluates.
     uint32_t wid = 0, prev = 0, cur = 0, hop = 0, attempt = 0;
-    uint32_t deg = 0, pdeg = 0;
+    uint32_t deg = 0, pdeg = 0, bucket = 0, pbucket = 0, magic = 0;
     uint64_t head = 0, phead = 0, h = 0;
-    U4 r{0, 0, 0, 0};
     StepThr t{0.f, 0.f, 0.f};
     uint32_t n_trials = 0;  // trials not yet added to s_ws
 
-    auto flush_trials = [&]() {
-        atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
-        n_trials = 0;
-    };
     // A walker's steps are its hops: every accepted trial moves it one hop.
     auto finish = [&]() {
         a.hashes[wid - a.out_base] = h;
         a.lens[wid - a.out_base] = hop + 1;
-        atomicAdd(&s_ws[warp][kWsSteps], (unsigned long long)hop);
-        atomicAdd(&s_ws[warp][kWsDone], 1ull);
-        atomicAdd(&s_ws[warp][kWsHash], (unsigned long long)h);
-        flush_trials();
+        s_steps[threadIdx.x] += hop;
+        s_hash[threadIdx.x] += h;
+        s_done[threadIdx.x] += 1;
         active = false;
     };
 
@@ -97,26 +103,22 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
                 const uint32_t src = walker_source(a.init, wid);
                 prev = cur = src;
                 hop = 0;
+                attempt = 0;
                 h = hash_init(src);
                 if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride] = src;
-                if (src >= a.nverts) {
-                    atomicOr(a.err, kErrSource);
-                    finish();
-                } else if (maxhops == 0) {
-                    finish();
+                Vertex vx{0, 0, 0, 0};
+                if (src >= a.nverts) atomicOr(a.err, kErrSource);
+                else if (maxhops != 0) vx = load_vertex(a, src);
+                deg = vx.deg;
+                if (deg == 0) {
+                    finish();  // bad source, no steps asked for, or a dead end (engine/engine.hpp:196-199)
                 } else {
-                    head = __ldg(beg + src);
-                    deg = (uint32_t)(__ldg(beg + src + 1) - head);
-                    if (deg == 0) {
-                        finish();  // dead end (engine/engine.hpp:196-199)
-                    } else {
-                        phead = head;
-                        pdeg = deg;
-                        t = step_thresholds<SOPR>(a.c, deg, pdeg);
-                        r = draw(a.c, wid, 0, 0);
-                        attempt = 1;
-                        active = true;
-                    }
+                    phead = head = vx.head;
+                    pbucket = bucket = vx.bucket;
+                    pdeg = deg;
+                    magic = vx.magic;
+                    t = step_thresholds<SOPR>(a.c, deg, pdeg);
+                    active = true;
                 }
             }
             q_next += min((uint32_t)__popc(need), avail);
@@ -124,12 +126,13 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
         if (!__any_sync(0xFFFFFFFFu, active)) break;
 
         // Walkers whose step keeps rejecting (a low-degree prev next to a hub
-        // under SOPR) are served one at a time by the whole warp; the lane
-        // then re-takes the accepting attempt below.  Meanwhile every lane's
-        // walker is parked in shared memory: the registers go to the attempt
-        // loop, and lane L's fields reach all lanes as broadcast loads.
+        // under SOPR) are served one at a time by the whole warp, which finds
+        // their accepting attempt; the lane then takes it below.  Meanwhile
+        // every lane's walker is parked in shared memory: the registers go to
+        // the attempt loop, and lane L's fields reach all lanes as broadcast
+        // loads.
         if (COOP) {
-            const unsigned hm = __ballot_sync(0xFFFFFFFFu, active && attempt > kHardAttempts);
+            const unsigned hm = __ballot_sync(0xFFFFFFFFu, active && attempt >= kHardAttempts);
             if (hm) {
                 uint32_t(*pk)[32] = s_park[COOP ? warp : 0];
                 pk[kPkWid][lane] = wid;
@@ -143,18 +146,19 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
                 pk[kPkHeadHi][lane] = (uint32_t)(head >> 32);
                 pk[kPkPheadLo][lane] = (uint32_t)phead;
                 pk[kPkPheadHi][lane] = (uint32_t)(phead >> 32);
+                pk[kPkBucket][lane] = bucket;
+                pk[kPkPbucket][lane] = pbucket;
+                pk[kPkMagic][lane] = magic;
                 pk[kPkHashLo][lane] = (uint32_t)h;
                 pk[kPkHashHi][lane] = (uint32_t)(h >> 32);
                 pk[kPkThr0][lane] = __float_as_uint(t.inv_deg);
                 pk[kPkThr1][lane] = __float_as_uint(t.sum);
                 pk[kPkThr2][lane] = __float_as_uint(t.t_prev);
-                pk[kPkRx][lane] = r.x;
-                pk[kPkRy][lane] = r.y;
                 pk[kPkTrials][lane] = n_trials;
                 __syncwarp();
                 for (unsigned m = hm; m; m &= m - 1) {
                     const int L = __ffs(m) - 1;
-                    const uint32_t p0 = pk[kPkAttempt][L] - 1;
+                    const uint32_t p0 = pk[kPkAttempt][L];
                     const uint32_t Lprev = pk[kPkPrev][L], Lcur = pk[kPkCur][L], Lpdeg = pk[kPkPdeg][L];
                     const uint64_t hd = ((uint64_t)pk[kPkHeadHi][L] << 32) | pk[kPkHeadLo][L];
                     const uint64_t ph = ((uint64_t)pk[kPkPheadHi][L] << 32) | pk[kPkPheadLo][L];
@@ -162,14 +166,16 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
                                      __uint_as_float(pk[kPkThr2][L])};
                     uint32_t xs;
                     const uint32_t astar = warp_first_accept<SOPR>(a.c, tl, pk[kPkWid][L], pk[kPkHop][L], p0,
-                                                                   kMaxAttempts, a.ix, hd, pk[kPkDeg][L], Lprev, Lcur,
-                                                                   a.ix, ph, Lpdeg, s_iv[warp], &xs);
+                                                                   kMaxAttempts, ix, hd, pk[kPkDeg][L],
+                                                                   Lprev, Lcur, ix, pk[kPkPbucket][L], ph, Lpdeg,
+                                                                   s_iv[COOP ? warp : 0], &xs);
+                    __syncwarp();  // every lane has read lane L's fields
                     if (lane == 0) {
-                        pk[kPkAstar][L] = astar;
+                        pk[kPkAttempt][L] = astar;
+                        pk[kPkTrials][L] += astar - p0;
                         const bool by_pos = Lpdeg < 32 && Lprev != Lcur;
-                        atomicAdd(&s_ws[warp][by_pos ? kWsCoopSmall : kWsCoopLarge], 1ull);
-                        atomicAdd(&s_ws[warp][by_pos ? kWsCoopSmallAtt : kWsCoopLargeAtt],
-                                  (unsigned long long)(astar - p0 + 1));
+                        s_ws[warp][by_pos ? kWsCoopSmall : kWsCoopLarge] += 1ull;
+                        s_ws[warp][by_pos ? kWsCoopSmallAtt : kWsCoopLargeAtt] += (unsigned long long)(astar - p0 + 1);
                     }
                 }
                 __syncwarp();
@@ -182,23 +188,17 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
                 pdeg = pk[kPkPdeg][lane];
                 head = ((uint64_t)pk[kPkHeadHi][lane] << 32) | pk[kPkHeadLo][lane];
                 phead = ((uint64_t)pk[kPkPheadHi][lane] << 32) | pk[kPkPheadLo][lane];
+                bucket = pk[kPkBucket][lane];
+                pbucket = pk[kPkPbucket][lane];
+                magic = pk[kPkMagic][lane];
                 h = ((uint64_t)pk[kPkHashHi][lane] << 32) | pk[kPkHashLo][lane];
                 t.inv_deg = __uint_as_float(pk[kPkThr0][lane]);
                 t.sum = __uint_as_float(pk[kPkThr1][lane]);
                 t.t_prev = __uint_as_float(pk[kPkThr2][lane]);
-                r.x = pk[kPkRx][lane];
-                r.y = pk[kPkRy][lane];
                 n_trials = pk[kPkTrials][lane];
-                if ((hm >> lane) & 1u) {
-                    const uint32_t astar = pk[kPkAstar][lane];
-                    n_trials += astar - (attempt - 1);
-                    if (astar >= kMaxAttempts) {
-                        atomicOr(a.err, kErrTrials);
-                        finish();
-                    } else {
-                        r = draw(a.c, wid, hop, astar);
-                        attempt = astar + 1;
-                    }
+                if (active && attempt >= kMaxAttempts) {
+                    atomicOr(a.err, kErrTrials);
+                    finish();
                 }
                 __syncwarp();
             }
@@ -206,7 +206,12 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
         if (!active) continue;
 
         // One rejection-sampling trial.
-        const uint32_t pos = r.x % deg;
+        const U4 r = draw(a.c, wid, hop, attempt);
+        if (attempt == 0 && hop != 0 && terminates(a.c, r.z)) {
+            finish();
+            continue;
+        }
+        const uint32_t pos = mod_by(r.x, deg, magic);
         const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
         uint32_t col = pos;
         if constexpr (W) {
@@ -215,55 +220,50 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
         }
         const uint32_t x = __ldg(csr + head + col);
         n_trials++;
-        if (accept_candidate<SOPR>(a.c, t, rv, x, prev, cur, a.ix, phead, pdeg)) {
+        int verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
+        // the record of a vertex that is, or may be, the next one
+        const bool last = hop + 1 >= maxhops, in_range = x < a.nverts;
+        Vertex vx{0, 0, 0, 0};
+        if (verdict != 0 && !last && in_range) vx = load_vertex(a, x);
+        if (verdict < 0)
+            verdict = csr_contains(ix, pbucket, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t);
+        if (verdict) {
             hop++;
             h = hash_step(h, x);
             if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride + hop] = x;
-            if (n_trials & 0x80000000u) flush_trials();  // a step adds < 2^27: no wrap
+            if (n_trials & 0x80000000u) {  // a step adds < 2^27: no wrap
+                atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
+                n_trials = 0;
+            }
+            attempt = 0;
             prev = cur;
             phead = head;
             pdeg = deg;
+            pbucket = bucket;
             cur = x;
-            if (hop >= maxhops) {
-                finish();
-            } else if (x >= a.nverts) {
-                atomicOr(a.err, kErrVertexRange);
-                finish();
-            } else if (a.c.term_prob > 0.0f) {
-                r = draw(a.c, wid, hop, 0);
-                attempt = 1;
-                if (terminates(a.c, r.z)) {
-                    finish();
-                } else {
-                    head = __ldg(beg + x);
-                    deg = (uint32_t)(__ldg(beg + x + 1) - head);
-                    if (deg == 0) finish();
-                    else t = step_thresholds<SOPR>(a.c, deg, pdeg);
-                }
-            } else {
-                head = __ldg(beg + x);
-                const uint64_t tail = __ldg(beg + x + 1);
-                r = draw(a.c, wid, hop, 0);
-                attempt = 1;
-                deg = (uint32_t)(tail - head);
-                if (deg == 0) finish();
-                else t = step_thresholds<SOPR>(a.c, deg, pdeg);
-            }
-        } else if (attempt >= kMaxAttempts) {
+            head = vx.head;
+            deg = vx.deg;
+            bucket = vx.bucket;
+            magic = vx.magic;
+            if (!last && !in_range) atomicOr(a.err, kErrVertexRange);
+            if (deg == 0) finish();  // the last hop, a bad id, or a dead end
+            else t = step_thresholds<SOPR>(a.c, deg, pdeg);
+        } else if (++attempt >= kMaxAttempts) {
             atomicOr(a.err, kErrTrials);
             finish();
-        } else {
-            r = draw(a.c, wid, hop, attempt);
-            attempt++;
         }
     }
 
     __syncwarp();
+    const unsigned long long trials = warp_sum((unsigned long long)n_trials);
+    const unsigned long long steps = warp_sum(s_steps[threadIdx.x]);
+    const unsigned long long hashes = warp_sum(s_hash[threadIdx.x]);
+    const unsigned long long done = warp_sum((unsigned long long)s_done[threadIdx.x]);
     if (lane == 0) {
-        atomicAdd(&a.ctr[kCtrSteps], s_ws[warp][kWsSteps]);
-        atomicAdd(&a.ctr[kCtrTrials], s_ws[warp][kWsTrials]);
-        atomicAdd(&a.ctr[kCtrDone], s_ws[warp][kWsDone]);
-        atomicAdd(&a.ctr[kCtrHashSum], s_ws[warp][kWsHash]);
+        atomicAdd(&a.ctr[kCtrSteps], steps);
+        atomicAdd(&a.ctr[kCtrTrials], trials + s_ws[warp][kWsTrials]);
+        atomicAdd(&a.ctr[kCtrDone], done);
+        atomicAdd(&a.ctr[kCtrHashSum], hashes);
         if (COOP) {
             atomicAdd(&a.ctr[kCtrCoopSmall], s_ws[warp][kWsCoopSmall]);
             atomicAdd(&a.ctr[kCtrCoopSmallAtt], s_ws[warp][kWsCoopSmallAtt]);
@@ -274,39 +274,117 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
 }
 
 // Memory-safety check of a resident CSR before any walk reads it: offsets
-// non-decreasing and within [0, nedges], every neighbour id < nverts.
-// (Adjacency order is a precondition -- the reference's `sorted` option --
-// and affects results, not safety.)
-__global__ void k_validate_csr(const uint64_t *__restrict__ beg, const uint32_t *__restrict__ csr,
-                               uint32_t nverts, uint64_t nedges, uint32_t *err)
+// non-decreasing and within [0, nedges], every neighbour id < nverts; the
+// vertex index is written from the same reads of the offsets.  (Adjacency
+// order is a precondition -- the reference's `sorted` option -- and affects
+// results, not safety.)  Bound by reading the CSR once: eight ids (one sector)
+// per thread and load.  A warp takes its vertices' buckets with one atomic.
+__global__ void __launch_bounds__(256) k_validate_csr(const __grid_constant__ CsrCheck a)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u;
     bool bad = false;
-    for (uint64_t v = t0; v < nverts; v += stride) {
-        const uint64_t a = beg[v], b = beg[v + 1];
-        bad |= (a > b) | (b > nedges);
+    for (uint64_t v0 = t0 - lane; v0 < a.nverts; v0 += stride) {
+        const uint64_t v = v0 + lane;
+        uint64_t b = 0, e = 0;
+        if (v < a.nverts) {
+            b = a.beg[v];
+            e = a.beg[v + 1];
+            bad |= (b > e) | (e > a.nedges);
+        }
+        if (a.verts) {
+            const uint32_t d = (uint32_t)(e - b);
+            const uint32_t n = table_buckets(d);
+            uint32_t x = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            unsigned long long base = 0;
+            if (lane == 31 && x) base = atomicAdd(a.nbuckets, (unsigned long long)x);
+            base = __shfl_sync(0xFFFFFFFFu, base, 31);
+            if (v < a.nverts) {
+                a.verts[v] = make_uint4((uint32_t)b, d, (uint32_t)base + x - n, d ? mod_magic(d) : 0u);
+                if (a.heads_hi) a.heads_hi[v] = (uint32_t)(b >> 32);
+            }
+        }
     }
-    for (uint64_t i = t0; i < nedges; i += stride) bad |= csr[i] >= nverts;
-    if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0) atomicOr(err, kErrVertexRange);
+    uint64_t done = 0;
+    if (((uintptr_t)a.csr & 31u) == 0) {
+        const uint64_t sectors = a.nedges / 8;
+        for (uint64_t j = t0; j < sectors; j += stride) {
+            uint32_t v[8];
+            load_sector(a.csr + 8 * j, v);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) bad |= v[i] >= a.nverts;
+        }
+        done = 8 * sectors;
+    }
+    for (uint64_t i = done + t0; i < a.nedges; i += stride) bad |= __ldg(a.csr + i) >= a.nverts;
+    if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(a.err, kErrVertexRange);
 }
 
-__global__ void k_sample_level(const uint32_t *__restrict__ src, uint64_t n, uint32_t *__restrict__ dst)
+cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s)
 {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) dst[j] = src[32 * j];
-}
-
-cudaError_t launch_sample_level(const uint32_t *src, uint64_t n, uint32_t *dst, int num_sms, cudaStream_t s)
-{
-    k_sample_level<<<num_sms * 8, 256, 0, s>>>(src, n, dst);
+    k_validate_csr<<<num_sms * 8, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
-cudaError_t launch_validate_csr(const uint64_t *beg, const uint32_t *csr, uint32_t nverts, uint64_t nedges,
-                                uint32_t *err, int num_sms, cudaStream_t s)
+// The membership tables: a thread takes 32 consecutive edges, finds the first
+// one's vertex by halving the offsets and goes on from there, so hubs and
+// isolated vertices cost alike.  An id claims the first free slot from its home
+// bucket on; an id met twice keeps one slot.  Bound by the claims, about two
+// atomics an edge into the L2.
+constexpr uint32_t kTableEdges = 32;
+__global__ void __launch_bounds__(256) k_build_table(const uint64_t *__restrict__ beg, const uint4 *__restrict__ verts,
+                                                     uint32_t nverts, const uint32_t *__restrict__ csr,
+                                                     uint64_t nedges, uint32_t *table)
 {
-    k_validate_csr<<<num_sms * 8, 256, 0, s>>>(beg, csr, nverts, nedges, err);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * kTableEdges;
+    for (uint64_t e0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * kTableEdges; e0 < nedges; e0 += stride) {
+        uint32_t v = 0, hi = nverts;  // beg[v] <= e0 < beg[hi]
+        while (hi - v > 1) {
+            const uint32_t m = v + ((hi - v) >> 1);
+            if (__ldg(beg + m) <= e0) v = m;
+            else hi = m;
+        }
+        uint64_t end = __ldg(beg + v + 1);
+        uint32_t buckets = 0, first = 0;
+        const uint64_t e1 = min(e0 + kTableEdges, nedges);
+        for (uint64_t e = e0; e < e1; ++e) {
+            while (e >= end) {
+                ++v;
+                end = __ldg(beg + v + 1);
+                buckets = 0;
+            }
+            if (buckets == 0) {
+                const uint4 r = __ldg(verts + v);
+                buckets = table_buckets(r.y);
+                first = r.z;
+            }
+            const uint32_t x = __ldg(csr + e);
+            uint32_t b = table_home(x, buckets);
+            for (bool placed = false; !placed;) {  // the slots outnumber the ids
+                uint32_t *slot = table + ((uint64_t)first + b) * 8u;
+                for (int k = 0; k < 8 && !placed; ++k) {
+                    const uint32_t was = atomicCAS(slot + k, kEmptySlot, x);
+                    placed = was == kEmptySlot || was == x;
+                }
+                b = b + 1 == buckets ? 0u : b + 1;
+            }
+        }
+    }
+}
+
+cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t nverts, const uint32_t *csr,
+                               uint64_t nedges, uint32_t *table, int num_sms, cudaStream_t s)
+{
+    const uint64_t need = (nedges + 256ull * kTableEdges - 1) / (256ull * kTableEdges);
+    if (need == 0) return cudaSuccess;
+    k_build_table<<<(int)(need < (uint64_t)num_sms * 8 ? need : (uint64_t)num_sms * 8), 256, 0, s>>>(
+        beg, verts, nverts, csr, nedges, table);
     return cudaGetLastError();
 }
 

@@ -22,8 +22,8 @@ constexpr uint32_t kHopDone = 0xFFFFFFFFu;  // hop word of a finished walker
 template <bool SOPR, bool PATHS>
 __global__ void __launch_bounds__(256) k_walk_hop(const __grid_constant__ IncoreArgs a, HopState st, uint32_t round)
 {
-    const uint64_t *__restrict__ beg = a.beg;
-    const uint32_t *__restrict__ csr = a.ix.csr;
+    const CsrIndex ix{a.csr, a.table};
+    const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     unsigned long long n_steps = 0, n_trials = 0, n_done = 0, n_hash = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -52,20 +52,22 @@ __global__ void __launch_bounds__(256) k_walk_hop(const __grid_constant__ Incore
         if (!done) {
             U4 r = draw(a.c, wid, hop, 0);
             uint32_t attempt = 1;
-            const uint64_t head = __ldg(beg + cur);
-            const uint32_t deg = (uint32_t)(__ldg(beg + cur + 1) - head);
+            const Vertex vc = load_vertex(a, cur);
+            const uint64_t head = vc.head;
+            const uint32_t deg = vc.deg;
             if ((hop > 0 && terminates(a.c, r.z)) || deg == 0) {
                 done = true;  // termination draw, or a dead end (engine/engine.hpp:196-199)
             } else {
-                const uint64_t phead = __ldg(beg + prev);
-                const uint32_t pdeg = (uint32_t)(__ldg(beg + prev + 1) - phead);
+                const Vertex vp = load_vertex(a, prev);
+                const uint64_t phead = vp.head;
+                const uint32_t pdeg = vp.deg;
                 const StepThr t = step_thresholds<SOPR>(a.c, deg, pdeg);
                 for (;;) {
                     const uint32_t pos = r.x % deg;
                     const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
                     const uint32_t x = __ldg(csr + head + pos);
                     n_trials++;
-                    if (accept_candidate<SOPR>(a.c, t, rv, x, prev, cur, a.ix, phead, pdeg)) {
+                    if (accept_candidate<SOPR>(a.c, t, rv, x, prev, cur, ix, vp.bucket, phead, pdeg)) {
                         hop++;
                         n_steps++;
                         h = hash_step(h, x);

@@ -185,8 +185,8 @@ int gw_handle::init_device()
     if ((st = cuda(cudaEventCreate(&ev_kernel0), "event"))) return st;
     if ((st = cuda(cudaEventCreate(&ev_kernel1), "event"))) return st;
     if ((st = cuda(cudaEventCreate(&ev_stop), "event"))) return st;
-    if ((st = cuda(cudaMalloc(&d_ctr, sizeof(unsigned long long) * kCtrCount), "counters"))) return st;
-    if ((st = cuda(cudaMalloc(&d_err, sizeof(uint32_t)), "error word"))) return st;
+    if ((st = cuda(cudaMalloc(&d_ctr, sizeof(unsigned long long) * (kCtrCount + 1)), "counters"))) return st;
+    d_err = reinterpret_cast<uint32_t *>(d_ctr + kCtrCount);
     if ((st = cuda(cudaMallocHost(&h_ctr, sizeof(unsigned long long) * (kCtrCount + 1)), "pinned counters")))
         return st;
     memset(h_ctr, 0, sizeof(unsigned long long) * (kCtrCount + 1));
@@ -209,7 +209,6 @@ void gw_handle::release()
     cudaFree(d_lens);
     cudaFree(d_hashes);
     cudaFree(d_ctr);
-    cudaFree(d_err);
     cudaFree(d_verts);
     cudaFree(d_heads_hi);
     cudaFree(d_table);
@@ -545,11 +544,10 @@ int gw_handle::validate_graph(cudaStream_t s)
         check.nbuckets = d_ctr;
     }
     uint64_t ends[2] = {1, 0};
-    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long), s), "memset")) ||
+    const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);
+    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, ctr_bytes, s), "memset")) ||
         (st = cuda(launch_validate_csr(check, num_sms, s), "validate")) ||
-        (st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s), "buckets")) ||
-        (st = cuda(cudaMemcpyAsync(h_ctr + kCtrCount, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-                   "error word D2H")) ||
+        (st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, ctr_bytes, cudaMemcpyDeviceToHost, s), "buckets D2H")) ||
         (st = cuda(cudaMemcpyAsync(&ends[0], dev_beg, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "beg[0]")) ||
         (st = cuda(cudaMemcpyAsync(&ends[1], dev_beg + nverts, sizeof(uint64_t), cudaMemcpyDeviceToHost, s), "beg[V]")) ||
         (st = cuda(cudaStreamSynchronize(s), "validate")))
@@ -613,7 +611,6 @@ int gw_handle::run_incore(gw_stats *stats)
     if (!resident) {
         if ((st = upload_whole_graph(s, &h2d))) return st;
     }
-    if ((st = cuda(cudaMemsetAsync(d_err, 0, sizeof(uint32_t), s), "memset"))) return st;
     if (!validated && (st = validate_graph(s))) return st;
     if (weighted) {
         if (cfg.algorithm != GW_NODE2VEC)
@@ -639,7 +636,6 @@ int gw_handle::run_incore(gw_stats *stats)
     a.nverts = nverts;
     a.nwalkers = (uint32_t)nwalkers;
     a.wid_base = wid_first;
-    a.wid_stride = 1;
     a.out_base = wid_first;
     a.paths = (cfg.record_paths == GW_PATHS_FULL) ? d_paths : nullptr;
     a.stride = cfg.maxhops + 1;
@@ -665,15 +661,14 @@ int gw_handle::run_incore(gw_stats *stats)
             return rc;
         }
         const uint32_t rounds = cfg.maxhops ? cfg.maxhops : 1;
-        if (!(rc = cuda(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long) * kCtrCount, s), "memset")) &&
+        if (!(rc = cuda(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long) * (kCtrCount + 1), s), "memset")) &&
             !(rc = cuda(cudaEventRecord(ev_kernel0, s), "event"))) {
             for (uint32_t k = 0; k < rounds && !rc; ++k) rc = cuda(launch_walk_hop(a, hs, sopr, k, num_sms, s), "hop launch");
         }
         if (!rc && !(rc = cuda(cudaEventRecord(ev_kernel1, s), "event")) &&
-            !(rc = cuda(cudaMemcpyAsync(h_ctr, d_ctr, sizeof(unsigned long long) * kCtrCount, cudaMemcpyDeviceToHost, s),
+            !(rc = cuda(cudaMemcpyAsync(h_ctr, d_ctr, sizeof(unsigned long long) * (kCtrCount + 1),
+                                        cudaMemcpyDeviceToHost, s),
                         "counters D2H")) &&
-            !(rc = cuda(cudaMemcpyAsync(h_ctr + kCtrCount, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-                        "error word D2H")) &&
             !(rc = cuda(cudaEventRecord(ev_stop, s), "event")))
             rc = cuda(cudaStreamSynchronize(s), "walk");
         cudaStreamSynchronize(s);
@@ -705,79 +700,18 @@ int gw_handle::run_incore(gw_stats *stats)
                         (unsigned long long)nwalkers);
         return GW_OK;
     }
-    // kernel class for the autotuner: (sopr, paths, coop), weighted Node2vec apart
-    const int combo = weighted ? 8 | (a.paths ? 2 : 0) : (sopr ? 4 : 0) | (a.paths ? 2 : 0) | (coop ? 1 : 0);
-    auto grid_of = [&](int v, bool paths_on) {
-        return weighted ? incore_grid_weighted(paths_on, v, num_sms) : incore_grid(sopr, paths_on, coop, v, num_sms);
-    };
-    auto launch = [&](const IncoreArgs &x, int v, int g) {
-        return weighted ? launch_walk_incore_weighted(x, v, g, s) : launch_walk_incore(x, sopr, coop, v, g, s);
-    };
-    int variant = tuned_variant[combo];
-    // Walkers per warp claim: few lanes idle at the end of a run with small
-    // claims, fewer atomics with large ones; the autotuner picks among these.
-    static const uint32_t kChunks[] = {16, 64, 256};
-    if (cfg.blockpergrid == 0 && variant < 0) {
-        // Autotuner: time each register-cap variant with each claim size on
-        // this run's walkers (their outputs are rewritten by the full run
-        // below) and keep the fastest pair for every later run of this kernel
-        // class.  Runs of up to 2^22 walkers are timed whole: with few walkers
-        // per lane the tail of the last round decides, and a part of the run
-        // would misrank the candidates.  Larger runs are timed on every 16th
-        // walker id, which keeps the run's mix of source degrees (R-MAT ids
-        // are not random in degree, so a contiguous range would not).  The
-        // candidates run in a forward then a reverse pass and keep their best
-        // time, so none gains from the caches the previous one warmed.
-        const uint32_t stride = nwalkers > (1ull << 22) ? 16u : 1u;
-        IncoreArgs c = a;
-        c.wid_base = wid_first;
-        c.wid_stride = stride;
-        c.nwalkers = (uint32_t)(nwalkers / stride);
-        constexpr int kCand = kIncoreVariants * 3;
-        float best = 1e30f;
-        float cand_ms[kCand];
-        for (float &m : cand_ms) m = 1e30f;
-        for (int i = 0; i < 2 * kCand; ++i) {
-            const int k = i < kCand ? i : 2 * kCand - 1 - i;
-            const int v = k / 3;
-            c.chunk = kChunks[k % 3];
-            if ((st = cuda(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long) * kCtrCount, s), "memset"))) return st;
-            if ((st = cuda(cudaEventRecord(ev_kernel0, s), "event"))) return st;
-            if ((st = cuda(launch(c, v, grid_of(v, c.paths != nullptr)), "walk kernel launch (tuning)")))
-                return st;
-            if ((st = cuda(cudaEventRecord(ev_kernel1, s), "event"))) return st;
-            if ((st = cuda(cudaEventSynchronize(ev_kernel1), "tuning"))) return st;
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, ev_kernel0, ev_kernel1);
-            cand_ms[k] = std::min(cand_ms[k], ms);
-        }
-        for (int k = 0; k < kCand; ++k) {
-            tuned_ms[combo][k / 3] = std::min(k % 3 == 0 ? 1e30f : tuned_ms[combo][k / 3], cand_ms[k]);
-            if (cand_ms[k] < best) {
-                best = cand_ms[k];
-                variant = k / 3;
-                tuned_chunk[combo] = kChunks[k % 3];
-            }
-        }
-        tuned_variant[combo] = variant;
-    }
-    if (variant < 0) variant = 1;
-    last_variant = variant;
-    a.chunk = tuned_chunk[combo] ? tuned_chunk[combo] : kChunk;
-    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, sizeof(unsigned long long) * kCtrCount, s), "memset"))) return st;
-    int grid = (int)cfg.blockpergrid;
-    if (grid <= 0) grid = grid_of(variant, a.paths != nullptr);
-    if ((st = cuda(cudaEventRecord(ev_kernel0, s), "event"))) return st;
-    if ((st = cuda(launch(a, variant, grid), "walk kernel launch"))) return st;
-    if ((st = cuda(cudaEventRecord(ev_kernel1, s), "event"))) return st;
-    if ((st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, sizeof(unsigned long long) * kCtrCount, cudaMemcpyDeviceToHost, s),
-                   "counters D2H")))
+    const IncorePlan plan = incore_plan(nwalkers, sopr, a.paths != nullptr, coop, weighted, index_ready,
+                                        (int)cfg.blockpergrid, num_sms);
+    a.lanes = plan.lanes;
+    a.chunk = plan.chunk;
+    const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);  // with the error word
+    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, ctr_bytes, s), "memset")) ||
+        (st = cuda(cudaEventRecord(ev_kernel0, s), "event")) ||
+        (st = cuda(launch_walk_incore(a, sopr, coop, plan.grid, s), "walk kernel launch")) ||
+        (st = cuda(cudaEventRecord(ev_kernel1, s), "event")) ||
+        (st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, ctr_bytes, cudaMemcpyDeviceToHost, s), "counters D2H")) ||
+        (st = cuda(cudaEventRecord(ev_stop, s), "event")) || (st = cuda(cudaStreamSynchronize(s), "walk")))
         return st;
-    if ((st = cuda(cudaMemcpyAsync(h_ctr + kCtrCount, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
-                   "error word D2H")))
-        return st;
-    if ((st = cuda(cudaEventRecord(ev_stop, s), "event"))) return st;
-    if ((st = cuda(cudaStreamSynchronize(s), "walk"))) return st;
     last_hash_sum = h_ctr[kCtrHashSum];
     last_steps = h_ctr[kCtrSteps];
     const uint32_t errw = (uint32_t)h_ctr[kCtrCount];
@@ -791,7 +725,7 @@ int gw_handle::run_incore(gw_stats *stats)
         stats->block_loads = h2d ? nblocks : 0;
         stats->iterations = 1;
         stats->launches = 1;
-        stats->kernel_variant = (uint32_t)variant;
+        stats->kernel_variant = plan.ctas_per_sm;
         stats->walker_chunk = a.chunk;
         stats->coop_small_steps = h_ctr[kCtrCoopSmall];
         stats->coop_small_attempts = h_ctr[kCtrCoopSmallAtt];

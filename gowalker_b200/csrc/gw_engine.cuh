@@ -72,18 +72,11 @@ struct gw_handle {
     uint32_t path_stride = 0;
 
     // counters
-    unsigned long long *d_ctr = nullptr;
-    uint32_t *d_err = nullptr;
+    unsigned long long *d_ctr = nullptr;  // kCtrCount counters, then the error word
+    uint32_t *d_err = nullptr;            // that word
     unsigned long long *h_ctr = nullptr;  // pinned: kCtrCount counters + error word
     uint64_t last_hash_sum = 0;
     uint64_t last_steps = 0;
-
-    // autotuner: best register-cap variant per in-core kernel class
-    // (sopr, paths, coop) and the measured times of each variant
-    int tuned_variant[16] = {-1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1, -1};
-    float tuned_ms[16][gw::kIncoreVariants] = {};
-    uint32_t tuned_chunk[16] = {};  // walkers per warp claim the autotuner picked per kernel class
-    int last_variant = -1;
 
     // out-of-core state (gw_ooc.cu)
     gw::OocState *ooc = nullptr;

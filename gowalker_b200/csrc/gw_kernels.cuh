@@ -7,7 +7,7 @@
 namespace gw {
 
 constexpr int kWalkThreads = 256;   // threads per CTA of the walk kernels
-constexpr uint32_t kChunk = 64;     // walkers a warp claims per atomic
+constexpr uint32_t kChunk = 64;     // walkers a warp of the out-of-core step claims per atomic
 
 // Work / statistics counters of one run (device, zeroed per run).
 enum Counter : int {
@@ -76,11 +76,11 @@ struct IncoreArgs {
     const uint32_t *heads_hi;  // high words of the first edges; null when all are 0
     const uint32_t *table;     // membership tables (table_has); set with verts
     uint32_t nverts;
-    uint32_t nwalkers;         // walkers of this launch: ids wid_base + i * wid_stride, i < nwalkers
+    uint32_t nwalkers;         // walkers of this launch: ids wid_base + i, i < nwalkers
     uint32_t wid_base;
-    uint32_t wid_stride;       // 1 for a run; > 1 for the autotuner's sample
     uint32_t out_base;         // first walker id of the population: outputs are indexed by wid - out_base
-    uint32_t chunk;            // walkers a warp claims per atomic (0: kChunk); the autotuner picks it
+    uint32_t chunk;            // walkers a warp claims per atomic (incore_plan)
+    uint32_t lanes;            // lanes of a warp that take walkers (incore_plan)
     uint32_t *paths;           // rows indexed by walker id, or null
     uint32_t stride;           // maxhops + 1
     uint32_t *lens;            // vertices per path
@@ -110,9 +110,11 @@ struct Vertex {
     uint32_t bucket; // first bucket of its membership table
     uint32_t magic;  // mod_magic(deg)
 };
+// INDEX: from the vertex index, else from the offsets.
+template <bool INDEX>
 __device__ __forceinline__ Vertex load_vertex(const IncoreArgs &a, uint32_t v)
 {
-    if (a.verts) {
+    if constexpr (INDEX) {
         const uint4 e = __ldg(a.verts + v);
         return Vertex{a.heads_hi ? ((uint64_t)__ldg(a.heads_hi + v) << 32) | e.x : e.x, e.y, e.z, e.w};
     }
@@ -128,14 +130,17 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
     return v;
 }
 
-// Grid size (CTAs) for a persistent walk kernel on this device.
-// `variant` selects the register cap (0: 4 CTAs/SM, 1: 5, 2: 6, 3: 8), see gw_walk.cu.
-constexpr int kIncoreVariants = 4;
-int incore_grid(bool sopr, bool paths, bool coop, int variant, int num_sms);
-cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int variant, int grid, cudaStream_t s);
-// Weighted Node2vec through the same kernel (candidates from a.alias).
-int incore_grid_weighted(bool paths, int variant, int num_sms);
-cudaError_t launch_walk_incore_weighted(const IncoreArgs &a, int variant, int grid, cudaStream_t s);
+// How an in-core run is launched.
+struct IncorePlan {
+    int grid;               // CTAs
+    uint32_t lanes, chunk;  // IncoreArgs
+    uint32_t ctas_per_sm;   // the kernel's register cap: CTAs of an SM it is built for
+};
+// `grid` CTAs as asked for, or (0) as many as are resident at once.
+IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, int grid,
+                       int num_sms);
+// a.alias set: weighted Node2vec.
+cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s);
 
 // One launch per hop (gw_walk_hop.cu): walker state between launches.
 struct HopState {

@@ -176,7 +176,6 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     a.csr = d_csr;  // no index: this entry point allocates nothing
     a.nverts = nverts;
     a.nwalkers = (uint32_t)nwalkers;
-    a.wid_stride = 1;
     a.paths = (cfg->record_paths == GW_PATHS_FULL) ? d_paths : nullptr;
     a.stride = cfg->maxhops + 1;
     a.lens = d_lens;
@@ -185,10 +184,11 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     a.err = err;
     const bool sopr = cfg->algorithm != GW_NODE2VEC;
     const bool coop = needs_coop(cfg->algorithm, a.c);
-    const int variant = 1;  // 5 CTAs per SM; this entry point keeps no tuning state
-    const int grid =
-        cfg->blockpergrid ? (int)cfg->blockpergrid : incore_grid(sopr, a.paths != nullptr, coop, variant, num_sms);
-    e = launch_walk_incore(a, sopr, coop, variant, grid, s);
+    const IncorePlan plan =
+        incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, false, (int)cfg->blockpergrid, num_sms);
+    a.lanes = plan.lanes;
+    a.chunk = plan.chunk;
+    e = launch_walk_incore(a, sopr, coop, plan.grid, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, sizeof(host_ctr), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {

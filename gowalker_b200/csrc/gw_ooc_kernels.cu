@@ -516,10 +516,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
             const uint64_t hd = shfl64(head, L), ph = shfl64(phead, L);
             const uint32_t *cc = shfl_ptr(ccsr, L), *pc = shfl_ptr(pcsr, L);
             uint32_t xs;
-            const CsrIndex cix{cc, nullptr}, pix{pc, nullptr};
+            const CsrIndex<false> pix{pc, nullptr};
             const uint32_t astar = warp_first_accept<SOPR>(
                 a.c, shfl_thr<SOPR>(t, L), __shfl_sync(0xFFFFFFFFu, wid, L), __shfl_sync(0xFFFFFFFFu, hop, L), p0,
-                kMaxAttempts, cix, hd, __shfl_sync(0xFFFFFFFFu, deg, L), __shfl_sync(0xFFFFFFFFu, prev, L),
+                kMaxAttempts, cc, hd, __shfl_sync(0xFFFFFFFFu, deg, L), __shfl_sync(0xFFFFFFFFu, prev, L),
                 __shfl_sync(0xFFFFFFFFu, cur, L), pix, 0u, ph, __shfl_sync(0xFFFFFFFFu, pdeg, L), s_iv[warp], &xs);
             if (lane == (uint32_t)L) {
                 n_trials += astar - p0;
@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         if (!ZC || s_mapped[cb]) zc_sectors += 1u;
         if (verdict < 0 && pcsr != nullptr) {
             if (!ZC || s_mapped[pb]) zc_sectors += search_sectors(pdeg);
-            verdict = (csr_contains(CsrIndex{pcsr, nullptr}, 0u, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
+            verdict = (csr_contains(CsrIndex<false>{pcsr, nullptr}, 0u, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
                                                                            : rv < thr_notfound<SOPR>(a.c, t))
                           ? 1
                           : 0;

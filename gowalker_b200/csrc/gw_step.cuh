@@ -119,11 +119,11 @@ __device__ __forceinline__ bool terminates(const StepConsts &c, uint32_t z)
 }
 
 // Neighbour array of the graph (or of one block), with the membership table of
-// its vertices when `table` is set (table_has); without it a search is a plain
-// binary search.
+// its vertices (table_has); without it a search is a plain binary search.
+template <bool TABLE>
 struct CsrIndex {
     const uint32_t *csr;
-    const uint32_t *table;  // buckets of eight ids, on 32-byte boundaries
+    const uint32_t *table;  // TABLE: buckets of eight ids, on 32-byte boundaries
 };
 
 // Membership table of one vertex's neighbours: table_buckets(d) buckets of
@@ -183,8 +183,8 @@ __device__ __forceinline__ uint64_t csr_lower_bound(const uint32_t *csr, uint64_
     return lo + a;
 }
 
-// Membership of x in the sorted csr[lo, lo + n), whose table (if any) starts
-// at bucket `first`.
+// Membership of x in the sorted csr[lo, lo + n), whose table starts at bucket
+// `first`.
 //
 // What bounds it: every probe of a search is a dependent load of a line of its
 // own and a warp waits for the longest chain of its lanes.  Halving takes 12
@@ -192,9 +192,11 @@ __device__ __forceinline__ uint64_t csr_lower_bound(const uint32_t *csr, uint64_
 // vertices walks visit most; a bucket is one load and eight compares.  Sample
 // levels of 32, eight-way levels and eight-way trees were all measured too:
 // fewer lines than halving, but no fewer instructions.
-__device__ __forceinline__ bool csr_contains(const CsrIndex &ix, uint32_t first, uint64_t lo, uint32_t n, uint32_t x)
+template <bool TABLE>
+__device__ __forceinline__ bool csr_contains(const CsrIndex<TABLE> &ix, uint32_t first, uint64_t lo, uint32_t n,
+                                             uint32_t x)
 {
-    if (ix.table != nullptr) return table_has(ix.table, first, n, x);
+    if constexpr (TABLE) return table_has(ix.table, first, n, x);
     const uint64_t p = csr_lower_bound(ix.csr, lo, lo + n, x);
     return p < lo + n && __ldg(ix.csr + p) == x;
 }
@@ -223,9 +225,9 @@ __device__ __forceinline__ int accept_without_prev(const StepConsts &c, const St
 // (three quarters of them) used to search.  The step kernels are bound by the
 // distinct lines their loads touch (one L1 tag access per cycle), most of
 // them probes of this search.
-template <bool SOPR>
+template <bool SOPR, bool TABLE>
 __device__ __forceinline__ bool accept_candidate(const StepConsts &c, const StepThr &t, float rv, uint32_t x,
-                                                 uint32_t prev, uint32_t cur, const CsrIndex &pix, uint32_t pbucket,
+                                                 uint32_t prev, uint32_t cur, const CsrIndex<TABLE> &pix, uint32_t pbucket,
                                                  uint64_t phead, uint32_t pdeg)
 {
     const int v = accept_without_prev<SOPR>(c, t, rv, x, prev, cur);
@@ -331,8 +333,8 @@ __device__ __forceinline__ uint32_t rand_bounds(const StepConsts &c, const StepT
 template <bool SOPR>
 __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, const StepThr &t, uint32_t wid,
                                                            uint32_t hop, uint32_t p0, uint32_t limit,
-                                                           const CsrIndex &cix, uint64_t head, uint32_t deg,
-                                                           uint32_t prev, const CsrIndex &pix, uint64_t phead,
+                                                           const uint32_t *ccsr, uint64_t head, uint32_t deg,
+                                                           uint32_t prev, const uint32_t *pcsr, uint64_t phead,
                                                            uint32_t pdeg, uint32_t *iv, uint32_t *x_out)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -342,10 +344,10 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
     // lane k < pdeg: run of N(prev)[k]; lane pdeg: run of prev
     uint32_t lo = 0, hi = 0;
     if (lane <= pdeg) {
-        const uint32_t y = (lane < pdeg) ? __ldg(pix.csr + phead + lane) : prev;
-        lo = (uint32_t)(csr_lower_bound(cix.csr, head, head + deg, y) - head);
+        const uint32_t y = (lane < pdeg) ? __ldg(pcsr + phead + lane) : prev;
+        lo = (uint32_t)(csr_lower_bound(ccsr, head, head + deg, y) - head);
         hi = lo;
-        while (hi < deg && __ldg(cix.csr + head + hi) == y) hi++;
+        while (hi < deg && __ldg(ccsr + head + hi) == y) hi++;
     }
     if (lane < pdeg) {
         iv[lane] = lo;
@@ -420,7 +422,7 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
             const bool first_half = m0 != 0;
             const int f = __ffs(first_half ? m0 : m1) - 1;
             const uint32_t xf = __shfl_sync(0xFFFFFFFFu, first_half ? x0 : x1, f);
-            *x_out = __ldg(cix.csr + head + fastmod(xf, M, deg));
+            *x_out = __ldg(ccsr + head + fastmod(xf, M, deg));
             __syncwarp();
             return base + (first_half ? 0u : 32u) + (uint32_t)f;
         }
@@ -435,16 +437,16 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
 // attempt in attempt order -- the one a single thread evaluating them one by
 // one would take -- and its candidate in *x_out.  Returns `limit` if none of
 // the attempts below `limit` accepts.
-template <bool SOPR>
+template <bool SOPR, bool TABLE>
 __device__ __forceinline__ uint32_t warp_first_accept(const StepConsts &c, const StepThr &t, uint32_t wid,
                                                       uint32_t hop, uint32_t p0, uint32_t limit,
-                                                      const CsrIndex &cix, uint64_t head, uint32_t deg,
-                                                      uint32_t prev, uint32_t cur, const CsrIndex &pix,
+                                                      const uint32_t *ccsr, uint64_t head, uint32_t deg,
+                                                      uint32_t prev, uint32_t cur, const CsrIndex<TABLE> &pix,
                                                       uint32_t pbucket, uint64_t phead, uint32_t pdeg, uint32_t *iv,
                                                       uint32_t *x_out)
 {
     if (pdeg < 32 && prev != cur)
-        return warp_first_accept_runs<SOPR>(c, t, wid, hop, p0, limit, cix, head, deg, prev, pix, phead, pdeg, iv,
+        return warp_first_accept_runs<SOPR>(c, t, wid, hop, p0, limit, ccsr, head, deg, prev, pix.csr, phead, pdeg, iv,
                                             x_out);
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t M = fastmod_magic(deg);
@@ -457,7 +459,7 @@ __device__ __forceinline__ uint32_t warp_first_accept(const StepConsts &c, const
             const U4 r = draw(c, wid, hop, att);
             const uint32_t pos = fastmod(r.x, M, deg);
             const float rv = rand_val(r.y, maxv);
-            x = __ldg(cix.csr + head + pos);
+            x = __ldg(ccsr + head + pos);
             acc = accept_candidate<SOPR>(c, t, rv, x, prev, cur, pix, pbucket, phead, pdeg);
         }
         const unsigned m = __ballot_sync(0xFFFFFFFFu, acc);

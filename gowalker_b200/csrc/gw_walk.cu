@@ -14,7 +14,9 @@
 // or written; per walker the kernel writes its path row (optional), length
 // and 64-bit path hash.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
+#include <type_traits>
 #include "gw_kernels.cuh"
 #include "../../include/gowalker.h"
 
@@ -27,6 +29,13 @@ enum ParkWord : int {
     kPkPheadHi, kPkBucket, kPkPbucket, kPkMagic, kPkHashLo, kPkHashHi, kPkThr0, kPkThr1, kPkThr2, kPkTrials, kPkCount
 };
 
+// CTAs of an SM the kernel is built for: 5 leave 48 registers a thread, 4 leave
+// 64.  Measured, 5 against 4: n2v_large-like 3.17 / 3.31 ms, SOPR over 128 M
+// edges 29.6 / 30.8, weighted 0.67 / 0.70, L2-resident Node2vec 1.75 / 1.72;
+// Node2vec with hard steps (p 0.25, q 4) spills at 48: 3.81 / 3.25.  (6 and 8
+// spill everywhere and lose 5-100 %.)
+__host__ __device__ constexpr int walk_ctas(bool sopr, bool coop) { return coop && !sopr ? 4 : 5; }
+
 // W: weighted Node2vec -- the trial's candidate is alias column r.x % deg,
 // kept when float(r.w >> 8) * 2^-24 < its probability, else its alias (the
 // alias tables of gw_weighted.cu); everything else is the unweighted step.
@@ -37,8 +46,8 @@ enum ParkWord : int {
 // longest lane in each part, so the parts that differ between lanes are kept
 // short: one draw for accepted, rejected and new walkers alike, a membership
 // table (csr_contains), one load for a vertex's record.
-template <bool SOPR, bool PATHS, bool COOP, int MINB, bool W = false>
-__global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid_constant__ IncoreArgs a)
+template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX>
+__global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_incore(const __grid_constant__ IncoreArgs a)
 {
     __shared__ uint32_t s_iv[COOP ? kWalkThreads / 32 : 1][kCoopScratchWords];  // scratch of warp_first_accept
     __shared__ unsigned long long s_ws[kWalkThreads / 32][kWsCount];  // per-warp statistics
@@ -52,10 +61,11 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
     s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
     s_done[threadIdx.x] = 0;
     __syncwarp();
-    const CsrIndex ix{a.csr, a.table};
+    const CsrIndex<INDEX> ix{a.csr, a.table};
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
-    const uint32_t chunk = a.chunk ? a.chunk : kChunk;
+    const uint32_t chunk = a.chunk;
+    const bool takes = lane < a.lanes;
 
     uint32_t q_next = 0, q_end = 0;  // warp-uniform claimed range
     bool exhausted = false;          // warp-uniform
@@ -83,7 +93,7 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
     for (;;) {
         // Hand walkers to idle lanes.
         for (;;) {
-            const unsigned need = __ballot_sync(0xFFFFFFFFu, !active);
+            const unsigned need = __ballot_sync(0xFFFFFFFFu, takes && !active);
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 unsigned long long base = 0;
@@ -98,8 +108,8 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
             }
             const uint32_t avail = q_end - q_next;
             const uint32_t rank = __popc(need & lt_mask);
-            if (!active && rank < avail) {
-                wid = a.wid_base + (q_next + rank) * a.wid_stride;
+            if (takes && !active && rank < avail) {
+                wid = a.wid_base + q_next + rank;
                 const uint32_t src = walker_source(a.init, wid);
                 prev = cur = src;
                 hop = 0;
@@ -108,7 +118,7 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
                 if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride] = src;
                 Vertex vx{0, 0, 0, 0};
                 if (src >= a.nverts) atomicOr(a.err, kErrSource);
-                else if (maxhops != 0) vx = load_vertex(a, src);
+                else if (maxhops != 0) vx = load_vertex<INDEX>(a, src);
                 deg = vx.deg;
                 if (deg == 0) {
                     finish();  // bad source, no steps asked for, or a dead end (engine/engine.hpp:196-199)
@@ -166,7 +176,7 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
                                      __uint_as_float(pk[kPkThr2][L])};
                     uint32_t xs;
                     const uint32_t astar = warp_first_accept<SOPR>(a.c, tl, pk[kPkWid][L], pk[kPkHop][L], p0,
-                                                                   kMaxAttempts, ix, hd, pk[kPkDeg][L],
+                                                                   kMaxAttempts, csr, hd, pk[kPkDeg][L],
                                                                    Lprev, Lcur, ix, pk[kPkPbucket][L], ph, Lpdeg,
                                                                    s_iv[COOP ? warp : 0], &xs);
                     __syncwarp();  // every lane has read lane L's fields
@@ -224,7 +234,7 @@ __global__ void __launch_bounds__(kWalkThreads, MINB) k_walk_incore(const __grid
         // the record of a vertex that is, or may be, the next one
         const bool last = hop + 1 >= maxhops, in_range = x < a.nverts;
         Vertex vx{0, 0, 0, 0};
-        if (verdict != 0 && !last && in_range) vx = load_vertex(a, x);
+        if (verdict != 0 && !last && in_range) vx = load_vertex<INDEX>(a, x);
         if (verdict < 0)
             verdict = csr_contains(ix, pbucket, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t);
         if (verdict) {
@@ -388,90 +398,62 @@ cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t
     return cudaGetLastError();
 }
 
-// Register-cap variants the autotuner chooses between: at 256 threads per CTA,
-// 4, 5, 6 or 8 resident CTAs per SM (<= 64, 51, 40, 32 registers per thread).
-template <int V>
-struct MinBlocks;
-template <> struct MinBlocks<0> { static constexpr int value = 4; };
-template <> struct MinBlocks<1> { static constexpr int value = 5; };
-template <> struct MinBlocks<2> { static constexpr int value = 6; };
-template <> struct MinBlocks<3> { static constexpr int value = 8; };
-
-template <bool SOPR, bool PATHS, bool COOP, int V, bool W = false>
-static int grid_for(int num_sms)
+template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX>
+static int resident_grid(int num_sms)
 {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, MinBlocks<V>::value, W>,
-                                                  kWalkThreads, 0);
-    if (per_sm < 1) per_sm = 1;
-    return per_sm * num_sms;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, INDEX>, kWalkThreads, 0);
+    return (per_sm < 1 ? 1 : per_sm) * num_sms;
 }
 
-template <bool SOPR, bool PATHS, bool COOP, int V, bool W = false>
-static void launch_one(const IncoreArgs &a, int grid, cudaStream_t s)
+// f called with the kernel's template arguments as compile-time constants.
+template <class F>
+static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool index, F &&f)
 {
-    k_walk_incore<SOPR, PATHS, COOP, MinBlocks<V>::value, W><<<grid, kWalkThreads, 0, s>>>(a);
+    const auto paths_index = [&](auto s, auto c, auto w) {
+        if (paths)
+            return index ? f(s, std::true_type{}, c, w, std::true_type{}) : f(s, std::true_type{}, c, w, std::false_type{});
+        return index ? f(s, std::false_type{}, c, w, std::true_type{}) : f(s, std::false_type{}, c, w, std::false_type{});
+    };
+    if (weighted) return paths_index(std::false_type{}, std::false_type{}, std::true_type{});
+    if (sopr) return paths_index(std::true_type{}, std::true_type{}, std::false_type{});  // SOPR steps get hard
+    return coop ? paths_index(std::false_type{}, std::true_type{}, std::false_type{})
+                : paths_index(std::false_type{}, std::false_type{}, std::false_type{});
 }
 
-template <bool SOPR, bool PATHS, bool COOP, bool W = false>
-static int grid_v(int variant, int num_sms)
+// Lanes and claims by the number of walkers, which is all that decides them:
+// - few walkers are spread over the warps, down to one lane each, as long as a
+//   scheduler then has about four warps: a round costs a warp the instructions
+//   of all its lanes' branches, so fewer lanes are faster until the schedulers
+//   are busy (1,024 walkers of length 30: 0.093 ms at one lane, 0.154 at 32;
+//   65,536: 0.23 ms at 32 lanes, 0.32 at 16);
+// - a claim fills a warp when the run is one wave, so that no more warps than
+//   needed share the walkers; later waves claim eight at a time, which evens
+//   out the end of the run (600,000 walkers: 1.75 ms at 8, 1.82 at 32, 1.98 at
+//   64; weighted 200,000: 0.67 / 0.77 / 0.76; hard Node2vec steps 3.25 / 4.44
+//   / 4.62; SOPR on 16.8 M walkers: no difference).
+IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, int grid,
+                       int num_sms)
 {
-    if (variant == 0) return grid_for<SOPR, PATHS, COOP, 0, W>(num_sms);
-    if (variant == 1) return grid_for<SOPR, PATHS, COOP, 1, W>(num_sms);
-    if (variant == 2) return grid_for<SOPR, PATHS, COOP, 2, W>(num_sms);
-    return grid_for<SOPR, PATHS, COOP, 3, W>(num_sms);
+    IncorePlan p{};
+    p.ctas_per_sm = (uint32_t)walk_ctas(sopr, coop);
+    p.grid = grid > 0 ? grid : walk_kernel(sopr, paths, coop, weighted, index, [&](auto s, auto pa, auto c, auto w, auto i) {
+        return resident_grid<s(), pa(), c(), w(), i()>(num_sms);
+    });
+    const uint64_t warps = (uint64_t)p.grid * (kWalkThreads / 32), busy = std::min<uint64_t>(warps, 16ull * num_sms);
+    p.lanes = 1;
+    while (p.lanes < 32 && p.lanes * busy < nwalkers) p.lanes *= 2;
+    p.chunk = nwalkers <= 32 * warps ? p.lanes : 8;
+    return p;
 }
 
-template <bool SOPR, bool PATHS, bool COOP, bool W = false>
-static void launch_v(const IncoreArgs &a, int variant, int grid, cudaStream_t s)
+cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s)
 {
-    if (variant == 0) launch_one<SOPR, PATHS, COOP, 0, W>(a, grid, s);
-    else if (variant == 1) launch_one<SOPR, PATHS, COOP, 1, W>(a, grid, s);
-    else if (variant == 2) launch_one<SOPR, PATHS, COOP, 2, W>(a, grid, s);
-    else launch_one<SOPR, PATHS, COOP, 3, W>(a, grid, s);
-}
-
-int incore_grid_weighted(bool paths, int variant, int num_sms)
-{
-    return paths ? grid_v<false, true, false, true>(variant, num_sms) : grid_v<false, false, false, true>(variant, num_sms);
-}
-
-cudaError_t launch_walk_incore_weighted(const IncoreArgs &a, int variant, int grid, cudaStream_t s)
-{
-    if (!a.alias) return cudaErrorInvalidValue;
-    if (a.paths) launch_v<false, true, false, true>(a, variant, grid, s);
-    else launch_v<false, false, false, true>(a, variant, grid, s);
-    return cudaGetLastError();
-}
-
-int incore_grid(bool sopr, bool paths, bool coop, int variant, int num_sms)
-{
-    const int v = (sopr ? 4 : 0) | (paths ? 2 : 0) | (coop ? 1 : 0);
-    switch (v) {
-    case 0: return grid_v<false, false, false>(variant, num_sms);
-    case 1: return grid_v<false, false, true>(variant, num_sms);
-    case 2: return grid_v<false, true, false>(variant, num_sms);
-    case 3: return grid_v<false, true, true>(variant, num_sms);
-    case 4: return grid_v<true, false, false>(variant, num_sms);
-    case 5: return grid_v<true, false, true>(variant, num_sms);
-    case 6: return grid_v<true, true, false>(variant, num_sms);
-    default: return grid_v<true, true, true>(variant, num_sms);
-    }
-}
-
-cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int variant, int grid, cudaStream_t s)
-{
-    const int v = (sopr ? 4 : 0) | (a.paths ? 2 : 0) | (coop ? 1 : 0);
-    switch (v) {
-    case 0: launch_v<false, false, false>(a, variant, grid, s); break;
-    case 1: launch_v<false, false, true>(a, variant, grid, s); break;
-    case 2: launch_v<false, true, false>(a, variant, grid, s); break;
-    case 3: launch_v<false, true, true>(a, variant, grid, s); break;
-    case 4: launch_v<true, false, false>(a, variant, grid, s); break;
-    case 5: launch_v<true, false, true>(a, variant, grid, s); break;
-    case 6: launch_v<true, true, false>(a, variant, grid, s); break;
-    default: launch_v<true, true, true>(a, variant, grid, s); break;
-    }
+    walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.verts != nullptr,
+                [&](auto so, auto pa, auto c, auto w, auto i) {
+                    k_walk_incore<so(), pa(), c(), w(), i()><<<grid, kWalkThreads, 0, s>>>(a);
+                    return 0;
+                });
     return cudaGetLastError();
 }
 

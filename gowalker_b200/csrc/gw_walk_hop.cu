@@ -22,7 +22,7 @@ constexpr uint32_t kHopDone = 0xFFFFFFFFu;  // hop word of a finished walker
 template <bool SOPR, bool PATHS>
 __global__ void __launch_bounds__(256) k_walk_hop(const __grid_constant__ IncoreArgs a, HopState st, uint32_t round)
 {
-    const CsrIndex ix{a.csr, a.table};
+    const CsrIndex<false> ix{a.csr, nullptr};
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     unsigned long long n_steps = 0, n_trials = 0, n_done = 0, n_hash = 0;
@@ -52,13 +52,13 @@ __global__ void __launch_bounds__(256) k_walk_hop(const __grid_constant__ Incore
         if (!done) {
             U4 r = draw(a.c, wid, hop, 0);
             uint32_t attempt = 1;
-            const Vertex vc = load_vertex(a, cur);
+            const Vertex vc = load_vertex<false>(a, cur);
             const uint64_t head = vc.head;
             const uint32_t deg = vc.deg;
             if ((hop > 0 && terminates(a.c, r.z)) || deg == 0) {
                 done = true;  // termination draw, or a dead end (engine/engine.hpp:196-199)
             } else {
-                const Vertex vp = load_vertex(a, prev);
+                const Vertex vp = load_vertex<false>(a, prev);
                 const uint64_t phead = vp.head;
                 const uint32_t pdeg = vp.deg;
                 const StepThr t = step_thresholds<SOPR>(a.c, deg, pdeg);

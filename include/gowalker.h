@@ -89,8 +89,8 @@ typedef struct gw_config {
     uint32_t maxhops;         /* walk length ("length") */
     uint32_t walkpersource;   /* walkers per vertex */
     uint32_t numwalks;        /* total walkers for SINGLE_SOURCE / RANDOM init */
-    uint32_t blockpergrid;    /* 0 = chosen by the autotuner */
-    uint32_t threadperblock;  /* 0 = chosen by the autotuner */
+    uint32_t blockpergrid;    /* 0 = as many CTAs as the device holds at once */
+    uint32_t threadperblock;  /* accepted; the kernels fix their own */
     uint32_t zero_threshold;  /* walkers a block must attract to be loaded */
     uint32_t zero_copy;       /* 1: finish stragglers reading mapped host CSR */
     uint32_t init_mode;       /* GW_INIT_* */
@@ -156,11 +156,11 @@ typedef struct gw_stats {
     float train_loss;            /* predictor training loss (mean squared, log1p scale) */
     float pred_error;            /* learned: mean |prediction - realised target| per block, the target
                                     log1p(mean demand over the next 3 iterations) */
-    uint32_t kernel_variant;     /* register-cap variant the autotuner picked (in-core) */
+    uint32_t kernel_variant;     /* CTAs of an SM the step kernel is built for (in-core) */
     float persist_error;         /* learned: the same error of the forecast without the network
                                     (this iteration's demand carried forward) */
     float bucket_ms;             /* out-of-core: time re-bucketing walkers (CUDA events) */
-    uint32_t walker_chunk;       /* in-core: walkers a warp claims per atomic (the autotuner's pick) */
+    uint32_t walker_chunk;       /* in-core: walkers a warp claims per atomic */
     uint64_t coop_small_steps;   /* hard steps decided from candidate positions (in-core) */
     uint64_t coop_small_attempts;
     uint64_t coop_large_steps;   /* hard steps evaluated with candidate loads (in-core) */

@@ -146,7 +146,10 @@ bool compress_block(const uint64_t *beg, const uint32_t *csr, uint32_t nv, uint6
         v &= ~31u;
         out.piece_v[k] = std::max(v, out.piece_v[k - 1]);
     }
-    for (uint32_t k = 0; k <= kPieces; ++k) out.piece_g[k] = (uint32_t)gstart[out.piece_v[k]];
+    for (uint32_t k = 0; k <= kPieces; ++k) {
+        out.piece_g[k] = (uint32_t)gstart[out.piece_v[k]];
+        out.piece_e[k] = beg[out.piece_v[k]] - e0;
+    }
     return true;
 }
 
@@ -200,21 +203,48 @@ constexpr uint32_t kWindowWords = 1024 + 36;  // a warp's shared-memory window o
 constexpr uint32_t kSlideAt = 1024;           // a chunk starting past this word of the window slides it
 constexpr uint32_t kDecodeThreads = 256;
 
-// Warp tasks: task t < ntv decodes vertices [32t, 32t + 32) that have at most
-// 32 chunks (lane i loads vertex 32t + i's payload offset and neighbour
-// range, coalesced, and the warp walks the 32 in turn); task ntv + g decodes
-// split group g (32 chunks of a larger vertex).  A task's chunks are read
-// from a window of the payload in shared memory, filled by the warp with
+// First vertex v in [lo, hi) with beg[v] >= t (hi if none), by the whole warp:
+// 32 probes a round.
+__device__ __forceinline__ uint32_t warp_first_vertex(const uint64_t *__restrict__ beg, uint32_t lo, uint32_t hi,
+                                                      uint64_t t, uint32_t lane)
+{
+    while (hi - lo > 32) {
+        const uint32_t q = lo + (uint32_t)((uint64_t)(hi - lo) * (lane + 1) / 33);
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, __ldg(beg + q) >= t);
+        const uint32_t below = (uint32_t)__popc(~m);  // offsets do not decrease: the first `below` probes are < t
+        const uint32_t q_lo = __shfl_sync(0xFFFFFFFFu, q, below ? below - 1 : 0);
+        const uint32_t q_hi = __shfl_sync(0xFFFFFFFFu, q, below < 32 ? below : 31);
+        if (below) lo = q_lo + 1;
+        if (below < 32) hi = q_hi;
+    }
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, lo + lane < hi && __ldg(beg + lo + lane) >= t);
+    return m ? lo + (uint32_t)__ffs(m) - 1 : hi;
+}
+
+// The vertices [v_lo, v_hi) of a block, whose ids are [e_lo, e_hi) of the
+// block's, and the split groups [g_lo, g_hi).
+//
+// Warp tasks: task t < nbt takes the vertices of at most 32 chunks whose first
+// id lies in [e_lo + t * per, + per), 32 at a time (lane i loads a vertex's
+// payload offset and neighbour range, coalesced); the tasks behind those each
+// decode one split group (32 chunks of a larger vertex).  A task's chunks are
+// read from a window of the payload in shared memory, filled by the warp with
 // coalesced, independent loads and slid forward when the next chunk would
 // run past it, so the only dependent chain -- each chunk's position follows
 // from the previous chunk's width byte -- runs through shared memory.  Every
 // id written is checked against nverts (the validation of a plain block
 // copy, done here in the same pass).
+//
+// What bounds it is the longest task: a vertex's chunks follow one another.
+// Tasks are therefore cut by ids, not by vertices: 32 vertices of up to 32
+// chunks each were one warp's work, a chain of 1,024 chunks, which took about
+// 80 us for each of a block's four pieces whatever its size; now a chain is at
+// most a task's ids and one vertex of 32 chunks.
 __global__ void __launch_bounds__(kDecodeThreads)
-    k_decode_block(const uint8_t *__restrict__ src, uint64_t split_off, uint32_t nsplit, uint64_t payload_off,
-                   uint64_t payload_bytes, uint32_t nv, const uint64_t *__restrict__ beg, uint32_t v0, uint64_t e0,
-                   uint64_t ne, uint32_t nverts, uint32_t *__restrict__ out, uint32_t *err, uint64_t t_lo,
-                   uint64_t t_hi, uint64_t g_lo, uint64_t g_hi)
+    k_decode_block(const uint8_t *__restrict__ src, uint64_t split_off, uint64_t payload_off, uint64_t payload_bytes,
+                   uint32_t nv, const uint64_t *__restrict__ beg, uint32_t v0, uint64_t e0, uint64_t ne,
+                   uint32_t nverts, uint32_t *__restrict__ out, uint32_t *err, uint32_t v_lo, uint32_t v_hi,
+                   uint64_t e_lo, uint64_t e_hi, uint32_t per, uint32_t g_lo, uint32_t g_hi)
 {
     __shared__ uint32_t s_win[kDecodeThreads / 32][kWindowWords];
     uint32_t *sm = s_win[threadIdx.x >> 5];
@@ -224,9 +254,7 @@ __global__ void __launch_bounds__(kDecodeThreads)
     const uint32_t *split = reinterpret_cast<const uint32_t *>(src + split_off);
     const uint32_t *pay_words = reinterpret_cast<const uint32_t *>(src + payload_off);
     const uint64_t limit = (payload_bytes + 8) >> 2;  // whole words of payload and padding
-    const uint64_t ntv = ((uint64_t)nv + 31) >> 5;
-    // this launch's tasks: vertex batches [t_lo, t_hi), then split groups [g_lo, g_hi)
-    const uint64_t nbt = t_hi - t_lo;
+    const uint64_t nbt = (e_hi - e_lo + per - 1) / per;
     const uint64_t ntasks = nbt + (g_hi - g_lo);
     bool bad_id = false, bad = false;
     uint64_t base = ~0ull;  // first payload word in the window (~0: empty)
@@ -240,19 +268,60 @@ __global__ void __launch_bounds__(kDecodeThreads)
         __syncwarp();
     };
     for (uint64_t task = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < ntasks; task += nwarps) {
-        const uint64_t t = task < nbt ? t_lo + task : ntv + g_lo + (task - nbt);
-        if (t < ntv) {
-            const uint64_t vi = (t << 5) + lane;
-            uint64_t mpos = 0, mb0 = 0, mb1 = 0;
-            if (vi < nv) {
-                mpos = __ldg(voff + vi);
-                mb0 = __ldg(beg + v0 + vi);
-                mb1 = __ldg(beg + v0 + vi + 1);
+        if (task >= nbt) {
+            const uint64_t g = g_lo + (task - nbt);
+            const uint32_t v = __ldg(split + 3 * g), c0 = __ldg(split + 3 * g + 1);
+            uint64_t pos = __ldg(split + 3 * g + 2);
+            if (v >= nv) {
+                bad = true;
+                continue;
             }
-            const uint32_t nvt = (uint32_t)min((uint64_t)32, (uint64_t)nv - (t << 5));
-            // the batch's payload: [first vertex's offset, the next batch's)
+            const uint64_t b0 = __ldg(beg + v0 + v), b1 = __ldg(beg + v0 + v + 1);
+            if (b1 < b0 || b0 < e0 || b1 - e0 > ne) {
+                bad = true;
+                continue;
+            }
+            const uint64_t d = b1 - b0;
+            const uint64_t nch = (d + kChunkIds - 1) / kChunkIds;
+            const uint64_t c1 = min(nch, (uint64_t)c0 + kChunkIds);
+            bool vbad = false;
+            for (uint64_t c = c0; c < c1 && !vbad; ++c) {
+                const uint32_t k = (uint32_t)min((uint64_t)kChunkIds, d - c * kChunkIds);
+                if (pos + 2 > payload_bytes) {
+                    vbad = true;
+                    break;
+                }
+                cover(pos);
+                pos = decode_chunk_sm(sm, base, pos, payload_bytes, k, lane, out + (b0 - e0) + c * kChunkIds, nverts,
+                                      bad_id, vbad);
+            }
+            bad |= vbad;
+            continue;
+        }
+        const uint64_t t_end = e0 + min(e_lo + (task + 1) * per, e_hi);  // first id past the task's
+        uint32_t vb = warp_first_vertex(beg + v0, v_lo, v_hi, e0 + e_lo + task * per, lane);
+        for (; vb < v_hi; vb += 32) {
+            const uint32_t nvt = min(32u, v_hi - vb);
+            uint64_t mpos = 0, mb0 = ~0ull, mb1 = ~0ull;
+            if (lane < nvt) {
+                mpos = __ldg(voff + vb + lane);
+                mb0 = __ldg(beg + v0 + vb + lane);
+                mb1 = __ldg(beg + v0 + vb + lane + 1);
+            }
+            if (__shfl_sync(0xFFFFFFFFu, mb0, 0) >= t_end) break;  // no vertex of the task is left
+            // a batch without ids: on to the next vertex that has some
+            if (__ballot_sync(0xFFFFFFFFu, lane < nvt && mb1 != mb0) == 0) {
+                const uint64_t at = __shfl_sync(0xFFFFFFFFu, mb0, 0);
+                // (the vertex before the first one that starts past `at`)
+                vb = max(vb + nvt, warp_first_vertex(beg + v0, vb + nvt, v_hi, at + 1, lane) - 1) - 32;
+                continue;
+            }
+            // lanes of the task's vertices; the others belong to the next task
+            const bool mine = lane < nvt && mb0 < t_end;
+            // the batch's payload: [first vertex's offset, past its last vertex's)
+            const uint32_t last = 31u - (uint32_t)__clz((int)__ballot_sync(0xFFFFFFFFu, mine));
             const uint64_t p0 = __shfl_sync(0xFFFFFFFFu, mpos, 0);
-            const uint64_t p1 = __ldg(voff + (t << 5) + nvt);
+            const uint64_t p1 = __ldg(voff + vb + last + 1);
             if (p1 < p0 || p1 > payload_bytes) {
                 bad = true;
                 continue;
@@ -268,7 +337,6 @@ __global__ void __launch_bounds__(kDecodeThreads)
                 for (uint32_t i = lane; i < nwords; i += 32)
                     sm[i] = (base + i < limit) ? __ldg(pay_words + base + i) : 0u;
                 __syncwarp();
-                const bool mine = (uint64_t)lane < nvt;
                 const bool range_ok = !mine || (mb1 >= mb0 && mb0 >= e0 && mb1 - e0 <= ne);
                 bad |= !range_ok;
                 const uint64_t d = (mine && range_ok) ? mb1 - mb0 : 0;
@@ -327,7 +395,7 @@ __global__ void __launch_bounds__(kDecodeThreads)
                 continue;
             }
             // ---- a batch larger than the window: vertex by vertex, sliding it
-            for (uint32_t j = 0; j < nvt; ++j) {
+            for (uint32_t j = 0; j <= last; ++j) {
                 uint64_t pos = __shfl_sync(0xFFFFFFFFu, mpos, j);
                 const uint64_t b0 = __shfl_sync(0xFFFFFFFFu, mb0, j), b1 = __shfl_sync(0xFFFFFFFFu, mb1, j);
                 if (b1 < b0 || b0 < e0 || b1 - e0 > ne) {
@@ -350,34 +418,6 @@ __global__ void __launch_bounds__(kDecodeThreads)
                 }
                 bad |= vbad;
             }
-        } else {
-            const uint64_t g = t - ntv;
-            const uint32_t v = __ldg(split + 3 * g), c0 = __ldg(split + 3 * g + 1);
-            uint64_t pos = __ldg(split + 3 * g + 2);
-            if (v >= nv) {
-                bad = true;
-                continue;
-            }
-            const uint64_t b0 = __ldg(beg + v0 + v), b1 = __ldg(beg + v0 + v + 1);
-            if (b1 < b0 || b0 < e0 || b1 - e0 > ne) {
-                bad = true;
-                continue;
-            }
-            const uint64_t d = b1 - b0;
-            const uint64_t nch = (d + kChunkIds - 1) / kChunkIds;
-            const uint64_t c1 = min(nch, (uint64_t)c0 + kChunkIds);
-            bool vbad = false;
-            for (uint64_t c = c0; c < c1 && !vbad; ++c) {
-                const uint32_t k = (uint32_t)min((uint64_t)kChunkIds, d - c * kChunkIds);
-                if (pos + 2 > payload_bytes) {
-                    vbad = true;
-                    break;
-                }
-                cover(pos);
-                pos = decode_chunk_sm(sm, base, pos, payload_bytes, k, lane, out + (b0 - e0) + c * kChunkIds, nverts,
-                                      bad_id, vbad);
-            }
-            bad |= vbad;
         }
     }
     if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(err, kErrBlock);
@@ -389,17 +429,19 @@ cudaError_t launch_decode_block(const uint8_t *src, const CompressedBlock &cb, u
                                 int num_sms, cudaStream_t s, int piece)
 {
     if (nv == 0) return cudaSuccess;
-    uint64_t t_lo = 0, t_hi = ((uint64_t)nv + 31) >> 5, g_lo = 0, g_hi = cb.nsplit;
-    if (piece >= 0) {
-        t_lo = cb.piece_v[piece] >> 5;
-        t_hi = ((uint64_t)cb.piece_v[piece + 1] + 31) >> 5;
-        g_lo = cb.piece_g[piece];
-        g_hi = cb.piece_g[piece + 1];
-        if (t_hi <= t_lo && g_hi <= g_lo) return cudaSuccess;
-    }
-    k_decode_block<<<num_sms * 4, kDecodeThreads, 0, s>>>(src, cb.split_off, cb.nsplit, cb.payload_off,
-                                                         cb.payload_bytes, nv, beg, v0, e0, ne, nverts, out, err, t_lo,
-                                                         t_hi, g_lo, g_hi);
+    const int k0 = piece < 0 ? 0 : piece, k1 = piece < 0 ? (int)kPieces : piece + 1;
+    const uint64_t ids = cb.piece_e[k1] - cb.piece_e[k0];
+    const uint32_t groups = cb.piece_g[k1] - cb.piece_g[k0];
+    if (ids == 0) return cudaSuccess;
+    // one task a warp as far as they go: a task of 128 ids costs its search
+    // for the first vertex and little more
+    const uint64_t warps = (uint64_t)num_sms * 4 * (kDecodeThreads / 32);
+    const uint32_t per = (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(128, (ids + warps - 1) / warps));
+    const uint64_t tasks = (ids + per - 1) / per + groups;
+    const uint64_t need = (tasks + kDecodeThreads / 32 - 1) / (kDecodeThreads / 32);
+    k_decode_block<<<(int)std::min<uint64_t>(need, (uint64_t)num_sms * 4), kDecodeThreads, 0, s>>>(
+        src, cb.split_off, cb.payload_off, cb.payload_bytes, nv, beg, v0, e0, ne, nverts, out, err, cb.piece_v[k0],
+        cb.piece_v[k1], cb.piece_e[k0], cb.piece_e[k1], per, cb.piece_g[k0], cb.piece_g[k1]);
     return cudaGetLastError();
 }
 

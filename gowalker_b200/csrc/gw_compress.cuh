@@ -62,6 +62,7 @@ struct CompressedBlock {
     uint64_t payload_bytes = 0;
     uint32_t piece_v[kPieces + 1] = {};  // first vertex of each piece (piece_v[kPieces] = nv)
     uint32_t piece_g[kPieces + 1] = {};  // first split group of each piece
+    uint64_t piece_e[kPieces + 1] = {};  // first id of each piece, from the block's first
 };
 
 // Encode block [beg[0], beg[nv]) (global edge ids; csr indexed from beg[0]).

@@ -871,6 +871,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     a.run_pre = o.d_run_pre;
     a.run_off = o.d_run_off;
     a.nrun = o.d_nrun;
+    a.busy_warps = 16u * (uint32_t)num_sms;
     a.paths = paths ? d_paths : nullptr;
     a.stride = stride;
     a.out_base = wid_first;

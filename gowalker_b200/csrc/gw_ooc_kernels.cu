@@ -379,40 +379,64 @@ __global__ void __launch_bounds__(1024) k_schedule(const uint32_t *__restrict__ 
 // binary search counts as its own sector).  Without ZC the same count is
 // taken as if every block were mapped (kCtrModelSectors): what these steps
 // would cost in the zero-copy tail, the learned policy's switch estimate.
+//
+// An iteration ends with its longest walk, a few dozen trials one after
+// another, so what bounds it is the chain of dependent loads in a trial: the
+// block table lives in shared memory, the next vertex's offsets load while
+// N(prev) is searched, resident lists are searched by quarters (list_has;
+// mapped ones by halving, which reads fewer sectors), and few walkers are
+// spread over many warps, a lane or two each, so that one lane's search does
+// not hold up the others.
 template <bool SOPR, bool PATHS, bool COOP, bool W = false, bool ZC = false>
 __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant__ OocStepArgs a)
 {
     __shared__ uint32_t s_vs[kMaxBlocks + 1];
+    __shared__ const uint32_t *s_csr[kMaxBlocks];  // block neighbours; null = absent
+    __shared__ uint64_t s_es[kMaxBlocks];          // first edge of each block
     __shared__ uint8_t s_mapped[ZC ? kMaxBlocks : 1];
-    if constexpr (ZC)
-        for (uint32_t i = threadIdx.x; i < a.nb; i += blockDim.x) s_mapped[i] = a.mapped[i];
+    __shared__ uint32_t s_iv[COOP ? kWalkThreads / 32 : 1][kCoopScratchWords];
+    __shared__ unsigned long long s_ws[kWalkThreads / 32][kWsCount];  // per-warp statistics
+    const uint32_t nrun = *a.nrun;
+    const uint32_t total = a.run_pre[nrun];
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.ctr[kCtrRunnable], (unsigned long long)total);
+    // lanes and claims by the number of walkers, as incore_plan chooses them
+    const uint32_t warps = gridDim.x * (kWalkThreads / 32);
+    uint32_t lanes = 1;
+    while (lanes < 32 && (uint64_t)lanes * a.busy_warps < total) lanes *= 2;
+    const uint32_t chunk = total <= 32ull * warps ? lanes : 8u;
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    if ((uint64_t)blockIdx.x * (kWalkThreads / 32) * chunk >= total && blockIdx.x != 0 && chunk == lanes)
+        return;  // one wave: the CTAs before this one take every walker
+    for (uint32_t i = threadIdx.x; i <= a.nb; i += blockDim.x) {
+        s_vs[i] = a.vstart[i];
+        if (i < a.nb) {
+            s_csr[i] = a.blk_csr[i];
+            s_es[i] = a.estart[i];
+            if constexpr (ZC) s_mapped[i] = a.mapped[i];
+        }
+    }
+    if (lane < kWsCount) s_ws[warp][lane] = 0;
+    __syncthreads();
+    constexpr int kSearch = ZC ? kHalve : kQuarter;
     uint32_t zc_sectors = 0;
     // sectors of a plain binary search over n ids plus the final read: at most
     // bit_length(n) + 1
     auto search_sectors = [](uint32_t n) { return 33u - (uint32_t)__clz(n); };
-    __shared__ uint32_t s_iv[kWalkThreads / 32][kCoopScratchWords];
-    __shared__ unsigned long long s_ws[kWalkThreads / 32][kWsCount];  // per-warp statistics
-    for (uint32_t i = threadIdx.x; i <= a.nb; i += blockDim.x) s_vs[i] = a.vstart[i];
-    const uint32_t warp = threadIdx.x >> 5;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (lane < kWsCount) s_ws[warp][lane] = 0;
-    __syncthreads();
 
     const uint32_t lt_mask = (1u << lane) - 1u;
-    const uint32_t nrun = *a.nrun;
-    const uint32_t total = a.run_pre[nrun];
     const uint32_t maxhops = a.c.maxhops;
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.ctr[kCtrRunnable], (unsigned long long)total);
+    const bool takes = lane < lanes;
 
     uint32_t q_next = 0, q_end = 0;
+    uint32_t bkt = 0, bkt_start = 0, bkt_end = 0;  // bucket of the claim's first walker; lane j: end of bucket bkt + j
     bool exhausted = false;
     bool active = false;
 
-    uint32_t wid = 0, prev = 0, cur = 0, hop = 0, hop0 = 0, attempt = 0, pb = 0, cb = 0, deg = 0, pdeg = 0;
-    uint64_t idx = 0, head = 0, phead = 0, h = 0;
-    const uint32_t *ccsr = nullptr, *pcsr = nullptr;
-    const uint2 *calias = nullptr;  // W: the current block's alias tables
-    U4 r{0, 0, 0, 0};
+    uint32_t wid = 0, prev = 0, cur = 0, hop = 0, hop0 = 0, attempt = 0, pb = 0, cb = 0, deg = 0, pdeg = 0, idx = 0;
+    uint64_t h = 0;
+    const uint32_t *cadj = nullptr, *padj = nullptr;  // N(cur), N(prev); padj null: prev's block is absent
+    const uint2 *calias = nullptr;                    // W: the current vertex's alias table
     StepThr t{0.f, 0.f, 0.f};
     uint32_t n_trials = 0;  // trials not yet added to s_ws
 
@@ -422,6 +446,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         atomicAdd(&s_ws[warp][kWsSteps], (unsigned long long)(hop - hop0));
         atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
         n_trials = 0;
+        active = false;
     };
     auto finish = [&]() {
         a.hashes[wid - a.out_base] = h;
@@ -430,56 +455,71 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         atomicAdd(&s_ws[warp][kWsHash], (unsigned long long)h);
         atomicAdd(&s_ws[warp][kWsDone], 1ull);
         flush();
-        active = false;
     };
-    // Enter a step at vertex cur (block cb), prev adjacency already set:
-    // termination draw, then cur's offsets (the order of the in-core kernel).
-    auto enter = [&]() {
-        r = draw(a.c, wid, hop, 0);
-        attempt = 1;
-        if (hop > 0 && terminates(a.c, r.z)) {
-            finish();
-            return;
-        }
-        ccsr = a.blk_csr[cb];
-        if constexpr (W) calias = a.blk_alias[cb];
-        const uint64_t b0 = __ldg(a.beg + cur), b1 = __ldg(a.beg + cur + 1);
-        head = b0 - a.estart[cb];
+    auto park = [&](uint32_t cur_blk) {
+        WalkerRec rec;
+        rec.wid = wid;
+        rec.prev = prev;
+        rec.cur = cur;
+        rec.hop = hop;
+        rec.prev_blk = pb;
+        rec.cur_blk = cur_blk;
+        rec.hash_lo = (uint32_t)h;
+        rec.hash_hi = (uint32_t)(h >> 32);
+        a.recs[__ldg(a.order + idx)] = rec;
+        a.keys[idx] = bucket_of(rec, a.nb);
+        flush();
+    };
+    // Enter a step at vertex cur (block cb, edges [b0, b1)), prev adjacency
+    // already set.  The termination draw is the step's first.
+    auto enter = [&](uint64_t b0, uint64_t b1) {
+        attempt = 0;
         deg = (uint32_t)(b1 - b0);
-        if (deg == 0) {
-            finish();
-            return;
-        }
-        t = step_thresholds<SOPR>(a.c, deg, pdeg);
-        active = true;
+        cadj = s_csr[cb] + (b0 - s_es[cb]);
+        if constexpr (W) calias = a.blk_alias[cb] + (b0 - s_es[cb]);
+        if (deg == 0) finish();
+        else t = step_thresholds<SOPR>(a.c, deg, pdeg);
     };
 
     for (;;) {
         for (;;) {
-            const unsigned need = __ballot_sync(0xFFFFFFFFu, !active);
+            const unsigned need = __ballot_sync(0xFFFFFFFFu, takes && !active);
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 uint32_t base = 0;
-                if (lane == 0) base = (uint32_t)atomicAdd(&a.ctr[kCtrCursor], (unsigned long long)kChunk);
+                if (lane == 0) base = (uint32_t)min(atomicAdd(&a.ctr[kCtrCursor], (unsigned long long)chunk), 0xFFFFFFFFull);
                 base = __shfl_sync(0xFFFFFFFFu, base, 0);
                 if (base >= total) {
                     exhausted = true;
                     break;
                 }
                 q_next = base;
-                q_end = min(base + kChunk, total);
+                q_end = min(base + chunk, total);
+                // its bucket: the last one that starts at or before it, 32
+                // probes a round.  Buckets are not empty, so the claim's
+                // walkers lie in this one and the 31 after it.
+                uint32_t lo = 0, hi = nrun;  // run_pre[lo] <= base < run_pre[hi]
+                while (hi - lo > 1) {
+                    const uint32_t step = (hi - lo + 32) / 33, q = lo + step * (lane + 1);
+                    const uint32_t c =
+                        (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, q < hi && __ldg(a.run_pre + q) <= base));
+                    hi = min(hi, lo + step * (c + 1));
+                    lo += step * c;
+                }
+                bkt = lo;
+                bkt_start = __ldg(a.run_pre + lo);
+                bkt_end = __ldg(a.run_pre + min(lo + 1 + lane, nrun));
             }
             const uint32_t avail = q_end - q_next;
             const uint32_t rank = __popc(need & lt_mask);
-            if (!active && rank < avail) {
-                const uint32_t g = q_next + rank;
-                uint32_t lo = 0, hi = nrun;  // run_pre[lo] <= g < run_pre[hi]
-                while (hi - lo > 1) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (__ldg(a.run_pre + mid) <= g) lo = mid;
-                    else hi = mid;
-                }
-                idx = (uint64_t)__ldg(a.run_off + lo) + (g - __ldg(a.run_pre + lo));
+            const uint32_t g = q_next + min(rank, avail - 1);
+            uint32_t k = 0;  // buckets of the window that end at or before g
+#pragma unroll
+            for (uint32_t o = 16; o > 0; o >>= 1)
+                if (__shfl_sync(0xFFFFFFFFu, bkt_end, (int)(k + o - 1)) <= g) k += o;
+            const uint32_t k_end = __shfl_sync(0xFFFFFFFFu, bkt_end, (int)(k ? k - 1 : 0));
+            if (takes && !active && rank < avail) {
+                idx = __ldg(a.run_off + bkt + k) + (g - (k ? k_end : bkt_start));
                 const WalkerRec rec = a.recs[__ldg(a.order + idx)];
                 wid = rec.wid;
                 prev = rec.prev;
@@ -489,9 +529,9 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                 pb = rec.prev_blk;
                 cb = rec.cur_blk & ~kNeedPrev;
                 h = ((uint64_t)rec.hash_hi << 32) | rec.hash_lo;
-                // lazy mode: the previous block may be absent (pcsr null); its
-                // offsets are resident, so deg(prev) is known either way
-                pcsr = hop < maxhops ? a.blk_csr[pb] : nullptr;
+                // lazy mode: the previous block may be absent; its offsets are
+                // resident, so deg(prev) is known either way
+                const uint32_t *pcsr = s_csr[pb];
                 if (hop >= maxhops) {
                     finish();
                 } else if (pcsr == nullptr && !a.lazy) {
@@ -499,9 +539,11 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                     finish();
                 } else {
                     const uint64_t p0 = __ldg(a.beg + prev), p1 = __ldg(a.beg + prev + 1);
-                    phead = p0 - a.estart[pb];
+                    const uint64_t c0 = __ldg(a.beg + cur), c1 = __ldg(a.beg + cur + 1);
                     pdeg = (uint32_t)(p1 - p0);
-                    enter();
+                    padj = pcsr ? pcsr + (p0 - s_es[pb]) : nullptr;
+                    active = true;
+                    enter(c0, c1);
                 }
             }
             q_next += min((uint32_t)__popc(need), avail);
@@ -509,75 +551,70 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         if (!__any_sync(0xFFFFFFFFu, active)) break;
 
         // hard steps: the whole warp evaluates 32 attempts per round
-        for (unsigned hm = COOP ? __ballot_sync(0xFFFFFFFFu, active && attempt > kHardAttempts) : 0u; hm;
+        for (unsigned hm = COOP ? __ballot_sync(0xFFFFFFFFu, active && attempt >= kHardAttempts) : 0u; hm;
              hm &= hm - 1) {
             const int L = __ffs(hm) - 1;
-            const uint32_t p0 = __shfl_sync(0xFFFFFFFFu, attempt, L) - 1;
-            const uint64_t hd = shfl64(head, L), ph = shfl64(phead, L);
-            const uint32_t *cc = shfl_ptr(ccsr, L), *pc = shfl_ptr(pcsr, L);
+            const uint32_t p0 = __shfl_sync(0xFFFFFFFFu, attempt, L);
             uint32_t xs;
-            const CsrIndex<false> pix{pc, nullptr};
+            const CsrIndex<kSearch> pix{shfl_ptr(padj, L), nullptr};
             const uint32_t astar = warp_first_accept<SOPR>(
                 a.c, shfl_thr<SOPR>(t, L), __shfl_sync(0xFFFFFFFFu, wid, L), __shfl_sync(0xFFFFFFFFu, hop, L), p0,
-                kMaxAttempts, cc, hd, __shfl_sync(0xFFFFFFFFu, deg, L), __shfl_sync(0xFFFFFFFFu, prev, L),
-                __shfl_sync(0xFFFFFFFFu, cur, L), pix, 0u, ph, __shfl_sync(0xFFFFFFFFu, pdeg, L), s_iv[warp], &xs);
+                kMaxAttempts, shfl_ptr(cadj, L), 0ull, __shfl_sync(0xFFFFFFFFu, deg, L),
+                __shfl_sync(0xFFFFFFFFu, prev, L), __shfl_sync(0xFFFFFFFFu, cur, L), pix, 0u, 0ull,
+                __shfl_sync(0xFFFFFFFFu, pdeg, L), s_iv[COOP ? warp : 0], &xs);
             if (lane == (uint32_t)L) {
                 n_trials += astar - p0;
                 if constexpr (ZC)  // every attempt: a candidate and, at most, a search of N(prev)
                     zc_sectors += (astar - p0) * ((s_mapped[cb] ? 1u : 0u) + (s_mapped[pb] ? search_sectors(pdeg) : 0u));
                 else
                     zc_sectors += (astar - p0) * (1u + search_sectors(pdeg));
+                attempt = astar;
                 if (astar >= kMaxAttempts) {
                     atomicOr(a.err, kErrTrials);
                     finish();
-                } else {
-                    r = draw(a.c, wid, hop, astar);
-                    attempt = astar + 1;
                 }
             }
         }
         if (!active) continue;
 
+        const U4 r = draw(a.c, wid, hop, attempt);
+        if (attempt == 0 && hop > 0 && terminates(a.c, r.z)) {
+            finish();
+            continue;
+        }
         const uint32_t pos = r.x % deg;
         const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
         uint32_t col = pos;
         if constexpr (W) {
-            const uint2 e = __ldg(calias + head + pos);
+            const uint2 e = __ldg(calias + pos);
             if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
         }
-        const uint32_t x = __ldg(ccsr + head + col);
+        const uint32_t x = __ldg(cadj + col);
         n_trials++;
+        int verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
+        if (!ZC || s_mapped[cb]) zc_sectors += 1u;
+        // offsets of a vertex that is, or may be, the next one
+        const bool last = hop + 1 >= maxhops, in_range = x < a.nverts;
+        uint64_t n0 = 0, n1 = 0;
+        if (verdict != 0 && !last && in_range) {
+            n0 = __ldg(a.beg + x);
+            n1 = __ldg(a.beg + x + 1);
+        }
         // N(prev) is searched only when the verdict depends on it, and then
         // only if its block is resident (or mapped); each search and each
         // candidate counts its sectors
-        int verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
-        if (!ZC || s_mapped[cb]) zc_sectors += 1u;
-        if (verdict < 0 && pcsr != nullptr) {
+        if (verdict < 0 && padj != nullptr) {
             if (!ZC || s_mapped[pb]) zc_sectors += search_sectors(pdeg);
-            verdict = (csr_contains(CsrIndex<false>{pcsr, nullptr}, 0u, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
-                                                                           : rv < thr_notfound<SOPR>(a.c, t))
-                          ? 1
-                          : 0;
+            const bool found = csr_contains(CsrIndex<kSearch>{padj, nullptr}, 0u, 0ull, pdeg, x);
+            verdict = (found ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t)) ? 1 : 0;
         }
         if (verdict < 0) {
             // Needs N(prev), whose block is absent: park the walker flagged in
             // bucket (prev block, cur block).  The step restarts at attempt 0
             // once both blocks are resident (the draws are counter-based), so
             // its attempts so far are not counted.
-            WalkerRec rec;
-            rec.wid = wid;
-            rec.prev = prev;
-            rec.cur = cur;
-            rec.hop = hop;
-            rec.prev_blk = pb;
-            rec.cur_blk = cb | kNeedPrev;
-            rec.hash_lo = (uint32_t)h;
-            rec.hash_hi = (uint32_t)(h >> 32);
-            a.recs[__ldg(a.order + idx)] = rec;
-            a.keys[idx] = bucket_of(rec, a.nb);
-            n_trials -= attempt;
-            flush();
-            active = false;
+            n_trials -= attempt + 1;
+            park(cb | kNeedPrev);
         } else if (verdict > 0) {
             hop++;
             h = hash_step(h, x);
@@ -588,43 +625,22 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
             }
             prev = cur;
             pb = cb;
-            phead = head;
             pdeg = deg;
-            pcsr = ccsr;
+            padj = cadj;
             cur = x;
-            if (hop >= maxhops) {
+            if (last) {
                 finish();
-            } else if (x >= a.nverts) {
+            } else if (!in_range) {
                 atomicOr(a.err, kErrVertexRange);
                 finish();
             } else {
-                const uint32_t nbx = (x >= s_vs[cb] && x < s_vs[cb + 1]) ? cb : block_of(s_vs, a.nb, x);
-                if (a.blk_csr[nbx] == nullptr) {
-                    // next block absent: park the walker in bucket (cb, nbx)
-                    WalkerRec rec;
-                    rec.wid = wid;
-                    rec.prev = prev;
-                    rec.cur = cur;
-                    rec.hop = hop;
-                    rec.prev_blk = pb;
-                    rec.cur_blk = nbx;
-                    rec.hash_lo = (uint32_t)h;
-                    rec.hash_hi = (uint32_t)(h >> 32);
-                    a.recs[__ldg(a.order + idx)] = rec;
-                    a.keys[idx] = bucket_of(rec, a.nb);
-                    flush();
-                    active = false;
-                } else {
-                    cb = nbx;
-                    enter();
-                }
+                if (x < s_vs[cb] || x >= s_vs[cb + 1]) cb = block_of(s_vs, a.nb, x);
+                if (s_csr[cb] == nullptr) park(cb);  // next block absent: bucket (pb, cb)
+                else enter(n0, n1);
             }
-        } else if (attempt >= kMaxAttempts) {
+        } else if (++attempt >= kMaxAttempts) {
             atomicOr(a.err, kErrTrials);
             finish();
-        } else {
-            r = draw(a.c, wid, hop, attempt);
-            attempt++;
         }
     }
 

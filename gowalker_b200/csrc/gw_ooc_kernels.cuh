@@ -40,6 +40,7 @@ struct OocStepArgs {
     const uint32_t *run_pre;         // [nrun+1] prefix of runnable bucket sizes
     const uint32_t *run_off;         // [nrun] first walker of each runnable bucket
     const uint32_t *nrun;            // runnable bucket count (device)
+    uint32_t busy_warps;             // warps that keep the device's schedulers busy
     uint32_t *paths;                 // or null
     uint32_t stride;
     uint32_t out_base;               // first walker id of the population: outputs at wid - out_base

@@ -119,11 +119,16 @@ __device__ __forceinline__ bool terminates(const StepConsts &c, uint32_t z)
 }
 
 // Neighbour array of the graph (or of one block), with the membership table of
-// its vertices (table_has); without it a search is a plain binary search.
-template <bool TABLE>
+// its vertices (table_has), and how a neighbour is searched.
+enum Search : int {
+    kHalve,    // mapped host memory: fewest sectors
+    kQuarter,  // device memory: fewest dependent loads without a table
+    kTable
+};
+template <int SEARCH>
 struct CsrIndex {
     const uint32_t *csr;
-    const uint32_t *table;  // TABLE: buckets of eight ids, on 32-byte boundaries
+    const uint32_t *table;  // kTable: buckets of eight ids, on 32-byte boundaries
 };
 
 // Membership table of one vertex's neighbours: table_buckets(d) buckets of
@@ -183,6 +188,25 @@ __device__ __forceinline__ uint64_t csr_lower_bound(const uint32_t *csr, uint64_
     return lo + a;
 }
 
+// Membership of x in the sorted p[0, n), quartering: three independent probes
+// a round, so half the dependent loads of halving for half as many again in
+// all -- what counts where no table is at hand and few walkers hide a load.
+__device__ __forceinline__ bool list_has(const uint32_t *__restrict__ p, uint32_t n, uint32_t x)
+{
+    uint32_t lo = 0, len = n;  // x can only be in [lo, lo + len)
+    while (len > 4) {
+        const uint32_t q = len >> 2;
+        const uint32_t v1 = __ldg(p + lo + q), v2 = __ldg(p + lo + 2 * q), v3 = __ldg(p + lo + 3 * q);
+        len = v3 <= x ? len - 3 * q : q;
+        lo += v3 <= x ? 3 * q : v2 <= x ? 2 * q : v1 <= x ? q : 0u;
+    }
+    bool found = false;
+#pragma unroll
+    for (uint32_t i = 0; i < 4; ++i)
+        if (i < len) found |= __ldg(p + lo + i) == x;
+    return found;
+}
+
 // Membership of x in the sorted csr[lo, lo + n), whose table starts at bucket
 // `first`.
 //
@@ -192,11 +216,12 @@ __device__ __forceinline__ uint64_t csr_lower_bound(const uint32_t *csr, uint64_
 // vertices walks visit most; a bucket is one load and eight compares.  Sample
 // levels of 32, eight-way levels and eight-way trees were all measured too:
 // fewer lines than halving, but no fewer instructions.
-template <bool TABLE>
-__device__ __forceinline__ bool csr_contains(const CsrIndex<TABLE> &ix, uint32_t first, uint64_t lo, uint32_t n,
+template <int SEARCH>
+__device__ __forceinline__ bool csr_contains(const CsrIndex<SEARCH> &ix, uint32_t first, uint64_t lo, uint32_t n,
                                              uint32_t x)
 {
-    if constexpr (TABLE) return table_has(ix.table, first, n, x);
+    if constexpr (SEARCH == kTable) return table_has(ix.table, first, n, x);
+    if constexpr (SEARCH == kQuarter) return list_has(ix.csr + lo, n, x);
     const uint64_t p = csr_lower_bound(ix.csr, lo, lo + n, x);
     return p < lo + n && __ldg(ix.csr + p) == x;
 }
@@ -225,9 +250,9 @@ __device__ __forceinline__ int accept_without_prev(const StepConsts &c, const St
 // (three quarters of them) used to search.  The step kernels are bound by the
 // distinct lines their loads touch (one L1 tag access per cycle), most of
 // them probes of this search.
-template <bool SOPR, bool TABLE>
+template <bool SOPR, int SEARCH>
 __device__ __forceinline__ bool accept_candidate(const StepConsts &c, const StepThr &t, float rv, uint32_t x,
-                                                 uint32_t prev, uint32_t cur, const CsrIndex<TABLE> &pix, uint32_t pbucket,
+                                                 uint32_t prev, uint32_t cur, const CsrIndex<SEARCH> &pix, uint32_t pbucket,
                                                  uint64_t phead, uint32_t pdeg)
 {
     const int v = accept_without_prev<SOPR>(c, t, rv, x, prev, cur);
@@ -437,11 +462,11 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
 // attempt in attempt order -- the one a single thread evaluating them one by
 // one would take -- and its candidate in *x_out.  Returns `limit` if none of
 // the attempts below `limit` accepts.
-template <bool SOPR, bool TABLE>
+template <bool SOPR, int SEARCH>
 __device__ __forceinline__ uint32_t warp_first_accept(const StepConsts &c, const StepThr &t, uint32_t wid,
                                                       uint32_t hop, uint32_t p0, uint32_t limit,
                                                       const uint32_t *ccsr, uint64_t head, uint32_t deg,
-                                                      uint32_t prev, uint32_t cur, const CsrIndex<TABLE> &pix,
+                                                      uint32_t prev, uint32_t cur, const CsrIndex<SEARCH> &pix,
                                                       uint32_t pbucket, uint64_t phead, uint32_t pdeg, uint32_t *iv,
                                                       uint32_t *x_out)
 {

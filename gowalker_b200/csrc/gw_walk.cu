@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
     s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
     s_done[threadIdx.x] = 0;
     __syncwarp();
-    const CsrIndex<INDEX> ix{a.csr, a.table};
+    const CsrIndex<INDEX ? kTable : kQuarter> ix{a.csr, a.table};
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     const uint32_t chunk = a.chunk;

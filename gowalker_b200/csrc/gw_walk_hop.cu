@@ -22,7 +22,7 @@ constexpr uint32_t kHopDone = 0xFFFFFFFFu;  // hop word of a finished walker
 template <bool SOPR, bool PATHS>
 __global__ void __launch_bounds__(256) k_walk_hop(const __grid_constant__ IncoreArgs a, HopState st, uint32_t round)
 {
-    const CsrIndex<false> ix{a.csr, nullptr};
+    const CsrIndex<kQuarter> ix{a.csr, nullptr};
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     unsigned long long n_steps = 0, n_trials = 0, n_done = 0, n_hash = 0;

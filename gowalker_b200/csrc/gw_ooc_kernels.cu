@@ -555,13 +555,12 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
              hm &= hm - 1) {
             const int L = __ffs(hm) - 1;
             const uint32_t p0 = __shfl_sync(0xFFFFFFFFu, attempt, L);
-            uint32_t xs;
+            const uint32_t Ldeg = __shfl_sync(0xFFFFFFFFu, deg, L);
             const CsrIndex<kSearch> pix{shfl_ptr(padj, L), nullptr};
             const uint32_t astar = warp_first_accept<SOPR>(
                 a.c, shfl_thr<SOPR>(t, L), __shfl_sync(0xFFFFFFFFu, wid, L), __shfl_sync(0xFFFFFFFFu, hop, L), p0,
-                kMaxAttempts, shfl_ptr(cadj, L), 0ull, __shfl_sync(0xFFFFFFFFu, deg, L),
-                __shfl_sync(0xFFFFFFFFu, prev, L), __shfl_sync(0xFFFFFFFFu, cur, L), pix, 0u, 0ull,
-                __shfl_sync(0xFFFFFFFFu, pdeg, L), s_iv[COOP ? warp : 0], &xs);
+                kMaxAttempts, shfl_ptr(cadj, L), Ldeg, mod_magic(Ldeg), __shfl_sync(0xFFFFFFFFu, prev, L),
+                __shfl_sync(0xFFFFFFFFu, cur, L), pix, 0u, __shfl_sync(0xFFFFFFFFu, pdeg, L), s_iv[COOP ? warp : 0]);
             if (lane == (uint32_t)L) {
                 n_trials += astar - p0;
                 if constexpr (ZC)  // every attempt: a candidate and, at most, a search of N(prev)

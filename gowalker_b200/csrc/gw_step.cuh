@@ -188,6 +188,28 @@ __device__ __forceinline__ uint64_t csr_lower_bound(const uint32_t *csr, uint64_
     return lo + a;
 }
 
+// How many of the sorted p[0, n) are below y, by quarters (see list_has).
+__device__ __forceinline__ uint32_t list_below(const uint32_t *__restrict__ p, uint32_t n, uint32_t y)
+{
+    uint32_t lo = 0, len = n;  // the answer lies in [lo, lo + len]
+    while (len > 3) {
+        const uint32_t q = len >> 2;
+        const uint32_t v1 = __ldg(p + lo + q), v2 = __ldg(p + lo + 2 * q), v3 = __ldg(p + lo + 3 * q);
+        if (v3 < y) {
+            lo += 3 * q + 1;
+            len -= 3 * q + 1;
+        } else {
+            len = v1 < y ? q - 1 : q;
+            lo += v2 < y ? 2 * q + 1 : v1 < y ? q + 1 : 0u;
+        }
+    }
+    uint32_t c = lo;
+#pragma unroll
+    for (uint32_t i = 0; i < 3; ++i)
+        if (i < len && __ldg(p + lo + i) < y) c = lo + i + 1;
+    return c;
+}
+
 // Membership of x in the sorted p[0, n), quartering: three independent probes
 // a round, so half the dependent loads of halving for half as many again in
 // all -- what counts where no table is at hand and few walkers hide a load.
@@ -314,10 +336,11 @@ __device__ __forceinline__ uint32_t rand_prefix(Pred pred)
 // Integer bounds of a step's four rand-value tests, found by the whole warp:
 // lanes 8w..8w+7 compute bound w (0: rv <= min, 1: rv < prev, 2: rv < found,
 // 3: rv < notfound) and lane 8w returns it.  Each group tests the eight k
-// around the estimate bound / maxv * 2^24, within two of the true bound when
-// maxv and the bound are normal floats (one rounding of k * 2^-24 * maxv moves
-// it by at most half an ulp, i.e. by at most one step of k); a group whose
-// window does not bracket the bound falls back to rand_prefix.
+// around the estimate bound / maxv * 2^24, within three of the true bound when
+// maxv and the bound are normal floats (the quotient is rounded once, and one
+// rounding of k * 2^-24 * maxv moves it by at most half an ulp: each at most
+// one step of k); a group whose window does not bracket the bound falls back
+// to rand_prefix.
 template <bool SOPR>
 __device__ __forceinline__ uint32_t rand_bounds(const StepConsts &c, const StepThr &t)
 {
@@ -330,10 +353,10 @@ __device__ __forceinline__ uint32_t rand_bounds(const StepConsts &c, const StepT
         const float rv = rand_val(k << 8, maxv);
         return which == 0 ? (rv <= bound) : (rv < bound);
     };
-    const double est = __dmul_rn(__ddiv_rn((double)bound, (double)maxv), 16777216.0);
-    const bool est_ok = est >= 0.0 && est <= 16777216.0;  // false for NaN
-    const int64_t base = (est_ok ? (int64_t)est : 0) - 4;
-    const int64_t kc = base + (int64_t)(lane & 7u);
+    const float est = __fmul_rn(__fdiv_rn(bound, maxv), 0x1p24f);
+    const bool est_ok = est >= 0.0f && est <= 0x1p24f;  // false for NaN
+    const int32_t base = (est_ok ? (int32_t)est : 0) - 4;
+    const int32_t kc = base + (int32_t)(lane & 7u);
     const bool q = kc < 0 ? true : (kc >= (1 << 24) ? false : pred((uint32_t)kc));
     const unsigned g = (__ballot_sync(0xFFFFFFFFu, q) >> (lane & 24u)) & 0xFFu;
     // a bracket: true at the first candidate, false at the last, ones then zeros
@@ -341,26 +364,43 @@ __device__ __forceinline__ uint32_t rand_bounds(const StepConsts &c, const StepT
     return rand_prefix(pred);
 }
 
+// Whether a hard step is decided from candidate positions
+// (warp_first_accept_runs) or by evaluating candidates 32 at a time.
+// Positions need prev's neighbours to fit a lane each.  Setting them up (a
+// search of N(cur) per neighbour, the filter) costs about as much as seven
+// rounds of 32 candidates, and an attempt then half of one; a SOPR trial
+// accepts with at least inv_deg / sum, so steps expected to take fewer than
+// 192 attempts are evaluated.
+template <bool SOPR>
+__device__ __forceinline__ bool by_position(const StepThr &t, uint32_t pdeg, uint32_t prev, uint32_t cur)
+{
+    return pdeg < 32 && prev != cur && !(SOPR && t.sum <= 192.0f * t.inv_deg);
+}
+
 // Hard steps whose prev has fewer than 32 neighbours are decided without
 // touching the candidate: a trial's verdict depends on x = N(cur)[pos] only
 // through "x == prev" and "x in N(prev)", i.e. through whether pos falls in
 // the run of prev, or of some y in N(prev), inside the sorted N(cur).  Those
-// runs are located once per step (one lower-bound search per lane).
+// runs are located once per step (one search per lane).
 //
 // Trials then run on integers only.  The rand-value tests become bounds on
-// k = y >> 8 (rand_prefix).  pos = x mod deg is never formed on the common
-// path: with Lemire's fraction f = M*x mod 2^64 (M = ceil(2^64/deg)), pos =
-// floor(f*deg / 2^64), so f lies in [pos, pos+1) * 2^64/deg and its top
-// kFilterBits bits name a bucket of positions.  A per-warp bitmap marks every
-// bucket a run can reach; a trial whose bucket is unmarked is in no run and
-// its verdict is k < max(k_min, k_notfound).  Only marked buckets take the
-// exact path (pos, run lookup in `iv`).
+// k = y >> 8 (rand_bounds).  pos = x mod deg is not formed on the common path:
+// the fraction f = R*x mod 2^64 (R = 2^64/deg less at most 2^12) is
+// pos * 2^64/deg less at most 2^44, so its top kFilterBits bits name a bucket
+// of positions.  A per-warp
+// bitmap marks every bucket a run can reach; a trial whose bucket is unmarked
+// is in no run and its verdict is k < max(k_min, k_notfound).  A round in
+// which some trial passes that or is marked is looked at again exactly (pos,
+// run lookup in `iv`).
+//
+// What bounds it: the Philox multiplies (17 wide products a draw, four cycles
+// each per warp: 70 of the cycles of 32 attempts), then the set-up's loads.
 template <bool SOPR>
 __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, const StepThr &t, uint32_t wid,
                                                            uint32_t hop, uint32_t p0, uint32_t limit,
-                                                           const uint32_t *ccsr, uint64_t head, uint32_t deg,
-                                                           uint32_t prev, const uint32_t *pcsr, uint64_t phead,
-                                                           uint32_t pdeg, uint32_t *iv, uint32_t *x_out)
+                                                           const uint32_t *cadj, uint32_t deg, uint32_t magic,
+                                                           uint32_t prev, const uint32_t *padj, uint32_t pdeg,
+                                                           uint32_t *iv)
 {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t *bm = iv + 64;
@@ -369,27 +409,30 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
     // lane k < pdeg: run of N(prev)[k]; lane pdeg: run of prev
     uint32_t lo = 0, hi = 0;
     if (lane <= pdeg) {
-        const uint32_t y = (lane < pdeg) ? __ldg(pcsr + phead + lane) : prev;
-        lo = (uint32_t)(csr_lower_bound(ccsr, head, head + deg, y) - head);
+        const uint32_t y = (lane < pdeg) ? __ldg(padj + lane) : prev;
+        lo = list_below(cadj, deg, y);
         hi = lo;
-        while (hi < deg && __ldg(ccsr + head + hi) == y) hi++;
+        while (hi < deg && __ldg(cadj + hi) == y) hi++;
     }
     if (lane < pdeg) {
         iv[lane] = lo;
         iv[32 + lane] = hi;
     }
-    const uint64_t M = fastmod_magic(deg);
+    // R: high word floor((2^32 - 1) / deg), low word from what that leaves
+    const float inv = __fdividef(1.0f, __uint2float_rn(deg));
+    const uint32_t r_lo = __float2uint_rd(__uint2float_rn(0u - magic * deg) * inv * (1.0f - 0x1p-21f) * 0x1p32f);
     __syncwarp();
     if (hi > lo) {
-        // buckets floor(p * 2^B / deg) for p in [lo, hi], widened by one below
-        // (umul64hi(M, P) exceeds floor(P / deg) by at most one); deg = 1 has
-        // M = 0 and covers everything.
+        // buckets of lo .. hi - 1 times 2^B / deg, a hundredth of a bucket
+        // more on either side for the roundings here and of R; a position so
+        // close to 0 may also wrap to the last bucket
         uint32_t b0 = 0, b1 = (1u << kFilterBits) - 1;
         if (deg > 1) {
-            const uint32_t e0 = (uint32_t)__umul64hi(M, (uint64_t)lo << kFilterBits);
-            const uint32_t e1 = (uint32_t)__umul64hi(M, (uint64_t)hi << kFilterBits);
-            b0 = e0 > 0 ? e0 - 1 : 0;
-            b1 = min(e1, b1);
+            const float s = inv * (float)(1u << kFilterBits);
+            const float f0 = __uint2float_rn(lo) * s - 0.01f;
+            b0 = __float2uint_rd(fmaxf(f0, 0.0f));
+            b1 = min(__float2uint_rd(__uint2float_rn(hi - 1) * s + 0.01f), b1);
+            if (f0 < 0.0f) atomicOr(bm + kFilterWords - 1, 0x80000000u);
         }
         for (uint32_t w = b0 >> 5; w <= (b1 >> 5); ++w) {
             const uint32_t from = (w == (b0 >> 5)) ? (b0 & 31u) : 0u;
@@ -404,13 +447,12 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
     const uint32_t k_found = __shfl_sync(0xFFFFFFFFu, kq, 16), k_nf = __shfl_sync(0xFFFFFFFFu, kq, 24);
     const uint32_t k_fast = max(k_min, k_nf);
     const uint32_t plo = __shfl_sync(0xFFFFFFFFu, lo, (int)pdeg), phi = __shfl_sync(0xFFFFFFFFu, hi, (int)pdeg);
-    const uint32_t m_lo = (uint32_t)M, m_hi = (uint32_t)(M >> 32);
     __syncwarp();
 
     // exact verdict of a trial whose bucket is marked
     auto exact = [&](uint32_t x, uint32_t k) -> bool {
         if (k < k_min) return true;
-        const uint32_t pos = fastmod(x, M, deg);
+        const uint32_t pos = mod_by(x, deg, magic);
         if (pos >= plo && pos < phi) return k < k_prev;
         // last run whose start is <= pos (runs are in N(prev) order, so sorted)
         int r = -1;
@@ -427,75 +469,62 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
         const bool found = r >= 0 && pos < iv[32 + r];
         return found ? (k < k_found) : (k < k_nf);
     };
-    auto judge = [&](uint32_t att, uint32_t &xr) -> bool {
-        if (att >= limit) return false;
-        const U4 r = draw(c, wid, hop, att);
-        xr = r.x;
-        const uint32_t k = r.y >> 8;
-        const uint32_t b = (m_hi * r.x + __umulhi(m_lo, r.x)) >> (32 - kFilterBits);
-        if ((bm[b >> 5] >> (b & 31u)) & 1u) return exact(r.x, k);
-        return k < k_fast;
+    auto marked = [&](uint32_t x) -> bool {
+        const uint32_t b = magic * x + __umulhi(r_lo, x);  // the top word of f
+        return (__funnelshift_r(bm[b >> (37 - kFilterBits)], 0u, b >> (32 - kFilterBits)) & 1u) != 0;
     };
     // 64 attempts per round, two independent Philox chains per lane
     for (uint32_t base = p0; base < limit; base += 64) {
-        uint32_t x0 = 0, x1 = 0;
-        const bool acc0 = judge(base + lane, x0);
-        const bool acc1 = judge(base + 32 + lane, x1);
+        const U4 r0 = draw(c, wid, hop, base + lane), r1 = draw(c, wid, hop, base + 32 + lane);
+        const uint32_t k0 = r0.y >> 8, k1 = r1.y >> 8;
+        const bool in0 = marked(r0.x), in1 = marked(r1.x);
+        if (!__any_sync(0xFFFFFFFFu, in0 || in1 || k0 < k_fast || k1 < k_fast)) continue;
+        const bool acc0 = base + lane < limit && (in0 ? exact(r0.x, k0) : k0 < k_fast);
+        const bool acc1 = base + 32 + lane < limit && (in1 ? exact(r1.x, k1) : k1 < k_fast);
         const unsigned m0 = __ballot_sync(0xFFFFFFFFu, acc0);
         const unsigned m1 = __ballot_sync(0xFFFFFFFFu, acc1);
-        if (m0 | m1) {
-            const bool first_half = m0 != 0;
-            const int f = __ffs(first_half ? m0 : m1) - 1;
-            const uint32_t xf = __shfl_sync(0xFFFFFFFFu, first_half ? x0 : x1, f);
-            *x_out = __ldg(ccsr + head + fastmod(xf, M, deg));
-            __syncwarp();
-            return base + (first_half ? 0u : 32u) + (uint32_t)f;
-        }
+        if (m0 | m1) return base + (m0 ? 0u : 32u) + (uint32_t)__ffs(m0 ? m0 : m1) - 1;
     }
-    *x_out = 0;
-    __syncwarp();
     return limit;
 }
 
 // All 32 lanes, with identical (broadcast) arguments, evaluate attempts
 // p0+lane, p0+32+lane, ... of one walker's step and return the first accepting
 // attempt in attempt order -- the one a single thread evaluating them one by
-// one would take -- and its candidate in *x_out.  Returns `limit` if none of
-// the attempts below `limit` accepts.
+// one would take.  Returns `limit` if none of the attempts below `limit`
+// accepts.  N(cur) is cadj[0, deg), magic its mod_magic; N(prev) is
+// pix.csr[0, pdeg), its table at bucket pbucket.
 template <bool SOPR, int SEARCH>
 __device__ __forceinline__ uint32_t warp_first_accept(const StepConsts &c, const StepThr &t, uint32_t wid,
                                                       uint32_t hop, uint32_t p0, uint32_t limit,
-                                                      const uint32_t *ccsr, uint64_t head, uint32_t deg,
+                                                      const uint32_t *cadj, uint32_t deg, uint32_t magic,
                                                       uint32_t prev, uint32_t cur, const CsrIndex<SEARCH> &pix,
-                                                      uint32_t pbucket, uint64_t phead, uint32_t pdeg, uint32_t *iv,
-                                                      uint32_t *x_out)
+                                                      uint32_t pbucket, uint32_t pdeg, uint32_t *iv)
 {
-    if (pdeg < 32 && prev != cur)
-        return warp_first_accept_runs<SOPR>(c, t, wid, hop, p0, limit, ccsr, head, deg, prev, pix.csr, phead, pdeg, iv,
-                                            x_out);
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t M = fastmod_magic(deg);
-    const float maxv = thr_max<SOPR>(c, t);
-    for (uint32_t base = p0; base < limit; base += 32) {
-        const uint32_t att = base + lane;
-        bool acc = false;
-        uint32_t x = 0;
-        if (att < limit) {
-            const U4 r = draw(c, wid, hop, att);
-            const uint32_t pos = fastmod(r.x, M, deg);
-            const float rv = rand_val(r.y, maxv);
-            x = __ldg(ccsr + head + pos);
-            acc = accept_candidate<SOPR>(c, t, rv, x, prev, cur, pix, pbucket, phead, pdeg);
-        }
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, acc);
-        if (m) {
-            const int f = __ffs(m) - 1;
-            *x_out = __shfl_sync(0xFFFFFFFFu, x, f);
-            return base + (uint32_t)f;
+    uint32_t first = limit;
+    if (by_position<SOPR>(t, pdeg, prev, cur)) {
+        first = warp_first_accept_runs<SOPR>(c, t, wid, hop, p0, limit, cadj, deg, magic, prev, pix.csr, pdeg, iv);
+    } else {
+        const uint32_t lane = threadIdx.x & 31u;
+        const float maxv = thr_max<SOPR>(c, t);
+        for (uint32_t base = p0; base < limit; base += 32) {
+            const uint32_t att = base + lane;
+            bool acc = false;
+            if (att < limit) {
+                const U4 r = draw(c, wid, hop, att);
+                const float rv = rand_val(r.y, maxv);
+                const uint32_t x = __ldg(cadj + mod_by(r.x, deg, magic));
+                acc = accept_candidate<SOPR>(c, t, rv, x, prev, cur, pix, pbucket, 0ull, pdeg);
+            }
+            const unsigned m = __ballot_sync(0xFFFFFFFFu, acc);
+            if (m) {
+                first = base + (uint32_t)__ffs(m) - 1;
+                break;
+            }
         }
     }
-    *x_out = 0;
-    return limit;
+    __syncwarp();
+    return first;
 }
 
 }  // namespace gw

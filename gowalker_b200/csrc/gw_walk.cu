@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
     s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
     s_done[threadIdx.x] = 0;
     __syncwarp();
-    const CsrIndex<INDEX ? kTable : kQuarter> ix{a.csr, a.table};
+    constexpr int kSearch = INDEX ? kTable : kQuarter;
+    const CsrIndex<kSearch> ix{a.csr, a.table};
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     const uint32_t chunk = a.chunk;
@@ -174,16 +175,15 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                     const uint64_t ph = ((uint64_t)pk[kPkPheadHi][L] << 32) | pk[kPkPheadLo][L];
                     const StepThr tl{__uint_as_float(pk[kPkThr0][L]), __uint_as_float(pk[kPkThr1][L]),
                                      __uint_as_float(pk[kPkThr2][L])};
-                    uint32_t xs;
-                    const uint32_t astar = warp_first_accept<SOPR>(a.c, tl, pk[kPkWid][L], pk[kPkHop][L], p0,
-                                                                   kMaxAttempts, csr, hd, pk[kPkDeg][L],
-                                                                   Lprev, Lcur, ix, pk[kPkPbucket][L], ph, Lpdeg,
-                                                                   s_iv[COOP ? warp : 0], &xs);
+                    const uint32_t astar = warp_first_accept<SOPR>(
+                        a.c, tl, pk[kPkWid][L], pk[kPkHop][L], p0, kMaxAttempts, csr + hd, pk[kPkDeg][L],
+                        pk[kPkMagic][L], Lprev, Lcur, CsrIndex<kSearch>{csr + ph, a.table}, pk[kPkPbucket][L], Lpdeg,
+                        s_iv[COOP ? warp : 0]);
                     __syncwarp();  // every lane has read lane L's fields
                     if (lane == 0) {
                         pk[kPkAttempt][L] = astar;
                         pk[kPkTrials][L] += astar - p0;
-                        const bool by_pos = Lpdeg < 32 && Lprev != Lcur;
+                        const bool by_pos = by_position<SOPR>(tl, Lpdeg, Lprev, Lcur);
                         s_ws[warp][by_pos ? kWsCoopSmall : kWsCoopLarge] += 1ull;
                         s_ws[warp][by_pos ? kWsCoopSmallAtt : kWsCoopLargeAtt] += (unsigned long long)(astar - p0 + 1);
                     }

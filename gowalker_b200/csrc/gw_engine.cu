@@ -11,7 +11,9 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
+#include <sys/mman.h>
 #include "gw_engine.cuh"
 
 using namespace gw;
@@ -176,9 +178,8 @@ int gw_handle::init_device()
     if (st) return st;
     if (cfg.device < 0 || cfg.device >= ndev) return fail(GW_ERR_ARG, "device %d of %d", cfg.device, ndev);
     if ((st = cuda(cudaSetDevice(cfg.device), "cudaSetDevice"))) return st;
-    cudaDeviceProp prop;
-    if ((st = cuda(cudaGetDeviceProperties(&prop, cfg.device), "cudaGetDeviceProperties"))) return st;
-    num_sms = prop.multiProcessorCount;
+    // the attribute alone: all of a device's properties take 2.4 ms to collect
+    if ((st = cuda(cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, cfg.device), "SM count"))) return st;
     if ((st = cuda(cudaStreamCreateWithFlags(&s_compute, cudaStreamNonBlocking), "stream"))) return st;
     if ((st = cuda(cudaStreamCreateWithFlags(&s_copy, cudaStreamNonBlocking), "stream"))) return st;
     if ((st = cuda(cudaEventCreate(&ev_start), "event"))) return st;
@@ -199,23 +200,17 @@ void gw_handle::release()
     if (s_compute) cudaStreamSynchronize(s_compute);
     if (s_copy) cudaStreamSynchronize(s_copy);
     cudaFree(own_beg);
-    cudaFree(own_csr);
     cudaFree(own_w);
     cudaFree(d_alias);
     own_w = nullptr;
     d_alias = nullptr;
     alias_ready = false;
     cudaFree(d_paths);
-    cudaFree(d_lens);
     cudaFree(d_hashes);
     cudaFree(d_ctr);
-    cudaFree(d_verts);
-    cudaFree(d_heads_hi);
-    cudaFree(d_table);
-    d_verts = nullptr;
-    d_heads_hi = nullptr;
-    d_table = nullptr;
-    verts_cap = heads_hi_cap = table_cap = 0;
+    cudaFree(d_index);
+    d_index = nullptr;
+    index_cap = 0;
     if (h_ctr) cudaFreeHost(h_ctr);
     ooc_release();
     if (ev_start) cudaEventDestroy(ev_start);
@@ -252,10 +247,9 @@ int gw_handle::upload_whole_graph(cudaStream_t s, uint64_t *h2d)
 {
     int st;
     if (!own_beg) {
-        if ((st = cuda(cudaMalloc(&own_beg, ((uint64_t)nverts + 1) * sizeof(uint64_t)), "graph offsets")))
-            return st;
-        if ((st = cuda(cudaMalloc(&own_csr, (nedges ? nedges : 1) * sizeof(uint32_t)), "graph neighbours")))
-            return st;
+        const uint64_t beg_bytes = (((uint64_t)nverts + 1) * sizeof(uint64_t) + 255) & ~255ull;
+        if ((st = cuda(cudaMalloc(&own_beg, beg_bytes + (nedges ? nedges : 1) * sizeof(uint32_t)), "graph"))) return st;
+        own_csr = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(own_beg) + beg_bytes);
     }
     uint64_t bytes = 0;
     for (uint32_t b = 0; b < nblocks; ++b) {
@@ -303,12 +297,13 @@ int gw_handle::ensure_outputs()
     const uint32_t stride = cfg.maxhops + 1;
     int st;
     if (n > cap_walkers) {
-        cudaFree(d_lens);
         cudaFree(d_hashes);
-        d_lens = nullptr;
         d_hashes = nullptr;
-        if ((st = cuda(cudaMalloc(&d_lens, n * sizeof(uint32_t)), "path lengths"))) return st;
-        if ((st = cuda(cudaMalloc(&d_hashes, n * sizeof(uint64_t)), "path hashes"))) return st;
+        d_lens = nullptr;
+        cap_walkers = 0;
+        if ((st = cuda(cudaMalloc(&d_hashes, n * (sizeof(uint64_t) + sizeof(uint32_t))), "path hashes and lengths")))
+            return st;
+        d_lens = reinterpret_cast<uint32_t *>(d_hashes + n);
         cap_walkers = n;
         cap_path_walkers = 0;
     }
@@ -361,7 +356,6 @@ extern "C" int gw_set_graph_meta(gw_handle *h, uint32_t nverts, uint64_t nedges,
     h->resident = false;
     h->validated = false;
     cudaFree(h->own_beg);
-    cudaFree(h->own_csr);
     h->own_beg = nullptr;
     h->own_csr = nullptr;
     h->ooc_release();
@@ -391,7 +385,6 @@ extern "C" int gw_device_graph(gw_handle *h, const uint64_t *d_beg, const uint32
     if (!d_beg || (!d_csr && h->nedges)) return h->fail(GW_ERR_ARG, "device graph pointers missing");
     cudaSetDevice(h->cfg.device);
     cudaFree(h->own_beg);
-    cudaFree(h->own_csr);
     h->own_beg = nullptr;
     h->own_csr = nullptr;
     h->dev_beg = d_beg;
@@ -503,23 +496,6 @@ extern "C" int gw_num_walkers(gw_handle *h, uint64_t *n)
 
 // ------------------------------------------------------------------ ABI: run
 
-// Device memory for `n` elements in *p, kept when it already holds as many.
-// An index is worth having, not needed: false when there is no room.
-template <typename T>
-static bool index_room(T **p, uint64_t *cap, uint64_t n, uint64_t bytes_each)
-{
-    if (n <= *cap) return true;
-    cudaFree(*p);
-    *p = nullptr;
-    *cap = 0;
-    if (cudaMalloc((void **)p, n * bytes_each) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    *cap = n;
-    return true;
-}
-
 // Checks the resident CSR and builds its index, once per graph: per vertex 16
 // bytes (first edge, degree, first bucket, the degree's reciprocal), which a
 // step loads at once in place of two offsets and a division, and the
@@ -529,9 +505,25 @@ int gw_handle::validate_graph(cudaStream_t s)
 {
     int st;
     index_ready = false;
-    index_wide = nedges >= (1ull << 32);
-    const bool index = index_room(&d_verts, &verts_cap, nverts, sizeof(uint4)) &&
-                       (!index_wide || index_room(&d_heads_hi, &heads_hi_cap, nverts, sizeof(uint32_t)));
+    const bool wide = nedges >= (1ull << 32);
+    // buckets: 5/16 of an edge's and one more per vertex at most (table_buckets)
+    const uint64_t most_buckets = nedges / 4 + nedges / 16 + nverts + 1;
+    const uint64_t verts_bytes = ((uint64_t)nverts * sizeof(uint4) + 255) & ~255ull;
+    const uint64_t hi_bytes = wide ? ((uint64_t)nverts * sizeof(uint32_t) + 255) & ~255ull : 0;
+    const uint64_t index_bytes = verts_bytes + hi_bytes + most_buckets * 32;
+    if (index_bytes > index_cap) {
+        cudaFree(d_index);
+        d_index = nullptr;
+        index_cap = 0;
+        // an index is worth having, not needed: a large one takes at most half
+        // of what is free, and none is no error
+        size_t free_bytes = 0, all_bytes = 0;
+        const bool room = index_bytes < (256ull << 20) ||
+                          (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && index_bytes <= free_bytes / 2);
+        if (room && cudaMalloc(&d_index, index_bytes) == cudaSuccess) index_cap = index_bytes;
+        cudaGetLastError();
+    }
+    const bool index = index_cap >= index_bytes && most_buckets < (1ull << 32);
     CsrCheck check{};
     check.beg = dev_beg;
     check.csr = dev_csr;
@@ -539,8 +531,11 @@ int gw_handle::validate_graph(cudaStream_t s)
     check.nedges = nedges;
     check.err = d_err;
     if (index) {
+        d_verts = reinterpret_cast<uint4 *>(d_index);
+        d_heads_hi = wide ? reinterpret_cast<uint32_t *>(d_index + verts_bytes) : nullptr;
+        d_table = reinterpret_cast<uint32_t *>(d_index + verts_bytes + hi_bytes);
         check.verts = d_verts;
-        check.heads_hi = index_wide ? d_heads_hi : nullptr;
+        check.heads_hi = d_heads_hi;
         check.nbuckets = d_ctr;
     }
     uint64_t ends[2] = {1, 0};
@@ -559,9 +554,8 @@ int gw_handle::validate_graph(cudaStream_t s)
     if (ends[0] != 0 || ends[1] != nedges)
         return fail(GW_ERR_GRAPH, "graph offsets must run from 0 to nedges (%llu..%llu)", (unsigned long long)ends[0],
                     (unsigned long long)ends[1]);
-    const uint64_t buckets = h_ctr[0];
-    if (index && buckets < (1ull << 32) && index_room(&d_table, &table_cap, buckets ? buckets : 1, 32)) {
-        if ((st = cuda(cudaMemsetAsync(d_table, 0xFF, buckets * 32, s), "memset")) ||
+    if (index) {
+        if ((st = cuda(cudaMemsetAsync(d_table, 0xFF, h_ctr[0] * 32, s), "memset")) ||
             (st = cuda(launch_build_table(dev_beg, d_verts, nverts, dev_csr, nedges, d_table, num_sms, s),
                        "membership tables")))
             return st;
@@ -615,7 +609,17 @@ int gw_handle::run_incore(gw_stats *stats)
     if (weighted) {
         if (cfg.algorithm != GW_NODE2VEC)
             return fail(GW_ERR_ARG, "weighted walks are Node2vec walks (algorithm %u given)", cfg.algorithm);
-        if (!alias_ready && (st = build_alias(s))) return st;
+        st = alias_ready ? GW_OK : build_alias(s);
+        if (st == GW_ERR_NOMEM && d_index) {
+            // the tables come before the index
+            cudaStreamSynchronize(s);
+            cudaFree(d_index);
+            d_index = nullptr;
+            index_cap = 0;
+            index_ready = false;
+            st = build_alias(s);
+        }
+        if (st) return st;
     }
     IncoreArgs a{};
     consts_from_config(cfg, a.c);
@@ -630,7 +634,7 @@ int gw_handle::run_incore(gw_stats *stats)
     a.csr = dev_csr;
     if (index_ready) {
         a.verts = d_verts;
-        a.heads_hi = index_wide ? d_heads_hi : nullptr;
+        a.heads_hi = d_heads_hi;
         a.table = d_table;
     }
     a.nverts = nverts;
@@ -776,12 +780,50 @@ __global__ void k_zero_tails(uint32_t *rows, const uint32_t *lens, uint64_t n, u
 }
 }  // namespace
 
+// Pages of a large pageable destination, brought in by several threads before
+// the copy: a device-to-host copy that meets fresh pages takes each fault on
+// its one thread (64 MB: 31 ms, 3.2 ms into resident pages).  A destination
+// that is pinned, or whose pages are there already, is left alone.
+static void touch_pages(void *dst, uint64_t bytes)
+{
+    constexpr uint64_t kPage = 4096, kLeast = 4ull << 20;
+    cudaPointerAttributes at{};
+    if (!dst || bytes < kLeast) return;
+    if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (at.type != cudaMemoryTypeUnregistered) return;
+    char *const p = (char *)dst;
+    uint64_t there = 0;
+    for (uint64_t k = 0; k < 16; ++k) {
+        unsigned char in = 0;
+        char *q = (char *)((uintptr_t)(p + (bytes - 1) / 16 * k) & ~(uintptr_t)(kPage - 1));
+        there += mincore(q, kPage, &in) == 0 && (in & 1u);
+    }
+    if (there == 16) return;
+    const unsigned n = std::max(1u, std::min(8u, std::thread::hardware_concurrency()));
+    const uint64_t part = (bytes / n + kPage - 1) / kPage * kPage;
+    auto touch = [=](uint64_t lo) {
+        for (uint64_t o = lo; o < std::min(lo + part, bytes); o += kPage) ((volatile char *)p)[o] = 0;
+    };
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve(n);
+        for (unsigned k = 1; k < n; ++k) pool.emplace_back(touch, k * part);
+    } catch (...) {  // fewer threads: the copy brings in the rest
+    }
+    touch(0);
+    for (auto &t : pool) t.join();
+}
+
 extern "C" int gw_path_lengths(gw_handle *h, uint64_t first, uint64_t n, uint32_t *lens)
 {
     if (!h || !lens) return GW_ERR_ARG;
     if (!h->walkers_ready || !h->d_lens) return h->fail(GW_ERR_STATE, "no walk has run");
     if (first + n > h->nwalkers) return h->fail(GW_ERR_ARG, "walker range out of bounds");
     cudaSetDevice(h->cfg.device);
+    touch_pages(lens, n * sizeof(uint32_t));
     return h->cuda(cudaMemcpy(lens, h->d_lens + first, n * sizeof(uint32_t), cudaMemcpyDeviceToHost), "lengths D2H");
 }
 
@@ -799,12 +841,14 @@ extern "C" int gw_get_paths(gw_handle *h, uint64_t first, uint64_t n, uint32_t *
         k_zero_tails<<<h->num_sms * 8, 256, 0, h->s_compute>>>(h->d_paths + first * h->path_stride, h->d_lens + first,
                                                               n, h->path_stride);
         if ((st = h->cuda(cudaGetLastError(), "path padding"))) return st;
+        touch_pages(out, n * h->path_stride * sizeof(uint32_t));
         if ((st = h->cuda(cudaMemcpyAsync(out, h->d_paths + first * h->path_stride,
                                           n * h->path_stride * sizeof(uint32_t), cudaMemcpyDeviceToHost, h->s_compute),
                           "paths D2H")))
             return st;
     }
     if (lens && n) {
+        touch_pages(lens, n * sizeof(uint32_t));
         if ((st = h->cuda(cudaMemcpyAsync(lens, h->d_lens + first, n * sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                           h->s_compute),
                           "lengths D2H")))
@@ -818,6 +862,7 @@ extern "C" int gw_path_hashes(gw_handle *h, uint64_t first, uint64_t n, uint64_t
     if (!h || !out) return GW_ERR_ARG;
     if (first + n > h->nwalkers) return h->fail(GW_ERR_ARG, "walker range out of bounds");
     cudaSetDevice(h->cfg.device);
+    touch_pages(out, n * sizeof(uint64_t));
     return h->cuda(cudaMemcpy(out, h->d_hashes + first, n * sizeof(uint64_t), cudaMemcpyDeviceToHost),
                    "hashes D2H");
 }

@@ -36,16 +36,19 @@ struct gw_handle {
     // whole graph on the device (in-core)
     const uint64_t *dev_beg = nullptr;
     const uint32_t *dev_csr = nullptr;
-    uint64_t *own_beg = nullptr;
+    uint64_t *own_beg = nullptr;  // one allocation: offsets, then neighbours
     uint32_t *own_csr = nullptr;
     bool resident = false;
     bool device_graph = false;
     bool validated = false;
-    // index of the resident CSR, rebuilt whenever it is validated
+    // index of the resident CSR, rebuilt whenever it is validated: one
+    // allocation, parts on 256-byte boundaries
+    char *d_index = nullptr;
+    uint64_t index_cap = 0;
     uint4 *d_verts = nullptr;
-    uint32_t *d_heads_hi = nullptr, *d_table = nullptr;
-    uint64_t verts_cap = 0, heads_hi_cap = 0, table_cap = 0;  // entries, entries, buckets
-    bool index_wide = false, index_ready = false;             // heads_hi in use; there is an index
+    uint32_t *d_heads_hi = nullptr;  // null: every offset is below 2^32
+    uint32_t *d_table = nullptr;
+    bool index_ready = false;
 
     // edge weights (weighted Node2vec, in-core): per host block, or resident
     std::vector<const float *> host_w;
@@ -64,8 +67,8 @@ struct gw_handle {
 
     // per-walker outputs
     uint32_t *d_paths = nullptr;
+    uint64_t *d_hashes = nullptr;  // one allocation: hashes, then lengths
     uint32_t *d_lens = nullptr;
-    uint64_t *d_hashes = nullptr;
     uint64_t cap_walkers = 0;
     uint64_t cap_path_words = 0;
     uint64_t cap_path_walkers = 0;

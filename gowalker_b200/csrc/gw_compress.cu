@@ -203,31 +203,37 @@ constexpr uint32_t kWindowWords = 1024 + 36;  // a warp's shared-memory window o
 constexpr uint32_t kSlideAt = 1024;           // a chunk starting past this word of the window slides it
 constexpr uint32_t kDecodeThreads = 256;
 
-// First vertex v in [lo, hi) with beg[v] >= t (hi if none), by the whole warp:
-// 32 probes a round.
+// Vertex v of a block lies at beg[v] + kVertexWeight * v on the line that tasks
+// cut: a batch of 32 vertices weighs what 128 ids do, whether it has ids or not.
+constexpr uint32_t kVertexWeight = 4;
+
+// First vertex v in [lo, hi) at or past t on that line (hi if none), by the
+// whole warp: 32 probes a round.
 __device__ __forceinline__ uint32_t warp_first_vertex(const uint64_t *__restrict__ beg, uint32_t lo, uint32_t hi,
                                                       uint64_t t, uint32_t lane)
 {
+    auto past = [&](uint32_t v) { return __ldg(beg + v) + (uint64_t)kVertexWeight * v >= t; };
     while (hi - lo > 32) {
         const uint32_t q = lo + (uint32_t)((uint64_t)(hi - lo) * (lane + 1) / 33);
-        const unsigned m = __ballot_sync(0xFFFFFFFFu, __ldg(beg + q) >= t);
-        const uint32_t below = (uint32_t)__popc(~m);  // offsets do not decrease: the first `below` probes are < t
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, past(q));
+        const uint32_t below = (uint32_t)__popc(~m);  // places increase: the first `below` probes are before t
         const uint32_t q_lo = __shfl_sync(0xFFFFFFFFu, q, below ? below - 1 : 0);
         const uint32_t q_hi = __shfl_sync(0xFFFFFFFFu, q, below < 32 ? below : 31);
         if (below) lo = q_lo + 1;
         if (below < 32) hi = q_hi;
     }
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, lo + lane < hi && __ldg(beg + lo + lane) >= t);
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, lo + lane < hi && past(lo + lane));
     return m ? lo + (uint32_t)__ffs(m) - 1 : hi;
 }
 
 // The vertices [v_lo, v_hi) of a block, whose ids are [e_lo, e_hi) of the
 // block's, and the split groups [g_lo, g_hi).
 //
-// Warp tasks: task t < nbt takes the vertices of at most 32 chunks whose first
-// id lies in [e_lo + t * per, + per), 32 at a time (lane i loads a vertex's
-// payload offset and neighbour range, coalesced); the tasks behind those each
-// decode one split group (32 chunks of a larger vertex).  A task's chunks are
+// Warp tasks: task t < nbt takes the vertices of at most 32 chunks that lie in
+// the t-th stretch of `per` on the line of ids and vertices above, 32 at a time
+// (lane i loads a vertex's payload offset and neighbour range, coalesced); the
+// tasks behind those each decode one split group (32 chunks of a larger
+// vertex).  A task's chunks are
 // read from a window of the payload in shared memory, filled by the warp with
 // coalesced, independent loads and slid forward when the next chunk would
 // run past it, so the only dependent chain -- each chunk's position follows
@@ -235,11 +241,11 @@ __device__ __forceinline__ uint32_t warp_first_vertex(const uint64_t *__restrict
 // id written is checked against nverts (the validation of a plain block
 // copy, done here in the same pass).
 //
-// What bounds it is the longest task: a vertex's chunks follow one another.
-// Tasks are therefore cut by ids, not by vertices: 32 vertices of up to 32
-// chunks each were one warp's work, a chain of 1,024 chunks, which took about
-// 80 us for each of a block's four pieces whatever its size; now a chain is at
-// most a task's ids and one vertex of 32 chunks.
+// What bounds it is the longest task: a vertex's chunks follow one another, and
+// so do a task's batches.  Cut by vertices alone, 32 vertices of up to 32 chunks
+// each were one warp's work, a chain of 1,024 chunks, about 80 us for each of a
+// block's four pieces whatever its size; by ids alone, 27 us, a few ids spread
+// over hundreds of vertices without any; by both, 22 us.
 __global__ void __launch_bounds__(kDecodeThreads)
     k_decode_block(const uint8_t *__restrict__ src, uint64_t split_off, uint64_t payload_off, uint64_t payload_bytes,
                    uint32_t nv, const uint64_t *__restrict__ beg, uint32_t v0, uint64_t e0, uint64_t ne,
@@ -254,7 +260,8 @@ __global__ void __launch_bounds__(kDecodeThreads)
     const uint32_t *split = reinterpret_cast<const uint32_t *>(src + split_off);
     const uint32_t *pay_words = reinterpret_cast<const uint32_t *>(src + payload_off);
     const uint64_t limit = (payload_bytes + 8) >> 2;  // whole words of payload and padding
-    const uint64_t nbt = (e_hi - e_lo + per - 1) / per;
+    const uint64_t line0 = e0 + e_lo + (uint64_t)kVertexWeight * v_lo;
+    const uint64_t nbt = (e_hi - e_lo + (uint64_t)kVertexWeight * (v_hi - v_lo) + per - 1) / per;
     const uint64_t ntasks = nbt + (g_hi - g_lo);
     bool bad_id = false, bad = false;
     uint64_t base = ~0ull;  // first payload word in the window (~0: empty)
@@ -298,28 +305,23 @@ __global__ void __launch_bounds__(kDecodeThreads)
             bad |= vbad;
             continue;
         }
-        const uint64_t t_end = e0 + min(e_lo + (task + 1) * per, e_hi);  // first id past the task's
-        uint32_t vb = warp_first_vertex(beg + v0, v_lo, v_hi, e0 + e_lo + task * per, lane);
+        const uint64_t t_end = line0 + (task + 1) * per;
+        uint32_t vb = warp_first_vertex(beg + v0, v_lo, v_hi, line0 + task * per, lane);
         for (; vb < v_hi; vb += 32) {
             const uint32_t nvt = min(32u, v_hi - vb);
-            uint64_t mpos = 0, mb0 = ~0ull, mb1 = ~0ull;
+            uint64_t mpos = 0, mb0 = 0, mb1 = 0;
             if (lane < nvt) {
                 mpos = __ldg(voff + vb + lane);
                 mb0 = __ldg(beg + v0 + vb + lane);
                 mb1 = __ldg(beg + v0 + vb + lane + 1);
             }
-            if (__shfl_sync(0xFFFFFFFFu, mb0, 0) >= t_end) break;  // no vertex of the task is left
-            // a batch without ids: on to the next vertex that has some
-            if (__ballot_sync(0xFFFFFFFFu, lane < nvt && mb1 != mb0) == 0) {
-                const uint64_t at = __shfl_sync(0xFFFFFFFFu, mb0, 0);
-                // (the vertex before the first one that starts past `at`)
-                vb = max(vb + nvt, warp_first_vertex(beg + v0, vb + nvt, v_hi, at + 1, lane) - 1) - 32;
-                continue;
-            }
             // lanes of the task's vertices; the others belong to the next task
-            const bool mine = lane < nvt && mb0 < t_end;
+            const bool mine = lane < nvt && mb0 + (uint64_t)kVertexWeight * (vb + lane) < t_end;
+            const unsigned ours = __ballot_sync(0xFFFFFFFFu, mine);
+            if (ours == 0) break;
+            if (__ballot_sync(0xFFFFFFFFu, mine && mb1 != mb0) == 0) continue;  // no ids in the batch
             // the batch's payload: [first vertex's offset, past its last vertex's)
-            const uint32_t last = 31u - (uint32_t)__clz((int)__ballot_sync(0xFFFFFFFFu, mine));
+            const uint32_t last = 31u - (uint32_t)__clz((int)ours);
             const uint64_t p0 = __shfl_sync(0xFFFFFFFFu, mpos, 0);
             const uint64_t p1 = __ldg(voff + vb + last + 1);
             if (p1 < p0 || p1 > payload_bytes) {
@@ -436,8 +438,9 @@ cudaError_t launch_decode_block(const uint8_t *src, const CompressedBlock &cb, u
     // one task a warp as far as they go: a task of 128 ids costs its search
     // for the first vertex and little more
     const uint64_t warps = (uint64_t)num_sms * 4 * (kDecodeThreads / 32);
-    const uint32_t per = (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(128, (ids + warps - 1) / warps));
-    const uint64_t tasks = (ids + per - 1) / per + groups;
+    const uint64_t line = ids + (uint64_t)kVertexWeight * (cb.piece_v[k1] - cb.piece_v[k0]);
+    const uint32_t per = (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(128, (line + warps - 1) / warps));
+    const uint64_t tasks = (line + per - 1) / per + groups;
     const uint64_t need = (tasks + kDecodeThreads / 32 - 1) / (kDecodeThreads / 32);
     k_decode_block<<<(int)std::min<uint64_t>(need, (uint64_t)num_sms * 4), kDecodeThreads, 0, s>>>(
         src, cb.split_off, cb.payload_off, cb.payload_bytes, nv, beg, v0, e0, ne, nverts, out, err, cb.piece_v[k0],

@@ -87,7 +87,7 @@ struct OocState {
     uint32_t *w_key[2] = {nullptr, nullptr};       // bucket per sorted position
     uint32_t w_cur = 0;
     uint64_t w_cap = 0;
-    uint32_t *d_n = nullptr, *h_n = nullptr;  // sorted positions (device; pinned host word to set it)
+    uint32_t *d_n = nullptr, *h_n = nullptr;  // sorted positions of each buffer (device; pinned host word to set one)
     // 2 * nb^2 buckets (unflagged, then kNeedPrev); d_pairs: nb^2 per-pair totals
     uint32_t *d_counts = nullptr, *d_offsets = nullptr, *d_cursor = nullptr, *d_pairs = nullptr;
     uint32_t *d_run_pre = nullptr, *d_run_off = nullptr, *d_nrun = nullptr;
@@ -374,7 +374,7 @@ static int ooc_setup(gw_handle *h)
         if ((st = h->cuda(cudaHostGetDevicePointer((void **)&o.dm_snap[k], o.h_snap[k], 0), "counter snapshot")))
             return st;
     }
-    if ((st = h->cuda(cudaMalloc(&o.d_n, sizeof(uint32_t)), "walker count"))) return st;
+    if ((st = h->cuda(cudaMalloc(&o.d_n, 2 * sizeof(uint32_t)), "walker count"))) return st;
     if ((st = h->cuda(cudaMallocHost(&o.h_n, sizeof(uint32_t)), "walker count"))) return st;
     if ((st = h->cuda(cudaMalloc(&o.d_vstart, (nb + 1) * sizeof(uint32_t)), "vstart"))) return st;
     if ((st = h->cuda(cudaMalloc(&o.d_estart, (nb + 1) * sizeof(uint64_t)), "estart"))) return st;
@@ -807,57 +807,39 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     cudaEvent_t ev_dec = nullptr;  // this iteration's decision has read the counts
     if ((st = cuda(cudaEventCreateWithFlags(&ev_dec, cudaEventDisableTiming), "event"))) return st;
 
-    // Re-bucketing: count, scan and scatter the sorted index from buffer c to
-    // c^1, per-pair totals, the new walker count into d_n, and the counter
-    // snapshot the next decision reads.  The sequence is captured once per
-    // run and buffer parity as a CUDA graph and replayed every iteration.
-    auto bucketize_ops = [&](uint32_t c) -> int {
-        int e;
-        if ((e = cuda(cudaMemsetAsync(o.d_counts, 0, nbk * sizeof(uint32_t), s), "memset"))) return e;
-        if ((e = cuda(launch_count(o.w_key[c], o.d_n, o.d_counts, num_sms, s), "count"))) return e;
-        if ((e = cuda(launch_scan(o.d_counts, (uint32_t)nbk, o.d_offsets, s), "scan"))) return e;
-        if ((e = cuda(cudaMemsetAsync(o.d_cursor, 0, nbk * sizeof(uint32_t), s), "memset"))) return e;
-        if ((e = cuda(launch_scatter(o.w_key[c], o.w_ord[c], o.d_n, o.d_offsets, o.d_cursor, o.w_key[c ^ 1],
-                                     o.w_ord[c ^ 1], num_sms, s),
-                      "scatter")))
-            return e;
-        if ((e = cuda(launch_combine(o.d_counts, nb, o.d_pairs, num_sms, s), "pair counts"))) return e;
-        if ((e = cuda(cudaMemcpyAsync(o.d_n, o.d_offsets + nbk, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s),
-                      "walker count")))
-            return e;
-        return cuda(launch_snapshot(d_ctr, d_err, o.dm_snap[c], s), "counter snapshot");
-    };
+    // Re-bucketing: count, plan and scatter the sorted index from buffer c to
+    // c^1, per-pair totals, the new walker count into d_n[c^1], and the counter
+    // snapshot the next decision reads.  The counts may be taken while the
+    // decision before still reads what the plan rewrites, so `decided` (or
+    // null) is waited for in between; the next decision needs only the plan
+    // (ev_buck), not the scatter.
     uint32_t snap_last = 0;  // snapshot parity of the last re-bucketing
-    cudaGraphExec_t bgraph[2] = {nullptr, nullptr};
-    auto bucketize = [&](uint64_t) -> int {
+    auto bucketize = [&](cudaEvent_t decided) -> int {
         const uint32_t c = o.w_cur;
         int e;
-        if (!bgraph[c]) {
-            cudaGraph_t g = nullptr;
-            if ((e = cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "capture"))) return e;
-            const int eo = bucketize_ops(c);
-            const cudaError_t ec = cudaStreamEndCapture(s, &g);
-            if (eo) {
-                if (g) cudaGraphDestroy(g);
-                return eo;
-            }
-            if ((e = cuda(ec, "capture"))) return e;
-            e = cuda(cudaGraphInstantiate(&bgraph[c], g, 0), "graph instantiate");
-            cudaGraphDestroy(g);
-            if (e) return e;
-        }
         snap_last = c;
         if ((e = cuda(bring.begin(s, bucket_ms), "event"))) return e;
-        if ((e = cuda(cudaGraphLaunch(bgraph[c], s), "bucketing graph"))) return e;
+        if ((e = cuda(launch_count(o.w_key[c], o.d_n + c, o.d_counts, num_sms, s), "count"))) return e;
+        if (decided && (e = cuda(cudaStreamWaitEvent(s, decided, 0), "decision wait"))) return e;
+        if ((e = cuda(launch_plan(o.d_counts, nb, o.d_offsets, o.d_cursor, o.d_pairs, o.d_n + (c ^ 1u), d_ctr, d_err,
+                                  o.dm_snap[c], num_sms, s),
+                      "bucket plan")))
+            return e;
+        if ((e = cuda(cudaEventRecord(ev_buck, s), "event"))) return e;
+        if ((e = cuda(launch_scatter(o.w_key[c], o.w_ord[c], o.d_n + c, o.d_cursor, o.w_key[c ^ 1], o.w_ord[c ^ 1],
+                                     num_sms, s),
+                      "scatter")))
+            return e;
         if ((e = cuda(bring.end(s), "event"))) return e;
-        launches += 4;
+        launches += nb > 64 ? 4 : 3;
         o.w_cur ^= 1u;  // the sorted index of the live walkers
-        return cuda(cudaEventRecord(ev_buck, s), "event");
+        return GW_OK;
     };
+    if ((st = cuda(cudaMemsetAsync(o.d_counts, 0, nbk * sizeof(uint32_t), s), "memset"))) return st;
     *o.h_n = (uint32_t)nwalkers;
     if ((st = cuda(cudaMemcpyAsync(o.d_n, o.h_n, sizeof(uint32_t), cudaMemcpyHostToDevice, s), "walker count")))
         return st;
-    if ((st = bucketize(nlive))) return st;
+    if ((st = bucketize(nullptr))) return st;
 
     OocStepArgs a{};
     consts_from_config(cfg, a.c);  // step constants as for the in-core kernel
@@ -893,15 +875,14 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         grid = ooc_grid(sopr, paths, coop, cfg.prefetch && num_sms > 8 ? num_sms - 1 : num_sms, o.weighted);
 
     // The step of an iteration -- runnable pass, cursor reset, step kernel --
-    // is captured once per run and sorted-index parity as a CUDA graph, like
-    // the re-bucketing after it (the step kernel's arguments differ only by
-    // that parity).  The zero-copy tail's launch and traced runs (events
-    // around the runnable pass) launch the kernels one by one.
+    // is captured once per run and sorted-index parity as a CUDA graph (the
+    // step kernel's arguments differ only by that parity).  The zero-copy
+    // tail's launch and traced runs (events around the runnable pass) launch
+    // the kernels one by one.
     cudaGraphExec_t sgraph[2] = {nullptr, nullptr};
     auto step_ops = [&](uint32_t c) -> int {
         int e;
-        if ((e = cuda(launch_runnable(o.d_counts, o.d_offsets, o.d_blk_csr, nb, a.lazy, o.d_run_pre, o.d_run_off,
-                                      o.d_nrun, s),
+        if ((e = cuda(launch_runnable(o.d_offsets, o.d_blk_csr, nb, a.lazy, o.d_run_pre, o.d_run_off, o.d_nrun, s),
                       "runnable")))
             return e;
         if ((e = cuda(cudaMemsetAsync(d_ctr + kCtrCursor, 0, sizeof(unsigned long long), s), "memset"))) return e;
@@ -936,8 +917,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
             return GW_OK;
         }
         if (trace) rring.begin(s, t_runnable_f);
-        if ((e = cuda(launch_runnable(o.d_counts, o.d_offsets, o.d_blk_csr, nb, a.lazy, o.d_run_pre, o.d_run_off,
-                                      o.d_nrun, s),
+        if ((e = cuda(launch_runnable(o.d_offsets, o.d_blk_csr, nb, a.lazy, o.d_run_pre, o.d_run_off, o.d_nrun, s),
                       "runnable")))
             return e;
         if (trace) rring.end(s);
@@ -1222,8 +1202,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         if (prefetch) {
             if ((st = cuda(cudaEventRecord(ev_dec, ds), "event"))) break;
             if ((st = step())) break;
-            if ((st = cuda(cudaStreamWaitEvent(s, ev_dec, 0), "decision wait"))) break;
-            if ((st = bucketize(nlive))) break;
+            if ((st = bucketize(ev_dec))) break;
             stepped = true;
         }
         const auto tw0 = std::chrono::steady_clock::now();
@@ -1356,7 +1335,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
             for (uint32_t b = 0; b < nb; ++b)
                 if (o.block_slot[b] < 0) o.h_blk_csr[b] = nullptr;
             if ((st = push_tables())) break;
-            if ((st = bucketize(nlive))) break;
+            if ((st = bucketize(nullptr))) break;
             iters++;
             done = true;
             break;
@@ -1457,7 +1436,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         if (!stepped) {
             if ((st = push_tables())) break;
             if ((st = step())) break;
-            if ((st = bucketize(nlive))) break;
+            if ((st = bucketize(nullptr))) break;
         }
 
         // ---- predictor training: once kTraceRing iterations are traced, and
@@ -1538,8 +1517,6 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     // a training still in flight finishes here; its weights are adopted by
     // the next run's first decision
     if (o.ts) cudaStreamSynchronize(o.ts);
-    for (auto &g : bgraph)
-        if (g) cudaGraphExecDestroy(g);
     for (auto &g : sgraph)
         if (g) cudaGraphExecDestroy(g);
     cudaEventDestroy(ev_buck);

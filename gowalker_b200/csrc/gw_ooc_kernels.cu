@@ -5,8 +5,9 @@
 //  k_count         walkers per (prev block, cur block) bucket, warp-aggregated
 //                  atomics (one atomic per distinct bucket per warp instead of
 //                  one per walker, gpu/gpuwalk.hpp:179)
-//  k_scan          exclusive scan of the bucket counts in one CTA (coalesced warp segments)
-//                  (the reference scans them on one thread, gpu/gpuwalk.hpp:321-338)
+//  k_plan          exclusive scan of the bucket counts in one CTA (coalesced warp segments;
+//                  the reference scans them on one thread, gpu/gpuwalk.hpp:321-338), with
+//                  everything else the next decision and the scatter read
 //  k_scatter       walkers into bucket order, finished walkers dropped
 //                  (gpu/gpuwalk.hpp:340-360 + the spill of engine/walk.hpp:484-525)
 //  k_runnable      ranges of the buckets whose two blocks are resident
@@ -81,9 +82,8 @@ __global__ void k_count(const uint32_t *__restrict__ keys, const uint32_t *__res
 }
 
 __global__ void k_scatter(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ order_in,
-                          const uint32_t *__restrict__ n_ptr, const uint32_t *__restrict__ offsets,
-                          uint32_t *__restrict__ cursor, uint32_t *__restrict__ keys_out,
-                          uint32_t *__restrict__ order_out)
+                          const uint32_t *__restrict__ n_ptr, uint32_t *__restrict__ cursor,
+                          uint32_t *__restrict__ keys_out, uint32_t *__restrict__ order_out)
 {
     const uint64_t n = *n_ptr;
     const uint32_t lane = threadIdx.x & 31u;
@@ -102,8 +102,8 @@ __global__ void k_scatter(const uint32_t *__restrict__ keys_in, const uint32_t *
             uint32_t pos = 0;
             if (lane == leader) pos = atomicAdd(&cursor[b], (uint32_t)__popc(grp));
             pos = __shfl_sync(grp, pos, leader) + (uint32_t)__popc(grp & lt);
-            keys_out[offsets[b] + pos] = b;
-            order_out[offsets[b] + pos] = r;
+            keys_out[pos] = b;
+            order_out[pos] = r;
         }
     }
 }
@@ -151,31 +151,52 @@ __device__ __forceinline__ uint32_t cta_warp_base(uint32_t wtotal, uint32_t *tot
     return b;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *__restrict__ in, uint32_t n,
-                                                       uint32_t *__restrict__ out)
+// Between the count and the scatter, all that needs one CTA: bucket offsets
+// (and the scatter's cursors, which start there), the new number of sorted
+// positions, per-pair totals (when `pairs` is given), the counts cleared for
+// the next count, and the counters and error word into mapped host memory.
+// Five launches and two copies of 2-5 us each before; the next decision may
+// start as soon as this is done, beside the scatter.
+__global__ void __launch_bounds__(kScanThreads) k_plan(uint32_t *__restrict__ counts, uint32_t nn,
+                                                       uint32_t *__restrict__ offsets, uint32_t *__restrict__ cursor,
+                                                       uint32_t *__restrict__ pairs, uint32_t *__restrict__ n_out,
+                                                       const unsigned long long *__restrict__ ctr,
+                                                       const uint32_t *__restrict__ err, unsigned long long *snap)
 {
     __shared__ uint32_t s_total;
+    const uint32_t n = 2 * nn;
+    if (threadIdx.x <= kCtrCount) {
+        snap[threadIdx.x] = threadIdx.x < kCtrCount ? ctr[threadIdx.x] : *err;
+        __threadfence_system();
+    }
+    if (pairs)
+        for (uint32_t k = threadIdx.x; k < nn; k += blockDim.x) pairs[k] = counts[k] + counts[nn + k];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const uint32_t seg = ((n + nw - 1) / nw + 31u) & ~31u;
     const uint32_t lo = min(warp * seg, n), hi = min(lo + seg, n);
     uint32_t part = 0;
 #pragma unroll 4
-    for (uint32_t i = lo + lane; i < hi; i += 32) part += in[i];
-    uint32_t base = cta_warp_base(warp_sum(part), &s_total);
+    for (uint32_t i = lo + lane; i < hi; i += 32) part += counts[i];
+    uint32_t base = cta_warp_base(warp_sum(part), &s_total);  // (every thread is past its pairs)
 #pragma unroll 4
     for (uint32_t i0 = lo; i0 < hi; i0 += 32) {
         const uint32_t i = i0 + lane;
-        const uint32_t v = i < hi ? in[i] : 0u;
+        const uint32_t v = i < hi ? counts[i] : 0u;
         const uint32_t inc = warp_incl_scan(v, lane);
-        if (i < hi) out[i] = base + inc - v;
+        if (i < hi) {
+            offsets[i] = cursor[i] = base + inc - v;
+            counts[i] = 0;
+        }
         base += __shfl_sync(0xFFFFFFFFu, inc, 31);
     }
     __syncthreads();
-    if (threadIdx.x == 0) out[n] = s_total;
+    if (threadIdx.x == 0) {
+        offsets[n] = s_total;
+        *n_out = s_total;
+    }
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__restrict__ counts,
-                                                           const uint32_t *__restrict__ offsets,
+__global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__restrict__ offsets,
                                                            const uint32_t *const *__restrict__ blk_csr, uint32_t nb,
                                                            uint32_t lazy, uint32_t *__restrict__ run_pre,
                                                            uint32_t *__restrict__ run_off, uint32_t *__restrict__ nrun)
@@ -199,7 +220,7 @@ __global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__res
     uint32_t pc = 0, ps = 0;
 #pragma unroll 4
     for (uint32_t b = lo + lane; b < hi; b += 32) {
-        const uint32_t c = counts[b];
+        const uint32_t c = offsets[b + 1] - offsets[b];
         if (c && runnable(b)) {
             pc++;
             ps += c;
@@ -210,7 +231,7 @@ __global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__res
 #pragma unroll 4
     for (uint32_t b0 = lo; b0 < hi; b0 += 32) {
         const uint32_t b = b0 + lane;
-        const uint32_t c = b < hi ? counts[b] : 0u;
+        const uint32_t c = b < hi ? offsets[b + 1] - offsets[b] : 0u;
         const bool f = c && runnable(b);
         const unsigned fm = __ballot_sync(0xFFFFFFFFu, f);
         const uint32_t v = f ? c : 0u;
@@ -773,53 +794,39 @@ cudaError_t launch_count(const uint32_t *keys, const uint32_t *n, uint32_t *coun
     return cudaGetLastError();
 }
 
-cudaError_t launch_scan(const uint32_t *counts, uint32_t n, uint32_t *offsets, cudaStream_t s)
-{
-    k_scan<<<1, kScanThreads, 0, s>>>(counts, n, offsets);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, const uint32_t *offsets,
-                           uint32_t *cursor, uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s)
-{
-    k_scatter<<<num_sms * 8, 256, 0, s>>>(keys_in, order_in, n, offsets, cursor, keys_out, order_out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_runnable(const uint32_t *counts, const uint32_t *offsets, const uint32_t *const *blk_csr,
-                            uint32_t nb, uint32_t lazy, uint32_t *run_pre, uint32_t *run_off, uint32_t *nrun,
-                            cudaStream_t s)
-{
-    k_runnable<<<1, kScanThreads, 0, s>>>(counts, offsets, blk_csr, nb, lazy, run_pre, run_off, nrun);
-    return cudaGetLastError();
-}
-
 __global__ void k_combine(const uint32_t *__restrict__ counts, uint32_t nn, uint32_t *__restrict__ combined)
 {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x)
         combined[k] = counts[k] + counts[nn + k];
 }
 
-// Counters and error word into out (mapped host memory): one thread each.
-__global__ void k_snapshot(const unsigned long long *__restrict__ ctr, const uint32_t *__restrict__ err,
-                           unsigned long long *out)
+cudaError_t launch_plan(uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
+                        uint32_t *n_out, const unsigned long long *ctr, const uint32_t *err, unsigned long long *snap,
+                        int num_sms, cudaStream_t s)
 {
-    const uint32_t i = threadIdx.x;
-    if (i < kCtrCount) out[i] = ctr[i];
-    else if (i == kCtrCount) out[i] = *err;
-    __threadfence_system();
-}
-
-cudaError_t launch_snapshot(const unsigned long long *ctr, const uint32_t *err, unsigned long long *out,
-                            cudaStream_t s)
-{
-    k_snapshot<<<1, 32, 0, s>>>(ctr, err, out);
+    // many blocks' pair totals are too much for one CTA (8 words a thread at 64
+    // blocks, 128 at 256)
+    const bool apart = nb > 64;
+    if (apart) {
+        k_combine<<<num_sms, 256, 0, s>>>(counts, nb * nb, pairs);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    k_plan<<<1, kScanThreads, 0, s>>>(counts, nb * nb, offsets, cursor, apart ? nullptr : pairs, n_out, ctr, err, snap);
     return cudaGetLastError();
 }
 
-cudaError_t launch_combine(const uint32_t *counts, uint32_t nb, uint32_t *combined, int num_sms, cudaStream_t s)
+cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, uint32_t *cursor,
+                           uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s)
 {
-    k_combine<<<num_sms, 256, 0, s>>>(counts, nb * nb, combined);
+    k_scatter<<<num_sms * 8, 256, 0, s>>>(keys_in, order_in, n, cursor, keys_out, order_out);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_runnable(const uint32_t *offsets, const uint32_t *const *blk_csr, uint32_t nb, uint32_t lazy,
+                            uint32_t *run_pre, uint32_t *run_off, uint32_t *nrun, cudaStream_t s)
+{
+    k_runnable<<<1, kScanThreads, 0, s>>>(offsets, blk_csr, nb, lazy, run_pre, run_off, nrun);
     return cudaGetLastError();
 }
 

@@ -67,22 +67,21 @@ struct Decision {
 cudaError_t launch_init_walkers(const WalkerInit &in, const uint32_t *vstart, uint32_t nb, uint32_t wid0, uint64_t n,
                                 WalkerRec *recs, uint32_t *order, uint32_t *keys, uint32_t *paths, uint32_t stride,
                                 int num_sms, cudaStream_t s);
-// `n` points at the number of sorted positions (a device word, so the
-// bucketing sequence can be captured once and replayed).
+// `n` points at the number of sorted positions (a device word).
 cudaError_t launch_count(const uint32_t *keys, const uint32_t *n, uint32_t *counts, int num_sms, cudaStream_t s);
-cudaError_t launch_scan(const uint32_t *counts, uint32_t n, uint32_t *offsets, cudaStream_t s);
-cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, const uint32_t *offsets,
-                           uint32_t *cursor, uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s);
+// After launch_count: offsets (2 * nb^2 + 1) and cursors from the counts, which
+// are cleared; pairs[k] = counts[k] + counts[nb^2 + k], walkers per (prev, cur)
+// block pair; *n_out, the sorted positions to come; counters (kCtrCount) and
+// error word into snap[0 .. kCtrCount] (mapped host memory).
+cudaError_t launch_plan(uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
+                        uint32_t *n_out, const unsigned long long *ctr, const uint32_t *err, unsigned long long *snap,
+                        int num_sms, cudaStream_t s);
+cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, uint32_t *cursor,
+                           uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s);
 // Buckets are 2 * nb^2: (prev_blk, cur_blk), then the same pairs for walkers
 // flagged kNeedPrev.
-cudaError_t launch_runnable(const uint32_t *counts, const uint32_t *offsets, const uint32_t *const *blk_csr,
-                            uint32_t nb, uint32_t lazy, uint32_t *run_pre, uint32_t *run_off, uint32_t *nrun,
-                            cudaStream_t s);
-// Counters (kCtrCount) and the error word into out[0 .. kCtrCount] (mapped host memory).
-cudaError_t launch_snapshot(const unsigned long long *ctr, const uint32_t *err, unsigned long long *out,
-                            cudaStream_t s);
-// combined[k] = counts[k] + counts[nb^2 + k]: walkers per (prev, cur) block pair.
-cudaError_t launch_combine(const uint32_t *counts, uint32_t nb, uint32_t *combined, int num_sms, cudaStream_t s);
+cudaError_t launch_runnable(const uint32_t *offsets, const uint32_t *const *blk_csr, uint32_t nb, uint32_t lazy,
+                            uint32_t *run_pre, uint32_t *run_off, uint32_t *nrun, cudaStream_t s);
 // `counts` are the nb^2 per-pair totals; `live` points at the live-walker count.
 cudaError_t launch_schedule(const uint32_t *counts, const uint32_t *live, uint32_t nb, const uint32_t *cached,
                             uint32_t ncached, uint32_t nslots, uint32_t zero_threshold, const float *pred,

@@ -706,7 +706,7 @@ int gw_handle::run_incore(gw_stats *stats)
     }
     const IncorePlan plan = incore_plan(nwalkers, sopr, a.paths != nullptr, coop, weighted, index_ready,
                                         (int)cfg.blockpergrid, num_sms);
-    a.lanes = plan.lanes;
+    a.slots = plan.slots;
     a.chunk = plan.chunk;
     const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);  // with the error word
     if ((st = cuda(cudaMemsetAsync(d_ctr, 0, ctr_bytes, s), "memset")) ||

@@ -80,7 +80,7 @@ struct IncoreArgs {
     uint32_t wid_base;
     uint32_t out_base;         // first walker id of the population: outputs are indexed by wid - out_base
     uint32_t chunk;            // walkers a warp claims per atomic (incore_plan)
-    uint32_t lanes;            // lanes of a warp that take walkers (incore_plan)
+    uint32_t slots;            // walkers of a warp at a time (incore_plan)
     uint32_t *paths;           // rows indexed by walker id, or null
     uint32_t stride;           // maxhops + 1
     uint32_t *lens;            // vertices per path
@@ -123,6 +123,38 @@ __device__ __forceinline__ Vertex load_vertex(const IncoreArgs &a, uint32_t v)
     return Vertex{head, deg, 0u, deg ? mod_magic(deg) : 0u};
 }
 
+// Lanes of a warp in groups of `size`, one walker a group: every lane of a
+// group holds the walker's whole state and evaluates one of its next `size`
+// attempts, and the first one in order that decides the step counts.  A walk is
+// a chain of trials, so where lanes are to spare -- few walkers, or the end of a
+// run -- groups shorten it by the attempts that reject.
+struct Group {
+    uint32_t shift = 0;  // size = 2^shift
+    __device__ uint32_t size() const { return 1u << shift; }
+    __device__ uint32_t sub(uint32_t lane) const { return lane & (size() - 1u); }
+    __device__ uint32_t base(uint32_t lane) const { return lane & ~(size() - 1u); }
+    // this lane's group's bits of a ballot, from bit 0
+    __device__ unsigned mine(unsigned ballot, uint32_t lane) const
+    {
+        return (ballot >> base(lane)) & (0xFFFFFFFFu >> (32u - size()));
+    }
+};
+constexpr uint32_t kMaxGroupShift = 3;  // 8 attempts: 1 step in 12 of a 0.27 acceptance needs more
+
+// Groups for a warp whose `act` (ballot) lanes hold the last walkers it will
+// get: grown while all walkers fit.  Returns the lane whose state this lane
+// takes over (itself when nothing changes), and whether it then holds a walker.
+__device__ __forceinline__ uint32_t regroup(Group &g, unsigned act, uint32_t lane, bool &holds)
+{
+    const unsigned bases[] = {0xFFFFFFFFu, 0x55555555u, 0x11111111u, 0x01010101u};
+    const unsigned b = act & bases[g.shift];  // a bit per walker
+    const uint32_t n = (uint32_t)__popc(b);
+    while (g.shift < kMaxGroupShift && (n << (g.shift + 1)) <= 32u) ++g.shift;
+    const uint32_t slot = lane >> g.shift;
+    holds = slot < n;
+    return holds ? __fns(b, 0, (int)slot + 1) : lane;
+}
+
 __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
 {
 #pragma unroll
@@ -133,7 +165,7 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
 // How an in-core run is launched.
 struct IncorePlan {
     int grid;               // CTAs
-    uint32_t lanes, chunk;  // IncoreArgs
+    uint32_t slots, chunk;  // IncoreArgs
     uint32_t ctas_per_sm;   // the kernel's register cap: CTAs of an SM it is built for
 };
 // `grid` CTAs as asked for, or (0) as many as are resident at once.

@@ -186,7 +186,7 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     const bool coop = needs_coop(cfg->algorithm, a.c);
     const IncorePlan plan =
         incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, false, (int)cfg->blockpergrid, num_sms);
-    a.lanes = plan.lanes;
+    a.slots = plan.slots;
     a.chunk = plan.chunk;
     e = launch_walk_incore(a, sopr, coop, plan.grid, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, sizeof(host_ctr), cudaMemcpyDeviceToHost, s);

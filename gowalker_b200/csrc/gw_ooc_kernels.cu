@@ -405,9 +405,10 @@ __global__ void __launch_bounds__(1024) k_schedule(const uint32_t *__restrict__ 
 // another, so what bounds it is the chain of dependent loads in a trial: the
 // block table lives in shared memory, the next vertex's offsets load while
 // N(prev) is searched, resident lists are searched by quarters (list_has;
-// mapped ones by halving, which reads fewer sectors), and few walkers are
-// spread over many warps, a lane or two each, so that one lane's search does
-// not hold up the others.
+// mapped ones by halving, which reads fewer sectors), few walkers are spread
+// over many warps, so that one lane's search does not hold up the others, and
+// lanes to spare share a walker's attempts (Group), from the start when the
+// walkers are few and at the end of every iteration.
 template <bool SOPR, bool PATHS, bool COOP, bool W = false, bool ZC = false>
 __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant__ OocStepArgs a)
 {
@@ -420,15 +421,17 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
     const uint32_t nrun = *a.nrun;
     const uint32_t total = a.run_pre[nrun];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.ctr[kCtrRunnable], (unsigned long long)total);
-    // lanes and claims by the number of walkers, as incore_plan chooses them
+    // slots and claims by the number of walkers, as incore_plan chooses them
     const uint32_t warps = gridDim.x * (kWalkThreads / 32);
-    uint32_t lanes = 1;
-    while (lanes < 32 && (uint64_t)lanes * a.busy_warps < total) lanes *= 2;
-    const uint32_t chunk = total <= 32ull * warps ? lanes : 8u;
+    uint32_t slots = 1;
+    while (slots < 32 && (uint64_t)slots * a.busy_warps < total) slots *= 2;
+    const uint32_t chunk = total <= 32ull * warps ? slots : 8u;
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
-    if ((uint64_t)blockIdx.x * (kWalkThreads / 32) * chunk >= total && blockIdx.x != 0 && chunk == lanes)
+    if ((uint64_t)blockIdx.x * (kWalkThreads / 32) * chunk >= total && blockIdx.x != 0 && chunk == slots)
         return;  // one wave: the CTAs before this one take every walker
+    Group grp;
+    while (grp.shift < kMaxGroupShift && (slots << (grp.shift + 1)) <= 32u) ++grp.shift;
     for (uint32_t i = threadIdx.x; i <= a.nb; i += blockDim.x) {
         s_vs[i] = a.vstart[i];
         if (i < a.nb) {
@@ -445,9 +448,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
     // bit_length(n) + 1
     auto search_sectors = [](uint32_t n) { return 33u - (uint32_t)__clz(n); };
 
-    const uint32_t lt_mask = (1u << lane) - 1u;
     const uint32_t maxhops = a.c.maxhops;
-    const bool takes = lane < lanes;
 
     uint32_t q_next = 0, q_end = 0;
     uint32_t bkt = 0, bkt_start = 0, bkt_end = 0;  // bucket of the claim's first walker; lane j: end of bucket bkt + j
@@ -461,15 +462,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
     StepThr t{0.f, 0.f, 0.f};
     uint32_t n_trials = 0;  // trials not yet added to s_ws
 
+    // Lane 0 of a group writes what its walker writes.
+    auto leads = [&]() { return grp.sub(lane) == 0; };
     // Statistics of the walker leaving this lane (finished or parked): its
     // steps in this launch are the hops it made since it was loaded.
-    auto flush = [&]() {
-        atomicAdd(&s_ws[warp][kWsSteps], (unsigned long long)(hop - hop0));
-        atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
-        n_trials = 0;
-        active = false;
-    };
+    auto flush = [&]() { atomicAdd(&s_ws[warp][kWsSteps], (unsigned long long)(hop - hop0)); };
     auto finish = [&]() {
+        active = false;
+        if (!leads()) return;
         a.hashes[wid - a.out_base] = h;
         a.lens[wid - a.out_base] = hop + 1;
         a.keys[idx] = kNoBucket;
@@ -478,6 +478,8 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         flush();
     };
     auto park = [&](uint32_t cur_blk) {
+        active = false;
+        if (!leads()) return;
         WalkerRec rec;
         rec.wid = wid;
         rec.prev = prev;
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
 
     for (;;) {
         for (;;) {
-            const unsigned need = __ballot_sync(0xFFFFFFFFu, takes && !active);
+            const unsigned need = __ballot_sync(0xFFFFFFFFu, !active && (lane >> grp.shift) < slots);
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 uint32_t base = 0;
@@ -532,14 +534,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                 bkt_end = __ldg(a.run_pre + min(lo + 1 + lane, nrun));
             }
             const uint32_t avail = q_end - q_next;
-            const uint32_t rank = __popc(need & lt_mask);
+            const uint32_t rank = __popc(need & ((1u << grp.base(lane)) - 1u)) >> grp.shift;
             const uint32_t g = q_next + min(rank, avail - 1);
             uint32_t k = 0;  // buckets of the window that end at or before g
 #pragma unroll
             for (uint32_t o = 16; o > 0; o >>= 1)
                 if (__shfl_sync(0xFFFFFFFFu, bkt_end, (int)(k + o - 1)) <= g) k += o;
             const uint32_t k_end = __shfl_sync(0xFFFFFFFFu, bkt_end, (int)(k ? k - 1 : 0));
-            if (takes && !active && rank < avail) {
+            if (((need >> lane) & 1u) && rank < avail) {
                 idx = __ldg(a.run_off + bkt + k) + (g - (k ? k_end : bkt_start));
                 const WalkerRec rec = a.recs[__ldg(a.order + idx)];
                 wid = rec.wid;
@@ -567,13 +569,34 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                     enter(c0, c1);
                 }
             }
-            q_next += min((uint32_t)__popc(need), avail);
+            q_next += min((uint32_t)__popc(need) >> grp.shift, avail);
         }
-        if (!__any_sync(0xFFFFFFFFu, active)) break;
+        const unsigned act = __ballot_sync(0xFFFFFFFFu, active);
+        if (act == 0) break;
+        if (exhausted && grp.shift < kMaxGroupShift && 2 * __popc(act) <= 32) {
+            // the last walkers spread over the lanes that have none left
+            const int from = (int)regroup(grp, act, lane, active);
+            wid = __shfl_sync(0xFFFFFFFFu, wid, from);
+            prev = __shfl_sync(0xFFFFFFFFu, prev, from);
+            cur = __shfl_sync(0xFFFFFFFFu, cur, from);
+            hop = __shfl_sync(0xFFFFFFFFu, hop, from);
+            hop0 = __shfl_sync(0xFFFFFFFFu, hop0, from);
+            attempt = __shfl_sync(0xFFFFFFFFu, attempt, from);
+            pb = __shfl_sync(0xFFFFFFFFu, pb, from);
+            cb = __shfl_sync(0xFFFFFFFFu, cb, from);
+            deg = __shfl_sync(0xFFFFFFFFu, deg, from);
+            pdeg = __shfl_sync(0xFFFFFFFFu, pdeg, from);
+            idx = __shfl_sync(0xFFFFFFFFu, idx, from);
+            h = shfl64(h, from);
+            cadj = shfl_ptr(cadj, from);
+            padj = shfl_ptr(padj, from);
+            if constexpr (W) calias = shfl_ptr(calias, from);
+            t = shfl_thr<SOPR>(t, from);
+        }
 
         // hard steps: the whole warp evaluates 32 attempts per round
-        for (unsigned hm = COOP ? __ballot_sync(0xFFFFFFFFu, active && attempt >= kHardAttempts) : 0u; hm;
-             hm &= hm - 1) {
+        for (unsigned hm = COOP ? __ballot_sync(0xFFFFFFFFu, active && leads() && attempt >= kHardAttempts) : 0u;
+             hm; hm &= hm - 1) {
             const int L = __ffs(hm) - 1;
             const uint32_t p0 = __shfl_sync(0xFFFFFFFFu, attempt, L);
             const uint32_t Ldeg = __shfl_sync(0xFFFFFFFFu, deg, L);
@@ -582,12 +605,14 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                 a.c, shfl_thr<SOPR>(t, L), __shfl_sync(0xFFFFFFFFu, wid, L), __shfl_sync(0xFFFFFFFFu, hop, L), p0,
                 kMaxAttempts, shfl_ptr(cadj, L), Ldeg, mod_magic(Ldeg), __shfl_sync(0xFFFFFFFFu, prev, L),
                 __shfl_sync(0xFFFFFFFFu, cur, L), pix, 0u, __shfl_sync(0xFFFFFFFFu, pdeg, L), s_iv[COOP ? warp : 0]);
-            if (lane == (uint32_t)L) {
-                n_trials += astar - p0;
-                if constexpr (ZC)  // every attempt: a candidate and, at most, a search of N(prev)
-                    zc_sectors += (astar - p0) * ((s_mapped[cb] ? 1u : 0u) + (s_mapped[pb] ? search_sectors(pdeg) : 0u));
-                else
-                    zc_sectors += (astar - p0) * (1u + search_sectors(pdeg));
+            if (grp.base(lane) == (uint32_t)L) {
+                if (leads()) {
+                    if constexpr (ZC)  // every attempt: a candidate and, at most, a search of N(prev)
+                        zc_sectors +=
+                            (astar - p0) * ((s_mapped[cb] ? 1u : 0u) + (s_mapped[pb] ? search_sectors(pdeg) : 0u));
+                    else
+                        zc_sectors += (astar - p0) * (1u + search_sectors(pdeg));
+                }
                 attempt = astar;
                 if (astar >= kMaxAttempts) {
                     atomicOr(a.err, kErrTrials);
@@ -595,54 +620,76 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                 }
             }
         }
-        if (!active) continue;
 
-        const U4 r = draw(a.c, wid, hop, attempt);
-        if (attempt == 0 && hop > 0 && terminates(a.c, r.z)) {
+        // One rejection-sampling trial a lane.
+        const bool last = hop + 1 >= maxhops;
+        bool end = false;  // the step's termination draw ends the walk
+        int verdict = 0;
+        uint32_t x = 0, sectors = 0;
+        uint64_t n0 = 0, n1 = 0;  // offsets of a vertex that is, or may be, the next one
+        if (active) {
+            const uint32_t att = attempt + grp.sub(lane);
+            const U4 r = draw(a.c, wid, hop, att);
+            end = att == 0 && hop > 0 && terminates(a.c, r.z);
+            const uint32_t pos = r.x % deg;
+            const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
+            uint32_t col = pos;
+            if constexpr (W) {
+                const uint2 e = __ldg(calias + pos);
+                if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
+            }
+            x = __ldg(cadj + col);
+            if (!end && att < kMaxAttempts) {
+                verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
+                if (!ZC || s_mapped[cb]) sectors += 1u;
+            }
+            if (verdict != 0 && !last && x < a.nverts) {
+                n0 = __ldg(a.beg + x);
+                n1 = __ldg(a.beg + x + 1);
+            }
+            // N(prev) is searched only when the verdict depends on it, and then
+            // only if its block is resident (or mapped); each search and each
+            // candidate counts its sectors
+            if (verdict < 0 && padj != nullptr) {
+                if (!ZC || s_mapped[pb]) sectors += search_sectors(pdeg);
+                const bool found = csr_contains(CsrIndex<kSearch>{padj, nullptr}, 0u, 0ull, pdeg, x);
+                verdict = (found ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t)) ? 1 : 0;
+            }
+        }
+        uint32_t first = 0;  // the deciding attempt, from `attempt`
+        if (grp.shift) {
+            const unsigned dec = grp.mine(__ballot_sync(0xFFFFFFFFu, verdict != 0), lane);
+            end = grp.mine(__ballot_sync(0xFFFFFFFFu, end), lane) != 0;
+            first = dec ? (uint32_t)__ffs(dec) - 1 : 0u;
+            if (dec && grp.sub(lane) > first) sectors = 0;  // one lane alone would not have come this far
+            const int from = (int)(grp.base(lane) + first);
+            verdict = __shfl_sync(0xFFFFFFFFu, verdict, from);
+            if (!dec) verdict = 0;
+            x = __shfl_sync(0xFFFFFFFFu, x, from);
+            n0 = shfl64(n0, from);
+            n1 = shfl64(n1, from);
+        }
+        if (!active) continue;
+        zc_sectors += end ? 0u : sectors;
+        if (end) {
             finish();
-            continue;
-        }
-        const uint32_t pos = r.x % deg;
-        const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
-        uint32_t col = pos;
-        if constexpr (W) {
-            const uint2 e = __ldg(calias + pos);
-            if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
-        }
-        const uint32_t x = __ldg(cadj + col);
-        n_trials++;
-        int verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
-        if (!ZC || s_mapped[cb]) zc_sectors += 1u;
-        // offsets of a vertex that is, or may be, the next one
-        const bool last = hop + 1 >= maxhops, in_range = x < a.nverts;
-        uint64_t n0 = 0, n1 = 0;
-        if (verdict != 0 && !last && in_range) {
-            n0 = __ldg(a.beg + x);
-            n1 = __ldg(a.beg + x + 1);
-        }
-        // N(prev) is searched only when the verdict depends on it, and then
-        // only if its block is resident (or mapped); each search and each
-        // candidate counts its sectors
-        if (verdict < 0 && padj != nullptr) {
-            if (!ZC || s_mapped[pb]) zc_sectors += search_sectors(pdeg);
-            const bool found = csr_contains(CsrIndex<kSearch>{padj, nullptr}, 0u, 0ull, pdeg, x);
-            verdict = (found ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t)) ? 1 : 0;
-        }
-        if (verdict < 0) {
+        } else if (verdict < 0) {
             // Needs N(prev), whose block is absent: park the walker flagged in
             // bucket (prev block, cur block).  The step restarts at attempt 0
             // once both blocks are resident (the draws are counter-based), so
             // its attempts so far are not counted.
-            n_trials -= attempt + 1;
             park(cb | kNeedPrev);
         } else if (verdict > 0) {
+            if (leads()) {
+                n_trials += attempt + first + 1;  // a step's trials are counted when it is taken
+                if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride + hop + 1] = x;
+                if (n_trials & 0x80000000u) {  // a step adds < 2^27: no wrap
+                    atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
+                    n_trials = 0;
+                }
+            }
             hop++;
             h = hash_step(h, x);
-            if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride + hop] = x;
-            if (n_trials & 0x80000000u) {  // a step adds < 2^27: no wrap
-                atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
-                n_trials = 0;
-            }
             prev = cur;
             pb = cb;
             pdeg = deg;
@@ -650,7 +697,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
             cur = x;
             if (last) {
                 finish();
-            } else if (!in_range) {
+            } else if (x >= a.nverts) {
                 atomicOr(a.err, kErrVertexRange);
                 finish();
             } else {
@@ -658,16 +705,20 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                 if (s_csr[cb] == nullptr) park(cb);  // next block absent: bucket (pb, cb)
                 else enter(n0, n1);
             }
-        } else if (++attempt >= kMaxAttempts) {
-            atomicOr(a.err, kErrTrials);
-            finish();
+        } else {
+            attempt += grp.size();
+            if (attempt >= kMaxAttempts) {
+                atomicOr(a.err, kErrTrials);
+                finish();
+            }
         }
     }
 
     __syncwarp();
+    const unsigned long long trials = warp_sum((unsigned long long)n_trials);
     if (lane == 0) {
         atomicAdd(&a.ctr[kCtrSteps], s_ws[warp][kWsSteps]);
-        atomicAdd(&a.ctr[kCtrTrials], s_ws[warp][kWsTrials]);
+        atomicAdd(&a.ctr[kCtrTrials], trials + s_ws[warp][kWsTrials]);
         atomicAdd(&a.ctr[kCtrDone], s_ws[warp][kWsDone]);
         atomicAdd(&a.ctr[kCtrHashSum], s_ws[warp][kWsHash]);
     }

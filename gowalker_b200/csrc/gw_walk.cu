@@ -45,8 +45,11 @@ __host__ __device__ constexpr int walk_ctas(bool sopr, bool coop) { return coop 
 // search of N(prev), in flight together.  A warp spends the time of its
 // longest lane in each part, so the parts that differ between lanes are kept
 // short: one draw for accepted, rejected and new walkers alike, a membership
-// table (csr_contains), one load for a vertex's record.
-template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX>
+// table (csr_contains), one load for a vertex's record.  GROUPS: with fewer
+// walkers than lanes several lanes share one (Group); runs that fill the lanes
+// are bound by instructions, and groups at their end alone lose (n2v_corpus-like
+// runs 1.70 / 1.88 ms without / with).
+template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX, bool GROUPS>
 __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_incore(const __grid_constant__ IncoreArgs a)
 {
     __shared__ uint32_t s_iv[COOP ? kWalkThreads / 32 : 1][kCoopScratchWords];  // scratch of warp_first_accept
@@ -56,7 +59,6 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
     __shared__ uint32_t s_park[COOP ? kWalkThreads / 32 : 1][kPkCount][32];  // lane state during hard steps
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lt_mask = (1u << lane) - 1u;
     if (lane < kWsCount) s_ws[warp][lane] = 0;
     s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
     s_done[threadIdx.x] = 0;
@@ -66,7 +68,9 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     const uint32_t chunk = a.chunk;
-    const bool takes = lane < a.lanes;
+    Group grp;
+    if constexpr (GROUPS)
+        while (grp.shift < kMaxGroupShift && (a.slots << (grp.shift + 1)) <= 32u) ++grp.shift;
 
     uint32_t q_next = 0, q_end = 0;  // warp-uniform claimed range
     bool exhausted = false;          // warp-uniform
@@ -82,19 +86,22 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
     uint32_t n_trials = 0;  // trials not yet added to s_ws
 
     // A walker's steps are its hops: every accepted trial moves it one hop.
+    // Lane 0 of a group writes what its walker writes.
+    auto leads = [&]() { return grp.sub(lane) == 0; };
     auto finish = [&]() {
+        active = false;
+        if (!leads()) return;
         a.hashes[wid - a.out_base] = h;
         a.lens[wid - a.out_base] = hop + 1;
         s_steps[threadIdx.x] += hop;
         s_hash[threadIdx.x] += h;
         s_done[threadIdx.x] += 1;
-        active = false;
     };
 
     for (;;) {
-        // Hand walkers to idle lanes.
+        // Hand walkers to idle groups.
         for (;;) {
-            const unsigned need = __ballot_sync(0xFFFFFFFFu, takes && !active);
+            const unsigned need = __ballot_sync(0xFFFFFFFFu, !active && (!GROUPS || (lane >> grp.shift) < a.slots));
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 unsigned long long base = 0;
@@ -108,15 +115,15 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                 q_end = (uint32_t)min(base + chunk, (unsigned long long)a.nwalkers);
             }
             const uint32_t avail = q_end - q_next;
-            const uint32_t rank = __popc(need & lt_mask);
-            if (takes && !active && rank < avail) {
+            const uint32_t rank = __popc(need & ((1u << grp.base(lane)) - 1u)) >> grp.shift;
+            if (((need >> lane) & 1u) && rank < avail) {
                 wid = a.wid_base + q_next + rank;
                 const uint32_t src = walker_source(a.init, wid);
                 prev = cur = src;
                 hop = 0;
                 attempt = 0;
                 h = hash_init(src);
-                if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride] = src;
+                if (PATHS && leads()) a.paths[(uint64_t)(wid - a.out_base) * a.stride] = src;
                 Vertex vx{0, 0, 0, 0};
                 if (src >= a.nverts) atomicOr(a.err, kErrSource);
                 else if (maxhops != 0) vx = load_vertex<INDEX>(a, src);
@@ -132,9 +139,28 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                     active = true;
                 }
             }
-            q_next += min((uint32_t)__popc(need), avail);
+            q_next += min((uint32_t)__popc(need) >> grp.shift, avail);
         }
-        if (!__any_sync(0xFFFFFFFFu, active)) break;
+        const unsigned act = __ballot_sync(0xFFFFFFFFu, active);
+        if (act == 0) break;
+        if (GROUPS && exhausted && grp.shift < kMaxGroupShift && 2 * __popc(act) <= 32) {
+            // the last walkers spread over the lanes that have none left
+            const int from = (int)regroup(grp, act, lane, active);
+            wid = __shfl_sync(0xFFFFFFFFu, wid, from);
+            prev = __shfl_sync(0xFFFFFFFFu, prev, from);
+            cur = __shfl_sync(0xFFFFFFFFu, cur, from);
+            hop = __shfl_sync(0xFFFFFFFFu, hop, from);
+            attempt = __shfl_sync(0xFFFFFFFFu, attempt, from);
+            deg = __shfl_sync(0xFFFFFFFFu, deg, from);
+            pdeg = __shfl_sync(0xFFFFFFFFu, pdeg, from);
+            bucket = __shfl_sync(0xFFFFFFFFu, bucket, from);
+            pbucket = __shfl_sync(0xFFFFFFFFu, pbucket, from);
+            magic = __shfl_sync(0xFFFFFFFFu, magic, from);
+            head = shfl64(head, from);
+            phead = shfl64(phead, from);
+            h = shfl64(h, from);
+            t = shfl_thr<SOPR>(t, from);
+        }
 
         // Walkers whose step keeps rejecting (a low-degree prev next to a hub
         // under SOPR) are served one at a time by the whole warp, which finds
@@ -143,7 +169,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
         // the attempt loop, and lane L's fields reach all lanes as broadcast
         // loads.
         if (COOP) {
-            const unsigned hm = __ballot_sync(0xFFFFFFFFu, active && attempt >= kHardAttempts);
+            const unsigned hm = __ballot_sync(0xFFFFFFFFu, active && attempt >= kHardAttempts && leads());
             if (hm) {
                 uint32_t(*pk)[32] = s_park[COOP ? warp : 0];
                 pk[kPkWid][lane] = wid;
@@ -182,7 +208,6 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                     __syncwarp();  // every lane has read lane L's fields
                     if (lane == 0) {
                         pk[kPkAttempt][L] = astar;
-                        pk[kPkTrials][L] += astar - p0;
                         const bool by_pos = by_position<SOPR>(tl, Lpdeg, Lprev, Lcur);
                         s_ws[warp][by_pos ? kWsCoopSmall : kWsCoopLarge] += 1ull;
                         s_ws[warp][by_pos ? kWsCoopSmallAtt : kWsCoopLargeAtt] += (unsigned long long)(astar - p0 + 1);
@@ -193,7 +218,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                 prev = pk[kPkPrev][lane];
                 cur = pk[kPkCur][lane];
                 hop = pk[kPkHop][lane];
-                attempt = pk[kPkAttempt][lane];
+                attempt = pk[kPkAttempt][grp.base(lane)];
                 deg = pk[kPkDeg][lane];
                 pdeg = pk[kPkPdeg][lane];
                 head = ((uint64_t)pk[kPkHeadHi][lane] << 32) | pk[kPkHeadLo][lane];
@@ -213,38 +238,64 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                 __syncwarp();
             }
         }
-        if (!active) continue;
 
-        // One rejection-sampling trial.
-        const U4 r = draw(a.c, wid, hop, attempt);
-        if (attempt == 0 && hop != 0 && terminates(a.c, r.z)) {
-            finish();
-            continue;
-        }
-        const uint32_t pos = mod_by(r.x, deg, magic);
-        const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
-        uint32_t col = pos;
-        if constexpr (W) {
-            const uint2 e = __ldg(a.alias + head + pos);
-            if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
-        }
-        const uint32_t x = __ldg(csr + head + col);
-        n_trials++;
-        int verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
-        // the record of a vertex that is, or may be, the next one
-        const bool last = hop + 1 >= maxhops, in_range = x < a.nverts;
+        // One rejection-sampling trial a lane.
+        if (!GROUPS && !active) continue;
+        const bool last = hop + 1 >= maxhops;
+        bool end = false;    // the step's termination draw ends the walk
+        int verdict = 0;
+        uint32_t x = 0;
         Vertex vx{0, 0, 0, 0};
-        if (verdict != 0 && !last && in_range) vx = load_vertex<INDEX>(a, x);
-        if (verdict < 0)
-            verdict = csr_contains(ix, pbucket, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t);
-        if (verdict) {
+        if (active) {
+            const uint32_t att = attempt + grp.sub(lane);
+            const U4 r = draw(a.c, wid, hop, att);
+            end = att == 0 && hop != 0 && terminates(a.c, r.z);
+            if (!GROUPS && end) {
+                finish();
+                continue;
+            }
+            const uint32_t pos = mod_by(r.x, deg, magic);
+            const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
+            uint32_t col = pos;
+            if constexpr (W) {
+                const uint2 e = __ldg(a.alias + head + pos);
+                if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
+            }
+            x = __ldg(csr + head + col);
+            if (!GROUPS || (!end && att < kMaxAttempts)) verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
+            // the record of a vertex that is, or may be, the next one
+            if (verdict != 0 && !last && x < a.nverts) vx = load_vertex<INDEX>(a, x);
+            if (verdict < 0)
+                verdict = csr_contains(ix, pbucket, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
+                                                                    : rv < thr_notfound<SOPR>(a.c, t);
+        }
+        uint32_t first = 0;  // the accepting attempt, from `attempt`
+        if (GROUPS && grp.shift) {
+            const unsigned acc = grp.mine(__ballot_sync(0xFFFFFFFFu, verdict != 0), lane);
+            end = grp.mine(__ballot_sync(0xFFFFFFFFu, end), lane) != 0;
+            first = acc ? (uint32_t)__ffs(acc) - 1 : 0u;
+            verdict = acc != 0;
+            const int from = (int)(grp.base(lane) + first);
+            x = __shfl_sync(0xFFFFFFFFu, x, from);
+            vx.head = shfl64(vx.head, from);
+            vx.deg = __shfl_sync(0xFFFFFFFFu, vx.deg, from);
+            vx.bucket = __shfl_sync(0xFFFFFFFFu, vx.bucket, from);
+            vx.magic = __shfl_sync(0xFFFFFFFFu, vx.magic, from);
+        }
+        if (GROUPS && !active) continue;
+        if (GROUPS && end) {
+            finish();
+        } else if (verdict) {
+            if (leads()) {
+                n_trials += attempt + first + 1;  // a step's trials are counted when it is taken
+                if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride + hop + 1] = x;
+                if (n_trials & 0x80000000u) {  // a step adds < 2^27: no wrap
+                    atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
+                    n_trials = 0;
+                }
+            }
             hop++;
             h = hash_step(h, x);
-            if (PATHS) a.paths[(uint64_t)(wid - a.out_base) * a.stride + hop] = x;
-            if (n_trials & 0x80000000u) {  // a step adds < 2^27: no wrap
-                atomicAdd(&s_ws[warp][kWsTrials], (unsigned long long)n_trials);
-                n_trials = 0;
-            }
             attempt = 0;
             prev = cur;
             phead = head;
@@ -255,12 +306,15 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
             deg = vx.deg;
             bucket = vx.bucket;
             magic = vx.magic;
-            if (!last && !in_range) atomicOr(a.err, kErrVertexRange);
+            if (!last && x >= a.nverts) atomicOr(a.err, kErrVertexRange);
             if (deg == 0) finish();  // the last hop, a bad id, or a dead end
             else t = step_thresholds<SOPR>(a.c, deg, pdeg);
-        } else if (++attempt >= kMaxAttempts) {
-            atomicOr(a.err, kErrTrials);
-            finish();
+        } else {
+            attempt += grp.size();
+            if (attempt >= kMaxAttempts) {
+                atomicOr(a.err, kErrTrials);
+                finish();
+            }
         }
     }
 
@@ -402,7 +456,8 @@ template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX>
 static int resident_grid(int num_sms)
 {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, INDEX>, kWalkThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, INDEX, false>,
+                                                  kWalkThreads, 0);
     return (per_sm < 1 ? 1 : per_sm) * num_sms;
 }
 
@@ -421,12 +476,12 @@ static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool in
                 : paths_index(std::false_type{}, std::false_type{}, std::false_type{});
 }
 
-// Lanes and claims by the number of walkers, which is all that decides them:
-// - few walkers are spread over the warps, down to one lane each, as long as a
+// Slots and claims by the number of walkers, which is all that decides them:
+// - few walkers are spread over the warps, down to one each, as long as a
 //   scheduler then has about four warps: a round costs a warp the instructions
-//   of all its lanes' branches, so fewer lanes are faster until the schedulers
-//   are busy (1,024 walkers of length 30: 0.093 ms at one lane, 0.154 at 32;
-//   65,536: 0.23 ms at 32 lanes, 0.32 at 16);
+//   of all its lanes' branches, so fewer walkers are faster until the schedulers
+//   are busy (1,024 walkers of length 30, one lane a walker: 0.093 ms at one a
+//   warp, 0.154 at 32; 65,536: 0.23 ms at 32, 0.32 at 16);
 // - a claim fills a warp when the run is one wave, so that no more warps than
 //   needed share the walkers; later waves claim eight at a time, which evens
 //   out the end of the run (600,000 walkers: 1.75 ms at 8, 1.82 at 32, 1.98 at
@@ -441,9 +496,9 @@ IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool
         return resident_grid<s(), pa(), c(), w(), i()>(num_sms);
     });
     const uint64_t warps = (uint64_t)p.grid * (kWalkThreads / 32), busy = std::min<uint64_t>(warps, 16ull * num_sms);
-    p.lanes = 1;
-    while (p.lanes < 32 && p.lanes * busy < nwalkers) p.lanes *= 2;
-    p.chunk = nwalkers <= 32 * warps ? p.lanes : 8;
+    p.slots = 1;
+    while (p.slots < 32 && p.slots * busy < nwalkers) p.slots *= 2;
+    p.chunk = nwalkers <= 32 * warps ? p.slots : 8;
     return p;
 }
 
@@ -451,7 +506,10 @@ cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int gr
 {
     walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.verts != nullptr,
                 [&](auto so, auto pa, auto c, auto w, auto i) {
-                    k_walk_incore<so(), pa(), c(), w(), i()><<<grid, kWalkThreads, 0, s>>>(a);
+                    if (a.slots < 32)
+                        k_walk_incore<so(), pa(), c(), w(), i(), true><<<grid, kWalkThreads, 0, s>>>(a);
+                    else
+                        k_walk_incore<so(), pa(), c(), w(), i(), false><<<grid, kWalkThreads, 0, s>>>(a);
                     return 0;
                 });
     return cudaGetLastError();

@@ -166,12 +166,21 @@ __global__ void k_validate_offsets(const uint64_t *beg, uint32_t nverts, const u
     if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0) atomicOr(err, kErrVertexRange);
 }
 
-// Neighbour ids of a block just copied into a slot.
-__global__ void k_validate_block(const uint32_t *csr, uint64_t ne, uint32_t nverts, uint32_t *err)
+// Neighbour ids of a block just copied into a slot (which starts on a 16-byte
+// boundary): four ids a load, all of a thread's loads in flight.  It stands
+// between the copy and the step.
+__global__ void __launch_bounds__(256) k_validate_block(const uint32_t *csr, uint64_t ne, uint32_t nverts, uint32_t *err)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint4 *q = reinterpret_cast<const uint4 *>(csr);
     bool bad = false;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < ne; i += stride) bad |= csr[i] >= nverts;
+#pragma unroll 4
+    for (uint64_t i = t0; i < ne / 4; i += stride) {
+        const uint4 v = q[i];
+        bad |= v.x >= nverts || v.y >= nverts || v.z >= nverts || v.w >= nverts;
+    }
+    for (uint64_t i = (ne & ~3ull) + t0; i < ne; i += stride) bad |= csr[i] >= nverts;
     if (__any_sync(0xFFFFFFFFu, bad) && (threadIdx.x & 31u) == 0) atomicOr(err, kErrVertexRange);
 }
 
@@ -1025,7 +1034,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         return fail(GW_ERR_ARG, "prefetch needs a cache of at least 3 blocks (has %u)", o.nslots);
     }
     cudaEvent_t staged_ev = nullptr;
-    if (prefetch) cudaEventCreateWithFlags(&staged_ev, cudaEventDisableTiming);
+    cudaEventCreateWithFlags(&staged_ev, cudaEventDisableTiming);
     // A prefetched compressed block is decoded on a stream of its own, piece
     // by piece behind its copy, so neither the compute stream (install, step,
     // re-bucketing) nor the next copy waits for the decode.  The decode
@@ -1042,11 +1051,17 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         for (auto &e : ev_decoded) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     }
     bool staged_decoded = false;
-    // Decisions run on their own stream when prefetching: they read the
-    // counts of the last re-bucketing (ev_buck) and never wait for a copy,
-    // so the next block's upload queues right behind the one in flight.
-    cudaStream_t ds = s;
-    if (prefetch) cudaStreamCreateWithFlags(&ds, cudaStreamNonBlocking);
+    // Decisions run on their own stream: they read the counts of the last
+    // re-bucketing (ev_buck, before its scatter) and never wait for a copy, so
+    // with prefetch the next block's upload queues right behind the one in
+    // flight, and without it the upload runs beside the scatter.
+    cudaStream_t ds = nullptr;
+    if ((st = cuda(cudaStreamCreateWithFlags(&ds, cudaStreamNonBlocking), "decision stream"))) {
+        kring.destroy();
+        bring.destroy();
+        rring.destroy();
+        return st;
+    }
     uint32_t upload_stage = 0, staged_stage = 0;
     while (!done) {
         if (++iters > kMaxIters) {
@@ -1418,7 +1433,12 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
             const uint64_t ne = eblocks[b + 1] - eblocks[b];
             uint32_t *sc = o.slot_csr + (uint64_t)slot * o.slot_stride_words;
             uint64_t bytes = 0;
-            if ((st = upload_block(b, sc, s, 0, &bytes)) || (st = decode_block(b, sc, s, 0))) break;
+            // the step that read the slot has ended (the decision followed its
+            // counts), so the copy need not wait for the compute stream
+            if ((st = upload_block(b, sc, s_copy, 0, &bytes)) ||
+                (st = cuda(cudaEventRecord(staged_ev, s_copy), "event")) ||
+                (st = cuda(cudaStreamWaitEvent(s, staged_ev, 0), "block copy")) || (st = decode_block(b, sc, s, 0)))
+                break;
             h2d += bytes;
             loads++;
             if (!o.compressed) {  // a decoded block was checked by its decoder
@@ -1510,10 +1530,8 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         cudaEventDestroy(ev_up);
         for (auto &e : ev_decoded) cudaEventDestroy(e);
     }
-    if (ds != s) {
-        cudaStreamSynchronize(ds);
-        cudaStreamDestroy(ds);
-    }
+    cudaStreamSynchronize(ds);
+    cudaStreamDestroy(ds);
     // a training still in flight finishes here; its weights are adopted by
     // the next run's first decision
     if (o.ts) cudaStreamSynchronize(o.ts);

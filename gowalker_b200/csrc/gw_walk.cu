@@ -396,18 +396,21 @@ cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// The membership tables: a thread takes 32 consecutive edges, finds the first
+// The membership tables: a thread takes `per` consecutive edges, finds the first
 // one's vertex by halving the offsets and goes on from there, so hubs and
 // isolated vertices cost alike.  An id claims the first free slot from its home
 // bucket on; an id met twice keeps one slot.  Bound by the claims, about two
-// atomics an edge into the L2.
-constexpr uint32_t kTableEdges = 32;
+// atomics an edge into the L2, one after another in a thread: a small graph's
+// edges are spread over all threads (30,000 edges: 106 us at 32 a thread, 14 us
+// so), a large one's taken 16 at a time (63 M: 4.8 / 4.1 / 3.2 / 3.1 / 3.4 ms at
+// 2 / 4 / 8 / 16 / 32; fewer repeat the search, more lengthen the last wave).
+constexpr uint64_t kTableEdges = 16;
 __global__ void __launch_bounds__(256) k_build_table(const uint64_t *__restrict__ beg, const uint4 *__restrict__ verts,
                                                      uint32_t nverts, const uint32_t *__restrict__ csr,
-                                                     uint64_t nedges, uint32_t *table)
+                                                     uint64_t nedges, uint32_t per, uint32_t *table)
 {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * kTableEdges;
-    for (uint64_t e0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * kTableEdges; e0 < nedges; e0 += stride) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * per;
+    for (uint64_t e0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * per; e0 < nedges; e0 += stride) {
         uint32_t v = 0, hi = nverts;  // beg[v] <= e0 < beg[hi]
         while (hi - v > 1) {
             const uint32_t m = v + ((hi - v) >> 1);
@@ -416,7 +419,7 @@ __global__ void __launch_bounds__(256) k_build_table(const uint64_t *__restrict_
         }
         uint64_t end = __ldg(beg + v + 1);
         uint32_t buckets = 0, first = 0;
-        const uint64_t e1 = min(e0 + kTableEdges, nedges);
+        const uint64_t e1 = min(e0 + per, nedges);
         for (uint64_t e = e0; e < e1; ++e) {
             while (e >= end) {
                 ++v;
@@ -445,10 +448,12 @@ __global__ void __launch_bounds__(256) k_build_table(const uint64_t *__restrict_
 cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t nverts, const uint32_t *csr,
                                uint64_t nedges, uint32_t *table, int num_sms, cudaStream_t s)
 {
-    const uint64_t need = (nedges + 256ull * kTableEdges - 1) / (256ull * kTableEdges);
-    if (need == 0) return cudaSuccess;
-    k_build_table<<<(int)(need < (uint64_t)num_sms * 8 ? need : (uint64_t)num_sms * 8), 256, 0, s>>>(
-        beg, verts, nverts, csr, nedges, table);
+    if (nedges == 0) return cudaSuccess;
+    const uint64_t threads = 2048ull * num_sms;  // all resident
+    const uint32_t per = (uint32_t)std::min(kTableEdges, (nedges + threads - 1) / threads);
+    const uint64_t need = (nedges + 256ull * per - 1) / (256ull * per);
+    k_build_table<<<(int)std::min<uint64_t>(need, 8ull * num_sms), 256, 0, s>>>(beg, verts, nverts, csr, nedges, per,
+                                                                              table);
     return cudaGetLastError();
 }
 

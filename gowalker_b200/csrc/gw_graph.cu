@@ -207,21 +207,77 @@ __global__ void k_thin(const uint64_t *in, uint64_t U, uint64_t k, uint64_t *out
     }
 }
 
-// Degrees from the runs of a source-sorted key list (key = src << sh | dst):
-// the first key of a run adds -i and the last adds i+1 to cnt[src] (mod 2^64),
-// so cnt[v] ends as the run length; two uncontended atomics per vertex
-// whatever the gaps between sources.  csr[i] = dst of key i.
-__global__ void k_runs(const uint64_t *__restrict__ keys, uint64_t n, uint32_t sh, unsigned long long *cnt,
-                       uint32_t *__restrict__ csr)
+// Offsets and neighbour ids of a source-sorted key list (key = src << sh | dst)
+// in one pass: csr[i] = dst of key i, and where the source changes from p to s
+// at key i, beg[p + 1 .. s] = i (beg[0 .. s] = 0 at the first key, beg[.. V] = n
+// past the last).  Long gaps (many vertices without edges in a row) go to a list
+// that k_fill_gaps spreads over the GPU, so no thread walks one alone.  Memory
+// bound: reads the keys, writes ids and offsets once.  Degrees by atomics, a
+// clear and a scan took four passes and two more allocations: an edge list of
+// 100 M directed edges to a CSR (with this function's scratch taken from the
+// sort's buffers) 14.0 -> 11.5 ms, of 20 M 5.1 -> 3.0, of 300 k 1.9 -> 0.9.
+struct Gap {
+    uint32_t first, last;  // beg[first .. last] = value
+    uint64_t value;
+    uint32_t piece;        // pieces of the gaps before it in the list
+};
+constexpr uint32_t kLongGap = 64;     // offsets a thread of k_csr writes by itself
+constexpr uint32_t kGapPiece = 1024;  // offsets of a piece
+// count: gaps in the high 32 bits, pieces in the low ones; one atomic moves both,
+// so the list is in the order of its pieces.
+__global__ void __launch_bounds__(256) k_csr(const uint64_t *__restrict__ keys, uint64_t n, uint32_t sh, uint32_t V,
+                                             uint64_t *__restrict__ beg, uint32_t *__restrict__ csr, Gap *gaps,
+                                             unsigned long long *count)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t mask = (1ull << sh) - 1;
+    auto fill = [&](uint32_t first, uint32_t last, uint64_t value) {
+        const uint32_t more = last - first;
+        if (more < kLongGap) {
+            for (uint32_t k = 0; k <= more; ++k) beg[first + k] = value;
+        } else {
+            const unsigned long long at = atomicAdd(count, (1ull << 32) + (more / kGapPiece + 1));
+            gaps[at >> 32] = Gap{first, last, value, (uint32_t)at};
+        }
+    };
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const uint64_t k = keys[i];
-        const uint64_t s = k >> sh;
-        if (i == 0 || (keys[i - 1] >> sh) != s) atomicAdd(cnt + s, 0ull - (unsigned long long)i);
-        if (i + 1 == n || (keys[i + 1] >> sh) != s) atomicAdd(cnt + s, (unsigned long long)(i + 1));
+        const uint32_t s = (uint32_t)(k >> sh);
+        const uint32_t from = i ? (uint32_t)(keys[i - 1] >> sh) + 1 : 0u;
+        if (from <= s) fill(from, s, i);
+        if (i + 1 == n) fill(s + 1, V, n);
         csr[i] = (uint32_t)(k & mask);
+    }
+}
+
+// A warp fills an equal run of the pieces.
+__global__ void __launch_bounds__(256) k_fill_gaps(const Gap *__restrict__ gaps, const unsigned long long *count,
+                                                   uint64_t *__restrict__ beg)
+{
+    const uint32_t ngaps = (uint32_t)(*count >> 32), pieces = (uint32_t)*count;
+    const uint64_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t piece = (uint32_t)(pieces * warp / warps);
+    const uint32_t end = (uint32_t)(pieces * (warp + 1) / warps);
+    if (piece == end) return;
+    uint32_t g = 0;  // the last gap that starts at or before the piece
+    for (uint32_t len = ngaps; len > 1;) {
+        const uint32_t half = len / 2;
+        if (gaps[g + half].piece <= piece) {
+            g += half;
+            len -= half;
+        } else {
+            len = half;
+        }
+    }
+    while (piece < end) {
+        const Gap x = gaps[g++];
+        const uint32_t own = (x.last - x.first) / kGapPiece + 1;
+        const uint32_t stop = min(end, x.piece + own);
+        const uint64_t from = x.first + (uint64_t)(piece - x.piece) * kGapPiece;
+        const uint64_t to = min((uint64_t)x.last + 1, x.first + (uint64_t)(stop - x.piece) * kGapPiece);
+        for (uint64_t v = from + lane; v < to; v += 32) beg[v] = x.value;
+        piece = stop;
     }
 }
 
@@ -433,36 +489,43 @@ __global__ void k_split_equal(const uint64_t *beg, uint32_t V, uint32_t nblocks,
     }
 }
 
-// offsets + neighbour ids from n sorted keys src << sh | dst (sources <
-// nverts).  Allocates *beg_out and *csr_out; s is synchronised before return.
-static cudaError_t csr_from_sorted(const uint64_t *keys, uint64_t n, uint32_t sh, uint32_t nverts, cudaStream_t s,
-                                   uint64_t **beg_out, uint32_t **csr_out)
+// Offsets and neighbour ids from n sorted keys src << sh | dst (sources <
+// nverts).  Allocates *beg_out and *csr_out; `scratch` (scratch_bytes, 16-byte
+// aligned, not the keys) holds the gap list when it is large enough.  s is
+// synchronised before return.
+static cudaError_t csr_from_sorted(const uint64_t *keys, uint64_t n, uint32_t sh, uint32_t nverts, void *scratch,
+                                   uint64_t scratch_bytes, cudaStream_t s, uint64_t **beg_out, uint32_t **csr_out)
 {
-    unsigned long long *cnt = nullptr;
     uint64_t *beg = nullptr;
     uint32_t *csr = nullptr;
-    void *tmp = nullptr;
-    size_t tmp_bytes = 0;
+    char *own = nullptr;
     const uint64_t nb = (uint64_t)nverts + 1;
+    // a count, then at most one gap for every kLongGap offsets
+    const uint64_t gap_bytes = 16 + (nb / kLongGap + 1) * sizeof(Gap);
     cudaError_t e;
     do {
-        if ((e = cudaMalloc(&cnt, nb * sizeof(uint64_t))) != cudaSuccess) break;
         if ((e = cudaMalloc(&beg, nb * sizeof(uint64_t))) != cudaSuccess) break;
         if ((e = cudaMalloc(&csr, (n ? n : 1) * sizeof(uint32_t))) != cudaSuccess) break;
-        if ((e = cudaMemsetAsync(cnt, 0, nb * sizeof(uint64_t), s)) != cudaSuccess) break;
-        if (n) {
-            k_runs<<<148 * 16, 256, 0, s>>>(keys, n, sh, cnt, csr);
+        if (n == 0) {
+            if ((e = cudaMemsetAsync(beg, 0, nb * sizeof(uint64_t), s)) != cudaSuccess) break;
+        } else {
+            char *p = (char *)scratch;
+            if (scratch_bytes < gap_bytes) {
+                if ((e = cudaMalloc(&own, gap_bytes)) != cudaSuccess) break;
+                p = own;
+            }
+            unsigned long long *count = (unsigned long long *)p;
+            Gap *gaps = (Gap *)(p + 16);
+            if ((e = cudaMemsetAsync(count, 0, sizeof(*count), s)) != cudaSuccess) break;
+            const uint64_t need = (n + 255) / 256;
+            k_csr<<<(int)std::min<uint64_t>(need, 148 * 16), 256, 0, s>>>(keys, n, sh, nverts, beg, csr, gaps, count);
+            if ((e = cudaGetLastError()) != cudaSuccess) break;
+            k_fill_gaps<<<148 * 4, 256, 0, s>>>(gaps, count, beg);
             if ((e = cudaGetLastError()) != cudaSuccess) break;
         }
-        if ((e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (const uint64_t *)cnt, beg, nb, s)) != cudaSuccess)
-            break;
-        if ((e = cudaMalloc(&tmp, tmp_bytes)) != cudaSuccess) break;
-        if ((e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, (const uint64_t *)cnt, beg, nb, s)) != cudaSuccess)
-            break;
         e = cudaStreamSynchronize(s);
     } while (0);
-    cudaFree(cnt);
-    cudaFree(tmp);
+    cudaFree(own);
     if (e != cudaSuccess) {
         cudaFree(beg);
         cudaFree(csr);
@@ -524,7 +587,7 @@ static int sampled_csr(const Sampler &smp, uint64_t nsamples, uint32_t nverts, b
     int64_t *d_nsel = nullptr, nsel = 0;
     void *tmp = nullptr;
     size_t tmp_bytes = 0, tb2 = 0;
-    uint64_t U = 0;
+    uint64_t U = 0, scratch = 0;  // scratch: bytes of alt
     int rc = GW_OK;
     cudaError_t e = cudaSuccess;
 #define SC_CHECK(x)                       \
@@ -543,7 +606,8 @@ static int sampled_csr(const Sampler &smp, uint64_t nsamples, uint32_t nverts, b
     SC_CHECK(cudaStreamSynchronize(s));
     U = h_cur;
     SC_CHECK(cudaMalloc(&keys, (U ? U : 1) * sizeof(uint64_t)));
-    SC_CHECK(cudaMalloc(&alt, (U ? U : 1) * sizeof(uint64_t)));
+    scratch = (U ? U : 1) * sizeof(uint64_t);
+    SC_CHECK(cudaMalloc(&alt, scratch));
     SC_CHECK(cudaMemsetAsync(d_cur, 0, sizeof(unsigned long long), s));
     k_sample_keys<Sampler, false><<<blocks, 256, 0, s>>>(smp, nsamples, sh, symmetric ? 1 : 0, keys, d_cur);
     SC_CHECK(cudaGetLastError());
@@ -575,7 +639,7 @@ static int sampled_csr(const Sampler &smp, uint64_t nsamples, uint32_t nverts, b
             U = target_edges;
         }
     }
-    SC_CHECK(csr_from_sorted(keys, U, sh, nverts, s, &beg, &csr));
+    SC_CHECK(csr_from_sorted(keys, U, sh, nverts, alt, scratch, s, &beg, &csr));
     *d_beg = beg;
     *d_csr = csr;
     *nedges = U;
@@ -696,7 +760,7 @@ extern "C" int gw_web_csr(uint32_t scale, uint32_t nverts, const uint32_t thr[3]
             U = target_edges;
         }
     }
-    WB_CHECK(csr_from_sorted(keys, U, sh, nverts, s, &beg, &csr));
+    WB_CHECK(csr_from_sorted(keys, U, sh, nverts, alt, (M ? M : 1) * sizeof(uint64_t), s, &beg, &csr));
     *d_beg = beg;
     *d_csr = csr;
     *nedges = U;
@@ -734,11 +798,12 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
     PhaseTrace trace(s);
     uint64_t *keys = nullptr, *alt = nullptr, *beg = nullptr;
     uint32_t *csr = nullptr, *stage = nullptr;
+    char *scratch = nullptr, *own_tmp = nullptr;
     unsigned int *d_max = nullptr, *d_err = nullptr;
     unsigned long long *d_cnt = nullptr;  // [0] kept edges, [1] compaction cursor
     int64_t *d_nsel = nullptr;
     void *tmp = nullptr;
-    size_t tmp_bytes = 0, tb2 = 0;
+    size_t tmp_bytes = 0, tb2 = 0, tmp_room = 0;
     unsigned int h_max = 0, h_err = 0;
     unsigned long long h_kept = 0;
     uint64_t U = 0;
@@ -753,15 +818,32 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
     // when nverts is given (otherwise repacked once the largest id is known).
     if (sorted && nverts) sh = bit_length32(nverts - 1);
 
-    GEN_CHECK(cudaMalloc(&keys, (m ? m : 1) * sizeof(uint64_t)));
-    GEN_CHECK(cudaMalloc(&alt, (m ? m : 1) * sizeof(uint64_t)));
-    GEN_CHECK(cudaMalloc(&d_max, 2 * sizeof(unsigned int)));
-    GEN_CHECK(cudaMalloc(&d_cnt, 2 * sizeof(unsigned long long)));
-    GEN_CHECK(cudaMalloc(&d_nsel, sizeof(int64_t)));
-    d_err = d_max + 1;
-    GEN_CHECK(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned int), s));
-    GEN_CHECK(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), s));
-    if (!in_place) GEN_CHECK(cudaMalloc(&stage, 2 * chunk * sizeof(uint32_t)));
+    {
+        // all scratch in one allocation (a call's other time is the sort's, and
+        // every allocation and free of this size costs as much as a pass of it):
+        // the keys twice, the counters, the sort's own scratch for all m keys.
+        const uint64_t key_bytes = ((m ? m : 1) * sizeof(uint64_t) + 255) & ~255ull;
+        cub::DoubleBuffer<uint64_t> db(nullptr, nullptr);
+        if (m) {
+            GEN_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, db, m, 0, 64, s));
+            if (dedup) {
+                GEN_CHECK(cub::DeviceSelect::Unique(nullptr, tb2, keys, alt, d_nsel, (int64_t)m, s));
+                tmp_bytes = std::max(tmp_bytes, tb2);
+            }
+        }
+        tmp_room = (tmp_bytes + 255) & ~size_t(255);
+        GEN_CHECK(cudaMalloc(&scratch, 2 * key_bytes + 256 + tmp_room));
+        keys = (uint64_t *)scratch;
+        alt = (uint64_t *)(scratch + key_bytes);
+        char *small = scratch + 2 * key_bytes;
+        d_cnt = (unsigned long long *)small;
+        d_nsel = (int64_t *)(small + 16);
+        d_max = (unsigned int *)(small + 24);
+        d_err = d_max + 1;
+        tmp = small + 256;
+        if (!in_place) stage = (uint32_t *)alt;  // 2 * chunk ids <= m keys; the sort takes alt over
+        GEN_CHECK(cudaMemsetAsync(small, 0, 256, s));
+    }
     trace.mark("alloc");
     for (uint64_t i0 = 0; i0 < n; i0 += chunk) {
         const uint64_t k = std::min(chunk, n - i0);
@@ -817,7 +899,10 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
             GEN_CHECK(cub::DeviceSelect::Unique(nullptr, tb2, keys, alt, d_nsel, (int64_t)U, s));
             tmp_bytes = std::max(tmp_bytes, tb2);
         }
-        GEN_CHECK(cudaMalloc(&tmp, tmp_bytes));
+        if (tmp_bytes > tmp_room) {  // fewer keys should not need more, but nothing says so
+            GEN_CHECK(cudaMalloc(&own_tmp, tmp_bytes));
+            tmp = own_tmp;
+        }
         GEN_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, db, nsort, b0, b1, s));
         keys = db.Current();
         alt = db.Alternate();
@@ -832,7 +917,7 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
             trace.mark("unique");
         }
     }
-    GEN_CHECK(csr_from_sorted(keys, U, sh, V, s, &beg, &csr));
+    GEN_CHECK(csr_from_sorted(keys, U, sh, V, alt, (m ? m : 1) * sizeof(uint64_t), s, &beg, &csr));
     trace.mark("csr");
     *d_beg = beg;
     *d_csr = csr;
@@ -841,13 +926,8 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
     beg = nullptr;
     csr = nullptr;
 done:
-    cudaFree(keys);
-    cudaFree(alt);
-    cudaFree(stage);
-    cudaFree(tmp);
-    cudaFree(d_max);
-    cudaFree(d_cnt);
-    cudaFree(d_nsel);
+    cudaFree(scratch);
+    cudaFree(own_tmp);
     cudaFree(beg);
     cudaFree(csr);
     trace.mark("free");

@@ -79,7 +79,7 @@ struct OocState {
     unsigned long long *h_snap[2] = {nullptr, nullptr}, *dm_snap[2] = {nullptr, nullptr};
     uint32_t *d_vstart = nullptr;
     uint64_t *d_estart = nullptr;
-    uint32_t *h_cached = nullptr;  // pinned and mapped: the decision kernels read it in place
+    uint32_t *h_cached = nullptr;  // pinned and mapped: the annealed choice reads it in place
     uint32_t *d_cached = nullptr;  // h_cached's device alias
 
     WalkerRec *w_rec = nullptr;                    // records, never moved
@@ -684,15 +684,18 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     for (uint32_t b = 0; b < 2 * nb; ++b) o.h_blk_csr[b] = nullptr;
     const uint32_t **pin_last = o.h_blk_pin[0];
     uint32_t pin_last_idx = 0;
-    auto push_tables = [&]() -> int {
+    // The table of the next step as the decision stream reads it (mapped host
+    // memory).  Two in turn: what read the one before last ended before the step
+    // whose counts the last decision read.
+    auto push_tables = [&]() {
         pin_last = o.h_blk_pin[o.pin_next];
         pin_last_idx = o.pin_next;
         o.pin_next ^= 1u;
         memcpy((void *)pin_last, o.h_blk_csr, 2 * nb * sizeof(void *));
-        return cuda(cudaMemcpyAsync((void *)o.d_blk_csr, pin_last, 2 * nb * sizeof(void *), cudaMemcpyHostToDevice, s),
-                    "block table");
     };
-    if ((st = push_tables())) return st;
+    push_tables();
+    std::vector<const uint32_t *> step_blk(2 * nb, nullptr);  // o.d_blk_csr as of the last step
+    if ((st = cuda(cudaMemsetAsync((void *)o.d_blk_csr, 0, 2 * nb * sizeof(void *), s), "block table"))) return st;
     // A block's neighbour list towards slot memory `sc` on stream `cs`: a
     // plain copy into the slot, or the compressed copy into the staging
     // buffer `stage`; decode_block then expands a compressed one into the
@@ -752,7 +755,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
             if (va == vb) continue;
             // the payload of the piece, plus the 8 bytes a decoder may read past it
             const uint64_t lo = done ? cb.payload_off + hvoff[va] : 0;
-            const uint64_t hi = k + 1 == kPieces ? cb.bytes : std::min(cb.payload_off + hvoff[vb] + 8, cb.bytes);
+            const uint64_t hi = vb == nv ? cb.bytes : std::min(cb.payload_off + hvoff[vb] + 8, cb.bytes);
             if ((e = put(lo, hi, "compressed block payload"))) return e;
             done = hi;
             if ((e = cuda(cudaEventRecord(ev, cs), "event")) || (e = cuda(cudaStreamWaitEvent(ds_dec, ev, 0), "event")))
@@ -815,6 +818,9 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     if ((st = cuda(cudaEventCreateWithFlags(&ev_buck, cudaEventDisableTiming), "event"))) return st;
     cudaEvent_t ev_dec = nullptr;  // this iteration's decision has read the counts
     if ((st = cuda(cudaEventCreateWithFlags(&ev_dec, cudaEventDisableTiming), "event"))) return st;
+    cudaEvent_t ev_run = nullptr;  // the next step's runnable ranges and block table are there
+    if ((st = cuda(cudaEventCreateWithFlags(&ev_run, cudaEventDisableTiming), "event"))) return st;
+    cudaStream_t ds = nullptr, s_run = nullptr;  // decisions, runnable passes: created below
 
     // Re-bucketing: count, plan and scatter the sorted index from buffer c to
     // c^1, per-pair totals, the new walker count into d_n[c^1], and the counter
@@ -883,54 +889,47 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     if (grid <= 0)
         grid = ooc_grid(sopr, paths, coop, cfg.prefetch && num_sms > 8 ? num_sms - 1 : num_sms, o.weighted);
 
-    // The step of an iteration -- runnable pass, cursor reset, step kernel --
-    // is captured once per run and sorted-index parity as a CUDA graph (the
-    // step kernel's arguments differ only by that parity).  The zero-copy
-    // tail's launch and traced runs (events around the runnable pass) launch
-    // the kernels one by one.
-    cudaGraphExec_t sgraph[2] = {nullptr, nullptr};
-    auto step_ops = [&](uint32_t c) -> int {
+    // What the step kernel reads besides the walkers -- the runnable ranges, the
+    // block table, its cursor -- needs the plan alone, so it is written on a
+    // stream of its own: beside the scatter and the decision, and without
+    // prefetch beside the block's copy.  In front of the step kernel, with a
+    // copy of the table and a clear of the cursor, it held the compute stream
+    // for about 20 us of an iteration; on the decision stream, the next copy.
+    // 725 iterations of 149 us -> 139, without prefetch 95 of 218 -> 210.
+    auto prepare_step = [&]() -> int {
         int e;
-        if ((e = cuda(launch_runnable(o.d_offsets, o.d_blk_csr, nb, a.lazy, o.d_run_pre, o.d_run_off, o.d_nrun, s),
+        if ((e = cuda(cudaStreamWaitEvent(s_run, ev_buck, 0), "plan wait"))) return e;
+        TablePatch patch{};
+        uint32_t changes = 0;
+        for (uint32_t b = 0; b < nb; ++b) {
+            if (step_blk[b] == o.h_blk_csr[b] && step_blk[nb + b] == o.h_blk_csr[nb + b]) continue;
+            if (changes < TablePatch::kMax) {
+                patch.block[changes] = b;
+                patch.csr[changes] = o.h_blk_csr[b];
+                patch.alias[changes] = o.h_blk_csr[nb + b];
+            }
+            ++changes;
+        }
+        std::copy(o.h_blk_csr, o.h_blk_csr + 2 * nb, step_blk.begin());
+        patch.n = changes;
+        if (changes > TablePatch::kMax) {  // around the zero-copy tail
+            patch.n = 0;
+            if ((e = cuda(cudaMemcpyAsync((void *)o.d_blk_csr, pin_last, 2 * nb * sizeof(void *),
+                                          cudaMemcpyHostToDevice, s_run),
+                          "block table")))
+                return e;
+        }
+        if (trace) rring.begin(s_run, t_runnable_f);
+        if ((e = cuda(launch_runnable(o.d_offsets, patch, nb, a.lazy, o.d_blk_csr,
+                                      d_ctr + kCtrCursor, o.d_run_pre, o.d_run_off, o.d_nrun, s_run),
                       "runnable")))
             return e;
-        if ((e = cuda(cudaMemsetAsync(d_ctr + kCtrCursor, 0, sizeof(unsigned long long), s), "memset"))) return e;
-        OocStepArgs ac = a;
-        ac.recs = o.w_rec;
-        ac.order = o.w_ord[c];
-        ac.keys = o.w_key[c];
-        return cuda(launch_walk_ooc(ac, sopr, coop, o.weighted, grid, s), "walk kernel");
+        if (trace) rring.end(s_run);
+        return cuda(cudaEventRecord(ev_run, s_run), "event");
     };
     auto step = [&]() -> int {
         int e;
-        if (!trace && !a.mapped) {
-            const uint32_t c = o.w_cur;
-            if (!sgraph[c]) {
-                cudaGraph_t g = nullptr;
-                if ((e = cuda(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal), "capture"))) return e;
-                const int eo = step_ops(c);
-                const cudaError_t ec = cudaStreamEndCapture(s, &g);
-                if (eo) {
-                    if (g) cudaGraphDestroy(g);
-                    return eo;
-                }
-                if ((e = cuda(ec, "capture"))) return e;
-                e = cuda(cudaGraphInstantiate(&sgraph[c], g, 0), "graph instantiate");
-                cudaGraphDestroy(g);
-                if (e) return e;
-            }
-            if ((e = cuda(kring.begin(s, kernel_ms), "event"))) return e;
-            if ((e = cuda(cudaGraphLaunch(sgraph[c], s), "step graph"))) return e;
-            if ((e = cuda(kring.end(s), "event"))) return e;
-            launches += 2;
-            return GW_OK;
-        }
-        if (trace) rring.begin(s, t_runnable_f);
-        if ((e = cuda(launch_runnable(o.d_offsets, o.d_blk_csr, nb, a.lazy, o.d_run_pre, o.d_run_off, o.d_nrun, s),
-                      "runnable")))
-            return e;
-        if (trace) rring.end(s);
-        if ((e = cuda(cudaMemsetAsync(d_ctr + kCtrCursor, 0, sizeof(unsigned long long), s), "memset"))) return e;
+        if ((e = cuda(cudaStreamWaitEvent(s, ev_run, 0), "runnable wait"))) return e;
         a.recs = o.w_rec;
         a.order = o.w_ord[o.w_cur];
         a.keys = o.w_key[o.w_cur];
@@ -1055,8 +1054,8 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     // re-bucketing (ev_buck, before its scatter) and never wait for a copy, so
     // with prefetch the next block's upload queues right behind the one in
     // flight, and without it the upload runs beside the scatter.
-    cudaStream_t ds = nullptr;
-    if ((st = cuda(cudaStreamCreateWithFlags(&ds, cudaStreamNonBlocking), "decision stream"))) {
+    if ((st = cuda(cudaStreamCreateWithFlags(&s_run, cudaStreamNonBlocking), "runnable stream")) ||
+        (st = cuda(cudaStreamCreateWithFlags(&ds, cudaStreamNonBlocking), "decision stream"))) {
         kring.destroy();
         bring.destroy();
         rring.destroy();
@@ -1105,20 +1104,21 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
                         break;
                     }
             staged_block = -1;
-            if ((st = push_tables())) break;
+            push_tables();
             if (trace) {
                 cudaEventRecord(tin1, s);
                 tin_live = true;
             }
         }
         const uint32_t ncached = (uint32_t)o.cached.size();
-        for (uint32_t j = 0; j < ncached; ++j) o.h_cached[j] = o.cached[j];
+        if (policy == GW_POLICY_SA) std::copy(o.cached.begin(), o.cached.end(), o.h_cached);
         if ((st = cuda(cudaStreamWaitEvent(ds, ev_buck, 0), "decision wait"))) break;
-        // The cached list and (for the learned features) the block table are
-        // read in place from mapped host memory -- the last decision on ds
-        // has finished, and the table's ring slot is not rewritten before this
-        // one does -- so the decision's path has no host-to-device copy to
-        // queue behind the block copy in flight.
+        if (prefetch && (st = prepare_step())) break;
+        // The cached list is an argument of the plain choice.  The annealed
+        // choice reads it, and the learned features the block table, in place
+        // from mapped host memory -- the last decision on ds has finished, and
+        // the table's ring slot is not rewritten before this one does -- so the
+        // decision's path has no copy to queue behind the block copy in flight.
         // ---- learned policy: features (traces while training), prediction, choice
         const bool learned = policy == GW_POLICY_LEARNED;
         // a training that has finished (host-side query: never a wait) hands
@@ -1192,7 +1192,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         const bool learned_decides = learned_active && !stall_next;
         const float *forecast =
             learned_decides && (lmode & GW_LEARNED_EVICT) ? (o.trained ? o.d_pred : ring_col) : nullptr;
-        if ((st = cuda(launch_schedule(o.d_pairs, o.d_offsets + nbk, nb, o.d_cached, ncached, capacity,
+        if ((st = cuda(launch_schedule(o.d_pairs, o.d_offsets + nbk, nb, o.cached.data(), ncached, capacity,
                                        cost_switch ? 0u : cfg.zero_threshold,
                                        forecast, 1.f, o.d_dec, ds),
                        "schedule")))
@@ -1323,14 +1323,14 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
             if (!o.d_mapped && (st = cuda(cudaMalloc(&o.d_mapped, nb), "mapped-block flags"))) break;
             if ((st = cuda(cudaMemcpyAsync(o.d_mapped, mapped.data(), nb, cudaMemcpyHostToDevice, s), "mapped flags")))
                 break;
-            if ((st = push_tables())) break;
+            push_tables();
             unsigned long long before[kCtrCount];
             if ((st = cuda(cudaMemcpyAsync(before, d_ctr, sizeof(before), cudaMemcpyDeviceToHost, s), "counters")) ||
                 (st = cuda(cudaStreamSynchronize(s), "counters")))
                 break;
             a.mapped = o.d_mapped;
             const auto tz0 = std::chrono::steady_clock::now();
-            st = step();
+            if (!(st = prepare_step())) st = step();
             a.mapped = nullptr;
             if (st) break;
             if ((st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, sizeof(before), cudaMemcpyDeviceToHost, s), "counters")))
@@ -1349,7 +1349,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
             // restore the table to device slots only
             for (uint32_t b = 0; b < nb; ++b)
                 if (o.block_slot[b] < 0) o.h_blk_csr[b] = nullptr;
-            if ((st = push_tables())) break;
+            push_tables();
             if ((st = bucketize(nullptr))) break;
             iters++;
             done = true;
@@ -1454,7 +1454,8 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
 
         // ---- walk every runnable bucket, then re-bucket
         if (!stepped) {
-            if ((st = push_tables())) break;
+            push_tables();
+            if ((st = prepare_step())) break;
             if ((st = step())) break;
             if ((st = bucketize(nullptr))) break;
         }
@@ -1532,13 +1533,14 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     }
     cudaStreamSynchronize(ds);
     cudaStreamDestroy(ds);
+    cudaStreamSynchronize(s_run);
+    cudaStreamDestroy(s_run);
     // a training still in flight finishes here; its weights are adopted by
     // the next run's first decision
     if (o.ts) cudaStreamSynchronize(o.ts);
-    for (auto &g : sgraph)
-        if (g) cudaGraphExecDestroy(g);
     cudaEventDestroy(ev_buck);
     cudaEventDestroy(ev_dec);
+    cudaEventDestroy(ev_run);
     kring.drain(kernel_ms);
     bring.drain(bucket_ms);
     if (trace) rring.drain(t_runnable_f);
@@ -1656,21 +1658,19 @@ extern "C" int gw_plain_choose_block(const uint32_t *counts, uint32_t nblocks, c
         seen[cached[j]] = 1;
     }
     const uint64_t nn = (uint64_t)nblocks * nblocks;
-    uint32_t *d_counts = nullptr, *d_cached = nullptr, *d_live = nullptr;
+    uint32_t *d_counts = nullptr, *d_live = nullptr;
     Decision *d_dec = nullptr;
     Decision h{};
     int rc = GW_OK;
     do {
         if (cudaMalloc(&d_counts, nn * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&d_cached, (ncached ? ncached : 1) * sizeof(uint32_t)) != cudaSuccess ||
             cudaMalloc(&d_live, sizeof(uint32_t)) != cudaSuccess || cudaMalloc(&d_dec, sizeof(Decision)) != cudaSuccess) {
             rc = GW_ERR_NOMEM;
             break;
         }
         if (cudaMemcpy(d_counts, counts, nn * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess ||
-            (ncached && cudaMemcpy(d_cached, cached, ncached * sizeof(uint32_t), cudaMemcpyHostToDevice) != cudaSuccess) ||
             cudaMemset(d_live, 0, sizeof(uint32_t)) != cudaSuccess ||
-            launch_schedule(d_counts, d_live, nblocks, d_cached, ncached, nslots, zero_threshold, nullptr, 1.f, d_dec,
+            launch_schedule(d_counts, d_live, nblocks, cached, ncached, nslots, zero_threshold, nullptr, 1.f, d_dec,
                             0) != cudaSuccess ||
             cudaMemcpy(&h, d_dec, sizeof(Decision), cudaMemcpyDeviceToHost) != cudaSuccess) {
             rc = GW_ERR_CUDA;
@@ -1682,7 +1682,6 @@ extern "C" int gw_plain_choose_block(const uint32_t *counts, uint32_t nblocks, c
     } while (0);
     if (rc != GW_OK) cudaGetLastError();
     cudaFree(d_counts);
-    cudaFree(d_cached);
     cudaFree(d_live);
     cudaFree(d_dec);
     return rc;

@@ -80,10 +80,21 @@ cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, co
                            uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s);
 // Buckets are 2 * nb^2: (prev_blk, cur_blk), then the same pairs for walkers
 // flagged kNeedPrev.
-cudaError_t launch_runnable(const uint32_t *offsets, const uint32_t *const *blk_csr, uint32_t nb, uint32_t lazy,
-                            uint32_t *run_pre, uint32_t *run_off, uint32_t *nrun, cudaStream_t s);
-// `counts` are the nb^2 per-pair totals; `live` points at the live-walker count.
-cudaError_t launch_schedule(const uint32_t *counts, const uint32_t *live, uint32_t nb, const uint32_t *cached,
+// Changes of the block table since the last step, as kernel arguments: a read of
+// mapped host memory waits behind the block copy in flight (60 us and more).
+struct TablePatch {
+    static constexpr uint32_t kMax = 4;
+    uint32_t n;
+    uint32_t block[kMax];
+    const uint32_t *csr[kMax], *alias[kMax];
+};
+// Also applies the patch to blk_csr and clears the step's cursor.
+cudaError_t launch_runnable(const uint32_t *offsets, const TablePatch &patch, uint32_t nb, uint32_t lazy,
+                            const uint32_t **blk_csr, unsigned long long *cursor, uint32_t *run_pre,
+                            uint32_t *run_off, uint32_t *nrun, cudaStream_t s);
+// `counts` are the nb^2 per-pair totals; `live` points at the live-walker count;
+// `h_cached` is host memory, taken as a kernel argument.
+cudaError_t launch_schedule(const uint32_t *counts, const uint32_t *live, uint32_t nb, const uint32_t *h_cached,
                             uint32_t ncached, uint32_t nslots, uint32_t zero_threshold, const float *pred,
                             float pred_weight, Decision *out, cudaStream_t s);
 // ---- SOWalker annealing policy (gw_sa.cu): the block set held across

@@ -138,10 +138,11 @@ bool compress_block(const uint64_t *beg, const uint32_t *csr, uint32_t nv, uint6
         for (uint32_t v = a; v < b; ++v) encode_vertex(csr + (beg[v] - e0), beg[v + 1] - beg[v], pay + off[v]);
     });
     // pieces of about equal payload, cut at multiples of 32 vertices
+    const uint32_t pieces = (uint32_t)std::clamp<uint64_t>(payload / kPieceBytes, 1, kPieces);
     out.piece_v[0] = 0;
-    out.piece_v[kPieces] = nv;
-    for (uint32_t k = 1; k < kPieces; ++k) {
-        const uint64_t target = payload * k / kPieces;
+    for (uint32_t k = pieces; k <= kPieces; ++k) out.piece_v[k] = nv;
+    for (uint32_t k = 1; k < pieces; ++k) {
+        const uint64_t target = payload * k / pieces;
         uint32_t v = (uint32_t)(std::lower_bound(off.begin(), off.begin() + nv, target) - off.begin());
         v &= ~31u;
         out.piece_v[k] = std::max(v, out.piece_v[k - 1]);

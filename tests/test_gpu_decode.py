@@ -44,3 +44,29 @@ def test_decoded_blocks_walk_like_oracle(gw, oracle, name, prefetch):
     assert st["block_loads"] > 0
     assert np.array_equal(eng.hashes(), ref["hashes"])
     eng.close()
+
+
+@pytest.mark.parametrize("prefetch", [0, 1])
+def test_blocks_of_one_to_four_pieces(gw, oracle, prefetch):
+    """A prefetched block arrives in one to four pieces by its payload (2 MB
+    each at least): blocks of 0.5 to 4.5 M ids, about 2 bytes an id."""
+    rng = np.random.default_rng(3)
+    deg = 64
+    sizes = [4_500_000, 500_000, 2_200_000, 3_200_000, 1_200_000] * 2
+    vb = np.concatenate([[0], np.cumsum([n // deg for n in sizes])]).astype(np.uint32)
+    V = int(vb[-1])
+    csr = np.sort(rng.integers(0, V, (V, deg), dtype=np.uint32), axis=1).ravel()
+    beg = np.arange(V + 1, dtype=np.uint64) * deg
+    eb = beg[vb]
+    slot = max(sizes) * 4 + 64
+    cache = (V + 1) * 8 + (1 + prefetch) * slot * 5 // 8 + 3 * slot
+    assert cache < (V + 1) * 8 + 4 * len(csr)
+    eng = gw.WalkEngine(algorithm=0, maxhops=5, p=0.5, q=2.0, seed=4, walkpersource=1, compress_blocks=1,
+                        prefetch=prefetch, cache_size=cache)
+    eng.set_host_graph(beg, csr, vb, eb)
+    eng.init_walkers(0, 1, 4)
+    st = eng.run()
+    ref = oracle.walk(beg, csr, oracle.make_cfg(algo=0, maxhops=5, p=0.5, q=2.0, seed=4, wps=1), 0, V, paths=False)
+    assert st["block_loads"] > 0
+    assert np.array_equal(eng.hashes(), ref["hashes"])
+    eng.close()

@@ -2,18 +2,20 @@
 // block choice of engine/schedule.hpp:70-138).
 //
 //  k_init_walkers  walker records from ids (engine/walk.hpp:32-95)
-//  k_count         walkers per (prev block, cur block) bucket, warp-aggregated
-//                  atomics (one atomic per distinct bucket per warp instead of
-//                  one per walker, gpu/gpuwalk.hpp:179)
+//  k_count         walkers per (prev block, cur block) bucket before the first
+//                  step, warp-aggregated atomics (one atomic per distinct bucket
+//                  per warp instead of one per walker, gpu/gpuwalk.hpp:179)
 //  k_plan          exclusive scan of the bucket counts in one CTA (coalesced warp segments;
 //                  the reference scans them on one thread, gpu/gpuwalk.hpp:321-338), with
 //                  everything else the next decision and the scatter read
 //  k_scatter       walkers into bucket order, finished walkers dropped
 //                  (gpu/gpuwalk.hpp:340-360 + the spill of engine/walk.hpp:484-525)
-//  k_runnable      ranges of the buckets whose two blocks are resident
+//  k_runnable      ranges of the buckets whose two blocks are resident, and their
+//                  counts cleared
 //  k_schedule      GOwalker_scheduler_t::max_choose_blocks on the device
 //  k_walk_ooc      the step kernel over runnable walkers; a walker stops when
-//                  its next vertex lies in a block that is not resident
+//                  its next vertex lies in a block that is not resident, and
+//                  counts itself in its new bucket
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "gw_ooc_kernels.cuh"
@@ -151,13 +153,13 @@ __device__ __forceinline__ uint32_t cta_warp_base(uint32_t wtotal, uint32_t *tot
     return b;
 }
 
-// Between the count and the scatter, all that needs one CTA: bucket offsets
+// Between the step and the scatter, all that needs one CTA: bucket offsets
 // (and the scatter's cursors, which start there), the new number of sorted
-// positions, per-pair totals (when `pairs` is given), the counts cleared for
-// the next count, and the counters and error word into mapped host memory.
-// Five launches and two copies of 2-5 us each before; the next decision may
-// start as soon as this is done, beside the scatter.
-__global__ void __launch_bounds__(kScanThreads) k_plan(uint32_t *__restrict__ counts, uint32_t nn,
+// positions, per-pair totals (when `pairs` is given), and the counters and error
+// word into mapped host memory.  Five launches and two copies of 2-5 us each
+// before; the next decision may start as soon as this is done, beside the
+// scatter.
+__global__ void __launch_bounds__(kScanThreads) k_plan(const uint32_t *__restrict__ counts, uint32_t nn,
                                                        uint32_t *__restrict__ offsets, uint32_t *__restrict__ cursor,
                                                        uint32_t *__restrict__ pairs, uint32_t *__restrict__ n_out,
                                                        const unsigned long long *__restrict__ ctr,
@@ -185,7 +187,6 @@ __global__ void __launch_bounds__(kScanThreads) k_plan(uint32_t *__restrict__ co
         const uint32_t inc = warp_incl_scan(v, lane);
         if (i < hi) {
             offsets[i] = cursor[i] = base + inc - v;
-            counts[i] = 0;
         }
         base += __shfl_sync(0xFFFFFFFFu, inc, 31);
     }
@@ -198,7 +199,8 @@ __global__ void __launch_bounds__(kScanThreads) k_plan(uint32_t *__restrict__ co
 
 __global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__restrict__ offsets,
                                                            const __grid_constant__ TablePatch patch, uint32_t nb,
-                                                           uint32_t lazy, const uint32_t **__restrict__ blk_csr,
+                                                           uint32_t lazy, uint32_t *__restrict__ counts,
+                                                           const uint32_t **__restrict__ blk_csr,
                                                            unsigned long long *cursor, uint32_t *__restrict__ run_pre,
                                                            uint32_t *__restrict__ run_off, uint32_t *__restrict__ nrun)
 {
@@ -251,6 +253,7 @@ __global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__res
             const uint32_t k = kb + (uint32_t)__popc(fm & lt);
             run_off[k] = offsets[b];
             run_pre[k] = sb + inc - v;
+            counts[b] = 0;  // the step takes all of them, and counts each where it stops
         }
         kb += (uint32_t)__popc(fm);
         sb += __shfl_sync(0xFFFFFFFFu, inc, 31);
@@ -528,7 +531,9 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         rec.hash_lo = (uint32_t)h;
         rec.hash_hi = (uint32_t)(h >> 32);
         a.recs[__ldg(a.order + idx)] = rec;
-        a.keys[idx] = bucket_of(rec, a.nb);
+        const uint32_t b = bucket_of(rec, a.nb);
+        a.keys[idx] = b;
+        atomicAdd(a.counts + b, 1u);
         flush();
     };
     // Enter a step at vertex cur (block cb, edges [b0, b1)), prev adjacency
@@ -889,7 +894,7 @@ __global__ void k_combine(const uint32_t *__restrict__ counts, uint32_t nn, uint
         combined[k] = counts[k] + counts[nn + k];
 }
 
-cudaError_t launch_plan(uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
+cudaError_t launch_plan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
                         uint32_t *n_out, const unsigned long long *ctr, const uint32_t *err, unsigned long long *snap,
                         int num_sms, cudaStream_t s)
 {
@@ -913,10 +918,10 @@ cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, co
 }
 
 cudaError_t launch_runnable(const uint32_t *offsets, const TablePatch &patch, uint32_t nb, uint32_t lazy,
-                            const uint32_t **blk_csr, unsigned long long *cursor, uint32_t *run_pre,
+                            uint32_t *counts, const uint32_t **blk_csr, unsigned long long *cursor, uint32_t *run_pre,
                             uint32_t *run_off, uint32_t *nrun, cudaStream_t s)
 {
-    k_runnable<<<1, kScanThreads, 0, s>>>(offsets, patch, nb, lazy, blk_csr, cursor, run_pre, run_off, nrun);
+    k_runnable<<<1, kScanThreads, 0, s>>>(offsets, patch, nb, lazy, counts, blk_csr, cursor, run_pre, run_off, nrun);
     return cudaGetLastError();
 }
 

@@ -37,6 +37,7 @@ struct OocStepArgs {
     WalkerRec *recs;                 // one record per walker, never moved
     const uint32_t *order;           // record of each bucket-sorted position
     uint32_t *keys;                  // bucket of each sorted position; kNoBucket once finished
+    uint32_t *counts;                // walkers per bucket; the runnable ones' are 0 before the step
     const uint32_t *run_pre;         // [nrun+1] prefix of runnable bucket sizes
     const uint32_t *run_off;         // [nrun] first walker of each runnable bucket
     const uint32_t *nrun;            // runnable bucket count (device)
@@ -69,11 +70,11 @@ cudaError_t launch_init_walkers(const WalkerInit &in, const uint32_t *vstart, ui
                                 int num_sms, cudaStream_t s);
 // `n` points at the number of sorted positions (a device word).
 cudaError_t launch_count(const uint32_t *keys, const uint32_t *n, uint32_t *counts, int num_sms, cudaStream_t s);
-// After launch_count: offsets (2 * nb^2 + 1) and cursors from the counts, which
-// are cleared; pairs[k] = counts[k] + counts[nb^2 + k], walkers per (prev, cur)
+// Offsets (2 * nb^2 + 1) and cursors from the counts (of launch_count, kept up by
+// the steps); pairs[k] = counts[k] + counts[nb^2 + k], walkers per (prev, cur)
 // block pair; *n_out, the sorted positions to come; counters (kCtrCount) and
 // error word into snap[0 .. kCtrCount] (mapped host memory).
-cudaError_t launch_plan(uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
+cudaError_t launch_plan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
                         uint32_t *n_out, const unsigned long long *ctr, const uint32_t *err, unsigned long long *snap,
                         int num_sms, cudaStream_t s);
 cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, uint32_t *cursor,
@@ -88,9 +89,10 @@ struct TablePatch {
     uint32_t block[kMax];
     const uint32_t *csr[kMax], *alias[kMax];
 };
-// Also applies the patch to blk_csr and clears the step's cursor.
+// Also applies the patch to blk_csr, and clears the step's cursor and the counts
+// of the buckets it lists.
 cudaError_t launch_runnable(const uint32_t *offsets, const TablePatch &patch, uint32_t nb, uint32_t lazy,
-                            const uint32_t **blk_csr, unsigned long long *cursor, uint32_t *run_pre,
+                            uint32_t *counts, const uint32_t **blk_csr, unsigned long long *cursor, uint32_t *run_pre,
                             uint32_t *run_off, uint32_t *nrun, cudaStream_t s);
 // `counts` are the nb^2 per-pair totals; `live` points at the live-walker count;
 // `h_cached` is host memory, taken as a kernel argument.

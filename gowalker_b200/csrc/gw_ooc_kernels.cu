@@ -670,12 +670,13 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         int verdict = 0;
         uint32_t x = 0, sectors = 0;
         uint64_t n0 = 0, n1 = 0;  // offsets of a vertex that is, or may be, the next one
+        float rv = 0.0f;
         if (active) {
             const uint32_t att = attempt + grp.sub(lane);
             const U4 r = draw(a.c, wid, hop, att);
             end = att == 0 && hop > 0 && terminates(a.c, r.z);
             const uint32_t pos = r.x % deg;
-            const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
+            rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
             uint32_t col = pos;
             if constexpr (W) {
                 const uint2 e = __ldg(calias + pos);
@@ -690,14 +691,20 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
                 n0 = __ldg(a.beg + x);
                 n1 = __ldg(a.beg + x + 1);
             }
-            // N(prev) is searched only when the verdict depends on it, and then
-            // only if its block is resident (or mapped); each search and each
-            // candidate counts its sectors
-            if (verdict < 0 && padj != nullptr) {
-                if (!ZC || s_mapped[pb]) sectors += search_sectors(pdeg);
-                const bool found = csr_contains(CsrIndex<kSearch>{padj, nullptr}, 0u, 0ull, pdeg, x);
-                verdict = (found ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t)) ? 1 : 0;
-            }
+        }
+        // N(prev) is searched only when the verdict depends on it, then only if
+        // its block is resident (or mapped), and only if no attempt before this
+        // one decides the step without: the whole warp waits for a search.  Each
+        // search and each candidate counts its sectors.
+        bool search = verdict < 0 && padj != nullptr;
+        if (grp.shift) {
+            const unsigned sure = grp.mine(__ballot_sync(0xFFFFFFFFu, end || (verdict != 0 && !search)), lane);
+            if (sure & ((1u << grp.sub(lane)) - 1u)) search = false;
+        }
+        if (search) {
+            if (!ZC || s_mapped[pb]) sectors += search_sectors(pdeg);
+            const bool found = csr_contains(CsrIndex<kSearch>{padj, nullptr}, 0u, 0ull, pdeg, x);
+            verdict = (found ? rv < thr_found<SOPR>(a.c, t) : rv < thr_notfound<SOPR>(a.c, t)) ? 1 : 0;
         }
         uint32_t first = 0;  // the deciding attempt, from `attempt`
         if (grp.shift) {

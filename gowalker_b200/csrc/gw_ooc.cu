@@ -91,6 +91,7 @@ struct OocState {
     // 2 * nb^2 buckets (unflagged, then kNeedPrev); d_pairs: nb^2 per-pair totals
     uint32_t *d_counts = nullptr, *d_offsets = nullptr, *d_cursor = nullptr, *d_pairs = nullptr;
     uint32_t *d_run_pre = nullptr, *d_run_off = nullptr, *d_nrun = nullptr;
+    OocClock *d_clock = nullptr;  // behind d_nrun
     Decision *d_dec = nullptr, *h_dec = nullptr;  // pinned, mapped: the decision kernels write it in place
     SaState *d_sa = nullptr;  // annealing policy: the held block set
 
@@ -397,7 +398,8 @@ static int ooc_setup(gw_handle *h)
     if ((st = h->cuda(cudaMalloc(&o.d_cursor, nbk * sizeof(uint32_t)), "bucket cursors"))) return st;
     if ((st = h->cuda(cudaMalloc(&o.d_run_pre, (nbk + 1) * sizeof(uint32_t)), "runnable prefix"))) return st;
     if ((st = h->cuda(cudaMalloc(&o.d_run_off, nbk * sizeof(uint32_t)), "runnable offsets"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_nrun, sizeof(uint32_t)), "runnable count"))) return st;
+    if ((st = h->cuda(cudaMalloc(&o.d_nrun, 16 + sizeof(OocClock)), "runnable count"))) return st;
+    o.d_clock = reinterpret_cast<OocClock *>(o.d_nrun + 4);
 
     if ((st = h->cuda(cudaMalloc(&o.d_sa, sizeof(SaState)), "annealing state"))) return st;
     if ((st = h->cuda(cudaHostAlloc((void **)&o.h_dec, sizeof(Decision), cudaHostAllocMapped), "decision"))) return st;
@@ -646,7 +648,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     const bool paths = cfg.record_paths == GW_PATHS_FULL;
     uint64_t h2d = 0, loads = 0, zc_steps = 0, zc_sectors = 0;
     uint32_t iters = 0, launches = 0;
-    float kernel_ms = 0.f, bucket_ms = 0.f;
+    OocClock clock{};
     // GOWALKER_TRACE: per-run phase totals on stderr (install = wait for the
     // staged copy + decode + validation on the compute stream; decision =
     // host time blocked on the decision stream; copy = prefetch uploads)
@@ -670,9 +672,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         cudaEventCreate(&pr[0]);
         cudaEventCreate(&pr[1]);
     }
-    EvRing bring, kring, rring;  // re-bucketing, step kernel, runnable pass (trace)
-    bring.create();
-    kring.create();
+    EvRing rring;  // runnable pass (trace)
     if (trace) rring.create();
     float t_runnable_f = 0.f;
 
@@ -834,24 +834,23 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         const uint32_t c = o.w_cur;
         int e;
         snap_last = c;
-        if ((e = cuda(bring.begin(s, bucket_ms), "event"))) return e;
         if (first && (e = cuda(launch_count(o.w_key[c], o.d_n + c, o.d_counts, num_sms, s), "count"))) return e;
         if (decided && (e = cuda(cudaStreamWaitEvent(s, decided, 0), "decision wait"))) return e;
         if ((e = cuda(launch_plan(o.d_counts, nb, o.d_offsets, o.d_cursor, o.d_pairs, o.d_n + (c ^ 1u), d_ctr, d_err,
-                                  o.dm_snap[c], num_sms, s),
+                                  o.dm_snap[c], o.d_clock, num_sms, s),
                       "bucket plan")))
             return e;
         if ((e = cuda(cudaEventRecord(ev_buck, s), "event"))) return e;
         if ((e = cuda(launch_scatter(o.w_key[c], o.w_ord[c], o.d_n + c, o.d_cursor, o.w_key[c ^ 1], o.w_ord[c ^ 1],
-                                     num_sms, s),
+                                     o.d_clock, num_sms, s),
                       "scatter")))
             return e;
-        if ((e = cuda(bring.end(s), "event"))) return e;
         launches += (nb > 64 ? 3 : 2) + (first ? 1 : 0);
         o.w_cur ^= 1u;  // the sorted index of the live walkers
         return GW_OK;
     };
     if ((st = cuda(cudaMemsetAsync(o.d_counts, 0, nbk * sizeof(uint32_t), s), "memset"))) return st;
+    if ((st = cuda(cudaMemsetAsync(o.d_clock, 0, sizeof(OocClock), s), "memset"))) return st;
     *o.h_n = (uint32_t)nwalkers;
     if ((st = cuda(cudaMemcpyAsync(o.d_n, o.h_n, sizeof(uint32_t), cudaMemcpyHostToDevice, s), "walker count")))
         return st;
@@ -870,6 +869,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     a.run_off = o.d_run_off;
     a.nrun = o.d_nrun;
     a.counts = o.d_counts;
+    a.clock = o.d_clock;
     a.busy_warps = 16u * (uint32_t)num_sms;
     a.paths = paths ? d_paths : nullptr;
     a.stride = stride;
@@ -935,9 +935,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
         a.recs = o.w_rec;
         a.order = o.w_ord[o.w_cur];
         a.keys = o.w_key[o.w_cur];
-        if ((e = cuda(kring.begin(s, kernel_ms), "event"))) return e;
         if ((e = cuda(launch_walk_ooc(a, sopr, coop, o.weighted, grid, s), "walk kernel"))) return e;
-        if ((e = cuda(kring.end(s), "event"))) return e;
         launches += 2;
         return GW_OK;
     };
@@ -946,23 +944,17 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     bool done = false;
     // learned-policy state of this run
     if (policy == GW_POLICY_LEARNED && (st = learned_setup(this))) {
-        kring.destroy();
-        bring.destroy();
         rring.destroy();
         return st;
     }
     if (policy == GW_POLICY_LEARNED) {
         if ((st = cuda(cudaMemsetAsync(o.d_prev_col, 0, sizeof(float) * nb, s), "memset")) ||
             (st = cuda(cudaMemsetAsync(o.d_ema, 0, sizeof(float) * nb, s), "memset"))) {
-            kring.destroy();
-            bring.destroy();
             rring.destroy();
             return st;
         }
     }
     if (policy == GW_POLICY_SA && (st = cuda(cudaMemsetAsync(o.d_sa, 0, sizeof(SaState), s), "memset"))) {
-        kring.destroy();
-        bring.destroy();
         rring.destroy();
         return st;
     }
@@ -1029,8 +1021,6 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     const uint32_t capacity = prefetch ? o.nslots - 1 : o.nslots;
     int staged_block = -1, staged_pos = -1, staging_slot = prefetch ? 0 : -1;
     if (prefetch && o.nslots < 3) {
-        kring.destroy();
-        bring.destroy();
         rring.destroy();
         return fail(GW_ERR_ARG, "prefetch needs a cache of at least 3 blocks (has %u)", o.nslots);
     }
@@ -1058,8 +1048,6 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     // flight, and without it the upload runs beside the scatter.
     if ((st = cuda(cudaStreamCreateWithFlags(&s_run, cudaStreamNonBlocking), "runnable stream")) ||
         (st = cuda(cudaStreamCreateWithFlags(&ds, cudaStreamNonBlocking), "decision stream"))) {
-        kring.destroy();
-        bring.destroy();
         rring.destroy();
         return st;
     }
@@ -1513,6 +1501,8 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
                        "counters D2H")) == GW_OK &&
             (st = cuda(cudaMemcpyAsync(h_ctr + kCtrCount, d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, s),
                        "error word")) == GW_OK &&
+            (st = cuda(cudaMemcpyAsync(&clock, o.d_clock, sizeof(clock), cudaMemcpyDeviceToHost, s), "clock")) ==
+                GW_OK &&
             (st = cuda(cudaEventRecord(ev_stop, s), "event")) == GW_OK)
             st = cuda(cudaStreamSynchronize(s), "run");
     } else {
@@ -1543,12 +1533,8 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     cudaEventDestroy(ev_buck);
     cudaEventDestroy(ev_dec);
     cudaEventDestroy(ev_run);
-    kring.drain(kernel_ms);
-    bring.drain(bucket_ms);
     if (trace) rring.drain(t_runnable_f);
     t_runnable += t_runnable_f;
-    kring.destroy();
-    bring.destroy();
     rring.destroy();
     cudaGetLastError();
     if (trace) {
@@ -1564,6 +1550,8 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     if (st) return st;
     last_hash_sum = h_ctr[kCtrHashSum];
     last_steps = h_ctr[kCtrSteps];
+    const float kernel_ms = (float)(clock.walk_ns * 1e-6);
+    const float bucket_ms = (float)((clock.bucket_ns + clock.scatter_end - clock.plan_start) * 1e-6);
     if (stats) {
         memset(stats, 0, sizeof(*stats));
         stats->steps = h_ctr[kCtrSteps];

@@ -23,6 +23,13 @@
 namespace gw {
 
 
+__device__ __forceinline__ unsigned long long global_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 __device__ __forceinline__ uint32_t block_of(const uint32_t *vs, uint32_t nb, uint32_t v)
 {
     // largest b with vs[b] <= v (vs[nb] = nverts > v)
@@ -83,31 +90,46 @@ __global__ void k_count(const uint32_t *__restrict__ keys, const uint32_t *__res
     }
 }
 
-__global__ void k_scatter(const uint32_t *__restrict__ keys_in, const uint32_t *__restrict__ order_in,
-                          const uint32_t *__restrict__ n_ptr, uint32_t *__restrict__ cursor,
-                          uint32_t *__restrict__ keys_out, uint32_t *__restrict__ order_out)
+// Half the threads an SM holds, so that the runnable pass and the block choice
+// (1,024 threads each) find room beside it instead of behind it: they start 3 us
+// after the plan, not 8.  Four rounds of 32 walkers in flight a warp make up for
+// it (10 us for a million walkers either way).
+__global__ void __launch_bounds__(256) k_scatter(const uint32_t *__restrict__ keys_in,
+                                                 const uint32_t *__restrict__ order_in,
+                                                 const uint32_t *__restrict__ n_ptr, uint32_t *__restrict__ cursor,
+                                                 uint32_t *__restrict__ keys_out, uint32_t *__restrict__ order_out,
+                                                 OocClock *clock)
 {
+    constexpr uint32_t R = 4;
     const uint64_t n = *n_ptr;
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lt = (1u << lane) - 1u;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t base = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull; base < n; base += step) {
-        const uint64_t i = base + lane;
-        uint32_t r = 0, b = kNoBucket;
-        if (i < n) {
-            b = keys_in[i];
-            r = order_in[i];
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x * R;
+    for (uint64_t base = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) & ~31ull) * R; base < n; base += step) {
+        uint32_t r[R], b[R], pos[R];
+        unsigned grp[R];
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k) {
+            const uint64_t i = base + 32 * k + lane;
+            b[k] = i < n ? keys_in[i] : kNoBucket;
+            r[k] = i < n ? order_in[i] : 0u;
         }
-        const unsigned grp = __match_any_sync(0xFFFFFFFFu, b);
-        if (b != kNoBucket) {
-            const uint32_t leader = (uint32_t)(__ffs(grp) - 1);
-            uint32_t pos = 0;
-            if (lane == leader) pos = atomicAdd(&cursor[b], (uint32_t)__popc(grp));
-            pos = __shfl_sync(grp, pos, leader) + (uint32_t)__popc(grp & lt);
-            keys_out[pos] = b;
-            order_out[pos] = r;
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k) {
+            grp[k] = __match_any_sync(0xFFFFFFFFu, b[k]);
+            pos[k] = 0;
+            if (b[k] != kNoBucket && (grp[k] & lt) == 0) pos[k] = atomicAdd(&cursor[b[k]], (uint32_t)__popc(grp[k]));
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k) {
+            const uint32_t at = __shfl_sync(0xFFFFFFFFu, pos[k], __ffs(grp[k]) - 1) + (uint32_t)__popc(grp[k] & lt);
+            if (b[k] != kNoBucket) {
+                keys_out[at] = b[k];
+                order_out[at] = r[k];
+            }
         }
     }
+    if (threadIdx.x == 0) atomicMax(&clock->scatter_end, global_ns());
 }
 
 // One-CTA scans over at most 2^20 entries (nblocks <= 1024).
@@ -163,9 +185,17 @@ __global__ void __launch_bounds__(kScanThreads) k_plan(const uint32_t *__restric
                                                        uint32_t *__restrict__ offsets, uint32_t *__restrict__ cursor,
                                                        uint32_t *__restrict__ pairs, uint32_t *__restrict__ n_out,
                                                        const unsigned long long *__restrict__ ctr,
-                                                       const uint32_t *__restrict__ err, unsigned long long *snap)
+                                                       const uint32_t *__restrict__ err, unsigned long long *snap,
+                                                       OocClock *clock)
 {
     __shared__ uint32_t s_total;
+    if (threadIdx.x == 0) {
+        const unsigned long long now = global_ns();
+        if (clock->walk_start) clock->walk_ns += now - clock->walk_start;
+        if (clock->plan_start) clock->bucket_ns += clock->scatter_end - clock->plan_start;
+        clock->walk_start = 0;
+        clock->plan_start = now;
+    }
     const uint32_t n = 2 * nn;
     if (threadIdx.x <= kCtrCount) {
         snap[threadIdx.x] = threadIdx.x < kCtrCount ? ctr[threadIdx.x] : *err;
@@ -461,7 +491,10 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
     __shared__ unsigned long long s_ws[kWalkThreads / 32][kWsCount];  // per-warp statistics
     const uint32_t nrun = *a.nrun;
     const uint32_t total = a.run_pre[nrun];
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&a.ctr[kCtrRunnable], (unsigned long long)total);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        a.clock->walk_start = global_ns();
+        atomicAdd(&a.ctr[kCtrRunnable], (unsigned long long)total);
+    }
     // slots and claims by the number of walkers, as incore_plan chooses them
     const uint32_t warps = gridDim.x * (kWalkThreads / 32);
     uint32_t slots = 1;
@@ -903,7 +936,7 @@ __global__ void k_combine(const uint32_t *__restrict__ counts, uint32_t nn, uint
 
 cudaError_t launch_plan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
                         uint32_t *n_out, const unsigned long long *ctr, const uint32_t *err, unsigned long long *snap,
-                        int num_sms, cudaStream_t s)
+                        OocClock *clock, int num_sms, cudaStream_t s)
 {
     // many blocks' pair totals are too much for one CTA (8 words a thread at 64
     // blocks, 128 at 256)
@@ -913,14 +946,15 @@ cudaError_t launch_plan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, 
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    k_plan<<<1, kScanThreads, 0, s>>>(counts, nb * nb, offsets, cursor, apart ? nullptr : pairs, n_out, ctr, err, snap);
+    k_plan<<<1, kScanThreads, 0, s>>>(counts, nb * nb, offsets, cursor, apart ? nullptr : pairs, n_out, ctr, err, snap,
+                                    clock);
     return cudaGetLastError();
 }
 
 cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, uint32_t *cursor,
-                           uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s)
+                           uint32_t *keys_out, uint32_t *order_out, OocClock *clock, int num_sms, cudaStream_t s)
 {
-    k_scatter<<<num_sms * 8, 256, 0, s>>>(keys_in, order_in, n, cursor, keys_out, order_out);
+    k_scatter<<<num_sms * 4, 256, 0, s>>>(keys_in, order_in, n, cursor, keys_out, order_out, clock);
     return cudaGetLastError();
 }
 

@@ -24,6 +24,15 @@ constexpr uint32_t kMaxBlocks = 1024;        // block table kept in shared memor
 // absent (lazy mode); such walkers sit in the second half of the buckets.
 constexpr uint32_t kNeedPrev = 0x80000000u;
 
+// Time in the steps and the re-bucketings of a run, kept by the kernels
+// (nanoseconds of the device's clock): four events that take a time hold the
+// compute stream for about 12 us of a 100 us iteration.
+struct OocClock {
+    unsigned long long walk_start, plan_start, scatter_end;  // of the last ones
+    unsigned long long walk_ns;                              // step kernels, start to the plan behind them
+    unsigned long long bucket_ns;                            // plan to the end of the scatter, but for the last
+};
+
 struct OocStepArgs {
     StepConsts c;
     const uint64_t *beg;             // [nverts+1] offsets of every vertex (global edge ids), resident
@@ -48,6 +57,7 @@ struct OocStepArgs {
     uint32_t *lens;
     uint64_t *hashes;
     unsigned long long *ctr;
+    OocClock *clock;
     uint32_t *err;
 };
 
@@ -76,9 +86,9 @@ cudaError_t launch_count(const uint32_t *keys, const uint32_t *n, uint32_t *coun
 // error word into snap[0 .. kCtrCount] (mapped host memory).
 cudaError_t launch_plan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, uint32_t *cursor, uint32_t *pairs,
                         uint32_t *n_out, const unsigned long long *ctr, const uint32_t *err, unsigned long long *snap,
-                        int num_sms, cudaStream_t s);
+                        OocClock *clock, int num_sms, cudaStream_t s);
 cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, const uint32_t *n, uint32_t *cursor,
-                           uint32_t *keys_out, uint32_t *order_out, int num_sms, cudaStream_t s);
+                           uint32_t *keys_out, uint32_t *order_out, OocClock *clock, int num_sms, cudaStream_t s);
 // Buckets are 2 * nb^2: (prev_blk, cur_blk), then the same pairs for walkers
 // flagged kNeedPrev.
 // Changes of the block table since the last step, as kernel arguments: a read of

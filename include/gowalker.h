@@ -147,8 +147,8 @@ typedef struct gw_stats {
     uint64_t zero_copy_steps; /* steps taken in the mapped-host tail mode */
     uint32_t iterations;      /* scheduler iterations */
     uint32_t launches;        /* kernels launched by this run */
-    float kernel_ms;          /* time inside the step kernels (CUDA events; out-of-core untraced
-                                 runs include each iteration's runnable-bucket pass) */
+    float kernel_ms;          /* time inside the step kernels (CUDA events; out-of-core: device clock,
+                                 to the start of the re-bucketing behind each) */
     float total_ms;           /* whole run (CUDA events) */
     uint32_t learned_iterations; /* decisions the learned parts changed or took: forecast evictions,
                                     and the switch to the zero-copy tail */
@@ -159,7 +159,7 @@ typedef struct gw_stats {
     uint32_t kernel_variant;     /* CTAs of an SM the step kernel is built for (in-core) */
     float persist_error;         /* learned: the same error of the forecast without the network
                                     (this iteration's demand carried forward) */
-    float bucket_ms;             /* out-of-core: time re-bucketing walkers (CUDA events) */
+    float bucket_ms;             /* out-of-core: time re-bucketing walkers (device clock) */
     uint32_t walker_chunk;       /* in-core: walkers a warp claims per atomic */
     uint64_t coop_small_steps;   /* hard steps decided from candidate positions (in-core) */
     uint64_t coop_small_attempts;

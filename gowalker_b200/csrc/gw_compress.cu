@@ -154,55 +154,99 @@ bool compress_block(const uint64_t *beg, const uint32_t *csr, uint32_t nv, uint6
     return true;
 }
 
-// One chunk of k ids at byte `pos` of the payload, decoded by the warp from
-// its shared-memory window of the payload words [base, base + kWindowWords):
-// lane 0 takes the first id, lane i < k delta i (its bits read straight from
-// the window), and a warp prefix sum (mod 2^32) rebuilds the ids.  `end` is
-// the byte past the chunks this task may read; a chunk reaching past it is
-// malformed.  A chunk spans at most 3 + 5 + 124 bytes (alignment, code and
-// first id, deltas), so its words lie in
-// [off, off + 35) with off = pos / 4 - base; the caller keeps off <= kSlideAt.
-__device__ __forceinline__ uint64_t decode_chunk_sm(const uint32_t *sm, uint64_t base, uint64_t pos, uint64_t end,
-                                                    uint32_t k, uint32_t lane, uint32_t *__restrict__ row,
-                                                    uint32_t nverts, bool &bad_id, bool &bad)
+// Up to kBatchChunks chunks, `left` ids, from byte `pos` of the payload, decoded
+// by the warp from its shared-memory window of the payload words
+// [base, base + kWindowWords): lane 0 takes a chunk's first id, lane i < 32 delta
+// i (its bits read straight from the window), and a warp prefix sum (mod 2^32)
+// rebuilds the ids.  `end` is the byte past the chunks this task may read; a
+// chunk reaching past it is malformed.  A chunk's place follows from the width
+// byte of the one before, but nothing else does: four at a time take 0.1 us each,
+// one by one 0.35.
+constexpr uint32_t kBatchChunks = 4;
+__device__ __forceinline__ uint64_t decode_chunks_sm(const uint32_t *sm, uint64_t base, uint64_t pos, uint64_t end,
+                                                     uint64_t left, uint32_t lane, uint32_t *__restrict__ row,
+                                                     uint32_t nverts, bool &bad_id, bool &bad)
 {
-    const uint32_t off = (uint32_t)((pos >> 2) - base);
-    const uint32_t sh = (uint32_t)(pos & 3u) * 8u;
-    const uint64_t head = (((uint64_t)sm[off + 1] << 32) | sm[off]) >> sh;
-    const uint32_t code = (uint32_t)head & 0xFFu, w = chunk_width(code), fb = chunk_first_bytes(code);
-    const uint32_t zz = chunk_plain(code) ? 0u : 1u;  // zigzag-coded deltas
-    const uint64_t size = chunk_bytes(code, k);
-    if (pos + size > end) {
-        bad = true;
-        return pos;
-    }
-    const uint32_t bp = lane ? (lane - 1) * w : 0u;
-    const uint32_t bo = sh + 8u + 8u * fb + bp;
-    const uint32_t q = off + (bo >> 5);
-    uint32_t x = 0;
-    if (lane == 0) {
-        x = (uint32_t)((head >> 8) & (0xFFFFFFFFull >> (32u - 8u * fb)));
-    } else if (lane < k && w != 0) {
-        const uint64_t acc = ((uint64_t)sm[q + 1] << 32) | sm[q];
-        const uint64_t mask = (w == 32) ? 0xFFFFFFFFull : ((1ull << w) - 1);
-        const uint32_t z = (uint32_t)((acc >> (bo & 31u)) & mask);
-        x = zz ? (z >> 1) ^ (0u - (z & 1u)) : z;
+    uint32_t x[kBatchChunks], ids[kBatchChunks];
+#pragma unroll
+    for (uint32_t i = 0; i < kBatchChunks; ++i) {
+        const uint32_t k = left > kChunkIds * i ? (uint32_t)min((uint64_t)kChunkIds, left - kChunkIds * i) : 0u;
+        x[i] = ids[i] = 0;
+        if (k == 0 || bad) continue;
+        if (pos + 2 > end) {
+            bad = true;
+            continue;
+        }
+        const uint32_t off = (uint32_t)((pos >> 2) - base);
+        const uint32_t sh = (uint32_t)(pos & 3u) * 8u;
+        const uint64_t head = (((uint64_t)sm[off + 1] << 32) | sm[off]) >> sh;
+        const uint32_t code = (uint32_t)head & 0xFFu, w = chunk_width(code), fb = chunk_first_bytes(code);
+        const uint32_t zz = chunk_plain(code) ? 0u : 1u;  // zigzag-coded deltas
+        const uint64_t size = chunk_bytes(code, k);
+        if (pos + size > end) {
+            bad = true;
+            continue;
+        }
+        ids[i] = k;
+        pos += size;
+        const uint32_t bo = sh + 8u + 8u * fb + (lane ? (lane - 1) * w : 0u);
+        const uint32_t q = off + (bo >> 5);
+        if (lane == 0) {
+            x[i] = (uint32_t)((head >> 8) & (0xFFFFFFFFull >> (32u - 8u * fb)));
+        } else if (lane < k && w != 0) {
+            const uint64_t acc = ((uint64_t)sm[q + 1] << 32) | sm[q];
+            const uint64_t mask = (w == 32) ? 0xFFFFFFFFull : ((1ull << w) - 1);
+            const uint32_t z = (uint32_t)((acc >> (bo & 31u)) & mask);
+            x[i] = zz ? (z >> 1) ^ (0u - (z & 1u)) : z;
+        }
     }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= (uint32_t)o) x += y;
+#pragma unroll
+        for (uint32_t i = 0; i < kBatchChunks; ++i) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x[i], o);
+            if (lane >= (uint32_t)o) x[i] += y;
+        }
     }
-    if (lane < k) {
-        row[lane] = x;
-        bad_id |= x >= nverts;
-    }
-    return pos + size;
+#pragma unroll
+    for (uint32_t i = 0; i < kBatchChunks; ++i)
+        if (lane < ids[i]) {
+            row[kChunkIds * i + lane] = x[i];
+            bad_id |= x[i] >= nverts;
+        }
+    return pos;
 }
 
-constexpr uint32_t kWindowWords = 1024 + 36;  // a warp's shared-memory window of the payload (4.1 KB)
-constexpr uint32_t kSlideAt = 1024;           // a chunk starting past this word of the window slides it
+// A warp's shared-memory window of the payload (4.3 KB), filled 16 bytes a lane.
+// A chunk spans at most 5 + 124 bytes, so kBatchChunks of them from byte `pos`
+// on lie in the 131 words from pos / 4, and one word more is read: kSlideAt is
+// the last word of the window that they may start in.
+constexpr uint32_t kWindowWords = 1088;
+constexpr uint32_t kSlideAt = kWindowWords - 132;
+// Payload words [base, base + n) to the window; base and n are multiples of 4.
+// Three loads of a lane in flight: one after another, 33 of a word each were
+// 24 us of a 34 us decode.
+__device__ __forceinline__ void fill_window(uint32_t *sm, const uint32_t *__restrict__ pay_words, uint64_t base,
+                                            uint32_t n, uint64_t limit, uint32_t lane)
+{
+    constexpr uint32_t R = 3;
+    for (uint32_t i0 = 4 * lane; i0 < n; i0 += 128 * R) {
+        uint4 r[R];
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k) {
+            const uint32_t i = i0 + 128 * k;
+            r[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (i < n && base + i < limit) r[k] = __ldg(reinterpret_cast<const uint4 *>(pay_words + base + i));
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < R; ++k) {
+            const uint32_t i = i0 + 128 * k;
+            if (i < n) *reinterpret_cast<uint4 *>(sm + i) = r[k];
+        }
+    }
+}
 constexpr uint32_t kDecodeThreads = 256;
+constexpr uint32_t kDecodeCtas = 3;  // of an SM
 
 // Vertex v of a block lies at beg[v] + kVertexWeight * v on the line that tasks
 // cut: a batch of 32 vertices weighs what 128 ids do, whether it has ids or not.
@@ -247,13 +291,13 @@ __device__ __forceinline__ uint32_t warp_first_vertex(const uint64_t *__restrict
 // each were one warp's work, a chain of 1,024 chunks, about 80 us for each of a
 // block's four pieces whatever its size; by ids alone, 27 us, a few ids spread
 // over hundreds of vertices without any; by both, 22 us.
-__global__ void __launch_bounds__(kDecodeThreads)
+__global__ void __launch_bounds__(kDecodeThreads, 4)
     k_decode_block(const uint8_t *__restrict__ src, uint64_t split_off, uint64_t payload_off, uint64_t payload_bytes,
                    uint32_t nv, const uint64_t *__restrict__ beg, uint32_t v0, uint64_t e0, uint64_t ne,
                    uint32_t nverts, uint32_t *__restrict__ out, uint32_t *err, uint32_t v_lo, uint32_t v_hi,
                    uint64_t e_lo, uint64_t e_hi, uint32_t per, uint32_t g_lo, uint32_t g_hi)
 {
-    __shared__ uint32_t s_win[kDecodeThreads / 32][kWindowWords];
+    __shared__ __align__(16) uint32_t s_win[kDecodeThreads / 32][kWindowWords];
     uint32_t *sm = s_win[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -266,13 +310,13 @@ __global__ void __launch_bounds__(kDecodeThreads)
     const uint64_t ntasks = nbt + (g_hi - g_lo);
     bool bad_id = false, bad = false;
     uint64_t base = ~0ull;  // first payload word in the window (~0: empty)
-    // make the window hold the chunk at byte `pos` (warp-uniform)
+    // make the window hold the chunks from byte `pos` on (warp-uniform)
     auto cover = [&](uint64_t pos) {
         const uint64_t w = pos >> 2;
         if (base != ~0ull && w >= base && w - base <= kSlideAt) return;
         __syncwarp();  // every lane is done with the old window
-        base = w;
-        for (uint32_t i = lane; i < kWindowWords; i += 32) sm[i] = (base + i < limit) ? __ldg(pay_words + base + i) : 0u;
+        base = w & ~3ull;
+        fill_window(sm, pay_words, base, kWindowWords, limit, lane);
         __syncwarp();
     };
     for (uint64_t task = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < ntasks; task += nwarps) {
@@ -293,15 +337,11 @@ __global__ void __launch_bounds__(kDecodeThreads)
             const uint64_t nch = (d + kChunkIds - 1) / kChunkIds;
             const uint64_t c1 = min(nch, (uint64_t)c0 + kChunkIds);
             bool vbad = false;
-            for (uint64_t c = c0; c < c1 && !vbad; ++c) {
-                const uint32_t k = (uint32_t)min((uint64_t)kChunkIds, d - c * kChunkIds);
-                if (pos + 2 > payload_bytes) {
-                    vbad = true;
-                    break;
-                }
+            const uint64_t ids_end = min(d, c1 * kChunkIds);
+            for (uint64_t i = (uint64_t)c0 * kChunkIds; i < ids_end && !vbad; i += kBatchChunks * kChunkIds) {
                 cover(pos);
-                pos = decode_chunk_sm(sm, base, pos, payload_bytes, k, lane, out + (b0 - e0) + c * kChunkIds, nverts,
-                                      bad_id, vbad);
+                pos = decode_chunks_sm(sm, base, pos, payload_bytes, ids_end - i, lane, out + (b0 - e0) + i, nverts,
+                                       bad_id, vbad);
             }
             bad |= vbad;
             continue;
@@ -330,15 +370,14 @@ __global__ void __launch_bounds__(kDecodeThreads)
                 continue;
             }
             // every chunk of the batch reads words [p0 / 4, p1 / 4 + 2)
-            const uint64_t b_base = p0 >> 2, nwords = ((p1 + 3) >> 2) - b_base + 2;
+            const uint64_t b_base = (p0 >> 2) & ~3ull, nwords = (((p1 + 3) >> 2) - b_base + 2 + 3) & ~3ull;
             if (nwords <= kWindowWords) {
                 // ---- the whole batch in the window: one fill, then each lane
                 // decodes its own vertex when it has one chunk (most do), and
                 // the warp decodes the chunks of the batch's larger vertices
                 __syncwarp();
                 base = b_base;
-                for (uint32_t i = lane; i < nwords; i += 32)
-                    sm[i] = (base + i < limit) ? __ldg(pay_words + base + i) : 0u;
+                fill_window(sm, pay_words, base, (uint32_t)nwords, limit, lane);
                 __syncwarp();
                 const bool range_ok = !mine || (mb1 >= mb0 && mb0 >= e0 && mb1 - e0 <= ne);
                 bad |= !range_ok;
@@ -381,17 +420,10 @@ __global__ void __launch_bounds__(kDecodeThreads)
                     uint64_t pos = __shfl_sync(0xFFFFFFFFu, mpos, j);
                     const uint64_t b0 = __shfl_sync(0xFFFFFFFFu, mb0, j);
                     const uint64_t dj = __shfl_sync(0xFFFFFFFFu, d, j);
-                    const uint64_t nch = (dj + kChunkIds - 1) / kChunkIds;
-                    bool vbad = false;
-                    for (uint64_t c = 0; c < nch && !vbad; ++c) {
-                        const uint32_t k = (uint32_t)min((uint64_t)kChunkIds, dj - c * kChunkIds);
-                        if (pos < p0 || pos + 2 > p1) {
-                            vbad = true;
-                            break;
-                        }
-                        pos = decode_chunk_sm(sm, base, pos, p1, k, lane, out + (b0 - e0) + c * kChunkIds, nverts,
-                                              bad_id, vbad);
-                    }
+                    bool vbad = pos < p0;
+                    for (uint64_t i = 0; i < dj && !vbad; i += kBatchChunks * kChunkIds)
+                        pos = decode_chunks_sm(sm, base, pos, p1, dj - i, lane, out + (b0 - e0) + i, nverts, bad_id,
+                                               vbad);
                     bad |= vbad;
                 }
                 base = ~0ull;  // the window holds this batch's words only
@@ -408,16 +440,10 @@ __global__ void __launch_bounds__(kDecodeThreads)
                 const uint64_t d = b1 - b0;
                 const uint64_t nch = (d + kChunkIds - 1) / kChunkIds;
                 if (nch > kChunkIds) continue;  // decoded by its split groups
-                bool vbad = false;
-                for (uint64_t c = 0; c < nch && !vbad; ++c) {
-                    const uint32_t k = (uint32_t)min((uint64_t)kChunkIds, d - c * kChunkIds);
-                    if (pos < p0 || pos + 2 > p1) {
-                        vbad = true;
-                        break;
-                    }
+                bool vbad = pos < p0;
+                for (uint64_t i = 0; i < d && !vbad; i += kBatchChunks * kChunkIds) {
                     cover(pos);
-                    pos = decode_chunk_sm(sm, base, pos, p1, k, lane, out + (b0 - e0) + c * kChunkIds, nverts, bad_id,
-                                          vbad);
+                    pos = decode_chunks_sm(sm, base, pos, p1, d - i, lane, out + (b0 - e0) + i, nverts, bad_id, vbad);
                 }
                 bad |= vbad;
             }
@@ -438,12 +464,13 @@ cudaError_t launch_decode_block(const uint8_t *src, const CompressedBlock &cb, u
     if (ids == 0) return cudaSuccess;
     // one task a warp as far as they go: a task of 128 ids costs its search
     // for the first vertex and little more
-    const uint64_t warps = (uint64_t)num_sms * 4 * (kDecodeThreads / 32);
+    const uint64_t all = (uint64_t)num_sms * kDecodeCtas * (kDecodeThreads / 32);
+    const uint64_t warps = all - std::min<uint64_t>(groups, all / 2);  // the others take a split group each
     const uint64_t line = ids + (uint64_t)kVertexWeight * (cb.piece_v[k1] - cb.piece_v[k0]);
     const uint32_t per = (uint32_t)std::min<uint64_t>(1024, std::max<uint64_t>(128, (line + warps - 1) / warps));
     const uint64_t tasks = (line + per - 1) / per + groups;
     const uint64_t need = (tasks + kDecodeThreads / 32 - 1) / (kDecodeThreads / 32);
-    k_decode_block<<<(int)std::min<uint64_t>(need, (uint64_t)num_sms * 4), kDecodeThreads, 0, s>>>(
+    k_decode_block<<<(int)std::min<uint64_t>(need, (uint64_t)num_sms * kDecodeCtas), kDecodeThreads, 0, s>>>(
         src, cb.split_off, cb.payload_off, cb.payload_bytes, nv, beg, v0, e0, ne, nverts, out, err, cb.piece_v[k0],
         cb.piece_v[k1], cb.piece_e[k0], cb.piece_e[k1], per, cb.piece_g[k0], cb.piece_g[k1]);
     return cudaGetLastError();

@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) k_scatter(const uint32_t *__restrict__ ke
     if (threadIdx.x == 0) atomicMax(&clock->scatter_end, global_ns());
 }
 
-// One-CTA scans over at most 2^20 entries (nblocks <= 1024).
+// One-CTA scans over at most 2^21 entries (nblocks <= 1024).
 constexpr int kScanThreads = 1024;
 
 
@@ -325,9 +325,10 @@ __device__ __forceinline__ unsigned long long warp_max(unsigned long long x)
 __device__ __forceinline__ unsigned long long warp_min(unsigned long long x) { return ~warp_max(~x); }
 
 struct CachedList {
-    uint16_t block[kMaxBlocks];  // an argument: mapped memory would be read behind the copy in flight
+    uint16_t block[kMaxBlocks];  // an argument: no read of mapped host memory on the decision's path
 };
-__global__ void __launch_bounds__(1024) k_schedule(const uint32_t *__restrict__ all_counts,
+// 32 registers: with 64 it waits for an SM of its own.
+__global__ void __launch_bounds__(1024, 2) k_schedule(const uint32_t *__restrict__ all_counts,
                                                    const uint32_t *__restrict__ live, uint32_t nb,
                                                    const __grid_constant__ CachedList cached, uint32_t ncached,
                                                    uint32_t nslots, uint32_t zero_threshold,

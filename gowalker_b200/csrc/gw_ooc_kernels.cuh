@@ -91,8 +91,8 @@ cudaError_t launch_scatter(const uint32_t *keys_in, const uint32_t *order_in, co
                            uint32_t *keys_out, uint32_t *order_out, OocClock *clock, int num_sms, cudaStream_t s);
 // Buckets are 2 * nb^2: (prev_blk, cur_blk), then the same pairs for walkers
 // flagged kNeedPrev.
-// Changes of the block table since the last step, as kernel arguments: a read of
-// mapped host memory waits behind the block copy in flight (60 us and more).
+// Changes of the block table since the last step, as kernel arguments: the pass
+// neither reads host memory nor waits for a copy of the table.
 struct TablePatch {
     static constexpr uint32_t kMax = 4;
     uint32_t n;

@@ -350,9 +350,10 @@ __global__ void __launch_bounds__(kDecodeThreads, 4)
         uint32_t vb = warp_first_vertex(beg + v0, v_lo, v_hi, line0 + task * per, lane);
         for (; vb < v_hi; vb += 32) {
             const uint32_t nvt = min(32u, v_hi - vb);
-            uint64_t mpos = 0, mb0 = 0, mb1 = 0;
+            uint64_t mpos = 0, mnext = 0, mb0 = 0, mb1 = 0;
             if (lane < nvt) {
                 mpos = __ldg(voff + vb + lane);
+                mnext = __ldg(voff + vb + lane + 1);
                 mb0 = __ldg(beg + v0 + vb + lane);
                 mb1 = __ldg(beg + v0 + vb + lane + 1);
             }
@@ -364,7 +365,7 @@ __global__ void __launch_bounds__(kDecodeThreads, 4)
             // the batch's payload: [first vertex's offset, past its last vertex's)
             const uint32_t last = 31u - (uint32_t)__clz((int)ours);
             const uint64_t p0 = __shfl_sync(0xFFFFFFFFu, mpos, 0);
-            const uint64_t p1 = __ldg(voff + vb + last + 1);
+            const uint64_t p1 = __shfl_sync(0xFFFFFFFFu, mnext, last);
             if (p1 < p0 || p1 > payload_bytes) {
                 bad = true;
                 continue;

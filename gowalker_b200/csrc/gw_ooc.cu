@@ -870,7 +870,9 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
     a.nrun = o.d_nrun;
     a.counts = o.d_counts;
     a.clock = o.d_clock;
-    a.busy_warps = 16u * (uint32_t)num_sms;
+    // 60,000 walkers a step: 16 / 24 / 32 / 48 / 64 warps an SM 67.4 / 66.4 / 65.0 /
+    // 65.4 / 64.6 ms a run (half as many walkers a warp, two attempts each)
+    a.busy_warps = 32u * (uint32_t)num_sms;
     a.paths = paths ? d_paths : nullptr;
     a.stride = stride;
     a.out_base = wid_first;

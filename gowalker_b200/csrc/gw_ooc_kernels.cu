@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(kScanThreads) k_runnable(const uint32_t *__res
 // One CTA on the path from a plan to the next block's copy.  Up to
 // kSchedShared blocks the counts come into shared memory in one round trip, and
 // the choices are reduced by shuffles, not by an atomic for every bucket: 7.5 us
-// at 64 blocks, 12 before.
+// at 24 blocks, 12 before.
 constexpr uint32_t kSchedShared = 64;  // 16 KB of counts
 __device__ __forceinline__ unsigned long long warp_max(unsigned long long x)
 {

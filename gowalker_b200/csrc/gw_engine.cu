@@ -39,6 +39,21 @@ int gw_handle::cuda(cudaError_t e, const char *what)
     return fail(st, "%s: %s", what, cudaGetErrorString(e));
 }
 
+int gw_handle::dev_alloc(void **p, uint64_t bytes, const char *what)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && d_index) {
+        cudaGetLastError();
+        cudaStreamSynchronize(s_compute);
+        cudaFree(d_index);
+        d_index = nullptr;
+        index_cap = 0;
+        index_ready = false;
+        e = cudaMalloc(p, bytes);
+    }
+    return cuda(e, what);
+}
+
 void gw::consts_from_config(const gw_config &c, StepConsts &k)
 {
     k.maxhops = c.maxhops;
@@ -248,7 +263,7 @@ int gw_handle::upload_whole_graph(cudaStream_t s, uint64_t *h2d)
     int st;
     if (!own_beg) {
         const uint64_t beg_bytes = (((uint64_t)nverts + 1) * sizeof(uint64_t) + 255) & ~255ull;
-        if ((st = cuda(cudaMalloc(&own_beg, beg_bytes + (nedges ? nedges : 1) * sizeof(uint32_t)), "graph"))) return st;
+        if ((st = dev_alloc(own_beg, beg_bytes + (nedges ? nedges : 1) * sizeof(uint32_t), "graph"))) return st;
         own_csr = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(own_beg) + beg_bytes);
     }
     uint64_t bytes = 0;
@@ -270,7 +285,7 @@ int gw_handle::upload_whole_graph(cudaStream_t s, uint64_t *h2d)
         }
     }
     if (weighted && !device_graph) {
-        if (!own_w && (st = cuda(cudaMalloc(&own_w, (nedges ? nedges : 1) * sizeof(float)), "edge weights")))
+        if (!own_w && (st = dev_alloc(own_w, (nedges ? nedges : 1) * sizeof(float), "edge weights")))
             return st;
         for (uint32_t b = 0; b < nblocks; ++b) {
             const uint64_t ne = eblocks[b + 1] - eblocks[b];
@@ -301,7 +316,7 @@ int gw_handle::ensure_outputs()
         d_hashes = nullptr;
         d_lens = nullptr;
         cap_walkers = 0;
-        if ((st = cuda(cudaMalloc(&d_hashes, n * (sizeof(uint64_t) + sizeof(uint32_t))), "path hashes and lengths")))
+        if ((st = dev_alloc(d_hashes, n * (sizeof(uint64_t) + sizeof(uint32_t)), "path hashes and lengths")))
             return st;
         d_lens = reinterpret_cast<uint32_t *>(d_hashes + n);
         cap_walkers = n;
@@ -312,7 +327,7 @@ int gw_handle::ensure_outputs()
         if (need > cap_path_words) {
             cudaFree(d_paths);
             d_paths = nullptr;
-            if ((st = cuda(cudaMalloc(&d_paths, need * sizeof(uint32_t)), "paths"))) return st;
+            if ((st = dev_alloc(d_paths, need * sizeof(uint32_t), "paths"))) return st;
             cap_path_words = need;
         }
         path_stride = stride;
@@ -570,12 +585,12 @@ int gw_handle::validate_graph(cudaStream_t s)
 int gw_handle::build_alias(cudaStream_t s)
 {
     int st;
-    if (!d_alias && (st = cuda(cudaMalloc(&d_alias, (nedges ? nedges : 1) * sizeof(AliasEntry)), "alias tables")))
+    if (!d_alias && (st = dev_alloc(d_alias, (nedges ? nedges : 1) * sizeof(AliasEntry), "alias tables")))
         return st;
     double *pd = nullptr;
     uint32_t *q = nullptr;
-    if ((st = cuda(cudaMalloc(&pd, (nedges ? nedges : 1) * sizeof(double)), "alias scratch"))) return st;
-    if ((st = cuda(cudaMalloc(&q, (2 * (nedges ? nedges : 1) + nverts + 2) * sizeof(uint32_t)), "alias scratch"))) {
+    if ((st = dev_alloc(pd, (nedges ? nedges : 1) * sizeof(double), "alias scratch"))) return st;
+    if ((st = dev_alloc(q, (2 * (nedges ? nedges : 1) + nverts + 2) * sizeof(uint32_t), "alias scratch"))) {
         cudaFree(pd);
         return st;
     }
@@ -609,17 +624,7 @@ int gw_handle::run_incore(gw_stats *stats)
     if (weighted) {
         if (cfg.algorithm != GW_NODE2VEC)
             return fail(GW_ERR_ARG, "weighted walks are Node2vec walks (algorithm %u given)", cfg.algorithm);
-        st = alias_ready ? GW_OK : build_alias(s);
-        if (st == GW_ERR_NOMEM && d_index) {
-            // the tables come before the index
-            cudaStreamSynchronize(s);
-            cudaFree(d_index);
-            d_index = nullptr;
-            index_cap = 0;
-            index_ready = false;
-            st = build_alias(s);
-        }
-        if (st) return st;
+        if (!alias_ready && (st = build_alias(s))) return st;
     }
     IncoreArgs a{};
     consts_from_config(cfg, a.c);
@@ -656,8 +661,8 @@ int gw_handle::run_incore(gw_stats *stats)
         HopState hs{};
         const uint64_t n = nwalkers;
         int rc = GW_OK;
-        if ((rc = cuda(cudaMalloc(&hs.prev, n * 4), "hop state")) || (rc = cuda(cudaMalloc(&hs.cur, n * 4), "hop state")) ||
-            (rc = cuda(cudaMalloc(&hs.hop, n * 4), "hop state")) || (rc = cuda(cudaMalloc(&hs.hash, n * 8), "hop state"))) {
+        if ((rc = dev_alloc(hs.prev, n * 4, "hop state")) || (rc = dev_alloc(hs.cur, n * 4, "hop state")) ||
+            (rc = dev_alloc(hs.hop, n * 4, "hop state")) || (rc = dev_alloc(hs.hash, n * 8, "hop state"))) {
             cudaFree(hs.prev);
             cudaFree(hs.cur);
             cudaFree(hs.hop);
@@ -705,7 +710,7 @@ int gw_handle::run_incore(gw_stats *stats)
         return GW_OK;
     }
     const IncorePlan plan = incore_plan(nwalkers, sopr, a.paths != nullptr, coop, weighted, index_ready,
-                                        (int)cfg.blockpergrid, num_sms);
+                                        sure_steps(sopr, a.c), (int)cfg.blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
     const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);  // with the error word

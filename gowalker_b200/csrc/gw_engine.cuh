@@ -86,6 +86,14 @@ struct gw_handle {
 
     int fail(int status, const char *fmt, ...);
     int cuda(cudaError_t e, const char *what);
+    // Device memory; the index of a resident CSR, which walks can do without,
+    // gives way to anything that they cannot.
+    int dev_alloc(void **p, uint64_t bytes, const char *what);
+    template <class T>
+    int dev_alloc(T *&p, uint64_t bytes, const char *what)
+    {
+        return dev_alloc((void **)&p, bytes, what);
+    }
     int init_device();
     void release();
     uint64_t graph_bytes() const;

@@ -7,7 +7,6 @@
 namespace gw {
 
 constexpr int kWalkThreads = 256;   // threads per CTA of the walk kernels
-constexpr uint32_t kChunk = 64;     // walkers a warp of the out-of-core step claims per atomic
 
 // Work / statistics counters of one run (device, zeroed per run).
 enum Counter : int {
@@ -169,8 +168,8 @@ struct IncorePlan {
     uint32_t ctas_per_sm;   // the kernel's register cap: CTAs of an SM it is built for
 };
 // `grid` CTAs as asked for, or (0) as many as are resident at once.
-IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, int grid,
-                       int num_sms);
+IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, bool sure,
+                       int grid, int num_sms);
 // a.alias set: weighted Node2vec.
 cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s);
 
@@ -192,6 +191,9 @@ inline bool needs_coop(uint32_t algo, const StepConsts &c)
 {
     return algo != 0u || c.n2v_maxv > 8.0f * c.n2v_minv;
 }
+// Whether every Node2vec trial accepts: 1/p, 1/q and 1 are one value, which no
+// rand value exceeds.
+inline bool sure_steps(bool sopr, const StepConsts &c) { return !sopr && c.n2v_maxv == c.n2v_minv; }
 // One pass over a resident CSR before any walk reads it: error bits for
 // offsets that are not monotone within [0, nedges] and ids >= nverts, and, in
 // the same pass, the vertex index (verts null: none) with a place for every

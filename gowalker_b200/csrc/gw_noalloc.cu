@@ -185,7 +185,8 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     const bool sopr = cfg->algorithm != GW_NODE2VEC;
     const bool coop = needs_coop(cfg->algorithm, a.c);
     const IncorePlan plan =
-        incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, false, (int)cfg->blockpergrid, num_sms);
+        incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, false, sure_steps(sopr, a.c),
+                    (int)cfg->blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
     e = launch_walk_incore(a, sopr, coop, plan.grid, s);

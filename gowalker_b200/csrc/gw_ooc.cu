@@ -363,10 +363,10 @@ static int ooc_setup(gw_handle *h)
     o.nslots = (uint32_t)ns;
     int st;
     for (uint32_t i = 0; cstage && i < o.nstage; ++i)
-        if ((st = h->cuda(cudaMalloc(&o.d_cstage[i], cstage), "compressed-block buffer"))) return st;
+        if ((st = h->dev_alloc(o.d_cstage[i], cstage, "compressed-block buffer"))) return st;
     beg_bytes = ((uint64_t)h->nverts + 1) * 8;
-    if ((st = h->cuda(cudaMalloc(&o.d_beg, beg_bytes), "vertex offsets"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.slot_csr, o.nslots * o.slot_stride_words * 4), "slot neighbours"))) return st;
+    if ((st = h->dev_alloc(o.d_beg, beg_bytes, "vertex offsets"))) return st;
+    if ((st = h->dev_alloc(o.slot_csr, o.nslots * o.slot_stride_words * 4, "slot neighbours"))) return st;
     if ((st = h->cuda(cudaMalloc((void **)&o.d_blk_csr, 2 * nb * sizeof(void *)), "block table"))) return st;
     if ((st = h->cuda(cudaMallocHost((void **)&o.h_blk_csr, 2 * nb * sizeof(void *)), "block table"))) return st;
     for (int k = 0; k < 2; ++k) {
@@ -428,10 +428,10 @@ static int ooc_walkers(gw_handle *h)
             o.w_ord[i] = o.w_key[i] = nullptr;
         }
         int st;
-        if ((st = h->cuda(cudaMalloc(&o.w_rec, h->nwalkers * sizeof(WalkerRec)), "walker records"))) return st;
+        if ((st = h->dev_alloc(o.w_rec, h->nwalkers * sizeof(WalkerRec), "walker records"))) return st;
         for (int i = 0; i < 2; ++i) {
-            if ((st = h->cuda(cudaMalloc(&o.w_ord[i], h->nwalkers * sizeof(uint32_t)), "walker order"))) return st;
-            if ((st = h->cuda(cudaMalloc(&o.w_key[i], h->nwalkers * sizeof(uint32_t)), "walker buckets"))) return st;
+            if ((st = h->dev_alloc(o.w_ord[i], h->nwalkers * sizeof(uint32_t), "walker order"))) return st;
+            if ((st = h->dev_alloc(o.w_key[i], h->nwalkers * sizeof(uint32_t), "walker buckets"))) return st;
         }
         o.w_cap = h->nwalkers;
     }

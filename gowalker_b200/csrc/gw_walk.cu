@@ -2,7 +2,7 @@
 //
 // In-core kernel: one persistent grid sized to fill the SMs.  Each lane owns
 // one walker at a time and takes it to the end; a warp claims walker ids in
-// chunks of kChunk with one atomic and hands them to its idle lanes, so lanes
+// claims of a few with one atomic and hands them to its idle lanes, so lanes
 // whose walks end early (SOPR termination, dead ends) pick up new walkers
 // instead of idling -- the work-stealing loop that replaces the reference's
 // grid-stride loop (gpu/gpuwalk.hpp:200) and its one-walker-per-thread
@@ -49,8 +49,15 @@ __host__ __device__ constexpr int walk_ctas(bool sopr, bool coop) { return coop 
 // walkers than lanes several lanes share one (Group); runs that fill the lanes
 // are bound by instructions, and groups at their end alone lose (n2v_corpus-like
 // runs 1.70 / 1.88 ms without / with).
-template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX, bool GROUPS>
-__global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_incore(const __grid_constant__ IncoreArgs a)
+//
+// SURE: every trial accepts (p = q = 1, first-order walks): no verdict, no
+// search, nothing of the previous vertex, and no groups, which only save
+// attempts that reject (3,878 walkers of length 80: 0.15 ms, 0.20 with groups;
+// 200,000 of length 40: 0.20 ms, 0.25 with the verdict).  8 CTAs an SM are 8 %
+// slower on a million walkers.
+template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX, bool GROUPS, bool SURE>
+__global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
+    k_walk_incore(const __grid_constant__ IncoreArgs a)
 {
     __shared__ uint32_t s_iv[COOP ? kWalkThreads / 32 : 1][kCoopScratchWords];  // scratch of warp_first_accept
     __shared__ unsigned long long s_ws[kWalkThreads / 32][kWsCount];  // per-warp statistics
@@ -101,7 +108,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
     for (;;) {
         // Hand walkers to idle groups.
         for (;;) {
-            const unsigned need = __ballot_sync(0xFFFFFFFFu, !active && (!GROUPS || (lane >> grp.shift) < a.slots));
+            const unsigned need = __ballot_sync(0xFFFFFFFFu, !active && (!(GROUPS || SURE) || (lane >> grp.shift) < a.slots));
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 unsigned long long base = 0;
@@ -262,10 +269,11 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP)) k_walk_in
                 if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
             }
             x = __ldg(csr + head + col);
-            if (!GROUPS || (!end && att < kMaxAttempts)) verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
+            if (SURE) verdict = 1;
+            else if (!GROUPS || (!end && att < kMaxAttempts)) verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
             // the record of a vertex that is, or may be, the next one
             if (verdict != 0 && !last && x < a.nverts) vx = load_vertex<INDEX>(a, x);
-            if (verdict < 0)
+            if (!SURE && verdict < 0)
                 verdict = csr_contains(ix, pbucket, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
                                                                     : rv < thr_notfound<SOPR>(a.c, t);
         }
@@ -457,28 +465,29 @@ cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t
     return cudaGetLastError();
 }
 
-template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX>
+template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX, bool SURE>
 static int resident_grid(int num_sms)
 {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, INDEX, false>,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, INDEX, false, SURE>,
                                                   kWalkThreads, 0);
     return (per_sm < 1 ? 1 : per_sm) * num_sms;
 }
 
 // f called with the kernel's template arguments as compile-time constants.
 template <class F>
-static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool index, F &&f)
+static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool index, bool sure, F &&f)
 {
-    const auto paths_index = [&](auto s, auto c, auto w) {
-        if (paths)
-            return index ? f(s, std::true_type{}, c, w, std::true_type{}) : f(s, std::true_type{}, c, w, std::false_type{});
-        return index ? f(s, std::false_type{}, c, w, std::true_type{}) : f(s, std::false_type{}, c, w, std::false_type{});
+    using yes = std::true_type;
+    using no = std::false_type;
+    const auto paths_index = [&](auto s, auto c, auto w, auto u) {
+        if (paths) return index ? f(s, yes{}, c, w, yes{}, u) : f(s, yes{}, c, w, no{}, u);
+        return index ? f(s, no{}, c, w, yes{}, u) : f(s, no{}, c, w, no{}, u);
     };
-    if (weighted) return paths_index(std::false_type{}, std::false_type{}, std::true_type{});
-    if (sopr) return paths_index(std::true_type{}, std::true_type{}, std::false_type{});  // SOPR steps get hard
-    return coop ? paths_index(std::false_type{}, std::true_type{}, std::false_type{})
-                : paths_index(std::false_type{}, std::false_type{}, std::false_type{});
+    if (weighted) return sure ? paths_index(no{}, no{}, yes{}, yes{}) : paths_index(no{}, no{}, yes{}, no{});
+    if (sopr) return paths_index(yes{}, yes{}, no{}, no{});  // SOPR steps get hard
+    if (sure) return paths_index(no{}, no{}, no{}, yes{});
+    return coop ? paths_index(no{}, yes{}, no{}, no{}) : paths_index(no{}, no{}, no{}, no{});
 }
 
 // Slots and claims by the number of walkers, which is all that decides them:
@@ -491,30 +500,33 @@ static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool in
 //   needed share the walkers; later waves claim eight at a time, which evens
 //   out the end of the run (600,000 walkers: 1.75 ms at 8, 1.82 at 32, 1.98 at
 //   64; weighted 200,000: 0.67 / 0.77 / 0.76; hard Node2vec steps 3.25 / 4.44
-//   / 4.62; SOPR on 16.8 M walkers: no difference).
-IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, int grid,
-                       int num_sms)
+//   / 4.62; SOPR on 16.8 M walkers: no difference); walks of sure steps end
+//   together, so a claim fills the warp again.
+IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, bool sure,
+                       int grid, int num_sms)
 {
     IncorePlan p{};
     p.ctas_per_sm = (uint32_t)walk_ctas(sopr, coop);
-    p.grid = grid > 0 ? grid : walk_kernel(sopr, paths, coop, weighted, index, [&](auto s, auto pa, auto c, auto w, auto i) {
-        return resident_grid<s(), pa(), c(), w(), i()>(num_sms);
-    });
+    p.grid = grid > 0 ? grid
+                      : walk_kernel(sopr, paths, coop, weighted, index, sure,
+                                    [&](auto s, auto pa, auto c, auto w, auto i, auto u) {
+                                        return resident_grid<s(), pa(), c(), w(), i(), u()>(num_sms);
+                                    });
     const uint64_t warps = (uint64_t)p.grid * (kWalkThreads / 32), busy = std::min<uint64_t>(warps, 16ull * num_sms);
     p.slots = 1;
     while (p.slots < 32 && p.slots * busy < nwalkers) p.slots *= 2;
-    p.chunk = nwalkers <= 32 * warps ? p.slots : 8;
+    p.chunk = nwalkers <= 32 * warps ? p.slots : sure ? 32 : 8;
     return p;
 }
 
 cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s)
 {
-    walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.verts != nullptr,
-                [&](auto so, auto pa, auto c, auto w, auto i) {
-                    if (a.slots < 32)
-                        k_walk_incore<so(), pa(), c(), w(), i(), true><<<grid, kWalkThreads, 0, s>>>(a);
+    walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.verts != nullptr, sure_steps(sopr, a.c),
+                [&](auto so, auto pa, auto c, auto w, auto i, auto u) {
+                    if (!u() && a.slots < 32)
+                        k_walk_incore<so(), pa(), c(), w(), i(), !u(), u()><<<grid, kWalkThreads, 0, s>>>(a);
                     else
-                        k_walk_incore<so(), pa(), c(), w(), i(), false><<<grid, kWalkThreads, 0, s>>>(a);
+                        k_walk_incore<so(), pa(), c(), w(), i(), false, u()><<<grid, kWalkThreads, 0, s>>>(a);
                     return 0;
                 });
     return cudaGetLastError();

@@ -57,3 +57,25 @@ def test_walks_on_borrowed_csr_at_any_word(gw, oracle, algo, offset):
     cfg = oracle.make_cfg(algo=algo, maxhops=30, p=0.5, q=2.0, alpha=0.2, term_prob=term, seed=3)
     assert np.array_equal(eng.hashes(), oracle.walk(beg, csr, cfg, 0, V, paths=False)["hashes"])
     eng.close()
+
+
+def test_index_gives_way_to_outputs(gw, oracle):
+    """With the device full, a population whose outputs fit only in the memory
+    of the index still walks, without it."""
+    import torch
+    dg = gw.DeviceGraph(18, nverts=1 << 18, edgefactor=16, seed=7, symmetric=True)
+    beg, csr = dg.to_host()
+    eng = gw.WalkEngine(algorithm=0, maxhops=4, p=0.5, q=2.0, seed=5)
+    eng.set_device_graph(dg.nverts, dg.nedges, dg.beg_ptr, dg.csr_ptr)
+    eng.init_walkers(0, 1, 5)
+    eng.run()  # builds the index: some 90 MB
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (60 << 20), dtype=torch.uint8, device="cuda")
+    eng.init_walkers(0, 32, 5)  # 12 bytes for each of 8.4 M walkers: 101 MB
+    eng.run()
+    got = eng.hashes()[:2000]
+    del fill
+    torch.cuda.empty_cache()
+    ref = oracle.walk(beg, csr, oracle.make_cfg(algo=0, maxhops=4, p=0.5, q=2.0, seed=5, wps=32), 0, 2000, paths=False)
+    assert np.array_equal(got, ref["hashes"])
+    eng.close()

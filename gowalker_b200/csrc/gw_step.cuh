@@ -133,20 +133,23 @@ struct CsrIndex {
 
 // Membership table of one vertex's neighbours: table_buckets(d) buckets of
 // eight slots, an id in its home bucket (table_home) or, that one being full,
-// in the next that was not, slots filled in order, empty ones kEmptySlot.  The
-// slots number more than d, so a search ends at a bucket with room.
+// in the next that was not, the eighth slot filled last, empty ones kEmptySlot.
+// The slots number more than d, so a search ends at a bucket with room.
 constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;  // no id: ids are below a 32-bit vertex count
 __host__ __device__ __forceinline__ uint32_t table_buckets(uint32_t d)
 {
     return d ? (d >> 2) + (d >> 4) + 1u : 0u;  // 3.2 ids a bucket: fewer than 1 in 100 buckets overflow
 }
-__device__ __forceinline__ uint32_t table_home(uint32_t id, uint32_t buckets)
+__device__ __forceinline__ uint32_t table_hash(uint32_t id)
 {
     // two rounds: the product alone sends some arithmetic progressions to one bucket
-    uint32_t h = id * 0x9E3779B1u;
-    h = (h ^ (h >> 15)) * 0x85EBCA77u;
-    return __umulhi(h, buckets);
+    const uint32_t h = id * 0x9E3779B1u;
+    return (h ^ (h >> 15)) * 0x85EBCA77u;
 }
+__device__ __forceinline__ uint32_t table_home(uint32_t id, uint32_t buckets) { return __umulhi(table_hash(id), buckets); }
+// The slot an id tries first, of the first seven (it goes round them, then to
+// the eighth): a hash of its own decides, so most find it empty.
+__device__ __forceinline__ uint32_t table_slot(uint32_t id) { return __umulhi(table_hash(id) * 0xC2B2AE3Du, 7u); }
 
 // One aligned 32-byte sector: eight consecutive words in one load.
 __device__ __forceinline__ void load_sector(const uint32_t *p, uint32_t (&v)[8])

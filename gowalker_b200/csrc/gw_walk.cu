@@ -406,12 +406,15 @@ cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s)
 
 // The membership tables: a thread takes `per` consecutive edges, finds the first
 // one's vertex by halving the offsets and goes on from there, so hubs and
-// isolated vertices cost alike.  An id claims the first free slot from its home
-// bucket on; an id met twice keeps one slot.  Bound by the claims, about two
-// atomics an edge into the L2, one after another in a thread: a small graph's
-// edges are spread over all threads (30,000 edges: 106 us at 32 a thread, 14 us
-// so), a large one's taken 16 at a time (63 M: 4.8 / 4.1 / 3.2 / 3.1 / 3.4 ms at
-// 2 / 4 / 8 / 16 / 32; fewer repeat the search, more lengthen the last wave).
+// isolated vertices cost alike.  An id claims the first free slot of its home
+// bucket, from its own first slot round (table_slot), and of the buckets after
+// it; an id met twice takes the same way and keeps one slot.  Bound by the
+// claims, atomics into the L2, one after another in a thread: from each bucket's
+// first slot on they were twice as many (31 M edges 1.43 ms, 1.05 so).  A small
+// graph's edges are spread over all threads (30,000 edges: 106 us at 32 a
+// thread, 14 us so), a large one's taken 16 at a time (63 M, claims from the
+// first slot: 4.8 / 4.1 / 3.2 / 3.1 / 3.4 ms at 2 / 4 / 8 / 16 / 32; fewer repeat
+// the search, more lengthen the last wave).
 constexpr uint64_t kTableEdges = 16;
 __global__ void __launch_bounds__(256) k_build_table(const uint64_t *__restrict__ beg, const uint4 *__restrict__ verts,
                                                      uint32_t nverts, const uint32_t *__restrict__ csr,
@@ -443,9 +446,11 @@ __global__ void __launch_bounds__(256) k_build_table(const uint64_t *__restrict_
             uint32_t b = table_home(x, buckets);
             for (bool placed = false; !placed;) {  // the slots outnumber the ids
                 uint32_t *slot = table + ((uint64_t)first + b) * 8u;
-                for (int k = 0; k < 8 && !placed; ++k) {
-                    const uint32_t was = atomicCAS(slot + k, kEmptySlot, x);
+                uint32_t k = table_slot(x);
+                for (uint32_t i = 0; i < 8 && !placed; ++i) {
+                    const uint32_t was = atomicCAS(slot + (i < 7 ? k : 7u), kEmptySlot, x);
                     placed = was == kEmptySlot || was == x;
+                    k = k == 6 ? 0u : k + 1;
                 }
                 b = b + 1 == buckets ? 0u : b + 1;
             }

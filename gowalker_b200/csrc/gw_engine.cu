@@ -327,6 +327,8 @@ int gw_handle::ensure_outputs()
         if (need > cap_path_words) {
             cudaFree(d_paths);
             d_paths = nullptr;
+            cap_path_words = 0;
+            cap_path_walkers = 0;
             if ((st = dev_alloc(d_paths, need * sizeof(uint32_t), "paths"))) return st;
             cap_path_words = need;
         }
@@ -492,11 +494,15 @@ extern "C" int gw_init_walker_range(gw_handle *h, uint32_t algo, uint32_t wps, u
         return h->fail(GW_ERR_ARG, "walker range [%llu, +%llu) outside the %llu walkers", (unsigned long long)first,
                        (unsigned long long)count, (unsigned long long)n);
     cudaSetDevice(h->cfg.device);
+    h->walkers_ready = false;  // until the new population has its outputs
     h->nwalkers = count;
     h->wid_first = (uint32_t)first;
     h->numwalks_eff = (uint32_t)n;
     int st = h->ensure_outputs();
-    if (st) return st;
+    if (st) {
+        h->nwalkers = 0;  // what is left of the outputs is no population's
+        return st;
+    }
     h->walkers_ready = true;
     h->ooc_walkers_stale = true;
     return GW_OK;

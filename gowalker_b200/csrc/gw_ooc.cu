@@ -420,6 +420,7 @@ static int ooc_walkers(gw_handle *h)
 {
     OocState &o = *h->ooc;
     if (h->nwalkers > o.w_cap) {
+        o.w_cap = 0;
         cudaFree(o.w_rec);
         o.w_rec = nullptr;
         for (int i = 0; i < 2; ++i) {

@@ -367,6 +367,8 @@ extern "C" int gw_set_graph_meta(gw_handle *h, uint32_t nverts, uint64_t nedges,
     h->dev_w = nullptr;
     cudaFree(h->own_w);
     h->own_w = nullptr;
+    cudaFree(h->d_alias);  // sized for the edges of the graph before
+    h->d_alias = nullptr;
     h->alias_ready = false;
     h->dev_beg = nullptr;
     h->dev_csr = nullptr;

@@ -793,6 +793,7 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
     const bool sorted = dedup || (flags & GW_EDGES_SORT);
     if (n > (symmetric ? (1ull << 62) : (1ull << 63)) / sizeof(uint64_t)) return GW_ERR_ARG;
     const uint64_t m = n * (symmetric ? 2 : 1);
+    if (m > (1ull << 56)) return GW_ERR_NOMEM;  // the scratch below is their sum: it must not wrap
     int rc = GW_OK;
     cudaStream_t s = 0;
     PhaseTrace trace(s);

@@ -49,6 +49,7 @@ struct gw_handle {
     uint32_t *d_heads_hi = nullptr;  // null: every offset is below 2^32
     uint32_t *d_table = nullptr;
     bool index_ready = false;
+    uint64_t index_sum = 0;  // borrowed CSR: sum of the contents the index was built from
 
     // edge weights (weighted Node2vec, in-core): per host block, or resident
     std::vector<const float *> host_w;
@@ -75,9 +76,9 @@ struct gw_handle {
     uint32_t path_stride = 0;
 
     // counters
-    unsigned long long *d_ctr = nullptr;  // kCtrCount counters, then the error word
+    unsigned long long *d_ctr = nullptr;  // kCtrWords: counters, error word, graph sum
     uint32_t *d_err = nullptr;            // that word
-    unsigned long long *h_ctr = nullptr;  // pinned: kCtrCount counters + error word
+    unsigned long long *h_ctr = nullptr;  // pinned, the same
     uint64_t last_hash_sum = 0;
     uint64_t last_steps = 0;
 

@@ -24,6 +24,9 @@ enum Counter : int {
     kCtrRunnable = 11,     // out-of-core: walkers handed to the step kernels (sum over launches)
     kCtrCount = 12
 };
+// Behind the counters of an in-core run: the error word, then the sum of the
+// graph's contents (CsrCheck::sum).
+constexpr int kCtrGraphSum = kCtrCount + 1, kCtrWords = kCtrCount + 2;
 
 // Per-warp statistics a walk kernel keeps in shared memory and adds to the
 // Counter slots when it ends.
@@ -74,6 +77,10 @@ struct IncoreArgs {
     const uint4 *verts;        // {first edge (low word), degree, first bucket, mod_magic(degree)} per vertex
     const uint32_t *heads_hi;  // high words of the first edges; null when all are 0
     const uint32_t *table;     // membership tables (table_has); set with verts
+    // a borrowed CSR: its contents now, and those the index was built from; the
+    // walk waits for a new index where they differ.  Null: the handle's own copy
+    const unsigned long long *sum;
+    unsigned long long sum_built;
     uint32_t nverts;
     uint32_t nwalkers;         // walkers of this launch: ids wid_base + i, i < nwalkers
     uint32_t wid_base;
@@ -207,6 +214,7 @@ struct CsrCheck {
     uint4 *verts;
     uint32_t *heads_hi;            // null: offsets below 2^32
     unsigned long long *nbuckets;
+    unsigned long long *sum;       // null, or a 64-bit sum over the contents is added here
 };
 cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s);
 // Fills the membership tables of a validated CSR; every slot is kEmptySlot before.

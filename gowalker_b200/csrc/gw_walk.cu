@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
     __shared__ uint32_t s_park[COOP ? kWalkThreads / 32 : 1][kPkCount][32];  // lane state during hard steps
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
+    if (INDEX && a.sum && *a.sum != a.sum_built) return;
     if (lane < kWsCount) s_ws[warp][lane] = 0;
     s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
     s_done[threadIdx.x] = 0;
@@ -351,12 +352,24 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
 // order is a precondition -- the reference's `sorted` option -- and affects
 // results, not safety.)  Bound by reading the CSR once: eight ids (one sector)
 // per thread and load.  A warp takes its vertices' buckets with one atomic.
+//
+// a.sum: a sum over every offset and id, each mixed with its place, by which a
+// later run sees that a borrowed CSR has been written.  One id's change always
+// changes it (each mix is a bijection of the word), several do but for one time
+// in 2^64.  Two ids a multiplication, so the pass stays bound by its reads.
+constexpr uint64_t kSumA = 0x9E3779B97F4A7C15ull, kSumB = 0xD1342543DE82EF95ull, kSumC = 0xBF58476D1CE4E5B9ull;
+__device__ __forceinline__ uint64_t sum_mix(uint64_t h, uint64_t w)
+{
+    h = (h ^ w) * kSumC;
+    return h ^ (h >> 32);
+}
 __global__ void __launch_bounds__(256) k_validate_csr(const __grid_constant__ CsrCheck a)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u;
     bool bad = false;
+    uint64_t sum = 0;
     for (uint64_t v0 = t0 - lane; v0 < a.nverts; v0 += stride) {
         const uint64_t v = v0 + lane;
         uint64_t b = 0, e = 0;
@@ -364,6 +377,7 @@ __global__ void __launch_bounds__(256) k_validate_csr(const __grid_constant__ Cs
             b = a.beg[v];
             e = a.beg[v + 1];
             bad |= (b > e) | (e > a.nedges);
+            if (a.sum) sum += sum_mix(v * kSumA, b * kSumB + e) * kSumB;
         }
         if (a.verts) {
             const uint32_t d = (uint32_t)(e - b);
@@ -391,16 +405,31 @@ __global__ void __launch_bounds__(256) k_validate_csr(const __grid_constant__ Cs
             load_sector(a.csr + 8 * j, v);
 #pragma unroll
             for (int i = 0; i < 8; ++i) bad |= v[i] >= a.nverts;
+            if (a.sum) {
+                uint64_t h = ~j * kSumA;
+#pragma unroll
+                for (int i = 0; i < 8; i += 2) h = sum_mix(h, ((uint64_t)v[i + 1] << 32) | v[i]);
+                sum += h * kSumB;
+            }
         }
         done = 8 * sectors;
     }
-    for (uint64_t i = done + t0; i < a.nedges; i += stride) bad |= __ldg(a.csr + i) >= a.nverts;
+    for (uint64_t i = done + t0; i < a.nedges; i += stride) {
+        const uint32_t x = __ldg(a.csr + i);
+        bad |= x >= a.nverts;
+        if (a.sum) sum += sum_mix(~i * kSumA, x) * kSumB;
+    }
+    if (a.sum) {
+        sum = warp_sum((unsigned long long)sum);
+        if (lane == 0) atomicAdd(a.sum, (unsigned long long)sum);
+    }
     if (__any_sync(0xFFFFFFFFu, bad) && lane == 0) atomicOr(a.err, kErrVertexRange);
 }
 
 cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s)
 {
-    k_validate_csr<<<num_sms * 8, 256, 0, s>>>(a);
+    const uint64_t need = (std::max<uint64_t>(a.nverts, a.nedges / 8) + 255) / 256;  // one round of every thread
+    k_validate_csr<<<(int)std::min<uint64_t>(need + 1, 8ull * num_sms), 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 

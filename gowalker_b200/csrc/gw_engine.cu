@@ -45,10 +45,8 @@ int gw_handle::dev_alloc(void **p, uint64_t bytes, const char *what)
     if (e == cudaErrorMemoryAllocation && d_index) {
         cudaGetLastError();
         cudaStreamSynchronize(s_compute);
-        cudaFree(d_index);
-        d_index = nullptr;
-        index_cap = 0;
-        index_ready = false;
+        drop_index();
+        index_refused = true;
         e = cudaMalloc(p, bytes);
     }
     return cuda(e, what);
@@ -223,9 +221,7 @@ void gw_handle::release()
     cudaFree(d_paths);
     cudaFree(d_hashes);
     cudaFree(d_ctr);
-    cudaFree(d_index);
-    d_index = nullptr;
-    index_cap = 0;
+    drop_index();
     if (h_ctr) cudaFreeHost(h_ctr);
     ooc_release();
     if (ev_start) cudaEventDestroy(ev_start);
@@ -519,34 +515,107 @@ extern "C" int gw_num_walkers(gw_handle *h, uint64_t *n)
 
 // ------------------------------------------------------------------ ABI: run
 
-// Checks the resident CSR and builds its index, once per graph: per vertex 16
-// bytes (first edge, degree, first bucket, the degree's reciprocal), which a
-// step loads at once in place of two offsets and a division, and the
-// membership tables (10 bytes per edge and up to 32 per vertex).  Where the
-// device has no room for them walks read the offsets and halve.
-int gw_handle::validate_graph(cudaStream_t s)
+// The index of a resident CSR for walks that search by `search`.
+// kTable: per vertex 16 bytes (first edge, degree, first bucket, the degree's
+// reciprocal), which a step loads at once in place of two offsets and a
+// division, and the membership tables (10 bytes per edge and up to 32 per
+// vertex).  kLevels: the sample levels (0.13 bytes per edge).
+gw_handle::IndexLayout gw_handle::index_layout(int search) const
+{
+    IndexLayout l{};
+    if (search == kTable) {
+        // buckets: 5/16 of an edge's and one more per vertex at most (table_buckets)
+        l.buckets = nedges / 4 + nedges / 16 + nverts + 1;
+        l.heads_hi = ((uint64_t)nverts * sizeof(uint4) + 255) & ~255ull;
+        l.table = l.heads_hi + (nedges >= (1ull << 32) ? ((uint64_t)nverts * sizeof(uint32_t) + 255) & ~255ull : 0);
+        l.bytes = l.table + l.buckets * 32;
+    } else if (search == kLevels) {
+        for (uint64_t m = nedges; l.nlevels < (uint32_t)kIdxLevels && m > 64; ++l.nlevels) {
+            m = (m + 31) / 32;
+            l.level[l.nlevels] = m;
+            l.bytes += m * sizeof(uint32_t);
+        }
+    }
+    return l;
+}
+
+// Memory for that index.  An index is worth having, not needed: a large one
+// takes at most half of what is free, and none is no error; after a refusal
+// another attempt is made only where it has room.
+bool gw_handle::reserve_index(int search)
+{
+    const IndexLayout l = index_layout(search);
+    if (l.buckets >= (1ull << 32)) return false;  // bucket numbers are 32-bit
+    if (l.bytes <= index_cap) return true;
+    size_t free_bytes = 0, all_bytes = 0;
+    if (l.bytes >= kSmallIndex || index_refused) {
+        if (cudaMemGetInfo(&free_bytes, &all_bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        if (l.bytes > (l.bytes >= kSmallIndex ? free_bytes / 2 : free_bytes)) {
+            index_refused = true;
+            return false;
+        }
+    }
+    drop_index();
+    index_refused = cudaMalloc(&d_index, l.bytes) != cudaSuccess;
+    if (index_refused) {
+        cudaGetLastError();
+        d_index = nullptr;
+        return false;
+    }
+    index_cap = l.bytes;
+    return true;
+}
+
+void gw_handle::drop_index()
+{
+    cudaFree(d_index);
+    d_index = nullptr;
+    index_cap = 0;
+    index_search = kQuarter;
+}
+
+// The search a run is worth an index for.  Tables cost a pass of atomics over
+// the edges (7.6 M edges 0.24 ms, 64 M 2.8 ms) and save part of each step, so
+// they are built when the steps of the runs on this graph so far and of this one
+// come to so many an edge:
+// - 1 where graph and tables fit the L2 (a first run of 27 steps an edge on 1.8 M
+//   edges 1.66 ms, 2.81 without; of 2.8 on 7.6 M 1.44 / 1.77; of 0.14 0.43 / 0.22),
+// - 3 past it (a first run of 2.6 on 64 M edges 6.0 / 4.5 ms, on 31 M 2.77 / 2.20;
+//   the run after it 3.3 / 4.3 and 1.53 / 2.13), 1 for SOPR and SOSR, whose steps
+//   take more trials (128 M edges, 0.8: 30.4 / 27.5 ms, then 24.3 / 27.2).
+// Steps that always accept search nothing.
+int gw_handle::wanted_search(bool sopr, bool sure) const
+{
+    if (cfg.launch_mode == GW_LAUNCH_PER_HOP || sure) return kQuarter;
+    const double steps = index_steps + run_steps();
+    if (steps >= (double)nedges * (sopr || 14 * nedges <= kL2Bytes ? 1.0 : 3.0)) return kTable;
+    return wants_levels(nwalkers, nedges, sopr, sure, num_sms) ? kLevels : kQuarter;
+}
+
+// Steps of a run at most: every walker to its last hop, or to its mean by the
+// termination draws.  Fewer walkers than lanes take as long as many.
+double gw_handle::run_steps() const
+{
+    double hops = cfg.maxhops;
+    if (cfg.term_prob > 0.f) hops = std::min(hops, 1.0 / (double)cfg.term_prob);
+    return (double)std::max(nwalkers, walk_lanes(num_sms)) * hops;
+}
+
+// Checks the resident CSR, and builds its index for walks that search by
+// `search`, where it has memory.
+int gw_handle::validate_graph(cudaStream_t s, int search)
 {
     int st;
-    index_ready = false;
-    const bool wide = nedges >= (1ull << 32);
-    // buckets: 5/16 of an edge's and one more per vertex at most (table_buckets)
-    const uint64_t most_buckets = nedges / 4 + nedges / 16 + nverts + 1;
-    const uint64_t verts_bytes = ((uint64_t)nverts * sizeof(uint4) + 255) & ~255ull;
-    const uint64_t hi_bytes = wide ? ((uint64_t)nverts * sizeof(uint32_t) + 255) & ~255ull : 0;
-    const uint64_t index_bytes = verts_bytes + hi_bytes + most_buckets * 32;
-    if (index_bytes > index_cap) {
-        cudaFree(d_index);
-        d_index = nullptr;
-        index_cap = 0;
-        // an index is worth having, not needed: a large one takes at most half
-        // of what is free, and none is no error
-        size_t free_bytes = 0, all_bytes = 0;
-        const bool room = index_bytes < (256ull << 20) ||
-                          (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && index_bytes <= free_bytes / 2);
-        if (room && cudaMalloc(&d_index, index_bytes) == cudaSuccess) index_cap = index_bytes;
-        cudaGetLastError();
-    }
-    const bool index = index_cap >= index_bytes && most_buckets < (1ull << 32);
+    index_search = kQuarter;
+    if (!reserve_index(search)) search = kQuarter;
+    // the memory of a small index is taken with the first check, so that the
+    // run that builds it, maybe a short one, does not wait for an allocation
+    if (search != kTable && !index_refused && index_layout(kTable).bytes < kSmallIndex) reserve_index(kTable);
+    const IndexLayout l = index_layout(search);
+    const bool index = search == kTable;
     CsrCheck check{};
     check.beg = dev_beg;
     check.csr = dev_csr;
@@ -556,8 +625,8 @@ int gw_handle::validate_graph(cudaStream_t s)
     check.sum = device_graph ? d_ctr + kCtrGraphSum : nullptr;
     if (index) {
         d_verts = reinterpret_cast<uint4 *>(d_index);
-        d_heads_hi = wide ? reinterpret_cast<uint32_t *>(d_index + verts_bytes) : nullptr;
-        d_table = reinterpret_cast<uint32_t *>(d_index + verts_bytes + hi_bytes);
+        d_heads_hi = l.table > l.heads_hi ? reinterpret_cast<uint32_t *>(d_index + l.heads_hi) : nullptr;
+        d_table = reinterpret_cast<uint32_t *>(d_index + l.table);
         check.verts = d_verts;
         check.heads_hi = d_heads_hi;
         check.nbuckets = d_ctr;
@@ -583,9 +652,17 @@ int gw_handle::validate_graph(cudaStream_t s)
             (st = cuda(launch_build_table(dev_beg, d_verts, nverts, dev_csr, nedges, d_table, num_sms, s),
                        "membership tables")))
             return st;
-        index_ready = true;
-        index_sum = h_ctr[kCtrGraphSum];
     }
+    const uint32_t *src = dev_csr;
+    uint32_t *dst = reinterpret_cast<uint32_t *>(d_index);
+    for (uint32_t i = 0; i < l.nlevels; ++i) {
+        if ((st = cuda(launch_sample_level(src, l.level[i], dst, num_sms, s), "sample level"))) return st;
+        levels.lvl[i] = src = dst;
+        dst += l.level[i];
+    }
+    levels.n = l.nlevels;
+    index_search = search;
+    index_sum = h_ctr[kCtrGraphSum];
     validated = true;
     return GW_OK;
 }
@@ -630,15 +707,21 @@ int gw_handle::run_incore(gw_stats *stats)
     if (!resident) {
         if ((st = upload_whole_graph(s, &h2d))) return st;
     }
-    const bool unchecked = !validated;
-    if (unchecked && (st = validate_graph(s))) return st;
+    StepConsts consts;
+    consts_from_config(cfg, consts);
+    const bool sopr = cfg.algorithm != GW_NODE2VEC;
+    const bool sure = sure_steps(sopr, consts);
+    if (!validated) index_steps = 0;
+    const int wanted = wanted_search(sopr, sure);
+    const bool unchecked = !validated || (wanted > index_search && reserve_index(wanted));
+    if (unchecked && (st = validate_graph(s, wanted))) return st;
     if (weighted) {
         if (cfg.algorithm != GW_NODE2VEC)
             return fail(GW_ERR_ARG, "weighted walks are Node2vec walks (algorithm %u given)", cfg.algorithm);
         if (!alias_ready && (st = build_alias(s))) return st;
     }
     IncoreArgs a{};
-    consts_from_config(cfg, a.c);
+    a.c = consts;
     a.init.mode = cfg.init_mode;
     a.init.algo = cfg.algorithm;
     a.init.wps = cfg.walkpersource;
@@ -648,11 +731,16 @@ int gw_handle::run_incore(gw_stats *stats)
     a.init.key1 = (uint32_t)(cfg.seed >> 32);
     a.beg = dev_beg;
     a.csr = dev_csr;
-    if (index_ready) {
-        a.verts = d_verts;
-        a.heads_hi = d_heads_hi;
-        a.table = d_table;
-    }
+    a.nedges = nedges;
+    // A borrowed CSR is summed before its index is read, so a run of few steps
+    // leaves the index alone and reads the CSR as it is
+    const bool indexed = !device_graph || unchecked || (!sure && 8.0 * run_steps() >= (double)nedges);
+    a.search = indexed ? index_search : kQuarter;
+    if (a.search == kLevels && !wants_levels(nwalkers, nedges, sopr, sure, num_sms)) a.search = kQuarter;
+    a.levels = levels;
+    a.verts = d_verts;
+    a.heads_hi = d_heads_hi;
+    a.table = d_table;
     a.nverts = nverts;
     a.nwalkers = (uint32_t)nwalkers;
     a.wid_base = wid_first;
@@ -663,7 +751,6 @@ int gw_handle::run_incore(gw_stats *stats)
     a.hashes = d_hashes;
     a.ctr = d_ctr;
     a.err = d_err;
-    const bool sopr = cfg.algorithm != GW_NODE2VEC;
     const bool coop = !weighted && needs_coop(cfg.algorithm, a.c);
     a.alias = weighted ? reinterpret_cast<const uint2 *>(d_alias) : nullptr;
     if (cfg.launch_mode == GW_LAUNCH_PER_HOP) {
@@ -720,33 +807,44 @@ int gw_handle::run_incore(gw_stats *stats)
                         (unsigned long long)nwalkers);
         return GW_OK;
     }
-    const IncorePlan plan = incore_plan(nwalkers, sopr, a.paths != nullptr, coop, weighted, index_ready,
-                                        sure_steps(sopr, a.c), (int)cfg.blockpergrid, num_sms);
+    const IncorePlan plan = incore_plan(nwalkers, sopr, a.paths != nullptr, coop, weighted, a.search, sure,
+                                        (int)cfg.blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
-    const size_t ctr_bytes = sizeof(unsigned long long) * kCtrWords;
-    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, ctr_bytes, s), "memset"))) return st;
+    const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);  // with the error word
     // A borrowed CSR may have been written since its index was built: its
-    // contents are summed again, and the walk goes ahead only if they are the
-    // same (64 M edges: 65 us beside a walk of 3.2 ms; 21,000: 5 us).
-    const bool summed = device_graph && index_ready && !unchecked;
-    if (summed) {
+    // contents are summed beside the walk, which is done again if they are not
+    // the same.  (Records, tables and levels of another graph of these sizes
+    // lead no read out of range.)  A walk that fills the device leaves the sum no
+    // room until its end, so there the sum goes first.  64 M edges: 65 us of a
+    // walk of 3.2 ms, and of one of 0.15 ms that leaves room.
+    const bool summed = device_graph && a.search != kQuarter && !unchecked;
+    const bool sum_first = nwalkers >= walk_lanes(num_sms);
+    auto sum_graph = [&]() {
         CsrCheck check{};
         check.beg = dev_beg;
         check.csr = dev_csr;
         check.nverts = nverts;
         check.nedges = nedges;
-        check.err = d_err;
         check.sum = d_ctr + kCtrGraphSum;
-        a.sum = check.sum;
-        a.sum_built = index_sum;
-        if ((st = cuda(launch_validate_csr(check, num_sms, s), "graph sum"))) return st;
-    }
-    if ((st = cuda(cudaEventRecord(ev_kernel0, s), "event")) ||
+        check.err = reinterpret_cast<uint32_t *>(check.sum + 1);
+        int e;
+        if ((e = cuda(cudaMemsetAsync(check.sum, 0, 2 * sizeof(unsigned long long), s_copy), "memset")) ||
+            (e = cuda(launch_validate_csr(check, num_sms, s_copy), "graph sum")))
+            return e;
+        return cuda(cudaMemcpyAsync(h_ctr + kCtrGraphSum, check.sum, sizeof(unsigned long long),
+                                    cudaMemcpyDeviceToHost, s_copy),
+                    "graph sum");
+    };
+    if (summed && sum_first && (st = sum_graph())) return st;
+    if ((st = cuda(cudaMemsetAsync(d_ctr, 0, ctr_bytes, s), "memset")) ||
+        (st = cuda(cudaEventRecord(ev_kernel0, s), "event")) ||
         (st = cuda(launch_walk_incore(a, sopr, coop, plan.grid, s), "walk kernel launch")) ||
         (st = cuda(cudaEventRecord(ev_kernel1, s), "event")) ||
+        (summed && !sum_first && (st = sum_graph())) ||
         (st = cuda(cudaMemcpyAsync(h_ctr, d_ctr, ctr_bytes, cudaMemcpyDeviceToHost, s), "counters D2H")) ||
-        (st = cuda(cudaEventRecord(ev_stop, s), "event")) || (st = cuda(cudaStreamSynchronize(s), "walk")))
+        (st = cuda(cudaEventRecord(ev_stop, s), "event")) || (st = cuda(cudaStreamSynchronize(s), "walk")) ||
+        (summed && (st = cuda(cudaStreamSynchronize(s_copy), "graph sum"))))
         return st;
     if (summed && h_ctr[kCtrGraphSum] != index_sum) {  // written: checked and indexed anew, then walked
         h_ctr[kCtrCount] = 0;
@@ -756,6 +854,7 @@ int gw_handle::run_incore(gw_stats *stats)
     }
     last_hash_sum = h_ctr[kCtrHashSum];
     last_steps = h_ctr[kCtrSteps];
+    index_steps += run_steps();
     const uint32_t errw = (uint32_t)h_ctr[kCtrCount];
     if (stats) {
         memset(stats, 0, sizeof(*stats));

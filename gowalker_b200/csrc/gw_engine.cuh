@@ -41,14 +41,18 @@ struct gw_handle {
     bool resident = false;
     bool device_graph = false;
     bool validated = false;
-    // index of the resident CSR, rebuilt whenever it is validated: one
-    // allocation, parts on 256-byte boundaries
+    // index of the resident CSR, built by the run that wants it: one allocation,
+    // the parts of tables on 256-byte boundaries
+    static constexpr uint64_t kSmallIndex = 256ull << 20;
     char *d_index = nullptr;
     uint64_t index_cap = 0;
+    int index_search = gw::kQuarter;  // what is built: kTable, kLevels or none
+    bool index_refused = false;       // the last attempt had no memory, or the index gave way
+    double index_steps = 0.0;         // run_steps() of the runs on this graph so far
     uint4 *d_verts = nullptr;
     uint32_t *d_heads_hi = nullptr;  // null: every offset is below 2^32
     uint32_t *d_table = nullptr;
-    bool index_ready = false;
+    gw::Levels levels{};
     uint64_t index_sum = 0;  // borrowed CSR: sum of the contents the index was built from
 
     // edge weights (weighted Node2vec, in-core): per host block, or resident
@@ -101,7 +105,17 @@ struct gw_handle {
     bool host_graph_complete() const;
     int upload_whole_graph(cudaStream_t s, uint64_t *h2d);
     int ensure_outputs();
-    int validate_graph(cudaStream_t s);
+    struct IndexLayout {
+        uint64_t bytes, buckets, heads_hi, table;  // kTable: offsets behind the records
+        uint64_t level[gw::kIdxLevels];            // kLevels: entries
+        uint32_t nlevels;
+    };
+    IndexLayout index_layout(int search) const;
+    bool reserve_index(int search);
+    void drop_index();
+    double run_steps() const;
+    int wanted_search(bool sopr, bool sure) const;
+    int validate_graph(cudaStream_t s, int search);
     int build_alias(cudaStream_t s);
     int run_incore(gw_stats *stats);
     int run_ooc(uint32_t policy, gw_stats *stats);

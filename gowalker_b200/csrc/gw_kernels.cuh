@@ -7,6 +7,7 @@
 namespace gw {
 
 constexpr int kWalkThreads = 256;   // threads per CTA of the walk kernels
+constexpr uint64_t kL2Bytes = 126ull << 20;
 
 // Work / statistics counters of one run (device, zeroed per run).
 enum Counter : int {
@@ -24,9 +25,9 @@ enum Counter : int {
     kCtrRunnable = 11,     // out-of-core: walkers handed to the step kernels (sum over launches)
     kCtrCount = 12
 };
-// Behind the counters of an in-core run: the error word, then the sum of the
-// graph's contents (CsrCheck::sum).
-constexpr int kCtrGraphSum = kCtrCount + 1, kCtrWords = kCtrCount + 2;
+// Behind the counters of an in-core run and the error word: the sum of a
+// borrowed graph's contents (CsrCheck::sum) and that check's own error word.
+constexpr int kCtrGraphSum = kCtrCount + 1, kCtrWords = kCtrCount + 3;
 
 // Per-warp statistics a walk kernel keeps in shared memory and adds to the
 // Counter slots when it ends.
@@ -73,14 +74,13 @@ struct IncoreArgs {
     WalkerInit init;
     const uint64_t *beg;       // nverts+1 global offsets
     const uint32_t *csr;       // nedges neighbour ids
-    // index of the resident CSR, built once per graph (verts null: none)
+    uint64_t nedges;
+    int search;                // Search: what of the index below the walk reads
+    Levels levels;             // kLevels
+    // kTable
     const uint4 *verts;        // {first edge (low word), degree, first bucket, mod_magic(degree)} per vertex
     const uint32_t *heads_hi;  // high words of the first edges; null when all are 0
-    const uint32_t *table;     // membership tables (table_has); set with verts
-    // a borrowed CSR: its contents now, and those the index was built from; the
-    // walk waits for a new index where they differ.  Null: the handle's own copy
-    const unsigned long long *sum;
-    unsigned long long sum_built;
+    const uint32_t *table;     // membership tables (table_has)
     uint32_t nverts;
     uint32_t nwalkers;         // walkers of this launch: ids wid_base + i, i < nwalkers
     uint32_t wid_base;
@@ -116,16 +116,18 @@ struct Vertex {
     uint32_t bucket; // first bucket of its membership table
     uint32_t magic;  // mod_magic(deg)
 };
-// INDEX: from the vertex index, else from the offsets.
-template <bool INDEX>
+// INDEX: from the vertex index, else from the offsets.  CHECK: offsets that are
+// no valid list's (a borrowed CSR, written since it was checked) give a dead end.
+template <bool INDEX, bool CHECK = false>
 __device__ __forceinline__ Vertex load_vertex(const IncoreArgs &a, uint32_t v)
 {
     if constexpr (INDEX) {
         const uint4 e = __ldg(a.verts + v);
         return Vertex{a.heads_hi ? ((uint64_t)__ldg(a.heads_hi + v) << 32) | e.x : e.x, e.y, e.z, e.w};
     }
-    const uint64_t head = __ldg(a.beg + v);
-    const uint32_t deg = (uint32_t)(__ldg(a.beg + v + 1) - head);
+    const uint64_t head = __ldg(a.beg + v), end = __ldg(a.beg + v + 1);
+    uint32_t deg = (uint32_t)(end - head);
+    if (CHECK && (head > end || end > a.nedges)) deg = 0;
     return Vertex{head, deg, 0u, deg ? mod_magic(deg) : 0u};
 }
 
@@ -175,7 +177,7 @@ struct IncorePlan {
     uint32_t ctas_per_sm;   // the kernel's register cap: CTAs of an SM it is built for
 };
 // `grid` CTAs as asked for, or (0) as many as are resident at once.
-IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, bool sure,
+IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
                        int grid, int num_sms);
 // a.alias set: weighted Node2vec.
 cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s);
@@ -217,6 +219,16 @@ struct CsrCheck {
     unsigned long long *sum;       // null, or a 64-bit sum over the contents is added here
 };
 cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s);
+// Walkers an in-core kernel holds at a time: the lanes of `walk_ctas` CTAs an SM.
+uint64_t walk_lanes(int num_sms);
+// Whether a run reads sample levels when it has no tables: Node2vec on a CSR
+// larger than the L2, with walkers for a quarter of the lanes (fewer wait for
+// the chain of loads, which is longer: 64 M edges, 10,000 walkers 0.45 ms, 0.39
+// by quarters, 100,000 0.67 / 0.82; SOPR searches little: 128 M edges 28.2 ms,
+// 27.3 by quarters).
+bool wants_levels(uint64_t nwalkers, uint64_t nedges, bool sopr, bool sure, int num_sms);
+// dst[j] = src[32 * j] for j < n.
+cudaError_t launch_sample_level(const uint32_t *src, uint64_t n, uint32_t *dst, int num_sms, cudaStream_t s);
 // Fills the membership tables of a validated CSR; every slot is kEmptySlot before.
 cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t nverts, const uint32_t *csr,
                                uint64_t nedges, uint32_t *table, int num_sms, cudaStream_t s);

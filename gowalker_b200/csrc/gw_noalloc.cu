@@ -173,7 +173,9 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     a.init.key0 = (uint32_t)cfg->seed;
     a.init.key1 = (uint32_t)(cfg->seed >> 32);
     a.beg = d_beg;
-    a.csr = d_csr;  // no index: this entry point allocates nothing
+    a.csr = d_csr;
+    a.nedges = nedges;
+    a.search = kQuarter;  // no index: this entry point allocates nothing
     a.nverts = nverts;
     a.nwalkers = (uint32_t)nwalkers;
     a.paths = (cfg->record_paths == GW_PATHS_FULL) ? d_paths : nullptr;
@@ -185,7 +187,7 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     const bool sopr = cfg->algorithm != GW_NODE2VEC;
     const bool coop = needs_coop(cfg->algorithm, a.c);
     const IncorePlan plan =
-        incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, false, sure_steps(sopr, a.c),
+        incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, kQuarter, sure_steps(sopr, a.c),
                     (int)cfg->blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;

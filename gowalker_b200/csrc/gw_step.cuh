@@ -122,13 +122,26 @@ __device__ __forceinline__ bool terminates(const StepConsts &c, uint32_t z)
 // its vertices (table_has), and how a neighbour is searched.
 enum Search : int {
     kHalve,    // mapped host memory: fewest sectors
-    kQuarter,  // device memory: fewest dependent loads without a table
+    kQuarter,  // device memory: fewest dependent loads without an index
+    kLevels,   // device memory past the L2: fewest lines without a table
     kTable
 };
 template <int SEARCH>
 struct CsrIndex {
     const uint32_t *csr;
     const uint32_t *table;  // kTable: buckets of eight ids, on 32-byte boundaries
+};
+// Sample levels of a whole CSR: level L holds csr[j * 32^L] for every j, about
+// 3 % of the CSR in all.
+constexpr int kIdxLevels = 6;
+struct Levels {
+    const uint32_t *lvl[kIdxLevels];
+    uint32_t n;
+};
+template <>
+struct CsrIndex<kLevels> {
+    const uint32_t *csr;  // the whole CSR: levels are by global position
+    const Levels *levels;
 };
 
 // Membership table of one vertex's neighbours: table_buckets(d) buckets of
@@ -232,6 +245,37 @@ __device__ __forceinline__ bool list_has(const uint32_t *__restrict__ p, uint32_
     return found;
 }
 
+// Membership of x in the sorted csr[lo, lo + n) through the sample levels: down
+// from the highest with more than two entries inside (level L qualifies when
+// the range is longer than 2 * 32^L), each a binary search that narrows the
+// range 32-fold, the last one in the CSR itself; 64 ids and fewer go there at
+// once.  All but that one stay in the L2.
+__device__ __forceinline__ bool levels_have(const CsrIndex<kLevels> &ix, uint64_t lo, uint32_t n, uint32_t x)
+{
+    const Levels &lv = *ix.levels;
+    const uint64_t end = lo + n;
+    uint64_t hi = end;
+    if (n > 64) {
+        int L = min((int)lv.n, (30 - __clz((int)n)) / 5);  // (floor(log2 n) - 1) / 5
+        for (; L >= 1; --L) {
+            const uint32_t sh = 5u * (uint32_t)L;
+            if (hi - lo <= (2ull << sh)) continue;
+            const uint32_t *__restrict__ g = lv.lvl[L - 1];
+            const uint64_t j0 = (lo + (1ull << sh) - 1) >> sh, j1 = (hi - 1) >> sh;
+            uint32_t a = 0, b = (uint32_t)(j1 - j0) + 1;  // first j in [j0, j1] with csr[j << sh] >= x
+            while (a < b) {
+                const uint32_t m = (a + b) >> 1;
+                if (__ldg(g + j0 + m) < x) a = m + 1;
+                else b = m;
+            }
+            if (a > 0) lo = ((j0 + a - 1) << sh) + 1;
+            if (j0 + a <= j1) hi = (j0 + a) << sh;
+        }
+    }
+    const uint64_t p = csr_lower_bound(ix.csr, lo, hi, x);
+    return p < end && __ldg(ix.csr + p) == x;
+}
+
 // Membership of x in the sorted csr[lo, lo + n), whose table starts at bucket
 // `first`.
 //
@@ -240,15 +284,24 @@ __device__ __forceinline__ bool list_has(const uint32_t *__restrict__ p, uint32_
 // probes (a hundred instructions) for the thousands of neighbours of the
 // vertices walks visit most; a bucket is one load and eight compares.  Sample
 // levels of 32, eight-way levels and eight-way trees were all measured too:
-// fewer lines than halving, but no fewer instructions.
+// fewer lines than halving, but no fewer instructions.  Fewer lines count where
+// the CSR is larger than the L2 and no table is there (Node2vec on 64 M edges:
+// 4.23 ms by levels of 32, 4.92 by quarters, 5.38 by halving, 3.25 by tables;
+// on 31 M 2.20 / 2.09 / 2.47 / 1.48).
 template <int SEARCH>
 __device__ __forceinline__ bool csr_contains(const CsrIndex<SEARCH> &ix, uint32_t first, uint64_t lo, uint32_t n,
                                              uint32_t x)
 {
-    if constexpr (SEARCH == kTable) return table_has(ix.table, first, n, x);
-    if constexpr (SEARCH == kQuarter) return list_has(ix.csr + lo, n, x);
-    const uint64_t p = csr_lower_bound(ix.csr, lo, lo + n, x);
-    return p < lo + n && __ldg(ix.csr + p) == x;
+    if constexpr (SEARCH == kTable) {
+        return table_has(ix.table, first, n, x);
+    } else if constexpr (SEARCH == kLevels) {
+        return levels_have(ix, lo, n, x);
+    } else if constexpr (SEARCH == kQuarter) {
+        return list_has(ix.csr + lo, n, x);
+    } else {
+        const uint64_t p = csr_lower_bound(ix.csr, lo, lo + n, x);
+        return p < lo + n && __ldg(ix.csr + p) == x;
+    }
 }
 
 // Verdict on candidate x drawn with rand value rv (engine/engine.hpp:209-258,

@@ -55,7 +55,7 @@ __host__ __device__ constexpr int walk_ctas(bool sopr, bool coop) { return coop 
 // attempts that reject (3,878 walkers of length 80: 0.15 ms, 0.20 with groups;
 // 200,000 of length 40: 0.20 ms, 0.25 with the verdict).  8 CTAs an SM are 8 %
 // slower on a million walkers.
-template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX, bool GROUPS, bool SURE>
+template <bool SOPR, bool PATHS, bool COOP, bool W, int SEARCH, bool GROUPS, bool SURE>
 __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
     k_walk_incore(const __grid_constant__ IncoreArgs a)
 {
@@ -66,13 +66,16 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
     __shared__ uint32_t s_park[COOP ? kWalkThreads / 32 : 1][kPkCount][32];  // lane state during hard steps
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31u;
-    if (INDEX && a.sum && *a.sum != a.sum_built) return;
     if (lane < kWsCount) s_ws[warp][lane] = 0;
     s_hash[threadIdx.x] = s_steps[threadIdx.x] = 0;
     s_done[threadIdx.x] = 0;
     __syncwarp();
-    constexpr int kSearch = INDEX ? kTable : kQuarter;
-    const CsrIndex<kSearch> ix{a.csr, a.table};
+    constexpr bool INDEX = SEARCH == kTable;
+    constexpr int kHard = INDEX ? kTable : kQuarter;  // a hard step's list stays in the L1
+    const auto ix = [&]() {
+        if constexpr (SEARCH == kLevels) return CsrIndex<kLevels>{a.csr, &a.levels};
+        else return CsrIndex<SEARCH>{a.csr, a.table};
+    }();
     const uint32_t *__restrict__ csr = a.csr;
     const uint32_t maxhops = a.c.maxhops;
     const uint32_t chunk = a.chunk;
@@ -134,7 +137,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
                 if (PATHS && leads()) a.paths[(uint64_t)(wid - a.out_base) * a.stride] = src;
                 Vertex vx{0, 0, 0, 0};
                 if (src >= a.nverts) atomicOr(a.err, kErrSource);
-                else if (maxhops != 0) vx = load_vertex<INDEX>(a, src);
+                else if (maxhops != 0) vx = load_vertex<INDEX, SEARCH == kLevels>(a, src);
                 deg = vx.deg;
                 if (deg == 0) {
                     finish();  // bad source, no steps asked for, or a dead end (engine/engine.hpp:196-199)
@@ -211,7 +214,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
                                      __uint_as_float(pk[kPkThr2][L])};
                     const uint32_t astar = warp_first_accept<SOPR>(
                         a.c, tl, pk[kPkWid][L], pk[kPkHop][L], p0, kMaxAttempts, csr + hd, pk[kPkDeg][L],
-                        pk[kPkMagic][L], Lprev, Lcur, CsrIndex<kSearch>{csr + ph, a.table}, pk[kPkPbucket][L], Lpdeg,
+                        pk[kPkMagic][L], Lprev, Lcur, CsrIndex<kHard>{csr + ph, a.table}, pk[kPkPbucket][L], Lpdeg,
                         s_iv[COOP ? warp : 0]);
                     __syncwarp();  // every lane has read lane L's fields
                     if (lane == 0) {
@@ -262,18 +265,19 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
                 finish();
                 continue;
             }
-            const uint32_t pos = mod_by(r.x, deg, magic);
+            const uint32_t pos = SURE && !INDEX ? r.x % deg : mod_by(r.x, deg, magic);
             const float rv = rand_val(r.y, thr_max<SOPR>(a.c, t));
             uint32_t col = pos;
             if constexpr (W) {
                 const uint2 e = __ldg(a.alias + head + pos);
-                if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y;
+                // (a column past the list: a borrowed graph was written since its tables were built)
+                if (!(__uint2float_rn(r.w >> 8) * 0x1p-24f < __uint_as_float(e.x))) col = e.y < deg ? e.y : pos;
             }
             x = __ldg(csr + head + col);
             if (SURE) verdict = 1;
             else if (!GROUPS || (!end && att < kMaxAttempts)) verdict = accept_without_prev<SOPR>(a.c, t, rv, x, prev, cur);
             // the record of a vertex that is, or may be, the next one
-            if (verdict != 0 && !last && x < a.nverts) vx = load_vertex<INDEX>(a, x);
+            if (verdict != 0 && !last && x < a.nverts) vx = load_vertex<INDEX, SEARCH == kLevels>(a, x);
             if (!SURE && verdict < 0)
                 verdict = csr_contains(ix, pbucket, phead, pdeg, x) ? rv < thr_found<SOPR>(a.c, t)
                                                                     : rv < thr_notfound<SOPR>(a.c, t);
@@ -499,29 +503,57 @@ cudaError_t launch_build_table(const uint64_t *beg, const uint4 *verts, uint32_t
     return cudaGetLastError();
 }
 
-template <bool SOPR, bool PATHS, bool COOP, bool W, bool INDEX, bool SURE>
+__global__ void __launch_bounds__(256) k_sample_level(const uint32_t *__restrict__ src, uint64_t n,
+                                                      uint32_t *__restrict__ dst)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += stride) dst[j] = __ldg(src + 32 * j);
+}
+
+cudaError_t launch_sample_level(const uint32_t *src, uint64_t n, uint32_t *dst, int num_sms, cudaStream_t s)
+{
+    k_sample_level<<<(int)std::min<uint64_t>((n + 255) / 256, 8ull * num_sms), 256, 0, s>>>(src, n, dst);
+    return cudaGetLastError();
+}
+
+bool wants_levels(uint64_t nwalkers, uint64_t nedges, bool sopr, bool sure, int num_sms)
+{
+    return !sopr && !sure && 4 * nedges > kL2Bytes && 4 * nwalkers > walk_lanes(num_sms);
+}
+
+uint64_t walk_lanes(int num_sms) { return (uint64_t)walk_ctas(false, false) * kWalkThreads * num_sms; }
+
+template <bool SOPR, bool PATHS, bool COOP, bool W, int SEARCH, bool SURE>
 static int resident_grid(int num_sms)
 {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, INDEX, false, SURE>,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_incore<SOPR, PATHS, COOP, W, SEARCH, false, SURE>,
                                                   kWalkThreads, 0);
     return (per_sm < 1 ? 1 : per_sm) * num_sms;
 }
 
 // f called with the kernel's template arguments as compile-time constants.
 template <class F>
-static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool index, bool sure, F &&f)
+static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, int search, bool sure, F &&f)
 {
     using yes = std::true_type;
     using no = std::false_type;
-    const auto paths_index = [&](auto s, auto c, auto w, auto u) {
-        if (paths) return index ? f(s, yes{}, c, w, yes{}, u) : f(s, yes{}, c, w, no{}, u);
-        return index ? f(s, no{}, c, w, yes{}, u) : f(s, no{}, c, w, no{}, u);
+    using quarter = std::integral_constant<int, kQuarter>;
+    using levels = std::integral_constant<int, kLevels>;
+    using table = std::integral_constant<int, kTable>;
+    const auto by_search = [&](auto s, auto p, auto c, auto w, auto u) {
+        if (search == kTable) return f(s, p, c, w, table{}, u);
+        if constexpr (!s() && !u())
+            if (search == kLevels) return f(s, p, c, w, levels{}, u);
+        return f(s, p, c, w, quarter{}, u);
     };
-    if (weighted) return sure ? paths_index(no{}, no{}, yes{}, yes{}) : paths_index(no{}, no{}, yes{}, no{});
-    if (sopr) return paths_index(yes{}, yes{}, no{}, no{});  // SOPR steps get hard
-    if (sure) return paths_index(no{}, no{}, no{}, yes{});
-    return coop ? paths_index(no{}, yes{}, no{}, no{}) : paths_index(no{}, no{}, no{}, no{});
+    const auto by_paths = [&](auto s, auto c, auto w, auto u) {
+        return paths ? by_search(s, yes{}, c, w, u) : by_search(s, no{}, c, w, u);
+    };
+    if (weighted) return sure ? by_paths(no{}, no{}, yes{}, yes{}) : by_paths(no{}, no{}, yes{}, no{});
+    if (sopr) return by_paths(yes{}, yes{}, no{}, no{});  // SOPR steps get hard
+    if (sure) return by_paths(no{}, no{}, no{}, yes{});
+    return coop ? by_paths(no{}, yes{}, no{}, no{}) : by_paths(no{}, no{}, no{}, no{});
 }
 
 // Slots and claims by the number of walkers, which is all that decides them:
@@ -536,13 +568,13 @@ static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, bool in
 //   64; weighted 200,000: 0.67 / 0.77 / 0.76; hard Node2vec steps 3.25 / 4.44
 //   / 4.62; SOPR on 16.8 M walkers: no difference); walks of sure steps end
 //   together, so a claim fills the warp again.
-IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, bool index, bool sure,
+IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
                        int grid, int num_sms)
 {
     IncorePlan p{};
     p.ctas_per_sm = (uint32_t)walk_ctas(sopr, coop);
     p.grid = grid > 0 ? grid
-                      : walk_kernel(sopr, paths, coop, weighted, index, sure,
+                      : walk_kernel(sopr, paths, coop, weighted, search, sure,
                                     [&](auto s, auto pa, auto c, auto w, auto i, auto u) {
                                         return resident_grid<s(), pa(), c(), w(), i(), u()>(num_sms);
                                     });
@@ -555,10 +587,11 @@ IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool
 
 cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s)
 {
-    walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.verts != nullptr, sure_steps(sopr, a.c),
+    walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.search, sure_steps(sopr, a.c),
                 [&](auto so, auto pa, auto c, auto w, auto i, auto u) {
-                    if (!u() && a.slots < 32)
-                        k_walk_incore<so(), pa(), c(), w(), i(), !u(), u()><<<grid, kWalkThreads, 0, s>>>(a);
+                    // (levels are read by runs that fill the lanes)
+                    if (!u() && i() != kLevels && a.slots < 32)
+                        k_walk_incore<so(), pa(), c(), w(), i(), !u() && i() != kLevels, u()><<<grid, kWalkThreads, 0, s>>>(a);
                     else
                         k_walk_incore<so(), pa(), c(), w(), i(), false, u()><<<grid, kWalkThreads, 0, s>>>(a);
                     return 0;

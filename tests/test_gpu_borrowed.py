@@ -65,6 +65,31 @@ def test_writes_between_runs_are_walked(gw, oracle, degrees, algo, p, q, offset)
     eng.close()
 
 
+def test_weights_and_offsets_written_and_given_again(gw, oracle):
+    import torch
+    rng = np.random.default_rng(4)
+    V = 2500
+    deg = np.minimum(rng.zipf(1.7, V) + 1, 700)
+    beg, csr = graph_of(deg, rng)
+    d = [torch.from_numpy(x.copy()).cuda() for x in (beg.view(np.int64), csr.view(np.int32), np.ones(len(csr), np.float32))]
+    eng = gw.WalkEngine(algorithm=0, maxhops=30, p=0.5, q=2.0, seed=9, walkpersource=4)
+    eng.set_device_graph(V, len(csr), d[0].data_ptr(), d[1].data_ptr())
+    for k in range(3):
+        beg, csr = graph_of(rng.permutation(deg), rng)
+        w = rng.lognormal(0, 1, len(csr)).astype(np.float32)
+        for t, x in zip(d, (beg.view(np.int64), csr.view(np.int32), w)):
+            t.copy_(torch.from_numpy(x))
+        torch.cuda.synchronize()
+        eng.set_device_weights(d[2].data_ptr())
+        for _ in range(2):
+            eng.init_walkers()
+            eng.run()
+            ref = oracle.walk(beg, csr, oracle.make_cfg(algo=0, maxhops=30, p=0.5, q=2.0, seed=9, wps=4), 0, 4 * V,
+                              paths=False, alias=oracle.build_alias(beg, w))
+            assert np.array_equal(eng.hashes(), ref["hashes"])
+    eng.close()
+
+
 def test_an_invalid_write_is_refused(gw, oracle):
     import torch
     rng = np.random.default_rng(3)

@@ -807,10 +807,11 @@ int gw_handle::run_incore(gw_stats *stats)
                         (unsigned long long)nwalkers);
         return GW_OK;
     }
-    const IncorePlan plan = incore_plan(nwalkers, sopr, a.paths != nullptr, coop, weighted, a.search, sure,
+    const IncorePlan plan = incore_plan(nwalkers, nedges, sopr, a.paths != nullptr, coop, weighted, a.search, sure,
                                         (int)cfg.blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
+    a.one_wave = plan.one_wave;
     const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);  // with the error word
     // A borrowed CSR may have been written since its index was built: its
     // contents are summed beside the walk, which is done again if they are not

@@ -87,6 +87,7 @@ struct IncoreArgs {
     uint32_t out_base;         // first walker id of the population: outputs are indexed by wid - out_base
     uint32_t chunk;            // walkers a warp claims per atomic (incore_plan)
     uint32_t slots;            // walkers of a warp at a time (incore_plan)
+    uint32_t one_wave;         // a claim for every warp: taken in order of the warps' places, not of their start
     uint32_t *paths;           // rows indexed by walker id, or null
     uint32_t stride;           // maxhops + 1
     uint32_t *lens;            // vertices per path
@@ -173,11 +174,11 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v)
 // How an in-core run is launched.
 struct IncorePlan {
     int grid;               // CTAs
-    uint32_t slots, chunk;  // IncoreArgs
+    uint32_t slots, chunk, one_wave;  // IncoreArgs
     uint32_t ctas_per_sm;   // the kernel's register cap: CTAs of an SM it is built for
 };
 // `grid` CTAs as asked for, or (0) as many as are resident at once.
-IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
+IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
                        int grid, int num_sms);
 // a.alias set: weighted Node2vec.
 cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s);

@@ -187,10 +187,11 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
     const bool sopr = cfg->algorithm != GW_NODE2VEC;
     const bool coop = needs_coop(cfg->algorithm, a.c);
     const IncorePlan plan =
-        incore_plan(nwalkers, sopr, a.paths != nullptr, coop, false, kQuarter, sure_steps(sopr, a.c),
+        incore_plan(nwalkers, nedges, sopr, a.paths != nullptr, coop, false, kQuarter, sure_steps(sopr, a.c),
                     (int)cfg->blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
+    a.one_wave = plan.one_wave;
     e = launch_walk_incore(a, sopr, coop, plan.grid, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, sizeof(host_ctr), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

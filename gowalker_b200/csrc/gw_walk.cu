@@ -116,8 +116,12 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(&a.ctr[kCtrCursor], (unsigned long long)chunk);
-                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                if (a.one_wave) {
+                    base = q_end ? a.nwalkers : (unsigned long long)(warp * gridDim.x + blockIdx.x) * chunk;
+                } else {
+                    if (lane == 0) base = atomicAdd(&a.ctr[kCtrCursor], (unsigned long long)chunk);
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                }
                 if (base >= a.nwalkers) {
                     exhausted = true;
                     break;
@@ -556,19 +560,30 @@ static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, int sea
     return coop ? by_paths(no{}, yes{}, no{}, no{}) : by_paths(no{}, no{}, no{}, no{});
 }
 
-// Slots and claims by the number of walkers, which is all that decides them:
+// Slots and claims by the number of walkers, which is what decides them first:
 // - few walkers are spread over the warps, down to one each, as long as a
 //   scheduler then has about four warps: a round costs a warp the instructions
 //   of all its lanes' branches, so fewer walkers are faster until the schedulers
 //   are busy (1,024 walkers of length 30, one lane a walker: 0.093 ms at one a
-//   warp, 0.154 at 32; 65,536: 0.23 ms at 32, 0.32 at 16);
+//   warp, 0.154 at 32; 65,536: 0.23 ms at 32, 0.32 at 16); walks of sure steps
+//   go four a warp at least (3,878 walkers 0.107 ms at two, 0.080 at four);
 // - a claim fills a warp when the run is one wave, so that no more warps than
 //   needed share the walkers; later waves claim eight at a time, which evens
 //   out the end of the run (600,000 walkers: 1.75 ms at 8, 1.82 at 32, 1.98 at
 //   64; weighted 200,000: 0.67 / 0.77 / 0.76; hard Node2vec steps 3.25 / 4.44
 //   / 4.62; SOPR on 16.8 M walkers: no difference); walks of sure steps end
-//   together, so a claim fills the warp again.
-IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
+//   together, so a claim fills the warp again; walks of a CSR past the L2
+//   without tables wait for memory, and sixteen lanes a warp wait less than
+//   thirty-two, so theirs are claims of eight in one wave too (100,000 walkers
+//   on 64 M edges 0.66 ms, 0.82 at 32, through levels 0.67 / 0.90);
+// - one wave's claims go to the first warp of every CTA, then to the second: taken
+//   as warps come, they fell to the CTAs that started first, on some devices
+//   several to an SM and none on others (180,000 walks of length 200 on one of
+//   them 2.70 ms, 1.47 so; 100,000 sure ones 0.084, 0.057; elsewhere the same);
+// - no more CTAs than walkers need where each gets an SM to itself: the others
+//   find none, but take 12 us to come and go (3,878 sure walks 0.080 -> 0.062
+//   ms, 1,024 of Node2vec 0.062 -> 0.049).
+IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
                        int grid, int num_sms)
 {
     IncorePlan p{};
@@ -579,9 +594,13 @@ IncorePlan incore_plan(uint64_t nwalkers, bool sopr, bool paths, bool coop, bool
                                         return resident_grid<s(), pa(), c(), w(), i(), u()>(num_sms);
                                     });
     const uint64_t warps = (uint64_t)p.grid * (kWalkThreads / 32), busy = std::min<uint64_t>(warps, 16ull * num_sms);
-    p.slots = 1;
+    p.slots = sure ? 4 : 1;
     while (p.slots < 32 && p.slots * busy < nwalkers) p.slots *= 2;
-    p.chunk = nwalkers <= 32 * warps ? p.slots : sure ? 32 : 8;
+    const bool waits = !sure && search != kTable && 4 * nedges > kL2Bytes;
+    p.chunk = nwalkers <= 32 * warps ? (waits ? std::min(p.slots, 8u) : p.slots) : sure ? 32 : 8;
+    const uint64_t need = (nwalkers + p.slots * (kWalkThreads / 32) - 1) / (p.slots * (kWalkThreads / 32));
+    if (grid <= 0 && need <= (uint64_t)num_sms) p.grid = (int)need;
+    p.one_wave = p.chunk == p.slots && need <= (uint64_t)p.grid;
     return p;
 }
 

@@ -9,12 +9,14 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <thread>
 #include <vector>
 #include <sys/mman.h>
 #include "gw_engine.cuh"
+#include "gw_memory.cuh"
 
 using namespace gw;
 
@@ -41,15 +43,50 @@ int gw_handle::cuda(cudaError_t e, const char *what)
 
 int gw_handle::dev_alloc(void **p, uint64_t bytes, const char *what)
 {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && d_index) {
-        cudaGetLastError();
-        cudaStreamSynchronize(s_compute);
-        drop_index();
-        index_refused = true;
-        e = cudaMalloc(p, bytes);
+    return cuda(device_malloc_any(p, bytes, this), what);
+}
+
+// Every engine, so that one's index can give way to another's allocation.  The
+// lists and gw_handle::in_call are guarded by the mutex; an index is dropped
+// under it, or by a call of its own engine, which others see by in_call.
+namespace {
+struct Engines {
+    std::mutex mu;
+    std::vector<gw_handle *> all;
+};
+Engines &engines()
+{
+    static Engines *e = new Engines;  // outlives every static
+    return *e;
+}
+struct InCall {
+    explicit InCall(gw_handle *h) : h(h) { set(true); }
+    ~InCall() { set(false); }
+    void set(bool v)
+    {
+        std::lock_guard<std::mutex> l(engines().mu);
+        h->in_call = v;
     }
-    return cuda(e, what);
+    gw_handle *h;
+};
+}  // namespace
+
+cudaError_t gw::device_malloc_any(void **p, size_t bytes, gw_handle *self)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> l(engines().mu);
+    for (gw_handle *h : engines().all) {
+        if (h->cfg.device != dev || (h->in_call && h != self) || !h->d_index) continue;
+        cudaGetLastError();
+        cudaStreamSynchronize(h->s_compute);
+        h->drop_index();
+        h->index_refused = true;
+        if ((e = cudaMalloc(p, bytes)) != cudaErrorMemoryAllocation) break;
+    }
+    return e;
 }
 
 void gw::consts_from_config(const gw_config &c, StepConsts &k)
@@ -199,16 +236,23 @@ int gw_handle::init_device()
     if ((st = cuda(cudaEventCreate(&ev_kernel0), "event"))) return st;
     if ((st = cuda(cudaEventCreate(&ev_kernel1), "event"))) return st;
     if ((st = cuda(cudaEventCreate(&ev_stop), "event"))) return st;
-    if ((st = cuda(cudaMalloc(&d_ctr, sizeof(unsigned long long) * kCtrWords), "counters"))) return st;
+    if ((st = dev_alloc(d_ctr, sizeof(unsigned long long) * kCtrWords, "counters"))) return st;
     d_err = reinterpret_cast<uint32_t *>(d_ctr + kCtrCount);
     if ((st = cuda(cudaMallocHost(&h_ctr, sizeof(unsigned long long) * kCtrWords), "pinned counters")))
         return st;
     memset(h_ctr, 0, sizeof(unsigned long long) * kCtrWords);
+    std::lock_guard<std::mutex> l(engines().mu);
+    engines().all.push_back(this);
     return GW_OK;
 }
 
 void gw_handle::release()
 {
+    {
+        std::lock_guard<std::mutex> l(engines().mu);
+        auto &all = engines().all;
+        all.erase(std::remove(all.begin(), all.end(), this), all.end());
+    }
     cudaSetDevice(cfg.device);
     if (s_compute) cudaStreamSynchronize(s_compute);
     if (s_copy) cudaStreamSynchronize(s_copy);
@@ -375,6 +419,9 @@ extern "C" int gw_set_graph_meta(gw_handle *h, uint32_t nverts, uint64_t nedges,
     h->own_csr = nullptr;
     h->ooc_release();
     h->walkers_ready = false;
+    std::lock_guard<std::mutex> l(engines().mu);
+    h->index_search = kQuarter;
+    if (h->index_cap >= gw_handle::kSmallIndex) h->drop_index();  // a small one's memory serves the next graph
     return GW_OK;
 }
 
@@ -540,7 +587,7 @@ gw_handle::IndexLayout gw_handle::index_layout(int search) const
 }
 
 // Memory for that index.  An index is worth having, not needed: a large one
-// takes at most half of what is free, and none is no error; after a refusal
+// takes at most a quarter of what is free, and none is no error; after a refusal
 // another attempt is made only where it has room.
 bool gw_handle::reserve_index(int search)
 {
@@ -553,7 +600,7 @@ bool gw_handle::reserve_index(int search)
             cudaGetLastError();
             return false;
         }
-        if (l.bytes > (l.bytes >= kSmallIndex ? free_bytes / 2 : free_bytes)) {
+        if (l.bytes > (l.bytes >= kSmallIndex ? free_bytes / 4 : free_bytes)) {
             index_refused = true;
             return false;
         }
@@ -890,6 +937,7 @@ extern "C" int gw_run(gw_handle *h, uint32_t policy, gw_stats *stats)
     if (h->nblocks == 0) return h->fail(GW_ERR_STATE, "no graph");
     if (!h->walkers_ready) return h->fail(GW_ERR_STATE, "call gw_init_walkers first");
     cudaSetDevice(h->cfg.device);
+    InCall in_call(h);
     int st = h->ensure_outputs();
     if (st) return st;
     const bool incore = h->device_graph || h->graph_bytes() <= h->cfg.cache_size;

@@ -91,8 +91,9 @@ struct gw_handle {
 
     int fail(int status, const char *fmt, ...);
     int cuda(cudaError_t e, const char *what);
-    // Device memory; the index of a resident CSR, which walks can do without,
-    // gives way to anything that they cannot.
+    bool in_call = false;  // a run of this engine, which may read its index
+    // Device memory (device_malloc): all that a handle allocates but its index,
+    // which gives way.
     int dev_alloc(void **p, uint64_t bytes, const char *what);
     template <class T>
     int dev_alloc(T *&p, uint64_t bytes, const char *what)

@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include "gw_fixedmath.cuh"
+#include "gw_memory.cuh"
 #include "gw_philox.cuh"
 #include "../../include/gowalker.h"
 
@@ -504,14 +505,14 @@ static cudaError_t csr_from_sorted(const uint64_t *keys, uint64_t n, uint32_t sh
     const uint64_t gap_bytes = 16 + (nb / kLongGap + 1) * sizeof(Gap);
     cudaError_t e;
     do {
-        if ((e = cudaMalloc(&beg, nb * sizeof(uint64_t))) != cudaSuccess) break;
-        if ((e = cudaMalloc(&csr, (n ? n : 1) * sizeof(uint32_t))) != cudaSuccess) break;
+        if ((e = device_malloc(&beg, nb * sizeof(uint64_t))) != cudaSuccess) break;
+        if ((e = device_malloc(&csr, (n ? n : 1) * sizeof(uint32_t))) != cudaSuccess) break;
         if (n == 0) {
             if ((e = cudaMemsetAsync(beg, 0, nb * sizeof(uint64_t), s)) != cudaSuccess) break;
         } else {
             char *p = (char *)scratch;
             if (scratch_bytes < gap_bytes) {
-                if ((e = cudaMalloc(&own, gap_bytes)) != cudaSuccess) break;
+                if ((e = device_malloc(&own, gap_bytes)) != cudaSuccess) break;
                 p = own;
             }
             unsigned long long *count = (unsigned long long *)p;
@@ -597,17 +598,17 @@ static int sampled_csr(const Sampler &smp, uint64_t nsamples, uint32_t nverts, b
             goto out;                     \
         }                                 \
     } while (0)
-    SC_CHECK(cudaMalloc(&d_cur, sizeof(unsigned long long)));
-    SC_CHECK(cudaMalloc(&d_nsel, sizeof(int64_t)));
+    SC_CHECK(device_malloc(&d_cur, sizeof(unsigned long long)));
+    SC_CHECK(device_malloc(&d_nsel, sizeof(int64_t)));
     SC_CHECK(cudaMemsetAsync(d_cur, 0, sizeof(unsigned long long), s));
     k_sample_keys<Sampler, true><<<blocks, 256, 0, s>>>(smp, nsamples, sh, symmetric ? 1 : 0, nullptr, d_cur);
     SC_CHECK(cudaGetLastError());
     SC_CHECK(cudaMemcpyAsync(&h_cur, d_cur, sizeof(h_cur), cudaMemcpyDeviceToHost, s));
     SC_CHECK(cudaStreamSynchronize(s));
     U = h_cur;
-    SC_CHECK(cudaMalloc(&keys, (U ? U : 1) * sizeof(uint64_t)));
+    SC_CHECK(device_malloc(&keys, (U ? U : 1) * sizeof(uint64_t)));
     scratch = (U ? U : 1) * sizeof(uint64_t);
-    SC_CHECK(cudaMalloc(&alt, scratch));
+    SC_CHECK(device_malloc(&alt, scratch));
     SC_CHECK(cudaMemsetAsync(d_cur, 0, sizeof(unsigned long long), s));
     k_sample_keys<Sampler, false><<<blocks, 256, 0, s>>>(smp, nsamples, sh, symmetric ? 1 : 0, keys, d_cur);
     SC_CHECK(cudaGetLastError());
@@ -617,7 +618,7 @@ static int sampled_csr(const Sampler &smp, uint64_t nsamples, uint32_t nverts, b
         SC_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, db, U, 0, b1, s));
         SC_CHECK(cub::DeviceSelect::Unique(nullptr, tb2, keys, alt, d_nsel, (int64_t)U, s));
         tmp_bytes = std::max(tmp_bytes, tb2);
-        SC_CHECK(cudaMalloc(&tmp, tmp_bytes));
+        SC_CHECK(device_malloc(&tmp, tmp_bytes));
         SC_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, db, U, 0, b1, s));
         keys = db.Current();
         alt = db.Alternate();
@@ -709,13 +710,13 @@ extern "C" int gw_web_csr(uint32_t scale, uint32_t nverts, const uint32_t thr[3]
             goto out;                     \
         }                                 \
     } while (0)
-    WB_CHECK(cudaMalloc(&deg, nb * sizeof(unsigned long long)));
-    WB_CHECK(cudaMalloc(&estart, nb * sizeof(unsigned long long)));
-    WB_CHECK(cudaMalloc(&d_nsel, sizeof(int64_t)));
+    WB_CHECK(device_malloc(&deg, nb * sizeof(unsigned long long)));
+    WB_CHECK(device_malloc(&estart, nb * sizeof(unsigned long long)));
+    WB_CHECK(device_malloc(&d_nsel, sizeof(int64_t)));
     k_web_degrees<<<148 * 8, 256, 0, s>>>(p, deg);
     WB_CHECK(cudaGetLastError());
     WB_CHECK(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, deg, estart, nb, s));
-    WB_CHECK(cudaMalloc(&tmp, tmp_bytes));
+    WB_CHECK(device_malloc(&tmp, tmp_bytes));
     WB_CHECK(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, deg, estart, nb, s));
     WB_CHECK(cudaMemcpyAsync(&M, estart + nverts, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
     WB_CHECK(cudaStreamSynchronize(s));
@@ -723,8 +724,8 @@ extern "C" int gw_web_csr(uint32_t scale, uint32_t nverts, const uint32_t thr[3]
     tmp = nullptr;
     cudaFree(deg);
     deg = nullptr;
-    WB_CHECK(cudaMalloc(&keys, (M ? M : 1) * sizeof(uint64_t)));
-    WB_CHECK(cudaMalloc(&alt, (M ? M : 1) * sizeof(uint64_t)));
+    WB_CHECK(device_malloc(&keys, (M ? M : 1) * sizeof(uint64_t)));
+    WB_CHECK(device_malloc(&alt, (M ? M : 1) * sizeof(uint64_t)));
     k_web_edges<<<148 * 16, 128, 0, s>>>(p, estart, sh, keys);
     WB_CHECK(cudaGetLastError());
     if (M) {
@@ -733,7 +734,7 @@ extern "C" int gw_web_csr(uint32_t scale, uint32_t nverts, const uint32_t thr[3]
         WB_CHECK(cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, db, M, 0, b1, s));
         WB_CHECK(cub::DeviceSelect::Unique(nullptr, tb2, keys, alt, d_nsel, (int64_t)M, s));
         tmp_bytes = std::max(tmp_bytes, tb2);
-        WB_CHECK(cudaMalloc(&tmp, tmp_bytes));
+        WB_CHECK(device_malloc(&tmp, tmp_bytes));
         WB_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, db, M, 0, b1, s));
         keys = db.Current();
         alt = db.Alternate();
@@ -833,7 +834,7 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
             }
         }
         tmp_room = (tmp_bytes + 255) & ~size_t(255);
-        GEN_CHECK(cudaMalloc(&scratch, 2 * key_bytes + 256 + tmp_room));
+        GEN_CHECK(device_malloc(&scratch, 2 * key_bytes + 256 + tmp_room));
         keys = (uint64_t *)scratch;
         alt = (uint64_t *)(scratch + key_bytes);
         char *small = scratch + 2 * key_bytes;
@@ -901,7 +902,7 @@ extern "C" int gw_edges_csr(const uint32_t *src, const uint32_t *dst, uint64_t n
             tmp_bytes = std::max(tmp_bytes, tb2);
         }
         if (tmp_bytes > tmp_room) {  // fewer keys should not need more, but nothing says so
-            GEN_CHECK(cudaMalloc(&own_tmp, tmp_bytes));
+            GEN_CHECK(device_malloc(&own_tmp, tmp_bytes));
             tmp = own_tmp;
         }
         GEN_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, db, nsort, b0, b1, s));
@@ -951,7 +952,7 @@ extern "C" int gw_split_blocks(const uint64_t *beg, uint32_t nverts, uint32_t mo
     uint32_t count = 0;
     const uint64_t slots = mode == GW_SPLIT_EQUAL_EDGES ? param + 1 : (uint64_t)cap + 1;
     if (!device_accessible(beg)) {
-        GEN_CHECK(cudaMalloc(&own, nv * sizeof(uint64_t)));
+        GEN_CHECK(device_malloc(&own, nv * sizeof(uint64_t)));
         GEN_CHECK(cudaMemcpy(own, beg, nv * sizeof(uint64_t), cudaMemcpyDefault));
         d_beg = own;
     }
@@ -960,9 +961,9 @@ extern "C" int gw_split_blocks(const uint64_t *beg, uint32_t nverts, uint32_t mo
         rc = GW_ERR_ARG;
         goto done;
     }
-    GEN_CHECK(cudaMalloc(&d_vb, slots * sizeof(uint32_t)));
-    GEN_CHECK(cudaMalloc(&d_eb, slots * sizeof(uint64_t)));
-    GEN_CHECK(cudaMalloc(&d_count, sizeof(uint32_t)));
+    GEN_CHECK(device_malloc(&d_vb, slots * sizeof(uint32_t)));
+    GEN_CHECK(device_malloc(&d_eb, slots * sizeof(uint64_t)));
+    GEN_CHECK(device_malloc(&d_count, sizeof(uint32_t)));
     if (mode == GW_SPLIT_REFERENCE) {
         k_split_reference<<<1, 32, 0, s>>>(d_beg, nv, param / sizeof(uint32_t), param / sizeof(uint64_t), cap, d_vb,
                                            d_eb, d_count);

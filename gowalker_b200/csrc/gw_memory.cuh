@@ -1,0 +1,20 @@
+// Device memory of the library (internal to libgowalker.so).
+#pragma once
+#include <cuda_runtime.h>
+#include <cstddef>
+
+struct gw_handle;
+
+namespace gw {
+
+// cudaMalloc.  On a full device the index of a resident CSR, which walks can do
+// without, gives way: that of any engine on the current device that no call is
+// using, and that of `self` (the engine whose call this is, or null).
+cudaError_t device_malloc_any(void **p, size_t bytes, gw_handle *self = nullptr);
+template <class T>
+inline cudaError_t device_malloc(T **p, size_t bytes)
+{
+    return device_malloc_any((void **)p, bytes);
+}
+
+}  // namespace gw

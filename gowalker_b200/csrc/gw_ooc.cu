@@ -17,6 +17,7 @@
 #include <cstring>
 #include <vector>
 #include "gw_engine.cuh"
+#include "gw_memory.cuh"
 #include "gw_ooc_kernels.cuh"
 #include "gw_mlp.cuh"
 #include "gw_compress.cuh"
@@ -255,7 +256,7 @@ static int learned_setup(gw_handle *h)
     if (o.learned_ready) return GW_OK;
     const uint32_t nb = o.nb;
     int st;
-    auto dalloc = [&](float **p, uint64_t n, const char *what) { return h->cuda(cudaMalloc(p, n * sizeof(float)), what); };
+    auto dalloc = [&](float **p, uint64_t n, const char *what) { return h->dev_alloc(*p, n * sizeof(float), what); };
     if ((st = dalloc(&o.d_params, kMlpParams, "predictor weights"))) return st;
     if ((st = dalloc(&o.d_params_train, kMlpParams, "predictor weights"))) return st;
     if ((st = h->cuda(cudaStreamCreateWithFlags(&o.ts, cudaStreamNonBlocking), "training stream"))) return st;
@@ -367,7 +368,7 @@ static int ooc_setup(gw_handle *h)
     beg_bytes = ((uint64_t)h->nverts + 1) * 8;
     if ((st = h->dev_alloc(o.d_beg, beg_bytes, "vertex offsets"))) return st;
     if ((st = h->dev_alloc(o.slot_csr, o.nslots * o.slot_stride_words * 4, "slot neighbours"))) return st;
-    if ((st = h->cuda(cudaMalloc((void **)&o.d_blk_csr, 2 * nb * sizeof(void *)), "block table"))) return st;
+    if ((st = h->dev_alloc(o.d_blk_csr, 2 * nb * sizeof(void *), "block table"))) return st;
     if ((st = h->cuda(cudaMallocHost((void **)&o.h_blk_csr, 2 * nb * sizeof(void *)), "block table"))) return st;
     for (int k = 0; k < 2; ++k) {
         if ((st = h->cuda(cudaHostAlloc((void **)&o.h_blk_pin[k], 2 * nb * sizeof(void *), cudaHostAllocMapped),
@@ -384,24 +385,24 @@ static int ooc_setup(gw_handle *h)
         if ((st = h->cuda(cudaHostGetDevicePointer((void **)&o.dm_snap[k], o.h_snap[k], 0), "counter snapshot")))
             return st;
     }
-    if ((st = h->cuda(cudaMalloc(&o.d_n, 2 * sizeof(uint32_t)), "walker count"))) return st;
+    if ((st = h->dev_alloc(o.d_n, 2 * sizeof(uint32_t), "walker count"))) return st;
     if ((st = h->cuda(cudaMallocHost(&o.h_n, sizeof(uint32_t)), "walker count"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_vstart, (nb + 1) * sizeof(uint32_t)), "vstart"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_estart, (nb + 1) * sizeof(uint64_t)), "estart"))) return st;
+    if ((st = h->dev_alloc(o.d_vstart, (nb + 1) * sizeof(uint32_t), "vstart"))) return st;
+    if ((st = h->dev_alloc(o.d_estart, (nb + 1) * sizeof(uint64_t), "estart"))) return st;
     if ((st = h->cuda(cudaHostAlloc((void **)&o.h_cached, nb * sizeof(uint32_t), cudaHostAllocMapped), "cached list")))
         return st;
     if ((st = h->cuda(cudaHostGetDevicePointer((void **)&o.d_cached, o.h_cached, 0), "cached list"))) return st;
     const uint64_t nbk = 2ull * nb * nb;
-    if ((st = h->cuda(cudaMalloc(&o.d_pairs, nbk / 2 * sizeof(uint32_t)), "pair counts"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_counts, nbk * sizeof(uint32_t)), "bucket counts"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_offsets, (nbk + 1) * sizeof(uint32_t)), "bucket offsets"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_cursor, nbk * sizeof(uint32_t)), "bucket cursors"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_run_pre, (nbk + 1) * sizeof(uint32_t)), "runnable prefix"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_run_off, nbk * sizeof(uint32_t)), "runnable offsets"))) return st;
-    if ((st = h->cuda(cudaMalloc(&o.d_nrun, 16 + sizeof(OocClock)), "runnable count"))) return st;
+    if ((st = h->dev_alloc(o.d_pairs, nbk / 2 * sizeof(uint32_t), "pair counts"))) return st;
+    if ((st = h->dev_alloc(o.d_counts, nbk * sizeof(uint32_t), "bucket counts"))) return st;
+    if ((st = h->dev_alloc(o.d_offsets, (nbk + 1) * sizeof(uint32_t), "bucket offsets"))) return st;
+    if ((st = h->dev_alloc(o.d_cursor, nbk * sizeof(uint32_t), "bucket cursors"))) return st;
+    if ((st = h->dev_alloc(o.d_run_pre, (nbk + 1) * sizeof(uint32_t), "runnable prefix"))) return st;
+    if ((st = h->dev_alloc(o.d_run_off, nbk * sizeof(uint32_t), "runnable offsets"))) return st;
+    if ((st = h->dev_alloc(o.d_nrun, 16 + sizeof(OocClock), "runnable count"))) return st;
     o.d_clock = reinterpret_cast<OocClock *>(o.d_nrun + 4);
 
-    if ((st = h->cuda(cudaMalloc(&o.d_sa, sizeof(SaState)), "annealing state"))) return st;
+    if ((st = h->dev_alloc(o.d_sa, sizeof(SaState), "annealing state"))) return st;
     if ((st = h->cuda(cudaHostAlloc((void **)&o.h_dec, sizeof(Decision), cudaHostAllocMapped), "decision"))) return st;
     if ((st = h->cuda(cudaHostGetDevicePointer((void **)&o.d_dec, o.h_dec, 0), "decision"))) return st;
     if ((st = h->cuda(cudaMemcpy(o.d_vstart, h->vblocks.data(), (nb + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice),
@@ -567,11 +568,11 @@ static int ooc_build_alias(gw_handle *h, cudaStream_t s, uint64_t *h2d)
     int st = GW_OK;
     o.halias.assign(nb, nullptr);
     do {
-        if ((st = h->cuda(cudaMalloc(&rel, (maxv + 1) * sizeof(uint64_t)), "alias build scratch")) ||
-            (st = h->cuda(cudaMalloc(&dw, maxe * sizeof(float)), "alias build scratch")) ||
-            (st = h->cuda(cudaMalloc(&pd, maxe * sizeof(double)), "alias build scratch")) ||
-            (st = h->cuda(cudaMalloc(&q, (2 * maxe + maxv + 2) * sizeof(uint32_t)), "alias build scratch")) ||
-            (st = h->cuda(cudaMalloc(&out, maxe * sizeof(AliasEntry)), "alias build scratch")))
+        if ((st = h->dev_alloc(rel, (maxv + 1) * sizeof(uint64_t), "alias build scratch")) ||
+            (st = h->dev_alloc(dw, maxe * sizeof(float), "alias build scratch")) ||
+            (st = h->dev_alloc(pd, maxe * sizeof(double), "alias build scratch")) ||
+            (st = h->dev_alloc(q, (2 * maxe + maxv + 2) * sizeof(uint32_t), "alias build scratch")) ||
+            (st = h->dev_alloc(out, maxe * sizeof(AliasEntry), "alias build scratch")))
             break;
         for (uint32_t b = 0; b < nb && !st; ++b) {
             const uint64_t ne = h->eblocks[b + 1] - h->eblocks[b];
@@ -1313,7 +1314,7 @@ int gw_handle::run_ooc(uint32_t policy, gw_stats *stats)
                     o.h_blk_csr[b] = o.map_csr[b];
                     mapped[b] = 1;
                 }
-            if (!o.d_mapped && (st = cuda(cudaMalloc(&o.d_mapped, nb), "mapped-block flags"))) break;
+            if (!o.d_mapped && (st = dev_alloc(o.d_mapped, nb, "mapped-block flags"))) break;
             if ((st = cuda(cudaMemcpyAsync(o.d_mapped, mapped.data(), nb, cudaMemcpyHostToDevice, s), "mapped flags")))
                 break;
             push_tables();
@@ -1656,8 +1657,8 @@ extern "C" int gw_plain_choose_block(const uint32_t *counts, uint32_t nblocks, c
     Decision h{};
     int rc = GW_OK;
     do {
-        if (cudaMalloc(&d_counts, nn * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&d_live, sizeof(uint32_t)) != cudaSuccess || cudaMalloc(&d_dec, sizeof(Decision)) != cudaSuccess) {
+        if (device_malloc(&d_counts, nn * sizeof(uint32_t)) != cudaSuccess ||
+            device_malloc(&d_live, sizeof(uint32_t)) != cudaSuccess || device_malloc(&d_dec, sizeof(Decision)) != cudaSuccess) {
             rc = GW_ERR_NOMEM;
             break;
         }

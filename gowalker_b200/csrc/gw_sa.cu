@@ -30,6 +30,7 @@
 #include <cstddef>
 #include <cstdint>
 #include "gw_fixedmath.cuh"
+#include "gw_memory.cuh"
 #include "gw_ooc_kernels.cuh"
 #include "gw_philox.cuh"
 #include "../../include/gowalker.h"
@@ -314,9 +315,9 @@ extern "C" int gw_sa_choose_blocks(const uint32_t *counts, uint32_t nblocks, con
     h.k = 0;
     h.calls = call;
     do {
-        if (cudaMalloc(&d_counts, (size_t)nblocks * nblocks * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&d_cached, (ncached ? ncached : 1) * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMalloc(&d_st, sizeof(SaState)) != cudaSuccess) {
+        if (device_malloc(&d_counts, (size_t)nblocks * nblocks * sizeof(uint32_t)) != cudaSuccess ||
+            device_malloc(&d_cached, (ncached ? ncached : 1) * sizeof(uint32_t)) != cudaSuccess ||
+            device_malloc(&d_st, sizeof(SaState)) != cudaSuccess) {
             rc = GW_ERR_NOMEM;
             break;
         }

@@ -262,7 +262,11 @@ int gw_init_walker_range(gw_handle *h, uint32_t algo, uint32_t walkpersource, ui
 /* Runs every walker to the end.  Replaces graph_engine::pipe_run
  * (engine/engine.hpp:517-638) with its pipeline / zero_gpujob launches
  * (406-515): the plain or learned block policy, device bucketing, and the
- * step kernels of gpu/gpuwalk.hpp. */
+ * step kernels of gpu/gpuwalk.hpp.  In-core runs that take many steps build an
+ * index of the graph, 10 to 13 bytes an edge and up to 48 a vertex: 256 MB, or a
+ * quarter of the memory that is free where that is more.  It is kept for later
+ * runs on the graph, and gives way where an allocation of this library, by this
+ * handle or another, finds the device full. */
 int gw_run(gw_handle *h, uint32_t policy, gw_stats *stats);
 
 /* Walker count of the current population. */

@@ -84,12 +84,46 @@ inline void philox_schedule(uint32_t k0, uint32_t k1, uint32_t *rk0, uint32_t *r
     }
 }
 
+// x % d with a precomputed m = floor((2^32 - 1) / d): m > 2^32 / d - 1 - 1 / d
+// and an integer, so m >= 2^32 / d - 1 and x m / 2^32 > x / d - 1; the quotient
+// falls short by at most one and one correction gives the remainder exactly.
+GW_HD uint32_t mod_magic(uint32_t d) { return 0xFFFFFFFFu / d; }
+GW_HD uint32_t mod_by(uint32_t x, uint32_t d, uint32_t m)
+{
+#if defined(__CUDA_ARCH__)
+    uint32_t r = x - __umulhi(x, m) * d;
+#else
+    uint32_t r = x - (uint32_t)(((uint64_t)x * m) >> 32) * d;
+#endif
+    if (r >= d) r -= d;
+    return r;
+}
+
 // Exact a % d for 32-bit a and d >= 1 by direct computation (Lemire, Kaser and
 // Kurz, "Faster remainder by direct computation", 2019): with the 64-bit
 // fraction M = ceil(2^64 / d), a % d = high64((M * a mod 2^64) * d).  M costs one
 // 64-bit division, so it pays off when one divisor serves many draws -- the
 // warp-uniform degree of a cooperative step.
 GW_HD uint64_t fastmod_magic(uint32_t d) { return ~0ull / d + 1; }
+// The same without a 64-bit division, from m = mod_magic(d) and 1 / d within
+// four units in the last place: 2^64 - 1 = (m 2^32 + q) d + rest, where q is the
+// quotient of n = (2^32 - 1 - m d) 2^32 + 2^32 - 1.  q is estimated from below by
+// at most 2^13 (n, 1 / d and their product are off by less than 2^-20 together),
+// what is left, below 2^46, is divided in turn, its quotient of 13 bits off by
+// one at most, and that one is put right.
+GW_HD uint64_t fastmod_magic_by(uint32_t d, uint32_t m, float inv)
+{
+    const uint32_t r = 0xFFFFFFFFu - m * d;
+    const uint64_t n = ((uint64_t)r << 32) | 0xFFFFFFFFu;
+    uint32_t q = (uint32_t)((float)(r + 1) * inv * ((1.0f - 0x1p-20f) * 0x1p32f));
+    int64_t left = (int64_t)(n - (uint64_t)q * d);
+    const uint32_t c = (uint32_t)(((float)(uint32_t)(left >> 32) * 0x1p32f + (float)(uint32_t)left) * inv);
+    q += c;
+    left -= (int64_t)((uint64_t)c * d);
+    if (left < 0) --q;
+    else if (left >= (int64_t)d) ++q;
+    return (((uint64_t)m << 32) | q) + 1;
+}
 GW_HD uint32_t fastmod(uint32_t a, uint64_t M, uint32_t d)
 {
     const uint64_t low = M * (uint64_t)a;
@@ -98,6 +132,24 @@ GW_HD uint32_t fastmod(uint32_t a, uint64_t M, uint32_t d)
 #else
     return (uint32_t)(((unsigned __int128)low * d) >> 64);
 #endif
+}
+
+// The top words of the fractions M * a mod 2^64 of the draws a = p, p + d, ... for
+// positions p in [lo, hi), hi <= d: first and last.  M d passes 2^64 by less than
+// d, so a draw's fraction passes M p by less than 2^32: by one in the top word.
+GW_HD uint32_t fraction_top(uint32_t a, uint64_t M)
+{
+#if defined(__CUDA_ARCH__)
+    return (uint32_t)(M >> 32) * a + __umulhi((uint32_t)M, a);
+#else
+    return (uint32_t)((M * a) >> 32);
+#endif
+}
+GW_HD uint32_t fraction_first(uint32_t lo, uint64_t M) { return fraction_top(lo, M); }
+GW_HD uint32_t fraction_last(uint32_t hi, uint64_t M)
+{
+    const uint32_t t = fraction_top(hi - 1, M);
+    return t + (t != 0xFFFFFFFFu ? 1u : 0u);
 }
 
 // FNV-1a over 32-bit words: the per-walker path hash.

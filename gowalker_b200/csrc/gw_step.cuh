@@ -97,17 +97,6 @@ __device__ __forceinline__ U4 draw(const StepConsts &c, uint32_t wid, uint32_t h
     return philox4x32_10_sched(wid, hop, attempt, kTagWalk, c.rk0, c.rk1);
 }
 
-// x % d with a precomputed m = floor((2^32 - 1) / d): m > 2^32 / d - 1 - 1 / d
-// and an integer, so m >= 2^32 / d - 1 and x m / 2^32 > x / d - 1; the quotient
-// falls short by at most one and one correction gives the remainder exactly.
-__host__ __device__ __forceinline__ uint32_t mod_magic(uint32_t d) { return 0xFFFFFFFFu / d; }
-__device__ __forceinline__ uint32_t mod_by(uint32_t x, uint32_t d, uint32_t m)
-{
-    uint32_t r = x - __umulhi(x, m) * d;
-    if (r >= d) r -= d;
-    return r;
-}
-
 __device__ __forceinline__ float rand_val(uint32_t y, float maxv)
 {
     return __fmul_rn(__uint2float_rn(y >> 8) * 0x1p-24f, maxv);
@@ -441,13 +430,12 @@ __device__ __forceinline__ bool by_position(const StepThr &t, uint32_t pdeg, uin
 //
 // Trials then run on integers only.  The rand-value tests become bounds on
 // k = y >> 8 (rand_bounds).  pos = x mod deg is not formed on the common path:
-// the fraction f = R*x mod 2^64 (R = 2^64/deg less at most 2^12) is
-// pos * 2^64/deg less at most 2^44, so its top kFilterBits bits name a bucket
-// of positions.  A per-warp
-// bitmap marks every bucket a run can reach; a trial whose bucket is unmarked
-// is in no run and its verdict is k < max(k_min, k_notfound).  A round in
-// which some trial passes that or is marked is looked at again exactly (pos,
-// run lookup in `iv`).
+// with Lemire's fraction f = M*x mod 2^64 (M = ceil(2^64/deg)), pos =
+// floor(f*deg / 2^64) and f lies in [M*pos, M*pos + 2^32), so its top kFilterBits
+// bits name a bucket of positions.  A per-warp bitmap marks every bucket a run
+// can reach; a trial whose bucket is unmarked is in no run and its verdict is
+// k < max(k_min, k_notfound).  A round in which some trial passes that or is
+// marked is looked at again exactly (pos, run lookup in `iv`).
 //
 // What bounds it: the Philox multiplies (17 wide products a draw, four cycles
 // each per warp: 70 of the cycles of 32 attempts), then the set-up's loads.
@@ -474,22 +462,10 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
         iv[lane] = lo;
         iv[32 + lane] = hi;
     }
-    // R: high word floor((2^32 - 1) / deg), low word from what that leaves
-    const float inv = __fdividef(1.0f, __uint2float_rn(deg));
-    const uint32_t r_lo = __float2uint_rd(__uint2float_rn(0u - magic * deg) * inv * (1.0f - 0x1p-21f) * 0x1p32f);
+    const uint64_t M = fastmod_magic_by(deg, magic, __frcp_rn(__uint2float_rn(deg)));
     __syncwarp();
     if (hi > lo) {
-        // buckets of lo .. hi - 1 times 2^B / deg, a hundredth of a bucket
-        // more on either side for the roundings here and of R; a position so
-        // close to 0 may also wrap to the last bucket
-        uint32_t b0 = 0, b1 = (1u << kFilterBits) - 1;
-        if (deg > 1) {
-            const float s = inv * (float)(1u << kFilterBits);
-            const float f0 = __uint2float_rn(lo) * s - 0.01f;
-            b0 = __float2uint_rd(fmaxf(f0, 0.0f));
-            b1 = min(__float2uint_rd(__uint2float_rn(hi - 1) * s + 0.01f), b1);
-            if (f0 < 0.0f) atomicOr(bm + kFilterWords - 1, 0x80000000u);
-        }
+        const uint32_t b0 = fraction_first(lo, M) >> (32 - kFilterBits), b1 = fraction_last(hi, M) >> (32 - kFilterBits);
         for (uint32_t w = b0 >> 5; w <= (b1 >> 5); ++w) {
             const uint32_t from = (w == (b0 >> 5)) ? (b0 & 31u) : 0u;
             const uint32_t to = (w == (b1 >> 5)) ? (b1 & 31u) : 31u;
@@ -508,7 +484,7 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
     // exact verdict of a trial whose bucket is marked
     auto exact = [&](uint32_t x, uint32_t k) -> bool {
         if (k < k_min) return true;
-        const uint32_t pos = mod_by(x, deg, magic);
+        const uint32_t pos = fastmod(x, M, deg);
         if (pos >= plo && pos < phi) return k < k_prev;
         // last run whose start is <= pos (runs are in N(prev) order, so sorted)
         int r = -1;
@@ -526,7 +502,7 @@ __device__ __forceinline__ uint32_t warp_first_accept_runs(const StepConsts &c, 
         return found ? (k < k_found) : (k < k_nf);
     };
     auto marked = [&](uint32_t x) -> bool {
-        const uint32_t b = magic * x + __umulhi(r_lo, x);  // the top word of f
+        const uint32_t b = fraction_top(x, M);
         return (__funnelshift_r(bm[b >> (37 - kFilterBits)], 0u, b >> (32 - kFilterBits)) & 1u) != 0;
     };
     // 64 attempts per round, two independent Philox chains per lane

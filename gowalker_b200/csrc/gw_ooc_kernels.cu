@@ -191,10 +191,10 @@ __global__ void __launch_bounds__(kScanThreads) k_plan(const uint32_t *__restric
     __shared__ uint32_t s_total;
     if (threadIdx.x == 0) {
         const unsigned long long now = global_ns();
-        if (clock->walk_start) clock->walk_ns += now - clock->walk_start;
+        if (clock->walk_start) clock->walk_ns += clock->walk_end - clock->walk_start;
         if (clock->plan_start) clock->bucket_ns += clock->scatter_end - clock->plan_start;
         clock->walk_start = 0;
-        clock->plan_start = now;
+        clock->plan_start = pairs ? now : clock->pairs_start;
     }
     const uint32_t n = 2 * nn;
     if (threadIdx.x <= kCtrCount) {
@@ -805,6 +805,7 @@ __global__ void __launch_bounds__(kWalkThreads) k_walk_ooc(const __grid_constant
         atomicAdd(&a.ctr[kCtrTrials], trials + s_ws[warp][kWsTrials]);
         atomicAdd(&a.ctr[kCtrDone], s_ws[warp][kWsDone]);
         atomicAdd(&a.ctr[kCtrHashSum], s_ws[warp][kWsHash]);
+        atomicMax(&a.clock->walk_end, global_ns());
     }
     {
         const unsigned long long zs = warp_sum((unsigned long long)zc_sectors);
@@ -929,8 +930,10 @@ cudaError_t launch_count(const uint32_t *keys, const uint32_t *n, uint32_t *coun
     return cudaGetLastError();
 }
 
-__global__ void k_combine(const uint32_t *__restrict__ counts, uint32_t nn, uint32_t *__restrict__ combined)
+__global__ void k_combine(const uint32_t *__restrict__ counts, uint32_t nn, uint32_t *__restrict__ combined,
+                          OocClock *clock)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0) clock->pairs_start = global_ns();
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += gridDim.x * blockDim.x)
         combined[k] = counts[k] + counts[nn + k];
 }
@@ -943,7 +946,7 @@ cudaError_t launch_plan(const uint32_t *counts, uint32_t nb, uint32_t *offsets, 
     // blocks, 128 at 256)
     const bool apart = nb > 64;
     if (apart) {
-        k_combine<<<num_sms, 256, 0, s>>>(counts, nb * nb, pairs);
+        k_combine<<<num_sms, 256, 0, s>>>(counts, nb * nb, pairs, clock);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -28,9 +28,10 @@ constexpr uint32_t kNeedPrev = 0x80000000u;
 // (nanoseconds of the device's clock): four events that take a time hold the
 // compute stream for about 12 us of a 100 us iteration.
 struct OocClock {
-    unsigned long long walk_start, plan_start, scatter_end;  // of the last ones
-    unsigned long long walk_ns;                              // step kernels, start to the plan behind them
-    unsigned long long bucket_ns;                            // plan to the end of the scatter, but for the last
+    unsigned long long walk_start, walk_end;                // of the last step kernel
+    unsigned long long pairs_start, plan_start, scatter_end;  // of the last re-bucketing; pairs: in a kernel of their own
+    unsigned long long walk_ns;    // step kernels
+    unsigned long long bucket_ns;  // first kernel of a re-bucketing to the end of its scatter, but for the last
 };
 
 struct OocStepArgs {

@@ -630,15 +630,16 @@ void gw_handle::drop_index()
 // come to so many an edge:
 // - 1 where graph and tables fit the L2 (a first run of 27 steps an edge on 1.8 M
 //   edges 1.66 ms, 2.81 without; of 2.8 on 7.6 M 1.44 / 1.77; of 0.14 0.43 / 0.22),
-// - 3 past it (a first run of 2.6 on 64 M edges 6.0 / 4.5 ms, on 31 M 2.77 / 2.20;
-//   the run after it 3.3 / 4.3 and 1.53 / 2.13), 1 for SOPR and SOSR, whose steps
-//   take more trials (128 M edges, 0.8: 30.4 / 27.5 ms, then 24.3 / 27.2).
+// - 6 past it (a first run of 2.6 on 64 M edges 6.0 / 4.5 ms, on 31 M 2.77 / 2.20,
+//   of 5.2 on 16 M with paths 2.34 / 1.89; the run after it 3.3 / 4.3, 1.53 / 2.20
+//   and 1.45 / 1.89), 1 for SOPR and SOSR, whose steps take more trials (128 M
+//   edges, 0.8: 30.4 / 27.5 ms, then 24.3 / 27.2).
 // Steps that always accept search nothing.
 int gw_handle::wanted_search(bool sopr, bool sure) const
 {
     if (cfg.launch_mode == GW_LAUNCH_PER_HOP || sure) return kQuarter;
     const double steps = index_steps + run_steps();
-    if (steps >= (double)nedges * (sopr || 14 * nedges <= kL2Bytes ? 1.0 : 3.0)) return kTable;
+    if (steps >= (double)nedges * (sopr || 14 * nedges <= kL2Bytes ? 1.0 : 6.0)) return kTable;
     return wants_levels(nwalkers, nedges, sopr, sure, num_sms) ? kLevels : kQuarter;
 }
 

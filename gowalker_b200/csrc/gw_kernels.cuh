@@ -8,6 +8,8 @@ namespace gw {
 
 constexpr int kWalkThreads = 256;   // threads per CTA of the walk kernels
 constexpr uint64_t kL2Bytes = 126ull << 20;
+// Whether a CSR's ids take more of the L2 than walks leave them (two thirds).
+inline bool past_l2(uint64_t nedges) { return 6 * nedges > kL2Bytes; }
 
 // Work / statistics counters of one run (device, zeroed per run).
 enum Counter : int {
@@ -222,11 +224,13 @@ struct CsrCheck {
 cudaError_t launch_validate_csr(const CsrCheck &a, int num_sms, cudaStream_t s);
 // Walkers an in-core kernel holds at a time: the lanes of `walk_ctas` CTAs an SM.
 uint64_t walk_lanes(int num_sms);
-// Whether a run reads sample levels when it has no tables: Node2vec on a CSR
-// larger than the L2, with walkers for a quarter of the lanes (fewer wait for
-// the chain of loads, which is longer: 64 M edges, 10,000 walkers 0.45 ms, 0.39
-// by quarters, 100,000 0.67 / 0.82; SOPR searches little: 128 M edges 28.2 ms,
-// 27.3 by quarters).
+// Whether a run reads sample levels when it has no tables: Node2vec past the L2
+// (one walker a vertex, without and with paths: 16 M edges 1.72 and 1.87 ms, by
+// quarters 1.52 and 1.83; 23 M 1.33 and 1.44 / 1.34 and 1.64; 31 M 2.21 and 2.47
+// / 2.09 to 2.42 and 3.14), with walkers for a quarter of the lanes (fewer wait
+// for the chain of loads, which is longer: 64 M edges, 10,000 walkers 0.45 ms,
+// 0.39 by quarters, 100,000 0.67 / 0.82; SOPR searches little: 128 M edges 28.2
+// ms, 27.3 by quarters).
 bool wants_levels(uint64_t nwalkers, uint64_t nedges, bool sopr, bool sure, int num_sms);
 // dst[j] = src[32 * j] for j < n.
 cudaError_t launch_sample_level(const uint32_t *src, uint64_t n, uint32_t *dst, int num_sms, cudaStream_t s);

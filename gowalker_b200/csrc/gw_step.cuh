@@ -274,9 +274,9 @@ __device__ __forceinline__ bool levels_have(const CsrIndex<kLevels> &ix, uint64_
 // vertices walks visit most; a bucket is one load and eight compares.  Sample
 // levels of 32, eight-way levels and eight-way trees were all measured too:
 // fewer lines than halving, but no fewer instructions.  Fewer lines count where
-// the CSR is larger than the L2 and no table is there (Node2vec on 64 M edges:
+// the L2 does not keep the CSR and no table is there (Node2vec on 64 M edges:
 // 4.23 ms by levels of 32, 4.92 by quarters, 5.38 by halving, 3.25 by tables;
-// on 31 M 2.20 / 2.09 / 2.47 / 1.48).
+// on 16 M 1.72 / 1.52 / - / 1.03).
 template <int SEARCH>
 __device__ __forceinline__ bool csr_contains(const CsrIndex<SEARCH> &ix, uint32_t first, uint64_t lo, uint32_t n,
                                              uint32_t x)

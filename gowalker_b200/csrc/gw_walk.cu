@@ -522,7 +522,7 @@ cudaError_t launch_sample_level(const uint32_t *src, uint64_t n, uint32_t *dst, 
 
 bool wants_levels(uint64_t nwalkers, uint64_t nedges, bool sopr, bool sure, int num_sms)
 {
-    return !sopr && !sure && 4 * nedges > kL2Bytes && 4 * nwalkers > walk_lanes(num_sms);
+    return !sopr && !sure && past_l2(nedges) && 4 * nwalkers > walk_lanes(num_sms);
 }
 
 uint64_t walk_lanes(int num_sms) { return (uint64_t)walk_ctas(false, false) * kWalkThreads * num_sms; }
@@ -596,7 +596,7 @@ IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths
     const uint64_t warps = (uint64_t)p.grid * (kWalkThreads / 32), busy = std::min<uint64_t>(warps, 16ull * num_sms);
     p.slots = sure ? 4 : 1;
     while (p.slots < 32 && p.slots * busy < nwalkers) p.slots *= 2;
-    const bool waits = !sure && search != kTable && 4 * nedges > kL2Bytes;
+    const bool waits = !sure && search != kTable && past_l2(nedges);
     p.chunk = nwalkers <= 32 * warps ? (waits ? std::min(p.slots, 8u) : p.slots) : sure ? 32 : 8;
     const uint64_t need = (nwalkers + p.slots * (kWalkThreads / 32) - 1) / (p.slots * (kWalkThreads / 32));
     if (grid <= 0 && need <= (uint64_t)num_sms) p.grid = (int)need;

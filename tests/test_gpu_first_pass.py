@@ -42,7 +42,7 @@ def test_short_runs_then_long_ones(gw, oracle, algo, p, q, weighted, device):
 
 @pytest.mark.parametrize("p,q", [(2.0, 0.5), (0.25, 4.0)])
 def test_levels_walk_as_tables(gw, oracle, p, q):
-    """A CSR larger than the L2: its first run reads sample levels, a run of few
+    """A CSR that the L2 does not keep: its first run reads sample levels, a run of few
     walkers none, a later one tables; the first's hashes against theirs, and
     against the oracle's for some walkers."""
     dg = gw.DeviceGraph(21, nverts=2_000_003, edgefactor=12, seed=5, symmetric=True)

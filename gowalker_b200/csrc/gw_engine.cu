@@ -859,7 +859,7 @@ int gw_handle::run_incore(gw_stats *stats)
                                         (int)cfg.blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
-    a.one_wave = plan.one_wave;
+    a.claims_end = plan.one_wave ? 0u : a.nwalkers;
     const size_t ctr_bytes = sizeof(unsigned long long) * (kCtrCount + 1);  // with the error word
     // A borrowed CSR may have been written since its index was built: its
     // contents are summed beside the walk, which is done again if they are not

@@ -89,7 +89,7 @@ struct IncoreArgs {
     uint32_t out_base;         // first walker id of the population: outputs are indexed by wid - out_base
     uint32_t chunk;            // walkers a warp claims per atomic (incore_plan)
     uint32_t slots;            // walkers of a warp at a time (incore_plan)
-    uint32_t one_wave;         // a claim for every warp: taken in order of the warps' places, not of their start
+    uint32_t claims_end;       // nwalkers; 0: a claim for every warp, by the warps' places and not by atomics
     uint32_t *paths;           // rows indexed by walker id, or null
     uint32_t stride;           // maxhops + 1
     uint32_t *lens;            // vertices per path

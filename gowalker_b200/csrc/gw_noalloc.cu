@@ -191,7 +191,7 @@ extern "C" int gw_walk_noalloc(const gw_config *cfg, const uint64_t *d_beg, cons
                     (int)cfg->blockpergrid, num_sms);
     a.slots = plan.slots;
     a.chunk = plan.chunk;
-    a.one_wave = plan.one_wave;
+    a.claims_end = plan.one_wave ? 0u : a.nwalkers;
     e = launch_walk_incore(a, sopr, coop, plan.grid, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(host_ctr, ctr, sizeof(host_ctr), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -84,6 +84,12 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
         while (grp.shift < kMaxGroupShift && (a.slots << (grp.shift + 1)) <= 32u) ++grp.shift;
 
     uint32_t q_next = 0, q_end = 0;  // warp-uniform claimed range
+    constexpr bool kOneWave = GROUPS || SURE;  // (the others, which fill the lanes, lose 9 % by these lines)
+    if (kOneWave && a.claims_end == 0) {
+        const unsigned long long base = (unsigned long long)(warp * gridDim.x + blockIdx.x) * chunk;
+        q_next = (uint32_t)min(base, (unsigned long long)a.nwalkers);
+        q_end = (uint32_t)min(base + chunk, (unsigned long long)a.nwalkers);
+    }
     bool exhausted = false;          // warp-uniform
     bool active = false;
 
@@ -116,13 +122,9 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
             if (need == 0 || exhausted) break;
             if (q_next >= q_end) {
                 unsigned long long base = 0;
-                if (a.one_wave) {
-                    base = q_end ? a.nwalkers : (unsigned long long)(warp * gridDim.x + blockIdx.x) * chunk;
-                } else {
-                    if (lane == 0) base = atomicAdd(&a.ctr[kCtrCursor], (unsigned long long)chunk);
-                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                }
-                if (base >= a.nwalkers) {
+                if (lane == 0) base = atomicAdd(&a.ctr[kCtrCursor], (unsigned long long)chunk);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                if (base >= (kOneWave ? a.claims_end : a.nwalkers)) {
                     exhausted = true;
                     break;
                 }
@@ -609,7 +611,7 @@ cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int gr
     walk_kernel(sopr, a.paths != nullptr, coop, a.alias != nullptr, a.search, sure_steps(sopr, a.c),
                 [&](auto so, auto pa, auto c, auto w, auto i, auto u) {
                     // (levels are read by runs that fill the lanes)
-                    if (!u() && i() != kLevels && a.slots < 32)
+                    if (!u() && i() != kLevels && (a.slots < 32 || a.claims_end == 0))
                         k_walk_incore<so(), pa(), c(), w(), i(), !u() && i() != kLevels, u()><<<grid, kWalkThreads, 0, s>>>(a);
                     else
                         k_walk_incore<so(), pa(), c(), w(), i(), false, u()><<<grid, kWalkThreads, 0, s>>>(a);

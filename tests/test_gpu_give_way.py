@@ -102,7 +102,7 @@ def test_to_the_next_graph(gw):
     """The index of 31 M edges, 340 MB, goes with its graph."""
     import torch
     dg = gw.DeviceGraph(20, nverts=1 << 20, edgefactor=16, seed=7, symmetric=True)
-    eng = gw.WalkEngine(algorithm=0, maxhops=120, p=0.5, q=2.0, seed=5)
+    eng = gw.WalkEngine(algorithm=0, maxhops=240, p=0.5, q=2.0, seed=5)  # eight steps an edge: tables
     eng.set_device_graph(dg.nverts, dg.nedges, dg.beg_ptr, dg.csr_ptr)
     eng.init_walkers()
     before = torch.cuda.mem_get_info()[0]

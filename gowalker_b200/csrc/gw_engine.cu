@@ -658,10 +658,11 @@ int gw_handle::validate_graph(cudaStream_t s, int search)
 {
     int st;
     index_search = kQuarter;
-    if (!reserve_index(search)) search = kQuarter;
     // the memory of a small index is taken with the first check, so that the
     // run that builds it, maybe a short one, does not wait for an allocation
+    // (first: a reservation that fails leaves nothing of the one before)
     if (search != kTable && !index_refused && index_layout(kTable).bytes < kSmallIndex) reserve_index(kTable);
+    if (!reserve_index(search)) search = kQuarter;
     const IndexLayout l = index_layout(search);
     const bool index = search == kTable;
     CsrCheck check{};

@@ -70,3 +70,27 @@ def test_levels_walk_as_tables(gw, oracle, p, q):
     assert np.array_equal(eng.hashes(), levels)
     eng.close()
     dg.free()
+
+
+def test_levels_where_tables_find_no_room(gw, oracle):
+    """23 M edges: the memory of tables (252 MB) is asked for ahead, and refused;
+    the levels (3 MB) that the run reads have room."""
+    import torch
+    dg = gw.DeviceGraph(19, nverts=1 << 19, edgefactor=24, nsamples=24 << 19, seed=3, symmetric=True)
+    assert 6 * dg.nedges > 126 << 20 and 10 * dg.nedges + 48 * dg.nverts < 256 << 20
+    beg, csr = dg.to_host()
+    eng = gw.WalkEngine(algorithm=0, maxhops=6, p=2.0, q=0.5, seed=4)
+    eng.set_device_graph(dg.nverts, dg.nedges, dg.beg_ptr, dg.csr_ptr)
+    eng.init_walkers()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (100 << 20), dtype=torch.uint8, device="cuda")
+    eng.run()
+    got = eng.hashes()[:4000]
+    del fill
+    torch.cuda.empty_cache()
+    ref = oracle.walk(beg, csr, oracle.make_cfg(algo=0, maxhops=6, p=2.0, q=0.5, seed=4), 0, 4000, paths=False)
+    assert np.array_equal(got, ref["hashes"])
+    eng.run()
+    assert np.array_equal(eng.hashes()[:4000], ref["hashes"])
+    eng.close()
+    dg.free()

@@ -879,7 +879,9 @@ int gw_handle::run_incore(gw_stats *stats)
         check.sum = d_ctr + kCtrGraphSum;
         check.err = reinterpret_cast<uint32_t *>(check.sum + 1);
         int e;
-        if ((e = cuda(cudaMemsetAsync(check.sum, 0, 2 * sizeof(unsigned long long), s_copy), "memset")) ||
+        // behind what the caller put on the compute stream before this run
+        if ((e = cuda(cudaStreamWaitEvent(s_copy, ev_start, 0), "graph sum")) ||
+            (e = cuda(cudaMemsetAsync(check.sum, 0, 2 * sizeof(unsigned long long), s_copy), "memset")) ||
             (e = cuda(launch_validate_csr(check, num_sms, s_copy), "graph sum")))
             return e;
         return cuda(cudaMemcpyAsync(h_ctr + kCtrGraphSum, check.sum, sizeof(unsigned long long),

@@ -214,8 +214,9 @@ int gw_host_block(gw_handle *h, uint32_t blk, const uint64_t *beg, const uint32_
 
 /* Whole graph already resident on this device (d_beg: nverts+1, d_csr:
  * nedges), borrowed.  The engine then runs in-core without host copies.  The
- * arrays may be written between runs (same sizes): each run walks what they
- * hold when it begins.  Weights and offsets that change under weighted walks
+ * arrays may be written between runs, by work that has ended or that is on the
+ * handle's stream, as long as they hold a valid CSR of the same sizes: each run
+ * walks what they hold when it begins.  Weights and offsets that change under weighted walks
  * are given again (gw_device_weights). */
 int gw_device_graph(gw_handle *h, const uint64_t *d_beg, const uint32_t *d_csr);
 

@@ -90,6 +90,34 @@ def test_weights_and_offsets_written_and_given_again(gw, oracle):
     eng.close()
 
 
+@pytest.mark.parametrize("count", [300, 12000])
+def test_writes_on_the_engine_stream_are_waited_for(gw, oracle, count):
+    """The new arrays arrive on the engine's own stream, behind work that takes a while."""
+    import torch
+    rng = np.random.default_rng(5)
+    V = 3000
+    beg, csr = graph_of(rng.integers(2, 30, V), rng)
+    beg2, csr2 = graph_of(rng.permutation(np.diff(beg.astype(np.int64))), rng)
+    d = [torch.from_numpy(x.copy()).cuda() for x in (beg.view(np.int64), csr.view(np.int32))]
+    new = [torch.from_numpy(x.copy()).cuda() for x in (beg2.view(np.int64), csr2.view(np.int32))]
+    busy = torch.zeros(1 << 28, dtype=torch.float32, device="cuda")
+    eng = gw.WalkEngine(algorithm=0, maxhops=30, p=0.5, q=2.0, seed=9, walkpersource=4)
+    eng.set_device_graph(V, len(csr), d[0].data_ptr(), d[1].data_ptr())
+    stream = torch.cuda.ExternalStream(eng.stream_handle())
+    eng.init_walkers(first=0, count=count)
+    eng.run()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for _ in range(8):
+            busy.add_(1.0)
+        d[0].copy_(new[0])
+        d[1].copy_(new[1])
+    eng.run()
+    cfg = oracle.make_cfg(algo=0, maxhops=30, p=0.5, q=2.0, seed=9, wps=4)
+    assert np.array_equal(eng.hashes(), oracle.walk(beg2, csr2, cfg, 0, count, paths=False)["hashes"])
+    eng.close()
+
+
 def test_an_invalid_write_is_refused(gw, oracle):
     import torch
     rng = np.random.default_rng(3)

@@ -99,7 +99,7 @@ def test_to_its_own_out_of_core_run(gw, oracle):
 
 
 def test_to_the_next_graph(gw):
-    """The index of 31 M edges, 340 MB, goes with its graph."""
+    """The index of 31 M edges, 340 MB, goes when a smaller graph comes."""
     import torch
     dg = gw.DeviceGraph(20, nverts=1 << 20, edgefactor=16, seed=7, symmetric=True)
     eng = gw.WalkEngine(algorithm=0, maxhops=240, p=0.5, q=2.0, seed=5)  # eight steps an edge: tables

@@ -256,7 +256,7 @@ void gw_handle::release()
     cudaSetDevice(cfg.device);
     if (s_compute) cudaStreamSynchronize(s_compute);
     if (s_copy) cudaStreamSynchronize(s_copy);
-    cudaFree(own_beg);
+    free_own_graph();
     cudaFree(own_w);
     cudaFree(d_alias);
     own_w = nullptr;
@@ -274,11 +274,17 @@ void gw_handle::release()
     if (ev_stop) cudaEventDestroy(ev_stop);
     if (s_compute) cudaStreamDestroy(s_compute);
     if (s_copy) cudaStreamDestroy(s_copy);
-    own_beg = nullptr;
-    own_csr = nullptr;
     d_paths = nullptr;
     d_lens = nullptr;
     d_hashes = nullptr;
+}
+
+void gw_handle::free_own_graph()
+{
+    cudaFree(own_beg);
+    cudaFree(own_csr_apart);
+    own_beg = nullptr;
+    own_csr = own_csr_apart = nullptr;
 }
 
 uint64_t gw_handle::graph_bytes() const
@@ -303,8 +309,17 @@ int gw_handle::upload_whole_graph(cudaStream_t s, uint64_t *h2d)
     int st;
     if (!own_beg) {
         const uint64_t beg_bytes = (((uint64_t)nverts + 1) * sizeof(uint64_t) + 255) & ~255ull;
-        if ((st = dev_alloc(own_beg, beg_bytes + (nedges ? nedges : 1) * sizeof(uint32_t), "graph"))) return st;
+        const uint64_t csr_bytes = (nedges ? nedges : 1) * sizeof(uint32_t);
+        const bool apart = beg_bytes < kShareBytes && csr_bytes < kShareBytes;
+        if ((st = dev_alloc(own_beg, beg_bytes + (apart ? 0 : csr_bytes), "graph"))) return st;
         own_csr = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(own_beg) + beg_bytes);
+        if (apart) {
+            if ((st = dev_alloc(own_csr_apart, csr_bytes, "graph"))) {
+                free_own_graph();
+                return st;
+            }
+            own_csr = own_csr_apart;
+        }
     }
     uint64_t bytes = 0;
     for (uint32_t b = 0; b < nblocks; ++b) {
@@ -414,9 +429,7 @@ extern "C" int gw_set_graph_meta(gw_handle *h, uint32_t nverts, uint64_t nedges,
     h->dev_csr = nullptr;
     h->resident = false;
     h->validated = false;
-    cudaFree(h->own_beg);
-    h->own_beg = nullptr;
-    h->own_csr = nullptr;
+    h->free_own_graph();
     h->ooc_release();
     h->walkers_ready = false;
     std::lock_guard<std::mutex> l(engines().mu);
@@ -447,9 +460,7 @@ extern "C" int gw_device_graph(gw_handle *h, const uint64_t *d_beg, const uint32
     if (h->nblocks == 0) return h->fail(GW_ERR_STATE, "set the graph meta first");
     if (!d_beg || (!d_csr && h->nedges)) return h->fail(GW_ERR_ARG, "device graph pointers missing");
     cudaSetDevice(h->cfg.device);
-    cudaFree(h->own_beg);
-    h->own_beg = nullptr;
-    h->own_csr = nullptr;
+    h->free_own_graph();
     h->dev_beg = d_beg;
     h->dev_csr = d_csr;
     h->resident = true;

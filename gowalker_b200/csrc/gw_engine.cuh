@@ -36,8 +36,8 @@ struct gw_handle {
     // whole graph on the device (in-core)
     const uint64_t *dev_beg = nullptr;
     const uint32_t *dev_csr = nullptr;
-    uint64_t *own_beg = nullptr;  // one allocation: offsets, then neighbours
-    uint32_t *own_csr = nullptr;
+    uint64_t *own_beg = nullptr;  // offsets, with the neighbours behind them or, small ones, apart
+    uint32_t *own_csr = nullptr, *own_csr_apart = nullptr;
     bool resident = false;
     bool device_graph = false;
     bool validated = false;
@@ -103,6 +103,7 @@ struct gw_handle {
     int init_device();
     void release();
     uint64_t graph_bytes() const;
+    void free_own_graph();
     bool host_graph_complete() const;
     int upload_whole_graph(cudaStream_t s, uint64_t *h2d);
     int ensure_outputs();

@@ -180,8 +180,8 @@ struct IncorePlan {
     uint32_t ctas_per_sm;   // the kernel's register cap: CTAs of an SM it is built for
 };
 // `grid` CTAs as asked for, or (0) as many as are resident at once.
-IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
-                       int grid, int num_sms);
+IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths, bool coop, bool weighted,
+                       int search, bool sure, int grid, int num_sms);
 // a.alias set: weighted Node2vec.
 cudaError_t launch_walk_incore(const IncoreArgs &a, bool sopr, bool coop, int grid, cudaStream_t s);
 

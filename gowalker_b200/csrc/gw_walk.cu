@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(kWalkThreads, walk_ctas(SOPR, COOP))
     uint32_t q_next = 0, q_end = 0;  // warp-uniform claimed range
     constexpr bool kOneWave = GROUPS || SURE;  // (the others, which fill the lanes, lose 9 % by these lines)
     if (kOneWave && a.claims_end == 0) {
-        const unsigned long long base = (unsigned long long)(warp * gridDim.x + blockIdx.x) * chunk;
+        const unsigned long long base = ((unsigned long long)warp * gridDim.x + blockIdx.x) * chunk;
         q_next = (uint32_t)min(base, (unsigned long long)a.nwalkers);
         q_end = (uint32_t)min(base + chunk, (unsigned long long)a.nwalkers);
     }
@@ -585,8 +585,8 @@ static auto walk_kernel(bool sopr, bool paths, bool coop, bool weighted, int sea
 // - no more CTAs than walkers need where each gets an SM to itself: the others
 //   find none, but take 12 us to come and go (3,878 sure walks 0.080 -> 0.062
 //   ms, 1,024 of Node2vec 0.062 -> 0.049).
-IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths, bool coop, bool weighted, int search, bool sure,
-                       int grid, int num_sms)
+IncorePlan incore_plan(uint64_t nwalkers, uint64_t nedges, bool sopr, bool paths, bool coop, bool weighted,
+                       int search, bool sure, int grid, int num_sms)
 {
     IncorePlan p{};
     p.ctas_per_sm = (uint32_t)walk_ctas(sopr, coop);
